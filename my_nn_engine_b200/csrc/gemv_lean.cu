@@ -6,15 +6,19 @@
 // allocation, tensor maps, mbarrier ring, a separate limb pre-pass launch, 128-row tiles that leave SMs idle) would dominate.
 // This kernel has none of it (the engine's counterpart is dequant_gemv, src/codegen/cuda/cpp/dequant_gemv.cuh:11-59: one
 // warp per row, one 16-byte load in flight per lane):
-//   * one CTA per SM with an equal share of the rows, so the grid is a single balanced wave; a warp takes up to four weight
-//     rows at a time and each lane issues all its 128-bit loads of those rows (up to 16) before it touches anything else, and
-//     before the programmatic-dependent-launch wait, so the weights are in flight while the preceding kernel drains;
-//   * the activation row(s) are held in shared memory as the same three signed 8-bit limbs of a 23-bit fixed-point value
-//     the tensor-core kernel uses (either copied from the workspace, where a fused producer left them, or computed here from
-//     the activation tensor: no extra launch), so a weight never needs converting: 16 weights x 3 limbs are 12 dp4a
-//     instructions with exact int32 accumulation;
-//   * warp-shuffle reduction, limbs recombined in int64, the same two roundings as the tensor-core kernel: the outputs are
-//     bit-identical to that kernel's, whichever of the two a shape is dispatched to.
+//   * one CTA per SM with an equal share of the rows, so the grid is a single balanced wave.  Its rows are tiles of 16; the sixteen warps
+//     deal out the contraction, so that every warp has the same piece of every row, and each lane issues all its 128-bit loads (up to 20)
+//     before it touches anything else, and before the programmatic-dependent-launch wait: the weights are in flight while
+//     the preceding kernel drains;
+//   * the activation row(s) are the same three signed 8-bit limbs of a 23-bit fixed-point value the tensor-core kernel uses, either read
+//     from the workspace, where a fused producer left them, or computed here in shared memory (no extra launch).  Three limbs of up to
+//     four rows are the columns of mma.m16n8k32 (int8, exact int32 sums).  The contraction index is permuted so that the 16 bytes a lane
+//     loads are its fragments of two MMAs, for weights and limbs alike; a warp needs its own piece of the limbs only;
+//   * the warps' int32 sums meet in shared memory once, limbs recombined in int64, the same two roundings as the tensor-core kernel:
+//     the outputs are bit-identical to that kernel's, whichever of the two a shape is dispatched to.
+// The legacy tensor path is enough here: 156 KB of weights per SM (gate/up of a 1B model) are 312 MMAs per eight columns, 0.3 us.  With
+// dp4a instead (12 per 16 weights and row, plus a warp reduction per output) the arithmetic took longer than the loads from two
+// rows on.
 // Measured against it and dropped: staging the weights through shared memory with untiled bulk copies (cp.async.bulk) so that
 // the next kernel's CTA fits beside this one (6.5 us against 4.3 us per launch on a 5632 x 2048 matrix), and 256-thread CTAs
 // two per SM (4.7 us).
@@ -24,6 +28,12 @@
 namespace mynn {
 
 constexpr int kLeanThreads = 512;
+constexpr int kLeanWarps = kLeanThreads / 32;
+constexpr int kLeanTiles = 8;                       // row tiles whose partial sums are kept at a time
+constexpr int kLeanFreeSms = 8;
+constexpr int kLeanPitch = 16 * kLeanTiles + 4;     // int32 per (warp, column): no two lanes of a store in one bank
+// limb rows in shared memory are this far apart: eight rows of a fragment load fall into different banks
+__host__ __device__ __forceinline__ int lean_limb_pitch(int K) { return (K + 127) / 128 * 128 + 64; }
 
 struct LeanParams {
     void *out;
@@ -45,7 +55,7 @@ __device__ __forceinline__ uint4 ldg_stream_16(const void *p) {
 // of the tensor-core kernel: |a| * 2^(22-e) rounded to an integer below 2^22, split into three signed bytes.  Rows of up to
 // 8 elements per thread stay in registers between the two passes.
 template <typename ActT>
-__device__ __forceinline__ void row_to_limbs(const ActT *row, int K, int8_t *l_s, int8_t *l_g, float *ascale_s, float *ascale_g,
+__device__ __forceinline__ void row_to_limbs(const ActT *row, int K, int pitch, int8_t *l_s, int8_t *l_g, float *ascale_s, float *ascale_g,
                                              float *red) {
     constexpr int kKeep = 8;
     float keep[kKeep];
@@ -86,8 +96,8 @@ __device__ __forceinline__ void row_to_limbs(const ActT *row, int K, int8_t *l_s
         const int d1 = (int)(int8_t)(A & 0xFF);
         A = (A - d1) >> 8;
         l_s[i] = (int8_t)d0;
-        l_s[K + i] = (int8_t)d1;
-        l_s[2 * K + i] = (int8_t)A;
+        l_s[pitch + i] = (int8_t)d1;
+        l_s[2 * pitch + i] = (int8_t)A;
         if (l_g) {
             l_g[i] = (int8_t)d0;
             l_g[K + i] = (int8_t)d1;
@@ -103,128 +113,141 @@ __device__ __forceinline__ void row_to_limbs(const ActT *row, int K, int8_t *l_s
     __syncthreads();  // red is reused by the next row
 }
 
-// One CTA per SM owns a contiguous range of weight rows, so that the whole grid is one balanced wave.  A warp takes groups
-// of RF consecutive rows; CPL = 16-byte chunks per lane and row (K <= 512 * CPL), so a group is RF * CPL <= 16 loads per lane,
-// all issued before anything else happens.  K % 16 == 0; wq and limbs 16-byte aligned.
-template <typename OutT, int M, int CPL, int RF>
+__device__ __forceinline__ void mma_i8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// One CTA per SM owns a contiguous range of weight rows, so that the whole grid is one balanced wave.  A warp owns NB blocks of 64 along K
+// (K <= 1024 NB) of all of them; TG tiles of 16 rows are in flight (2 NB TG <= 20 loads per lane, issued before anything else happens).
+// K % 16 == 0; wq and limbs 16-byte aligned.  Dynamic shared memory: limbs [3 M][pitch] (only with act), partial sums [warp][3 M][kLeanPitch].
+template <typename OutT, int M, int NB, int TG>
 __global__ void __launch_bounds__(kLeanThreads, 1) gemv_lean_kernel(const LeanParams p) {
-    extern __shared__ __align__(16) int8_t sm_limbs[];  // [M][3][K]
+    extern __shared__ __align__(16) int8_t sm_dyn[];
     __shared__ float sm_ascale[4];
-    __shared__ float red[kLeanThreads / 32];
-    constexpr int kWarps = kLeanThreads / 32;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int K = p.K, chunks = K >> 4;
-    const int cta_row0 = blockIdx.x * p.rows_per_cta;
-    const int cta_rows = min(p.rows_per_cta, p.N - cta_row0);
-    const int groups = (cta_rows + RF - 1) / RF;
+    __shared__ float red[kLeanWarps];
+    constexpr int C = 3 * M, NT = (C + 7) / 8;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, t = lane & 3;
+    const int K = p.K, chunks = K >> 4, pitch = lean_limb_pitch(K);
+    const int row0 = blockIdx.x * p.rows_per_cta, rows = min(p.rows_per_cta, p.N - row0), tiles = (rows + 15) >> 4;
+    int8_t *sm_limbs = sm_dyn;
+    int *sm_sum = reinterpret_cast<int *>(sm_dyn + (p.act ? (size_t)C * pitch : 0));
     const OutT *scale_p = reinterpret_cast<const OutT *>(p.scale);
     const OutT *resid_p = reinterpret_cast<const OutT *>(p.resid);
     OutT *out_p = reinterpret_cast<OutT *>(p.out);
 
-    uint4 w[RF][CPL];
-    auto load_group = [&](int g) {
+    const int c0 = warp * 4 * NB + t;  // this lane's 16-byte chunks of a row: c0 + 4 j
+    uint4 w[TG][NB][2];
+    auto load_tile = [&](uint4 (&x)[NB][2], int tile) {
 #pragma unroll
-        for (int r = 0; r < RF; r++) {
-            const int row = g * RF + r;
-            const int8_t *wr = p.wq + (size_t)(cta_row0 + (row < cta_rows ? row : 0)) * K;
+        for (int h = 0; h < 2; h++) {
+            const int row = 16 * tile + gq + 8 * h;
+            const int8_t *wr = p.wq + (size_t)(row0 + (row < rows ? row : 0)) * K;
 #pragma unroll
-            for (int j = 0; j < CPL; j++) {
-                const int c = lane + 32 * j;
-                w[r][j] = (row < cta_rows && c < chunks) ? ldg_stream_16(wr + 16 * (size_t)c) : make_uint4(0u, 0u, 0u, 0u);
+            for (int j = 0; j < NB; j++) {
+                const int c = c0 + 4 * j;
+                x[j][h] = row < rows && c < chunks ? ldg_stream_16(wr + 16 * (size_t)c) : make_uint4(0u, 0u, 0u, 0u);
             }
         }
     };
-    // the first group of weights and its row scales depend on nothing an earlier kernel writes: get them moving before the wait
-    if (warp < groups) load_group(warp);
-    float wscale_first = 0.f;
-    if (lane < RF && warp * RF + lane < cta_rows) wscale_first = to_f32<OutT>(scale_p[cta_row0 + warp * RF + lane]);
+    // the first tiles of weights and the row scale of this thread's output depend on nothing an earlier kernel writes
+#pragma unroll
+    for (int i = 0; i < TG; i++)
+        if (i < tiles) load_tile(w[i], i);
+    // outputs of the first pass: thread -> (row, activation row)
+    const int pass_rows = min(rows, 16 * kLeanTiles), my_m = threadIdx.x / pass_rows, my_r = threadIdx.x - my_m * pass_rows;
+    float wscale_first = 0.f, resv_first = 0.f;
+    if (my_m < M) wscale_first = to_f32<OutT>(scale_p[row0 + my_r]);
     pdl_trigger();
     pdl_wait();
-    float resv_first[M];
-#pragma unroll
-    for (int m = 0; m < M; m++)
-        resv_first[m] = (resid_p && lane < RF && warp * RF + lane < cta_rows) ? to_f32<OutT>(resid_p[(size_t)m * p.N + cta_row0 + warp * RF + lane]) : 0.f;
-    // activations -> limbs in shared memory
+    if (my_m < M && resid_p) resv_first = to_f32<OutT>(resid_p[(size_t)my_m * p.N + row0 + my_r]);
+    // limbs of this warp's piece of K: column gq (and gq + 8) of the MMAs is limb row gq (gq + 8) = 3 m + l
+    uint4 b[NT][NB];
     if (p.act != nullptr) {
         int8_t *lg = blockIdx.x == 0 ? p.limbs_g : nullptr;
         float *ag = blockIdx.x == 0 ? p.ascale_g : nullptr;
 #pragma unroll 1
         for (int m = 0; m < M; m++) {
-            int8_t *ls = sm_limbs + (size_t)m * 3 * K;
+            int8_t *ls = sm_limbs + (size_t)m * 3 * pitch;
             if (p.act_dtype == MYNN_F32)
-                row_to_limbs<float>((const float *)p.act + (size_t)m * K, K, ls, lg ? lg + (size_t)m * 3 * K : nullptr, &sm_ascale[m], ag ? ag + m : nullptr, red);
+                row_to_limbs<float>((const float *)p.act + (size_t)m * K, K, pitch, ls, lg ? lg + (size_t)m * 3 * K : nullptr, &sm_ascale[m], ag ? ag + m : nullptr, red);
             else if (p.act_dtype == MYNN_BF16)
-                row_to_limbs<__nv_bfloat16>((const __nv_bfloat16 *)p.act + (size_t)m * K, K, ls, lg ? lg + (size_t)m * 3 * K : nullptr, &sm_ascale[m], ag ? ag + m : nullptr, red);
+                row_to_limbs<__nv_bfloat16>((const __nv_bfloat16 *)p.act + (size_t)m * K, K, pitch, ls, lg ? lg + (size_t)m * 3 * K : nullptr, &sm_ascale[m], ag ? ag + m : nullptr, red);
             else
-                row_to_limbs<__half>((const __half *)p.act + (size_t)m * K, K, ls, lg ? lg + (size_t)m * 3 * K : nullptr, &sm_ascale[m], ag ? ag + m : nullptr, red);
+                row_to_limbs<__half>((const __half *)p.act + (size_t)m * K, K, pitch, ls, lg ? lg + (size_t)m * 3 * K : nullptr, &sm_ascale[m], ag ? ag + m : nullptr, red);
         }
+        __syncthreads();
+#pragma unroll
+        for (int n = 0; n < NT; n++)
+#pragma unroll
+            for (int j = 0; j < NB; j++) {
+                const int c = c0 + 4 * j, col = 8 * n + gq;
+                b[n][j] = col < C && c < chunks ? *reinterpret_cast<const uint4 *>(sm_limbs + (size_t)col * pitch + 16 * c) : make_uint4(0u, 0u, 0u, 0u);
+            }
     } else {
-        const uint4 *src = reinterpret_cast<const uint4 *>(p.limbs_g);
-        uint4 *dst = reinterpret_cast<uint4 *>(sm_limbs);
-        for (int i = threadIdx.x; i < (M * 3 * K) >> 4; i += kLeanThreads) dst[i] = __ldcg(src + i);
+#pragma unroll
+        for (int n = 0; n < NT; n++)
+#pragma unroll
+            for (int j = 0; j < NB; j++) {
+                const int c = c0 + 4 * j, col = 8 * n + gq;
+                b[n][j] = col < C && c < chunks ? __ldcg(reinterpret_cast<const uint4 *>(p.limbs_g + (size_t)col * K + 16 * (size_t)c)) : make_uint4(0u, 0u, 0u, 0u);
+            }
         if (threadIdx.x < M) sm_ascale[threadIdx.x] = __ldcg(p.ascale_g + threadIdx.x);
     }
-    __syncthreads();
 
-    for (int g = warp; g < groups; g += kWarps) {
-        if (g != warp) load_group(g);
-        // weight-row scales (and residuals) of the group: requested before the arithmetic
-        const int my_row = cta_row0 + g * RF + lane;  // lanes 0..RF-1 each finish one row of the group
-        const bool my_live = lane < RF && g * RF + lane < cta_rows;
-        float wscale = wscale_first;  // the first group's were requested at the top of the kernel
-        float resv[M];
+    for (int first = 0; first < tiles; first += kLeanTiles) {
+        const int last = min(first + kLeanTiles, tiles);
+        // kLeanTiles is not a multiple of TG: the register slot of a tile is its number modulo TG, walked slot by slot
+        for (int base = first / TG * TG; base < last; base += TG) {
 #pragma unroll
-        for (int m = 0; m < M; m++) resv[m] = resv_first[m];
-        if (g != warp) {
-            wscale = my_live ? to_f32<OutT>(scale_p[my_row]) : 0.f;
+            for (int i = 0; i < TG; i++) {
+                const int tile = base + i;
+                if (tile < first || tile >= last) continue;
+                int acc[NT][4];
 #pragma unroll
-            for (int m = 0; m < M; m++) resv[m] = (my_live && resid_p) ? to_f32<OutT>(resid_p[(size_t)m * p.N + my_row]) : 0.f;
-        }
-        int acc[RF][M][3];
+                for (int n = 0; n < NT; n++) {
+                    acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0;
 #pragma unroll
-        for (int r = 0; r < RF; r++)
+                    for (int j = 0; j < NB; j++) {
+                        mma_i8(acc[n], w[i][j][0].x, w[i][j][1].x, w[i][j][0].y, w[i][j][1].y, b[n][j].x, b[n][j].y);
+                        mma_i8(acc[n], w[i][j][0].z, w[i][j][1].z, w[i][j][0].w, w[i][j][1].w, b[n][j].z, b[n][j].w);
+                    }
+                }
+                if (tile + TG < tiles) load_tile(w[i], tile + TG);
+                // registers: (row gq, columns 2t, 2t + 1), (row gq + 8, the same columns)
+                const int r = 16 * (tile - first) + gq;
 #pragma unroll
-            for (int m = 0; m < M; m++) acc[r][m][0] = acc[r][m][1] = acc[r][m][2] = 0;
+                for (int n = 0; n < NT; n++)
 #pragma unroll
-        for (int j = 0; j < CPL; j++) {
-            const int c = lane + 32 * j;
-            if (c < chunks) {
-#pragma unroll
-                for (int m = 0; m < M; m++)
-#pragma unroll
-                    for (int l = 0; l < 3; l++) {
-                        const uint4 a = *reinterpret_cast<const uint4 *>(sm_limbs + ((size_t)(m * 3 + l)) * K + 16 * (size_t)c);
-#pragma unroll
-                        for (int r = 0; r < RF; r++) {
-                            int s = acc[r][m][l];
-                            s = __dp4a((int)w[r][j].x, (int)a.x, s);
-                            s = __dp4a((int)w[r][j].y, (int)a.y, s);
-                            s = __dp4a((int)w[r][j].z, (int)a.z, s);
-                            s = __dp4a((int)w[r][j].w, (int)a.w, s);
-                            acc[r][m][l] = s;
+                    for (int e = 0; e < 2; e++) {
+                        const int col = 8 * n + 2 * t + e;
+                        if (col < C) {
+                            int *at = sm_sum + (warp * C + col) * kLeanPitch + r;
+                            at[0] = acc[n][e];
+                            at[8] = acc[n][2 + e];
                         }
                     }
             }
         }
-        // warp reduction; lane r then finishes row r with the arithmetic of the tensor-core kernel's epilogue
+        __syncthreads();
+        const int beg = 16 * first, n_rows = min(rows, 16 * last) - beg;
+        for (int i = threadIdx.x; i < n_rows * M; i += kLeanThreads) {
+            const int m = i / n_rows, r = i - m * n_rows, row = row0 + beg + r;
+            const bool known = first == 0 && i == (int)threadIdx.x;  // requested at the top of the kernel
+            const float wscale = known ? wscale_first : to_f32<OutT>(scale_p[row]);
+            const float resv = known ? resv_first : resid_p ? to_f32<OutT>(resid_p[(size_t)m * p.N + row]) : 0.f;
+            int v[3] = {0, 0, 0};
 #pragma unroll
-        for (int r = 0; r < RF; r++)
+            for (int x = 0; x < kLeanWarps; x++)
 #pragma unroll
-            for (int m = 0; m < M; m++) {
-                int v0 = acc[r][m][0], v1 = acc[r][m][1], v2 = acc[r][m][2];
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    v0 += __shfl_xor_sync(0xffffffffu, v0, o);
-                    v1 += __shfl_xor_sync(0xffffffffu, v1, o);
-                    v2 += __shfl_xor_sync(0xffffffffu, v2, o);
-                }
-                const long long sum = (long long)v2 * 65536 + (long long)v1 * 256 + (long long)v0;
-                if (lane == r && my_live) {
-                    float v = __fmul_rn(__fmul_rn((float)sum, sm_ascale[m]), wscale);
-                    if (resid_p) v = __fadd_rn(round_store<OutT>(v), resv[m]);
-                    out_p[(size_t)m * p.N + my_row] = from_f32<OutT>(v);
-                }
-            }
+                for (int l = 0; l < 3; l++) v[l] += sm_sum[(x * C + 3 * m + l) * kLeanPitch + r];
+            const long long sum = (long long)v[2] * 65536 + (long long)v[1] * 256 + (long long)v[0];
+            float y = __fmul_rn(__fmul_rn((float)sum, sm_ascale[m]), wscale);
+            if (resid_p) y = __fadd_rn(round_store<OutT>(y), resv);
+            out_p[(size_t)m * p.N + row] = from_f32<OutT>(y);
+        }
+        if (last < tiles) __syncthreads();  // the sums are read before the next tiles' replace them
     }
 }
 
@@ -234,20 +257,26 @@ bool gemv_lean_supported(int M, int N, int K, const void *wq) {
            ((uintptr_t)wq % 16) == 0;
 }
 
-template <typename OutT, int M, int CPL, int RF>
+template <typename OutT, int M, int NB, int TG>
 static int launch_lean(cudaStream_t st, LeanParams p) {
-    const size_t smem = (size_t)3 * M * p.K;
-    auto kern = gemv_lean_kernel<OutT, M, CPL, RF>;
-    if (smem > 48 * 1024) MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const size_t smem = (p.act ? (size_t)3 * M * lean_limb_pitch(p.K) : 0) + (size_t)kLeanWarps * 3 * M * kLeanPitch * sizeof(int);
+    auto kern = gemv_lean_kernel<OutT, M, NB, TG>;
+    static bool attr_set = false;
+    if (!attr_set) {  // the most this form can need
+        constexpr int most = 3 * M * (1024 * NB + 64) + kLeanWarps * 3 * M * kLeanPitch * (int)sizeof(int);
+        static_assert(most <= 227 * 1024, "shared memory of a CTA");
+        MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+        attr_set = true;
+    }
     static int sms = 0;
     if (sms == 0) {
         int dev = 0;
         cudaGetDevice(&dev);
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
     }
-    // one CTA per SM, each with an equal share of the rows (a multiple of RF)
-    int rpc = (p.N + sms - 1) / sms;
-    rpc = (rpc + RF - 1) / RF * RF;
+    // One CTA per SM, each with an equal share of the rows; a few SMs stay free, where the CTAs of the row kernel behind this one (launched
+    // as its dependent) are resident by the time it ends.
+    const int ctas = sms > 4 * kLeanFreeSms ? sms - kLeanFreeSms : sms, rpc = (p.N + ctas - 1) / ctas;
     p.rows_per_cta = rpc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((p.N + rpc - 1) / rpc);
@@ -283,17 +312,18 @@ int gemv_lean_launch(cudaStream_t st, void *out, const void *act, const int8_t *
     p.K = K;
     p.act_dtype = act_dtype;
     p.rows_per_cta = 0;
-    // chunks per lane (K <= 2048 / 4096 / 6144) and rows in flight per warp: 16 loads per lane, at most 24 accumulators
-#define BY_K(OT, MV, RF4, RF8)                                \
-    if (K <= 2048) return launch_lean<OT, MV, 4, RF4>(st, p); \
-    if (K <= 4096) return launch_lean<OT, MV, 8, RF8>(st, p); \
-    return launch_lean<OT, MV, 12, 1>(st, p);
-#define GO(OT)                    \
-    switch (M) {                  \
-        case 1: BY_K(OT, 1, 4, 2) \
-        case 2: BY_K(OT, 2, 4, 2) \
-        case 3: BY_K(OT, 3, 2, 2) \
-        default: BY_K(OT, 4, 2, 2) \
+    // blocks of 64 per warp (K <= 1024 / 2048 / 4096 / 6144) and row tiles in flight
+#define BY_K(OT, MV)                                        \
+    if (K <= 1024) return launch_lean<OT, MV, 1, 8>(st, p); \
+    if (K <= 2048) return launch_lean<OT, MV, 2, 5>(st, p); \
+    if (K <= 4096) return launch_lean<OT, MV, 4, 2>(st, p); \
+    return launch_lean<OT, MV, 6, 1>(st, p);
+#define GO(OT)               \
+    switch (M) {             \
+        case 1: BY_K(OT, 1)  \
+        case 2: BY_K(OT, 2)  \
+        case 3: BY_K(OT, 3)  \
+        default: BY_K(OT, 4) \
     }
     if (out_dtype == MYNN_BF16) GO(__nv_bfloat16)
     if (out_dtype == MYNN_F16) GO(__half)

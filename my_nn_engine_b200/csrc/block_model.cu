@@ -306,6 +306,7 @@ static int mix_attention(Model &m, cudaStream_t st, const BlockLayer &L, const B
         ra.cache_rows = l.cache_rows;
         ra.B = B, ra.S = S, ra.Hq = l.heads, ra.G = l.kv_heads, ra.D = l.dim, ra.E = l.vdim;
         ra.past = m.past_dev;
+        ra.settled = 1;
         RC(launch_rotary_append(st, dt, ra));
     } else {
         ConvStep cv;
@@ -321,6 +322,7 @@ static int mix_attention(Model &m, cudaStream_t st, const BlockLayer &L, const B
         cv.cache_rows = l.cache_rows;
         cv.B = B, cv.S = S, cv.Hq = l.heads, cv.G = l.kv_heads, cv.D = l.dim, cv.E = l.vdim;
         cv.past = m.past_dev;
+        cv.settled = 1;
         RC(launch_conv_step(st, dt, cv));
     }
     WindowAttention at;
@@ -336,6 +338,7 @@ static int mix_attention(Model &m, cudaStream_t st, const BlockLayer &L, const B
     at.active = m.active_dev;
     at.workspace = m.attn_ws;
     at.workspace_bytes = m.attn_ws_bytes;
+    at.settled = 1;
     at.status_word = (int *)m.gemm_ws;
     return launch_window_attention(st, dt, at);
 }
@@ -426,6 +429,7 @@ static int mix_mlstm(Model &m, cudaStream_t st, const BlockLayer &L, const Block
     p.out = b.attn;
     p.B = b.c.batch, p.S = S, p.H = l.heads, p.D = l.dim, p.E = l.vdim;
     p.past = m.past_dev;
+    p.settled = 1;  // the state was last written by the step before, and the inputs' copies lie between
     p.status = (int *)m.gemm_ws;
     return launch_mlstm(st, dt, p);
 }
@@ -447,6 +451,7 @@ int block_forward(Model &m, cudaStream_t st, int S, int head_rows) {
         p.mult = c.residual_mult;
         p.eps = c.norm_eps;
         p.rms = c.rms_norm;
+        p.fixed_weights = 1;
         p.W = H;
         p.w2 = w2;
         p.b2 = b2;
@@ -535,6 +540,7 @@ int block_forward(Model &m, cudaStream_t st, int S, int head_rows) {
     f.w2 = b.fnw, f.b2 = b.fnb;
     f.eps = c.norm_eps;
     f.rms = c.rms_norm;
+    f.fixed_weights = 1;
     f.W = H;
     f.out = b.h;
     f.row_map = nullptr;

@@ -34,6 +34,7 @@ struct NormStep {
     float mult = 1.f, eps = 0.f;
     int add_x0 = 0;
     int rms = 0;
+    int fixed_weights = 0;  // no kernel in front of this one writes w1, b1, w2, b2: they may be read before it has finished
     void *out = nullptr;
     const int32_t *row_map = nullptr;
     int W = 0;
@@ -59,6 +60,7 @@ struct ConvStep {
     int cache_rows = 0;
     int B = 0, S = 0, Hq = 0, G = 0, D = 0, E = 0;
     const int32_t *past = nullptr;
+    int settled = 0;  // the kernels right in front write proj and nothing else that is read here (not hist, w, past)
 };
 int launch_conv_step(cudaStream_t st, int dtype, const ConvStep &p);
 
@@ -81,6 +83,7 @@ struct WindowAttention {
     const int32_t *active = nullptr;   // device: positions written so far, the new rows included
     void *workspace = nullptr;
     size_t workspace_bytes = 0;
+    int settled = 0;                   // decode: the kernels right in front write q and the newest key and value rows, nothing else read here
     int *status_word = nullptr;
 };
 int launch_window_attention(cudaStream_t st, int dtype, const WindowAttention &p);
@@ -115,6 +118,7 @@ struct RotaryAppend {
     int cache_rows = 0;
     int B = 0, S = 0, Hq = 0, G = 0, D = 0, E = 0;
     const int32_t *past = nullptr;
+    int settled = 0;  // as above
 };
 int launch_rotary_append(cudaStream_t st, int dtype, const RotaryAppend &p);
 
@@ -166,6 +170,7 @@ struct MlstmStep {
     void *out = nullptr;         // [B * S, H E]
     int B = 0, S = 0, H = 0, D = 0, E = 0;
     const int32_t *past = nullptr;
+    int settled = 0;             // nothing launched right in front of this step writes mem, sum, top or past: they may be read early
     int form = 0;                // 0: by size, 1: token by token, 2: chunkwise on mma.sync, 3: chunkwise on tcgen05 (both 16-bit)
     int *status = nullptr;       // status word of the bounded waits (tcgen05 form only)
 };

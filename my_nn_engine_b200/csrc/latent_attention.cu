@@ -98,10 +98,10 @@ int launch_latent_append(cudaStream_t st, int dtype, const LatentAppend &p) {
     const dim3 grid(2, p.B * p.S);
     const uintptr_t a = (uintptr_t)p.proj | (uintptr_t)p.q_out | (uintptr_t)p.cache | (uintptr_t)p.wq | (uintptr_t)p.wc;
     if (dtype != MYNN_F32 && p.Q % 8 == 0 && p.R % 8 == 0 && a % 16 == 0) {
-        if (dtype == MYNN_BF16) latent_append_kernel<__nv_bfloat16, 8><<<grid, 256, 0, st>>>(p);
-        else latent_append_kernel<__half, 8><<<grid, 256, 0, st>>>(p);
+        if (dtype == MYNN_BF16) MYNN_CUDA_OK(launch_dependent(latent_append_kernel<__nv_bfloat16, 8>, grid, dim3(256), 0, st, p));
+        else MYNN_CUDA_OK(launch_dependent(latent_append_kernel<__half, 8>, grid, dim3(256), 0, st, p));
     } else {
-        MYNN_DISPATCH_DTYPE(dtype, T, { latent_append_kernel<T, 1><<<grid, 256, 0, st>>>(p); });
+        MYNN_DISPATCH_DTYPE(dtype, T, { MYNN_CUDA_OK(launch_dependent(latent_append_kernel<T, 1>, grid, dim3(256), 0, st, p)); });
     }
     MYNN_LAUNCH_OK("latent_append_kernel");
     return MYNN_OK;
@@ -400,7 +400,7 @@ static int run_latent(cudaStream_t st, const LatParams &l, int queries) {
         MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         attr_set = true;
     }
-    kern<<<dim3(l.splits, queries, l.groups), lat_warps(R) * 32, smem, st>>>(l);
+    MYNN_CUDA_OK(launch_dependent(kern, dim3(l.splits, queries, l.groups), dim3(lat_warps(R) * 32), smem, st, l));
     MYNN_LAUNCH_OK("latent_attention_kernel");
     if (l.splits > 1) {
         MYNN_CUDA_OK(launch_dependent(latent_merge_kernel<T>, dim3((unsigned)((long long)queries * l.H)), dim3(R / 2), 0, st, l, R));

@@ -3,8 +3,9 @@
 // A sandwich-normed layer does x += mult * LN(sublayer output) and then feeds LN(x) to the next sublayer.  Both norms, the
 // residual sum, the combination of routed experts and the addition of the embedding output at the start of a repeated pass
 // are row operations, so one kernel does them with one read of the sublayer output and one read and write of x.
-// Mean and squared deviations are gathered per thread around the thread's own mean and merged pairwise (the update of Chan, Golub
-// and LeVeque), which needs one block reduction per norm and stays accurate when the mean is large against the deviations.
+// Two forms of the statistics, both accurate when the mean is large against the deviations.  Many rows: mean and squared deviations are
+// gathered per thread around the thread's own mean and merged pairwise (the update of Chan, Golub and LeVeque), one block reduction
+// per norm.  Few rows: sums, first for the mean and then for the deviations around it, because the merge's divisions are the longer chain.
 #include "block_ops.cuh"
 #include "common.cuh"
 
@@ -41,6 +42,27 @@ __device__ __forceinline__ Moments block_moments(Moments v, Moments *sm) {
     return t;
 }
 
+// Sums of two numbers over the block; every thread gets them.  sm holds two numbers per warp (32 pairs) and must not be the buffer of the
+// call before (calls take turns between two), so one barrier per call is enough.
+__device__ __forceinline__ float2 block_sum2(float a, float b, float2 *sm) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+    const int warps = blockDim.x >> 5, lane = threadIdx.x & 31;
+    if (lane == 0) sm[threadIdx.x >> 5] = make_float2(a, b);
+    __syncthreads();
+    float2 t = lane < warps ? sm[lane] : make_float2(0.f, 0.f);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        if (o >= warps) continue;  // the warps past the last one hold zeros
+        t.x += __shfl_xor_sync(0xffffffffu, t.x, o);
+        t.y += __shfl_xor_sync(0xffffffffu, t.y, o);
+    }
+    return make_float2(__shfl_sync(0xffffffffu, t.x, 0), __shfl_sync(0xffffffffu, t.y, 0));
+}
+
 template <typename T, int V>
 __device__ __forceinline__ void load_vec(const T *p, float (&v)[V]) {
     if constexpr (V == 4 && sizeof(T) == 2) {
@@ -54,6 +76,24 @@ __device__ __forceinline__ void load_vec(const T *p, float (&v)[V]) {
     } else {
 #pragma unroll
         for (int i = 0; i < V; i++) v[i] = to_f32<T>(p[i]);
+    }
+}
+// the same without the conversion
+template <typename T, int V>
+__device__ __forceinline__ void raw_vec(const T *p, T (&v)[V]) {
+    if constexpr (V == 4 && sizeof(T) == 2) {
+        const uint2 r = *reinterpret_cast<const uint2 *>(p);
+        const T *e = reinterpret_cast<const T *>(&r);
+#pragma unroll
+        for (int i = 0; i < 4; i++) v[i] = e[i];
+    } else if constexpr (V == 4) {
+        const float4 r = *reinterpret_cast<const float4 *>(p);
+        const T *e = reinterpret_cast<const T *>(&r);
+#pragma unroll
+        for (int i = 0; i < 4; i++) v[i] = e[i];
+    } else {
+#pragma unroll
+        for (int i = 0; i < V; i++) v[i] = p[i];
     }
 }
 template <typename T, int V>
@@ -73,47 +113,94 @@ __device__ __forceinline__ void store_vec(T *p, const float (&v)[V]) {
 }
 
 // grid = rows.  NV groups of V elements per thread live in registers between the passes (NV * V * blockDim.x >= W).
-template <typename T, int V, int NV>
-__global__ void __launch_bounds__(NV == 1 ? 256 : 1024) norm_step_kernel(const NormStep p) {
-    __shared__ Moments sm[32];
-    pdl_trigger();
-    pdl_wait();
+// FEW: a decode step, whose time is the chain of dependent steps: the weights are requested in front of the wait for the preceding kernel
+// when they are known not to come from it, the expert rows are requested together, and the statistics take the shorter chain.
+// For many rows that would only cost registers.
+template <typename T, int V, int NV, bool FEW>
+__global__ void __launch_bounds__(NV == 1 ? 256 : FEW ? 512 : 1024) norm_step_kernel(const NormStep p) {
+    __shared__ float2 sm[2][32];
+    __shared__ Moments sm_m[32];
     const int row = blockIdx.x, W = p.W;
+    const int step = blockDim.x * V, i0 = threadIdx.x * V;
+    constexpr bool EARLY = FEW;  // weights of both norms in registers
+    float we[EARLY ? 4 : 1][NV][V];
+    auto get_weights = [&]() {
+        const float *src[4] = {p.w1, p.rms ? nullptr : p.b1, p.w2, p.rms ? nullptr : p.b2};
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+#pragma unroll
+            for (int j = 0; j < NV; j++) {
+#pragma unroll
+                for (int k = 0; k < V; k++) we[q][j][k] = q & 1 ? 0.f : 1.f;
+                if (src[q] && i0 + j * step < W) load_vec<float, V>(src[q] + i0 + j * step, we[q][j]);
+            }
+    };
+    pdl_trigger();
+    if (!p.fixed_weights) pdl_wait();
+    if constexpr (EARLY) get_weights();
+    pdl_wait();
     const int src = p.row_map ? p.row_map[row] : row;
     float xv[NV][V];
-    const int step = blockDim.x * V, i0 = threadIdx.x * V;
-    auto moments = [&](const float (&v)[NV][V]) {
-        Moments m = {0.f, 0.f, 0.f};
-        float s = 0.f;
-        int n = 0;
+    int turn = 0;
+    // mean (0 for a norm by root mean square) and reciprocal deviation of the row.  The deviations are taken around the mean of the whole
+    // row, and what rounding left of their own mean corrects both.
+    auto norm_of = [&](const float (&v)[NV][V]) {
+        if constexpr (!FEW) {
+            Moments m = {0.f, 0.f, 0.f};
+            float s = 0.f;
+            int n = 0;
 #pragma unroll
-        for (int j = 0; j < NV; j++)
-            if (i0 + j * step < W) {
+            for (int j = 0; j < NV; j++)
+                if (i0 + j * step < W) {
 #pragma unroll
-                for (int e = 0; e < V; e++) s += v[j][e];
-                n += V;
-            }
-        m.n = (float)n;
-        m.mean = n ? s / (float)n : 0.f;
-#pragma unroll
-        for (int j = 0; j < NV; j++)
-            if (i0 + j * step < W) {
-#pragma unroll
-                for (int e = 0; e < V; e++) {
-                    const float d = v[j][e] - m.mean;
-                    m.m2 += d * d;
+                    for (int e = 0; e < V; e++) s += v[j][e];
+                    n += V;
                 }
+            m.n = (float)n;
+            m.mean = n ? s / (float)n : 0.f;
+#pragma unroll
+            for (int j = 0; j < NV; j++)
+                if (i0 + j * step < W) {
+#pragma unroll
+                    for (int e = 0; e < V; e++) {
+                        const float d = v[j][e] - m.mean;
+                        m.m2 += d * d;
+                    }
+                }
+            m = block_moments(m, sm_m);
+            float q = m.m2 / (float)W;
+            if (p.rms) {  // nothing is taken off, and mean(v^2) = var + mean^2
+                q += m.mean * m.mean;
+                m.mean = 0.f;
             }
-        return block_moments(m, sm);
-    };
-    // reciprocal deviation; for a norm by root mean square nothing is taken off, and mean(v^2) = var + mean^2
-    auto scale_of = [&](Moments &m) {
-        float v = m.m2 / (float)W;
-        if (p.rms) {
-            v += m.mean * m.mean;
-            m.mean = 0.f;
+            return make_float2(m.mean, 1.0f / sqrtf(q + p.eps));
         }
-        return 1.0f / sqrtf(v + p.eps);
+        float s = 0.f, q = 0.f, mean = 0.f;
+#pragma unroll
+        for (int pass = 0; pass < 2; pass++) {
+            if (pass == 0 && p.rms) continue;
+            s = q = 0.f;
+#pragma unroll
+            for (int j = 0; j < NV; j++)
+                if (i0 + j * step < W) {
+#pragma unroll
+                    for (int e = 0; e < V; e++) {
+                        const float d = v[j][e] - mean;
+                        s += d;
+                        if (pass) q += d * d;
+                    }
+                }
+            const float2 t = block_sum2(s, q, sm[turn]);
+            turn ^= 1;
+            s = t.x / (float)W;
+            q = t.y / (float)W;
+            if (pass == 0) mean = s;
+        }
+        if (!p.rms) {
+            mean += s;
+            q = fmaxf(q - s * s, 0.f);
+        }
+        return make_float2(mean, 1.0f / sqrtf(q + p.eps));
     };
     if (p.embed) {
         const long long id = min(max((long long)p.ids[row], 0ll), (long long)p.vocab - 1);
@@ -143,19 +230,33 @@ __global__ void __launch_bounds__(NV == 1 ? 256 : 1024) norm_step_kernel(const N
                 for (int j = 0; j < NV; j++)
 #pragma unroll
                     for (int k = 0; k < V; k++) sv[j][k] = 0.f;
-                for (int s = 0; s < p.top; s++) {
-                    const T *r = sub + (size_t)p.pair_row[(size_t)row * p.top + s] * W;
-                    const float g = p.pair_w[(size_t)row * p.top + s];
+                // rows in flight together: one after the other each would cost a trip to L2
+                constexpr int U = FEW ? 8 : 1;
+                for (int s0 = 0; s0 < p.top; s0 += U) {
+                    T t[U][NV][V];
+                    float g[U];
+                    int at[U];
 #pragma unroll
-                    for (int j = 0; j < NV; j++) {
-                        const int i = i0 + j * step;
-                        if (i < W) {
-                            float t[V];
-                            load_vec<T, V>(r + i, t);
-#pragma unroll
-                            for (int k = 0; k < V; k++) sv[j][k] += g * t[k];
-                        }
+                    for (int u = 0; u < U; u++) {
+                        const size_t pair = (size_t)row * p.top + min(s0 + u, p.top - 1);
+                        at[u] = p.pair_row[pair];
+                        g[u] = p.pair_w[pair];
                     }
+#pragma unroll
+                    for (int u = 0; u < U; u++)
+#pragma unroll
+                        for (int j = 0; j < NV; j++)
+                            if (i0 + j * step < W) raw_vec<T, V>(sub + (size_t)at[u] * W + i0 + j * step, t[u][j]);
+#pragma unroll
+                    for (int u = 0; u < U; u++)
+                        if (s0 + u < p.top) {
+#pragma unroll
+                            for (int j = 0; j < NV; j++)
+                                if (i0 + j * step < W) {
+#pragma unroll
+                                    for (int k = 0; k < V; k++) sv[j][k] += g[u] * to_f32<T>(t[u][j][k]);
+                                }
+                        }
                 }
             } else {
 #pragma unroll
@@ -164,25 +265,23 @@ __global__ void __launch_bounds__(NV == 1 ? 256 : 1024) norm_step_kernel(const N
                     if (i < W) load_vec<T, V>(sub + (size_t)row * W + i, sv[j]);
                 }
             }
-            Moments m = {0.f, 0.f, 0.f};
-            float inv = 1.f;
-            if (p.w1) {
-                m = moments(sv);
-                inv = scale_of(m);
-            }
+            float2 m = make_float2(0.f, 1.f);
+            if (p.w1) m = norm_of(sv);
 #pragma unroll
             for (int j = 0; j < NV; j++) {
                 const int i = i0 + j * step;
                 if (i < W) {
                     float w[V], b[V], z[V];
 #pragma unroll
-                    for (int k = 0; k < V; k++) w[k] = 1.f, b[k] = 0.f;
-                    if (p.w1) load_vec<float, V>(p.w1 + i, w);
-                    if (p.w1 && !p.rms) load_vec<float, V>(p.b1 + i, b);
+                    for (int k = 0; k < V; k++) w[k] = EARLY ? we[0][j][k] : 1.f, b[k] = EARLY ? we[EARLY ? 1 : 0][j][k] : 0.f;
+                    if constexpr (!EARLY) {
+                        if (p.w1) load_vec<float, V>(p.w1 + i, w);
+                        if (p.w1 && !p.rms) load_vec<float, V>(p.b1 + i, b);
+                    }
                     if (p.add_x0) load_vec<float, V>(p.x0 + (size_t)row * W + i, z);
 #pragma unroll
                     for (int k = 0; k < V; k++) {
-                        xv[j][k] += p.mult * ((sv[j][k] - m.mean) * inv * w[k] + b[k]);
+                        xv[j][k] += p.mult * ((sv[j][k] - m.x) * m.y * w[k] + b[k]);
                         if (p.add_x0) xv[j][k] += z[k];
                     }
                     store_vec<float, V>(p.x + (size_t)row * W + i, xv[j]);
@@ -191,20 +290,21 @@ __global__ void __launch_bounds__(NV == 1 ? 256 : 1024) norm_step_kernel(const N
         }
     }
     if (!p.out) return;
-    Moments m = moments(xv);
-    const float inv = scale_of(m);
+    const float2 m = norm_of(xv);
     T *out = reinterpret_cast<T *>(p.out) + (size_t)row * W;
 #pragma unroll
     for (int j = 0; j < NV; j++) {
         const int i = i0 + j * step;
         if (i < W) {
             float w[V], b[V], y[V];
-            load_vec<float, V>(p.w2 + i, w);
 #pragma unroll
-            for (int k = 0; k < V; k++) b[k] = 0.f;
-            if (!p.rms) load_vec<float, V>(p.b2 + i, b);
+            for (int k = 0; k < V; k++) w[k] = EARLY ? we[EARLY ? 2 : 0][j][k] : 1.f, b[k] = EARLY ? we[EARLY ? 3 : 0][j][k] : 0.f;
+            if constexpr (!EARLY) {
+                load_vec<float, V>(p.w2 + i, w);
+                if (!p.rms) load_vec<float, V>(p.b2 + i, b);
+            }
 #pragma unroll
-            for (int k = 0; k < V; k++) y[k] = (xv[j][k] - m.mean) * inv * w[k] + b[k];
+            for (int k = 0; k < V; k++) y[k] = (xv[j][k] - m.x) * m.y * w[k] + b[k];
             store_vec<T, V>(out + i, y);
         }
     }
@@ -213,16 +313,24 @@ __global__ void __launch_bounds__(NV == 1 ? 256 : 1024) norm_step_kernel(const N
 template <typename T, int V>
 static int run_norm(cudaStream_t st, const NormStep &p, int rows) {
     const int groups = (p.W + V - 1) / V;
+    // one wave of CTAs at most, rows of up to 4096 elements: measured inside a decode step of one row of 2048 (two norms, eight expert rows)
+    if (rows <= 148 && V == 4 && groups <= 1024) {
+        const int nv = groups <= 256 ? 1 : 2, threads = ((groups + nv - 1) / nv + 31) / 32 * 32;
+        if (nv == 1) MYNN_CUDA_OK(launch_dependent(norm_step_kernel<T, 4, 1, true>, dim3(rows), dim3(threads), 0, st, p));
+        else MYNN_CUDA_OK(launch_dependent(norm_step_kernel<T, 4, 2, true>, dim3(rows), dim3(threads), 0, st, p));
+        MYNN_LAUNCH_OK("norm_step_kernel");
+        return MYNN_OK;
+    }
     const int nv = groups <= 256 ? 1 : groups <= 2048 ? 2 : groups <= 4096 ? 4 : groups <= 8192 ? 8 : V == 1 && groups <= 32768 ? 32 : 0;
     if (!nv) return fail(MYNN_E_UNSUPPORTED, "layer_norm: rows of %d elements", p.W);
     const int threads = ((groups + nv - 1) / nv + 31) / 32 * 32;
     switch (nv) {
-        case 1: norm_step_kernel<T, V, 1><<<rows, threads, 0, st>>>(p); break;
-        case 2: norm_step_kernel<T, V, 2><<<rows, threads, 0, st>>>(p); break;
-        case 4: norm_step_kernel<T, V, 4><<<rows, threads, 0, st>>>(p); break;
-        case 8: norm_step_kernel<T, V, 8><<<rows, threads, 0, st>>>(p); break;
+        case 1: MYNN_CUDA_OK(launch_dependent(norm_step_kernel<T, V, 1, false>, dim3(rows), dim3(threads), 0, st, p)); break;
+        case 2: MYNN_CUDA_OK(launch_dependent(norm_step_kernel<T, V, 2, false>, dim3(rows), dim3(threads), 0, st, p)); break;
+        case 4: MYNN_CUDA_OK(launch_dependent(norm_step_kernel<T, V, 4, false>, dim3(rows), dim3(threads), 0, st, p)); break;
+        case 8: MYNN_CUDA_OK(launch_dependent(norm_step_kernel<T, V, 8, false>, dim3(rows), dim3(threads), 0, st, p)); break;
         default:
-            if constexpr (V == 1) norm_step_kernel<T, V, 32><<<rows, threads, 0, st>>>(p);
+            if constexpr (V == 1) MYNN_CUDA_OK(launch_dependent(norm_step_kernel<T, V, 32, false>, dim3(rows), dim3(threads), 0, st, p));
             break;
     }
     MYNN_LAUNCH_OK("norm_step_kernel");

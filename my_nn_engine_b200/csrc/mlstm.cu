@@ -86,7 +86,8 @@ __global__ void __launch_bounds__(256) mlstm_out_kernel(const MlstmStep p) {
 }
 
 // grid (ceil(E / 32), H, B), 256 threads.  Warp w holds rows [w NR, (w + 1) NR) of the memory tile, lane l column l.  ONE: a single token, which
-// is all about reading and writing the memory: four CTAs per SM keep enough of it on its way.
+// is all about reading and writing the memory: four CTAs per SM keep enough of it on its way, and where the state is settled the reads
+// start while the product in front still runs.
 template <typename T, int NR, bool ONE>
 __global__ void __launch_bounds__(kScanWarps * 32, ONE && NR <= 32 ? 4 : 1) mlstm_scan_kernel(const MlstmStep p) {
     constexpr int DP = kScanWarps * NR;  // rows with padding
@@ -95,7 +96,7 @@ __global__ void __launch_bounds__(kScanWarps * 32, ONE && NR <= 32 ? 4 : 1) mlst
     __shared__ float sm_ss[kScanWarps];
     __shared__ unsigned flag;
     pdl_trigger();
-    pdl_wait();
+    if (!p.settled) pdl_wait();
     const int h = blockIdx.y, b = blockIdx.z, pair = b * p.H + h, tiles = gridDim.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, col = blockIdx.x * kScanCols + lane;
     const bool fresh = *p.past == 0, in = col < p.E;
@@ -116,6 +117,7 @@ __global__ void __launch_bounds__(kScanWarps * 32, ONE && NR <= 32 ? 4 : 1) mlst
     }
     float m = fresh ? 0.f : p.top[pair];
     const float q_scale = 1.0f / sqrtf((float)p.D), bias_i = p.gate_bias[h], bias_f = p.gate_bias[p.H + h];
+    pdl_wait();  // the projections come from the kernel in front
     constexpr int PT = (DP + 255) / 256;  // elements of q and of k a thread stages
     auto stage = [&](int t) {
         const T *row = reinterpret_cast<const T *>(p.proj) + (size_t)(b * p.S + t) * C + (size_t)h * p.D;
@@ -563,10 +565,10 @@ static int run_out(cudaStream_t st, const MlstmStep &p) {
 template <typename T, bool ONE>
 static int run_scan(cudaStream_t st, const MlstmStep &p) {
     const dim3 grid((p.E + kScanCols - 1) / kScanCols, p.H, p.B);
-    if (p.D <= 64) mlstm_scan_kernel<T, 8, ONE><<<grid, 256, 0, st>>>(p);
-    else if (p.D <= 128) mlstm_scan_kernel<T, 16, ONE><<<grid, 256, 0, st>>>(p);
-    else if (p.D <= 256) mlstm_scan_kernel<T, 32, ONE><<<grid, 256, 0, st>>>(p);
-    else mlstm_scan_kernel<T, 64, ONE><<<grid, 256, 0, st>>>(p);
+    if (p.D <= 64) MYNN_CUDA_OK(launch_dependent(mlstm_scan_kernel<T, 8, ONE>, grid, dim3(256), 0, st, p));
+    else if (p.D <= 128) MYNN_CUDA_OK(launch_dependent(mlstm_scan_kernel<T, 16, ONE>, grid, dim3(256), 0, st, p));
+    else if (p.D <= 256) MYNN_CUDA_OK(launch_dependent(mlstm_scan_kernel<T, 32, ONE>, grid, dim3(256), 0, st, p));
+    else MYNN_CUDA_OK(launch_dependent(mlstm_scan_kernel<T, 64, ONE>, grid, dim3(256), 0, st, p));
     MYNN_LAUNCH_OK("mlstm_scan_kernel");
     return ONE ? MYNN_OK : run_out<T>(st, p);
 }

@@ -1,7 +1,7 @@
 // Expert routing: softmax over the router logits, the groups with the best member, the best experts of those groups, and the
 // (token, slot) pairs ordered by expert for the grouped matrix products.
 //
-// One warp per token makes the choice (logits in shared memory, repeated warp-wide maxima; equal scores go to the lower index).
+// One warp per token makes the choice (repeated warp-wide maxima; equal scores go to the lower index).
 // A step of a few tokens runs entirely in one CTA; longer ones count in global memory, order in a second kernel and scatter in a
 // third.  The order of the pairs of one expert is not fixed, and nothing depends on it: every pair is a row of its own.
 #include "block_ops.cuh"
@@ -49,82 +49,97 @@ MoeRoute moe_route_bind(void *base, int M, int experts, int top) {
     return r;
 }
 
-// larger value first, then the lower index
-__device__ __forceinline__ void warp_argmax(float &v, int &i) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float v2 = __shfl_xor_sync(0xffffffffu, v, o);
-        const int i2 = __shfl_xor_sync(0xffffffffu, i, o);
-        if (v2 > v || (v2 == v && i2 < i)) {
-            v = v2;
-            i = i2;
-        }
-    }
+// Floats as integers in the same order (zeros of both signs are one number); 0 is below every number and marks what is out of the race.
+__device__ __forceinline__ unsigned order_key(float v) {
+    const unsigned b = __float_as_uint(v + 0.0f);
+    return b ^ ((b >> 31) ? 0xffffffffu : 0x80000000u);
+}
+__device__ __forceinline__ float key_value(unsigned k) { return __uint_as_float(k ^ ((k >> 31) ? 0x80000000u : 0xffffffffu)); }
+
+// the largest key of the warp and, of those that have it, the lowest index
+__device__ __forceinline__ void warp_argmax(unsigned &key, int &i) {
+    const unsigned best = __reduce_max_sync(0xffffffffu, key);
+    i = (int)__reduce_min_sync(0xffffffffu, key == best ? (unsigned)i : 0x7fffffffu);
+    key = best;
 }
 
-// The choice for one token by one warp; z holds its E logits and is overwritten.  Slot s: expert in lane s's `e`, weight in `w`.
+// The choice for one token by one warp; z: room for its E logits in shared memory.  Slot s: expert in lane s's `e`, weight in `w`.
+// NU: logits per lane (E <= 32 NU), in registers as ordered integers, so that a slot costs two warp reductions: at one token the choice
+// is a chain of `keep + top` of them and nothing else (eight of 64 experts out of four of eight groups: 7.7 us with five shuffle steps of value and index over
+// shared memory, 4.3 us so).
+template <int NU>
 __device__ __forceinline__ void choose(float *z, const float *src, int E, int top, int groups, int keep, int &e_out, float &w_out) {
     const int lane = threadIdx.x & 31;
-    float mx = -INFINITY;
-    for (int i = lane; i < E; i += 32) {
-        const float v = src[i];
-        z[i] = fmaxf(v, -3.0e38f);  // also for NaN: every expert stays comparable, and above the excluded ones
-        mx = fmaxf(mx, z[i]);
+    float raw[NU], mx = -INFINITY;
+    unsigned key[NU];
+#pragma unroll
+    for (int u = 0; u < NU; u++) raw[u] = lane + 32 * u < E ? src[lane + 32 * u] : 0.f;
+#pragma unroll
+    for (int u = 0; u < NU; u++) {
+        key[u] = 0u;
+        if (lane + 32 * u < E) {
+            const float v = fmaxf(raw[u], -3.0e38f);  // also for NaN: every expert stays comparable, and above the excluded ones
+            key[u] = order_key(v);
+            mx = fmaxf(mx, v);
+            if (keep < groups) z[lane + 32 * u] = v;
+        }
     }
     mx = warp_max(mx);
     float sum = 0.f;
-    for (int i = lane; i < E; i += 32) sum += expf(src[i] - mx);  // a NaN logit makes the weights NaN
+#pragma unroll
+    for (int u = 0; u < NU; u++)
+        if (lane + 32 * u < E) sum += expf(raw[u] - mx);  // a NaN logit makes the weights NaN
     sum = warp_sum(sum);
     __syncwarp();
     if (keep < groups) {
         // softmax is monotonic, so group scores may be compared as logits
         const int per = E / groups;
-        unsigned kept_lo = 0, kept_hi = 0;  // this lane's groups lane, lane + 32
-        float gs[2];
+        unsigned gk[2], kept[2] = {0u, 0u};  // this lane's groups lane, lane + 32
 #pragma unroll
         for (int u = 0; u < 2; u++) {
             const int g = lane + 32 * u;
-            gs[u] = -INFINITY;
-            if (g < groups)
-                for (int i = 0; i < per; i++) gs[u] = fmaxf(gs[u], z[g * per + i]);
+            gk[u] = 0u;
+            if (g < groups) {
+                float v = -INFINITY;
+                for (int i = 0; i < per; i++) v = fmaxf(v, z[g * per + i]);
+                gk[u] = order_key(v);
+            }
         }
         for (int k = 0; k < keep; k++) {
-            float v = -INFINITY;
-            int g = 1 << 20;
-            if (lane < groups && !kept_lo) v = gs[0], g = lane;
-            if (lane + 32 < groups && !kept_hi && (gs[1] > v || g == 1 << 20)) v = gs[1], g = lane + 32;
+            unsigned v = gk[0];
+            int g = lane;
+            if (gk[1] > v) v = gk[1], g = lane + 32;
             warp_argmax(v, g);
-            if (g == lane) kept_lo = 1;
-            if (g == lane + 32) kept_hi = 1;
+            if (g == lane) gk[0] = 0u;
+            if (g == lane + 32) gk[1] = 0u;
+            kept[g >> 5] |= 1u << (g & 31);
         }
 #pragma unroll
-        for (int u = 0; u < 2; u++) {
-            const int g = lane + 32 * u;
-            if (g < groups && !(u ? kept_hi : kept_lo))
-                for (int i = 0; i < per; i++) z[g * per + i] = -INFINITY;
+        for (int u = 0; u < NU; u++) {
+            const int i = lane + 32 * u, g = i / per;
+            if (i < E && !((g < 32 ? kept[0] : kept[1]) >> (g & 31) & 1u)) key[u] = 0u;
         }
-        __syncwarp();
     }
     e_out = 0;
     w_out = 0.f;
+    unsigned mine = 0u;
     for (int s = 0; s < top; s++) {
-        float v = -INFINITY;
-        int e = 1 << 20;
-        for (int i = lane; i < E; i += 32)
-            if (z[i] > v || e == 1 << 20) v = z[i], e = i;
+        unsigned v = key[0];
+        int e = lane;
+#pragma unroll
+        for (int u = 1; u < NU; u++)
+            if (key[u] > v) v = key[u], e = lane + 32 * u;
         warp_argmax(v, e);
-        if (lane == s) {
-            e_out = e;
-            w_out = expf(v - mx) / sum;
-        }
-        __syncwarp();
-        if (lane == 0) z[e] = -INFINITY;
-        __syncwarp();
+        if (lane == s) e_out = e, mine = v;
+#pragma unroll
+        for (int u = 0; u < NU; u++)
+            if (e == lane + 32 * u) key[u] = 0u;
     }
+    if (lane < top) w_out = expf(key_value(mine) - mx) / sum;
 }
 
 // counts -> offsets, list of used experts, tiles; one warp.  Counts are cleared on the way.
-__device__ __forceinline__ void order_experts(const MoeRoute &r, int32_t *count, int E) {
+__device__ __forceinline__ void order_experts(const MoeRoute &r, int32_t *count, int E, int32_t *off_s = nullptr) {
     const int lane = threadIdx.x & 31;
     int off = 0, act = 0, tiles = 0;
     for (int base = 0; base < E; base += 32) {
@@ -139,6 +154,7 @@ __device__ __forceinline__ void order_experts(const MoeRoute &r, int32_t *count,
         const int my_off = off + so - c, my_tile = tiles + st - nt;
         if (e < E) {
             r.off[e] = my_off;
+            if (off_s) off_s[e] = my_off;
             if (used) r.active[act + su - 1] = e;
             for (int t = 0; t < nt; t++) {
                 r.tile_e[my_tile + t] = e;
@@ -157,44 +173,48 @@ __device__ __forceinline__ void order_experts(const MoeRoute &r, int32_t *count,
     }
 }
 
-// everything for a few tokens: one CTA; dynamic shared memory: E logits per warp, then E counts
+// everything for a few tokens: one CTA; dynamic shared memory: E logits per warp, E counts, E offsets, expert and place of every pair
+static size_t route_small_smem(int warps, int M, int E, int top) { return ((size_t)(warps + 2) * E + 2 * (size_t)M * top) * 4; }
+template <int NU>
 __global__ void __launch_bounds__(1024) moe_route_small_kernel(const MoeRoute r, const float *logits, int M, int E, int top, int groups, int keep) {
     extern __shared__ float sm[];
-    pdl_trigger();
-    pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     float *z = sm + (size_t)warp * E;
-    int32_t *count = reinterpret_cast<int32_t *>(sm + (size_t)warps * E);
+    int32_t *count = reinterpret_cast<int32_t *>(sm + (size_t)warps * E), *off = count + E, *pair_e = off + E, *place = pair_e + M * top;
     for (int i = threadIdx.x; i < E; i += blockDim.x) count[i] = 0;
+    pdl_trigger();
+    pdl_wait();
     __syncthreads();
     for (int t = warp; t < M; t += warps) {
         int e;
         float w;
-        choose(z, logits + (size_t)t * E, E, top, groups, keep, e, w);
+        choose<NU>(z, logits + (size_t)t * E, E, top, groups, keep, e, w);
         if (lane < top) {
-            const size_t pair = (size_t)t * top + lane;
+            const int pair = t * top + lane;
             r.pair_w[pair] = w;
             r.pair_e[pair] = e;
-            r.pair_row[pair] = atomicAdd(&count[e], 1);  // place inside the expert for now
+            pair_e[pair] = e;
+            place[pair] = atomicAdd(&count[e], 1);
         }
     }
     __syncthreads();
-    if (warp == 0) order_experts(r, count, E);
-    __syncthreads();  // global writes of this CTA are visible to it
+    if (warp == 0) order_experts(r, count, E, off);
+    __syncthreads();
     for (int i = threadIdx.x; i < M * top; i += blockDim.x) {
-        const int row = r.off[r.pair_e[i]] + r.pair_row[i];
+        const int row = off[pair_e[i]] + place[i];
         r.pair_row[i] = row;
         r.tok_of[row] = i / top;
     }
 }
 
+template <int NU>
 __global__ void __launch_bounds__(256) moe_choose_kernel(const MoeRoute r, const float *logits, int M, int E, int top, int groups, int keep) {
     extern __shared__ float sm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = blockIdx.x * (blockDim.x >> 5) + warp;
     if (t >= M) return;
     int e;
     float w;
-    choose(sm + (size_t)warp * E, logits + (size_t)t * E, E, top, groups, keep, e, w);
+    choose<NU>(sm + (size_t)warp * E, logits + (size_t)t * E, E, top, groups, keep, e, w);
     if (lane < top) {
         const size_t pair = (size_t)t * top + lane;
         r.pair_w[pair] = w;
@@ -216,15 +236,26 @@ int launch_moe_route(cudaStream_t st, const MoeRoute &r, const float *logits, in
         (long long)top > (long long)keep * (E / groups))
         return fail(MYNN_E_ARG, "moe_route: bad routing (%d experts, top %d, %d of %d groups)", E, top, keep, groups);
     if ((long long)M * top > (1ll << 30)) return fail(MYNN_E_UNSUPPORTED, "moe_route: too many tokens");
+#define BY_EXPERTS(LAUNCH) \
+    if (E <= 64) LAUNCH(2) else if (E <= 256) LAUNCH(8) else LAUNCH(32)
     if (M <= 64) {
         const int warps = M < 32 ? M : 32;
-        const size_t smem = (size_t)(warps + 1) * E * 4;
-        if (smem > 48 * 1024) MYNN_CUDA_OK(cudaFuncSetAttribute(moe_route_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        moe_route_small_kernel<<<1, warps * 32, smem, st>>>(r, logits, M, E, top, groups, keep);
+        const size_t smem = route_small_smem(warps, M, E, top);
+#define SMALL(NU)                                                                                                                              \
+    {                                                                                                                                          \
+        auto kern = moe_route_small_kernel<NU>;                                                                                                \
+        if (smem > 48 * 1024) MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));                \
+        MYNN_CUDA_OK(launch_dependent(kern, dim3(1), dim3(warps * 32), smem, st, r, logits, M, E, top, groups, keep));                         \
+    }
+        BY_EXPERTS(SMALL)
+#undef SMALL
         MYNN_LAUNCH_OK("moe_route_small_kernel");
         return MYNN_OK;
     }
-    moe_choose_kernel<<<(M + 7) / 8, 256, (size_t)8 * E * 4, st>>>(r, logits, M, E, top, groups, keep);
+#define CHOOSE(NU) moe_choose_kernel<NU><<<(M + 7) / 8, 256, (size_t)8 * E * 4, st>>>(r, logits, M, E, top, groups, keep);
+    BY_EXPERTS(CHOOSE)
+#undef CHOOSE
+#undef BY_EXPERTS
     MYNN_LAUNCH_OK("moe_choose_kernel");
     moe_order_kernel<<<1, 32, 0, st>>>(r, E);
     MYNN_LAUNCH_OK("moe_order_kernel");

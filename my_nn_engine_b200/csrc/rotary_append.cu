@@ -45,10 +45,11 @@ template <typename T, int V>
 __global__ void __launch_bounds__(kRotWarps * 32) rotary_append_kernel(const RotaryAppend p) {
     extern __shared__ float sm[];
     pdl_trigger();
-    pdl_wait();
+    if (!p.settled) pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, job = blockIdx.x * kRotWarps + warp;
     if (job >= p.Hq + 2 * p.G) return;
     const int b = blockIdx.y / p.S, s = blockIdx.y - b * p.S, pos = *p.past + s, slot = pos % p.cache_rows;
+    pdl_wait();  // the projections of this step
     const int C = (p.Hq + p.G) * p.D + p.G * p.E;
     const T *row = reinterpret_cast<const T *>(p.proj) + (size_t)blockIdx.y * C;
     if (job >= p.Hq + p.G) {  // a value head: copied
@@ -128,8 +129,8 @@ int launch_rotary_append(cudaStream_t st, int dtype, const RotaryAppend &p) {
     const dim3 grid((p.Hq + 2 * p.G + kRotWarps - 1) / kRotWarps, p.B * p.S);
     const size_t smem = (size_t)kRotWarps * p.D * sizeof(float);
     MYNN_DISPATCH_DTYPE(dtype, T, {
-        if (vec) rotary_append_kernel<T, 4><<<grid, kRotWarps * 32, smem, st>>>(p);
-        else rotary_append_kernel<T, 1><<<grid, kRotWarps * 32, smem, st>>>(p);
+        if (vec) MYNN_CUDA_OK(launch_dependent(rotary_append_kernel<T, 4>, grid, dim3(kRotWarps * 32), smem, st, p));
+        else MYNN_CUDA_OK(launch_dependent(rotary_append_kernel<T, 1>, grid, dim3(kRotWarps * 32), smem, st, p));
     });
     MYNN_LAUNCH_OK("rotary_append_kernel");
     return MYNN_OK;

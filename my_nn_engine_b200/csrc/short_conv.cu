@@ -30,7 +30,7 @@ __device__ __forceinline__ const T *conv_source(const ConvStep &p, int b, int s,
 template <typename T, int TAPS, int TPT>
 __global__ void __launch_bounds__(128) conv_step_vec_kernel(const ConvStep p, int write_hist) {
     pdl_trigger();
-    pdl_wait();
+    if (!p.settled) pdl_wait();
     const int Cq = p.Hq * p.D, Ck = p.G * p.D, C = Cq + Ck + p.G * p.E;
     const int c = (blockIdx.x * 128 + threadIdx.x) * 8;
     if (c >= C) return;
@@ -38,22 +38,28 @@ __global__ void __launch_bounds__(128) conv_step_vec_kernel(const ConvStep p, in
     const int past = *p.past;
     constexpr int LAG = TAPS > 0 ? TAPS - 1 : 0;
     uint4 raw[TPT + LAG];  // rows s0 - LAG .. s0 + TPT - 1
+    auto fetch = [&](bool earlier) {  // rows of earlier steps, rows of this one
 #pragma unroll
-    for (int i = 0; i < TPT + LAG; i++) {
-        raw[i] = make_uint4(0u, 0u, 0u, 0u);
-        const int s = s0 + i - LAG;
-        if (s < p.S) {
-            bool zero;
-            const T *src = conv_source<T>(p, b, s, 0, past, C, zero);
-            if (!zero) raw[i] = *reinterpret_cast<const uint4 *>(src + c);
+        for (int i = 0; i < TPT + LAG; i++) {
+            const int s = s0 + i - LAG;
+            if ((s < 0) != earlier) continue;
+            raw[i] = make_uint4(0u, 0u, 0u, 0u);
+            if (s < p.S) {
+                bool zero;
+                const T *src = conv_source<T>(p, b, s, 0, past, C, zero);
+                if (!zero) raw[i] = *reinterpret_cast<const uint4 *>(src + c);
+            }
         }
-    }
+    };
+    fetch(true);
     float w[TAPS > 0 ? TAPS : 1][8];
 #pragma unroll
     for (int j = 0; j < TAPS; j++) {
         const float4 a = *reinterpret_cast<const float4 *>(p.w + (size_t)j * C + c), d = *reinterpret_cast<const float4 *>(p.w + (size_t)j * C + c + 4);
         w[j][0] = a.x, w[j][1] = a.y, w[j][2] = a.z, w[j][3] = a.w, w[j][4] = d.x, w[j][5] = d.y, w[j][6] = d.z, w[j][7] = d.w;
     }
+    pdl_wait();  // the projections of this step
+    fetch(false);
     // where token 0 of the sequence's step goes, and how far apart tokens are
     int d, rows = 0;
     T *dst;
@@ -182,11 +188,11 @@ template <typename T, int TPT>
 static int run_conv_vec(cudaStream_t st, const ConvStep &p, int C, int fused) {
     const dim3 grid((C / 8 + 127) / 128, p.B * ((p.S + TPT - 1) / TPT));
     switch (p.taps) {
-        case 0: conv_step_vec_kernel<T, 0, TPT><<<grid, 128, 0, st>>>(p, fused); break;
-        case 1: conv_step_vec_kernel<T, 1, TPT><<<grid, 128, 0, st>>>(p, fused); break;
-        case 2: conv_step_vec_kernel<T, 2, TPT><<<grid, 128, 0, st>>>(p, fused); break;
-        case 3: conv_step_vec_kernel<T, 3, TPT><<<grid, 128, 0, st>>>(p, fused); break;
-        default: conv_step_vec_kernel<T, 4, TPT><<<grid, 128, 0, st>>>(p, fused); break;
+        case 0: MYNN_CUDA_OK(launch_dependent(conv_step_vec_kernel<T, 0, TPT>, grid, dim3(128), 0, st, p, fused)); break;
+        case 1: MYNN_CUDA_OK(launch_dependent(conv_step_vec_kernel<T, 1, TPT>, grid, dim3(128), 0, st, p, fused)); break;
+        case 2: MYNN_CUDA_OK(launch_dependent(conv_step_vec_kernel<T, 2, TPT>, grid, dim3(128), 0, st, p, fused)); break;
+        case 3: MYNN_CUDA_OK(launch_dependent(conv_step_vec_kernel<T, 3, TPT>, grid, dim3(128), 0, st, p, fused)); break;
+        default: MYNN_CUDA_OK(launch_dependent(conv_step_vec_kernel<T, 4, TPT>, grid, dim3(128), 0, st, p, fused)); break;
     }
     MYNN_LAUNCH_OK("conv_step_vec_kernel");
     return launch_history<T>(st, p, C, fused);

@@ -54,7 +54,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     constexpr int KCH = D / 32;  // 16-byte K chunks per lane per row
     constexpr int VH = D / 64;   // 16-byte V chunks per lane per row
     pdl_trigger();
-    pdl_wait();  // q, the newest kv row and the active length come from the preceding kernels
+    if (!p.settled) pdl_wait();  // else only q and the newest kv row come from the preceding kernels
     const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int G = p.G;
@@ -110,8 +110,16 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
         __syncthreads();
+        // with a settled cache the tiles that do not hold the newest row set out while the projection in front still runs (with the
+        // fused append no tile does: the new row never comes from the cache)
+        int j = 0;
+        if (lane == 0 && p.settled)
+            for (; j < min(ntile, kRingDepth) && (fused || first + 16 * kAttnWarps * j + 16 < active); j++) issue(j);
+        pdl_wait();
         if (lane == 0)
-            for (int j = 0; j < min(ntile, kRingDepth); j++) issue(j);
+            for (; j < min(ntile, kRingDepth); j++) issue(j);
+    } else {
+        pdl_wait();
     }
     // x rotated against its partner xp (the element half a head away): low half x c - xp s, high half x c + xp s, rounded to
     // the storage type as the stand-alone RoPE kernel rounds it
@@ -481,7 +489,7 @@ static int launch_decode(cudaStream_t st, const DecodeParams &p, int B, bool rin
             MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             attr_set = true;
         }
-        MYNN_CUDA_OK(launch_pdl(kern, dim3(p.splits, p.Hkv, B), dim3(kAttnWarps * 32), smem, st, mk, mv, p));
+        MYNN_CUDA_OK(launch_dependent(kern, dim3(p.splits, p.Hkv, B), dim3(kAttnWarps * 32), smem, st, mk, mv, p));
     } else {
         MYNN_CUDA_OK(launch_pdl(attention_decode_kernel<T, D, false, WIN>, dim3(p.splits, p.Hkv, B), dim3(kAttnWarps * 32), 0, st, mk, mv, p));
     }
@@ -627,6 +635,7 @@ int mynn::launch_attention(cudaStream_t st, void *out, const void *q, const void
         p.sin_t = fuse->sin_t;
         p.fused_pos = fuse->pos;
         p.fused_row = fuse->row;
+        p.settled = fuse->settled;
     }
     if (int rc = decode_bind_workspace(p, B, D, workspace, workspace_bytes)) return rc;
     if (dtype == MYNN_BF16) return D == 64 ? launch_decode<__nv_bfloat16, 64>(st, p, B, ring) : launch_decode<__nv_bfloat16, 128>(st, p, B, ring);
@@ -663,6 +672,7 @@ int mynn::launch_window_attention_decode(cudaStream_t st, int dtype, const Windo
     p.chunk = w.chunk;
     p.ring_cache = 1;
     p.softcap = w.softcap;
+    p.settled = w.settled;
     if (int rc = decode_bind_workspace(p, w.B, w.D, w.workspace, w.workspace_bytes)) return rc;
     if (dtype == MYNN_BF16) return w.D == 64 ? launch_decode<__nv_bfloat16, 64, true>(st, p, w.B, ring) : launch_decode<__nv_bfloat16, 128, true>(st, p, w.B, ring);
     return w.D == 64 ? launch_decode<__half, 64, true>(st, p, w.B, ring) : launch_decode<__half, 128, true>(st, p, w.B, ring);

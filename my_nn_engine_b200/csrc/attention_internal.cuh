@@ -117,6 +117,9 @@ struct DecodeParams {
     int window = 0, ring_cache = 0;
     int chunk = 0;  // and none before the query's own chunk of that many positions (counted from position 0)
     float softcap = 0.f;
+    // Of what the kernel reads, the kernels right in front of it write q and the newest key and value rows only: cached rows, positions and
+    // the active length may be read while they still run.
+    int settled = 0;
     int *status = nullptr;  // ring kernel: where a timed-out wait is recorded (null: the library's own word, see attention_check)
 };
 

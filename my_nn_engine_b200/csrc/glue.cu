@@ -308,12 +308,12 @@ int launch_rope_kv_append(cudaStream_t st, int dtype, void *q_out, void *k_cache
         const unsigned blocks = (unsigned)((units + 255) / 256);
         if (dtype == MYNN_BF16) {
             using T = __nv_bfloat16;
-            MYNN_CUDA_OK(launch_pdl(rope_kv_append_vec_kernel<T>, dim3(blocks), dim3(256), 0, st, (T *)q_out, (T *)k_cache, (T *)v_cache,
+            MYNN_CUDA_OK(launch_dependent(rope_kv_append_vec_kernel<T>, dim3(blocks), dim3(256), 0, st, (T *)q_out, (T *)k_cache, (T *)v_cache,
                                     (const T *)q, (const T *)k, (const T *)v, q_stride, k_stride, v_stride, (const T *)cos_t,
                                     (const T *)sin_t, positions, units, S, Hq, Hkv, D, cache_seq, past_len_dev, rotate_k));
         } else {
             using T = __half;
-            MYNN_CUDA_OK(launch_pdl(rope_kv_append_vec_kernel<T>, dim3(blocks), dim3(256), 0, st, (T *)q_out, (T *)k_cache, (T *)v_cache,
+            MYNN_CUDA_OK(launch_dependent(rope_kv_append_vec_kernel<T>, dim3(blocks), dim3(256), 0, st, (T *)q_out, (T *)k_cache, (T *)v_cache,
                                     (const T *)q, (const T *)k, (const T *)v, q_stride, k_stride, v_stride, (const T *)cos_t,
                                     (const T *)sin_t, positions, units, S, Hq, Hkv, D, cache_seq, past_len_dev, rotate_k));
         }

@@ -27,6 +27,8 @@
 
 #include <cstring>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "i8_gemm.cuh"
 #include "tcgen05.cuh"
@@ -609,6 +611,80 @@ rms_norm_limbs_kernel(int8_t *limbs, float *ascale, T *norm_out, T *sum_out, con
     MYNN_GLUE_END();
 }
 
+// The same for rows of at most 8 elements per thread, which stay in registers (blockDim.x = D / 8 rounded up to whole warps).  A row or a
+// few is a chain of dependent steps, so they are kept short: the norm's weights, which belong to the model, are requested in front of the
+// wait for the preceding kernel, and both block reductions are finished by every thread for itself.
+template <typename T>
+__global__ void __launch_bounds__(kRowThreads)
+rms_norm_limbs_row_kernel(int8_t *limbs, float *ascale, T *norm_out, T *sum_out, const T *x, const float *part, const T *w, float eps, int D) {
+    __shared__ float red_s[32], red_m[32];
+    MYNN_GLUE_BEGIN(1);
+    pdl_trigger();
+    const int m = blockIdx.x, i0 = 8 * threadIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    const size_t base = (size_t)m * D;
+    const bool in = i0 < D;
+    float wv[8], v[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) wv[j] = v[j] = 0.f;
+    if (in) load8<T>(w + i0, wv);
+    pdl_wait();
+    if (in) {
+        load8<T>(x + base + i0, v);
+        if (part != nullptr) {
+            float pp[8];
+            load8<float>(part + base + i0, pp);
+#pragma unroll
+            for (int j = 0; j < 8; j++) v[j] = round_store<T>(v[j] + round_store<T>(pp[j]));
+            store8<T>(sum_out + base + i0, v);
+        }
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; j++) ss += v[j] * v[j];
+    ss = warp_sum(ss);
+    if (lane == 0) red_s[warp] = ss;
+    __syncthreads();
+    float tot = 0.f;
+    for (int i = 0; i < warps; i++) tot += red_s[i];
+    const float inv = 1.0f / sqrtf(tot / (float)D + eps);
+    float mx = 0.f;
+    bool bad = false;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        v[j] = round_store<T>(v[j] * inv * wv[j]);
+        bad |= !(fabsf(v[j]) <= 3.0e38f);
+        mx = fmaxf(mx, fabsf(v[j]));
+    }
+    if (in && norm_out != nullptr) store8<T>(norm_out + base + i0, v);
+    mx = warp_max(mx);
+    if (lane == 0) red_m[warp] = mx;
+    const unsigned anybad = __syncthreads_or(in && bad);
+    float top = red_m[0];
+    for (int i = 1; i < warps; i++) top = fmaxf(top, red_m[i]);
+    int e = 0;
+    if (top > 0.f) frexpf(top, &e);
+    const float sc1 = top > 0.f ? ldexpf(1.0f, 22 - e) : 1.0f, sc = anybad ? 0.f : sc1;
+    if (threadIdx.x == 0) ascale[m] = anybad ? __int_as_float(0x7fc00000) : 1.0f / sc1;  // non-finite input -> NaN outputs
+    if (in) {
+        uint32_t l[3][2] = {};
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            int A = sc == 0.f ? 0 : __float2int_rn(v[j] * sc);
+            const int d0 = (int)(int8_t)(A & 0xFF);
+            A = (A - d0) >> 8;
+            const int d1 = (int)(int8_t)(A & 0xFF);
+            A = (A - d1) >> 8;
+            l[0][j >> 2] |= (uint32_t)(d0 & 0xFF) << (8 * (j & 3));
+            l[1][j >> 2] |= (uint32_t)(d1 & 0xFF) << (8 * (j & 3));
+            l[2][j >> 2] |= (uint32_t)(A & 0xFF) << (8 * (j & 3));
+        }
+        int8_t *out = limbs + (size_t)(3 * m) * D + i0;
+#pragma unroll
+        for (int k = 0; k < 3; k++) *reinterpret_cast<uint2 *>(out + (size_t)k * D) = make_uint2(l[k][0], l[k][1]);
+    }
+    MYNN_GLUE_END();
+}
+
 // h = round(swish(gate) * up) -> limbs; gate/up rows are in_stride elements apart.  F % 8 == 0, 16-byte aligned rows.
 template <typename T>
 __global__ void __launch_bounds__(kRowThreads)
@@ -656,7 +732,7 @@ swiglu_limbs_cluster_kernel(int8_t *limbs, float *ascale, const T *gate, const T
     const int seg = F / C, f0 = rank * seg;
     float mx = 0.f;
     bool bad = false;
-    for (int i = 8 * threadIdx.x; i < seg; i += 8 * kSegThreads) {
+    for (int i = 8 * threadIdx.x; i < seg; i += 8 * blockDim.x) {
         float g[8], u[8];
         load8<T>(gate + (size_t)m * in_stride + f0 + i, g);
         load8<T>(up + (size_t)m * in_stride + f0 + i, u);
@@ -674,7 +750,7 @@ swiglu_limbs_cluster_kernel(int8_t *limbs, float *ascale, const T *gate, const T
     __syncthreads();
     if (threadIdx.x < C) {  // thread r delivers this CTA's maximum to cluster rank r
         float t = 0.f;
-        for (int i = 0; i < kSegThreads / 32; i++) t = fmaxf(t, red[i]);
+        for (int i = 0; i < (int)(blockDim.x >> 5); i++) t = fmaxf(t, red[i]);
         if (anybad) t = -1.f;
         uint32_t remote;
         asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(&peer_max[rank])), "r"((uint32_t)threadIdx.x));
@@ -854,7 +930,7 @@ int i8_gemm_launch_tp(cudaStream_t st, void *out, const void *act, const int8_t 
     if (row_kernel) {                                                                                                    \
         auto kern = act_limbs_row_kernel<T>;                                                                             \
         if (smem > 48 * 1024) MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-        MYNN_CUDA_OK(launch_pdl(kern, dim3(M), dim3(kRowThreads), smem, st, limbs, ascale, (const T *)act, K));          \
+        MYNN_CUDA_OK(launch_dependent(kern, dim3(M), dim3(kRowThreads), smem, st, limbs, ascale, (const T *)act, K));          \
     } else {                                                                                                             \
         MYNN_CUDA_OK(launch_pdl(act_to_limbs_kernel<T>, dim3(M), dim3(256), 0, st, limbs, ascale, (const T *)act, K));   \
     }
@@ -933,11 +1009,19 @@ int launch_rms_norm_limbs(cudaStream_t st, int dtype, void *workspace, size_t wo
     float *ascale;
     int rc = fused_ws(workspace, workspace_bytes, rows, D, &limbs, &ascale);
     if (rc) return rc;
+    if (D <= 8 * kRowThreads) {
+        MYNN_DISPATCH_DTYPE(dtype, T, {
+            MYNN_CUDA_OK(launch_dependent(rms_norm_limbs_row_kernel<T>, dim3(rows), dim3((D / 8 + 31) / 32 * 32), 0, st, limbs, ascale, (T *)norm_out, (T *)sum_out,
+                                          (const T *)x, part, (const T *)w, eps, D));
+        });
+        MYNN_LAUNCH_OK("rms_norm_limbs_row_kernel");
+        return MYNN_OK;
+    }
     const size_t smem = (size_t)D * 4;
     MYNN_DISPATCH_DTYPE(dtype, T, {
         auto kern = rms_norm_limbs_kernel<T>;
         if (smem > 48 * 1024) MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        MYNN_CUDA_OK(launch_pdl(kern, dim3(rows), dim3(kRowThreads), smem, st, limbs, ascale, (T *)norm_out, (T *)sum_out, (const T *)x, part, (const T *)w, eps, D));
+        MYNN_CUDA_OK(launch_dependent(kern, dim3(rows), dim3(kRowThreads), smem, st, limbs, ascale, (T *)norm_out, (T *)sum_out, (const T *)x, part, (const T *)w, eps, D));
     });
     MYNN_LAUNCH_OK("rms_norm_limbs_kernel");
     return MYNN_OK;
@@ -963,16 +1047,18 @@ int launch_swiglu_limbs(cudaStream_t st, int dtype, void *workspace, size_t work
             if (smem > 48 * 1024) MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(C, rows, 1);
-            cfg.blockDim = dim3(kSegThreads, 1, 1);
+            cfg.blockDim = dim3(std::min(kSegThreads, (F / C / 8 + 31) / 32 * 32), 1, 1);
             cfg.dynamicSmemBytes = smem;
             cfg.stream = st;
-            cudaLaunchAttribute attr[1];
+            cudaLaunchAttribute attr[2];
             attr[0].id = cudaLaunchAttributeClusterDimension;
             attr[0].val.clusterDim.x = C;
             attr[0].val.clusterDim.y = 1;
             attr[0].val.clusterDim.z = 1;
+            attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[1].val.programmaticStreamSerializationAllowed = 1;
             cfg.attrs = attr;
-            cfg.numAttrs = 1;
+            cfg.numAttrs = 2;
             MYNN_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, limbs, ascale, (const T *)gate, (const T *)up, F, in_stride));
         });
         MYNN_LAUNCH_OK("swiglu_limbs_cluster_kernel");
@@ -982,7 +1068,7 @@ int launch_swiglu_limbs(cudaStream_t st, int dtype, void *workspace, size_t work
     MYNN_DISPATCH_DTYPE(dtype, T, {
         auto kern = swiglu_limbs_kernel<T>;
         if (smem > 48 * 1024) MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        MYNN_CUDA_OK(launch_pdl(kern, dim3(rows), dim3(kRowThreads), smem, st, limbs, ascale, (const T *)gate, (const T *)up, F, in_stride));
+        MYNN_CUDA_OK(launch_dependent(kern, dim3(rows), dim3(kRowThreads), smem, st, limbs, ascale, (const T *)gate, (const T *)up, F, in_stride));
     });
     MYNN_LAUNCH_OK("swiglu_limbs_kernel");
     return MYNN_OK;

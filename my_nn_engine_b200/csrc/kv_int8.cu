@@ -133,7 +133,7 @@ int launch_rope_kv_append_q8(cudaStream_t st, int dtype, void *q_out, void *k_ca
         slot0 = Hq;
     }
     MYNN_DISPATCH_DTYPE(dtype, T, {
-        MYNN_CUDA_OK(launch_pdl(rope_kv_append_q8_kernel<T>, dim3(B * S, Hq + 2 * Hkv - slot0), dim3(64), (size_t)D * 4, st, (T *)q_out,
+        MYNN_CUDA_OK(launch_dependent(rope_kv_append_q8_kernel<T>, dim3(B * S, Hq + 2 * Hkv - slot0), dim3(64), (size_t)D * 4, st, (T *)q_out,
                                 (int8_t *)k_cache, (int8_t *)v_cache, (T *)k_scale, (T *)v_scale, (const T *)q, (const T *)k,
                                 (const T *)v, q_stride, k_stride, v_stride, (const T *)cos_t, (const T *)sin_t, positions, S,
                                 Hq, Hkv, D, cache_seq, past_len_dev, slot0, rotate_k));
@@ -583,7 +583,7 @@ static int launch_decode_q8(cudaStream_t st, const DecodeParams &p, int B, bool 
                 MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
                 attr_set = true;
             }
-            MYNN_CUDA_OK(launch_pdl(kern, dim3(p.splits, p.Hkv, B), dim3(kAttnWarps * 32), smem, st, mk, mv, p));
+            MYNN_CUDA_OK(launch_dependent(kern, dim3(p.splits, p.Hkv, B), dim3(kAttnWarps * 32), smem, st, mk, mv, p));
             MYNN_LAUNCH_OK("attention_decode_q8_kernel");
             return MYNN_OK;
         }

@@ -195,7 +195,7 @@ static int enqueue_forward(Model &m, cudaStream_t st, int S, int head_rows = 0) 
             const bool fuse_rope = g_fuse_rope && attn_limbs && L.qkv_fused && qs % 8 == 0 && D % 32 == 0 &&
                                    (((uintptr_t)kb | (uintptr_t)vb) % 16) == 0;
             if (fuse_rope) {
-                const AttentionFuse fz = {kb, vb, qs, m.cos_t, m.sin_t, m.pos0_dev, m.past_dev};
+                const AttentionFuse fz = {kb, vb, qs, m.cos_t, m.sin_t, m.pos0_dev, m.past_dev, 1};  // the inputs' copy lies between two steps
                 RC(launch_attention(st, m.attn, qb, L.kc, L.vc, attn_scale, B, m.Hq, m.Hkv, S, D, c.max_seq_len, c.max_seq_len,
                                     m.active_dev, 0, dt, m.attn_ws, m.attn_ws_bytes, 1, (int8_t *)m.gemm_ws + 512,
                                     (float *)((char *)m.gemm_ws + 256), &fz, (int *)m.gemm_ws));

@@ -60,6 +60,7 @@ struct AttentionFuse {
     const void *cos_t, *sin_t;
     const int64_t *pos;
     const int32_t *row;
+    int settled;  // see DecodeParams
 };
 int launch_attention(cudaStream_t st, void *out, const void *q, const void *k, const void *v, float scale, int B,
                      int Hq, int Hkv, int Sq, int D, int cache_seq_len, int active_seq_kv,

@@ -86,7 +86,7 @@ int launch_rope_cache_rows(cudaStream_t st, int dtype, void *out, const void *x,
     MYNN_DISPATCH_DTYPE(dtype, T, {
         if (vec) {
             const long long n = (long long)bound * (D / 16);
-            MYNN_CUDA_OK(launch_pdl(rope_cache_rows_kernel<T>, dim3((unsigned)((n + 255) / 256), BH), dim3(256), 0, st, (T *)out, (const T *)x,
+            MYNN_CUDA_OK(launch_dependent(rope_cache_rows_kernel<T>, dim3((unsigned)((n + 255) / 256), BH), dim3(256), 0, st, (T *)out, (const T *)x,
                                     (const T *)cos_t, (const T *)sin_t, kv_position, cache_seq, D, active_host, active_dev));
         } else {
             const long long n = (long long)bound * (D / 2);

@@ -89,6 +89,53 @@ __global__ void __launch_bounds__(kDqThreads) dyn_quantize_kernel(void *y_, T *y
     }
 }
 
+// MODE 0 for 16-bit rows of up to 8192 elements (a multiple of 8, 16-byte aligned): the row is read once, 16 bytes at a time, and stays in
+// registers between the maximum and the rounding.  Bound by memory (6 MB in, 3 MB out for 777 x 4096); the general kernel above,
+// two bytes at a time and twice over the row, takes 9.5 us for that.
+constexpr int kDqRowThreads = 256, kDqRowVecs = 4;
+template <typename T>
+__global__ void __launch_bounds__(kDqRowThreads) dyn_quantize_row_kernel(int8_t *y, T *y_scale, int8_t *y_zp, const T *x, int inner) {
+    __shared__ float buf[kDqRowThreads / 32];
+    pdl_trigger();
+    pdl_wait();
+    const size_t slice = blockIdx.x;
+    const T *xs = x + slice * inner;
+    uint4 raw[kDqRowVecs];
+    float amax = 0.f;
+#pragma unroll
+    for (int u = 0; u < kDqRowVecs; u++) {
+        const int i = 8 * (threadIdx.x + u * kDqRowThreads);
+        raw[u] = i < inner ? *reinterpret_cast<const uint4 *>(xs + i) : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int u = 0; u < kDqRowVecs; u++) {
+        const T *e = reinterpret_cast<const T *>(&raw[u]);
+#pragma unroll
+        for (int j = 0; j < 8; j++) amax = fmaxf(amax, fabsf(to_f32<T>(e[j])));
+    }
+    amax = warp_max(amax);
+    if ((threadIdx.x & 31) == 0) buf[threadIdx.x >> 5] = amax;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kDqRowThreads / 32; i++) amax = fmaxf(amax, buf[i]);
+    const float sc = amax > 0.f ? __fdiv_rn(amax, 127.0f) : 1.0f;
+    const float inv = __fdiv_rn(1.0f, sc);
+    if (threadIdx.x == 0) {
+        y_scale[slice] = from_f32<T>(sc);
+        y_zp[slice] = 0;
+    }
+#pragma unroll
+    for (int u = 0; u < kDqRowVecs; u++) {
+        const int i = 8 * (threadIdx.x + u * kDqRowThreads);
+        if (i >= inner) break;
+        const T *e = reinterpret_cast<const T *>(&raw[u]);
+        __align__(8) int8_t q[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) q[j] = (int8_t)fmaxf(-127.f, fminf(127.f, roundf(__fmul_rn(to_f32<T>(e[j]), inv))));
+        *reinterpret_cast<uint2 *>(y + slice * inner + i) = *reinterpret_cast<const uint2 *>(q);
+    }
+}
+
 // one warp per output element group: warp (m, n-block of 32): lane handles n = n0 + lane, loops K bytes 4 at a time
 template <typename T>
 __global__ void quantized_matmul_generic_kernel(T *out, const int8_t *lhs, const T *lhs_scale, int ls_stride, const int8_t *rhs,
@@ -119,6 +166,15 @@ extern "C" int mynn_b200_dynamic_quantize_linear(void *stream, void *y, void *y_
     }
     if (blocks > 0x7fffffffLL) return fail(MYNN_E_UNSUPPORTED, "dynamic_quantize_linear: too many slices");
     cudaStream_t st = (cudaStream_t)stream;
+    if (symmetric && per_row && dtype != MYNN_F32 && inner % 8 == 0 && inner <= 8ll * kDqRowThreads * kDqRowVecs && (((uintptr_t)x | (uintptr_t)y) % 16) == 0) {
+        const dim3 grid((unsigned)blocks), block(kDqRowThreads);
+        if (dtype == MYNN_BF16)
+            MYNN_CUDA_OK(launch_dependent(dyn_quantize_row_kernel<__nv_bfloat16>, grid, block, 0, st, (int8_t *)y, (__nv_bfloat16 *)y_scale, (int8_t *)y_zero_point, (const __nv_bfloat16 *)x, (int)inner));
+        else
+            MYNN_CUDA_OK(launch_dependent(dyn_quantize_row_kernel<__half>, grid, block, 0, st, (int8_t *)y, (__half *)y_scale, (int8_t *)y_zero_point, (const __half *)x, (int)inner));
+        MYNN_LAUNCH_OK("dyn_quantize_row_kernel");
+        return MYNN_OK;
+    }
     MYNN_DISPATCH_DTYPE(dtype, T, {
         if (!symmetric)
             dyn_quantize_kernel<T, 2><<<(unsigned)blocks, kDqThreads, 0, st>>>(y, (T *)y_scale, y_zero_point, (const T *)x, len);

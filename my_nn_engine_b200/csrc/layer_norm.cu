@@ -3,44 +3,12 @@
 // A sandwich-normed layer does x += mult * LN(sublayer output) and then feeds LN(x) to the next sublayer.  Both norms, the
 // residual sum, the combination of routed experts and the addition of the embedding output at the start of a repeated pass
 // are row operations, so one kernel does them with one read of the sublayer output and one read and write of x.
-// Two forms of the statistics, both accurate when the mean is large against the deviations.  Many rows: mean and squared deviations are
-// gathered per thread around the thread's own mean and merged pairwise (the update of Chan, Golub and LeVeque), one block reduction
-// per norm.  Few rows: sums, first for the mean and then for the deviations around it, because the merge's divisions are the longer chain.
+// The row stays in registers, so the deviations are taken around its mean in a second pass, which stays accurate when the mean is
+// large against them.  (Merged moments, one block reduction in place of two, were slower: a division per merge in a chain of 13.)
 #include "block_ops.cuh"
 #include "common.cuh"
 
 namespace mynn {
-
-struct Moments {
-    float n, mean, m2;
-};
-__device__ __forceinline__ Moments merge(const Moments &a, const Moments &b) {
-    Moments r;
-    r.n = a.n + b.n;
-    const float d = b.mean - a.mean, f = r.n > 0.f ? b.n / r.n : 0.f;
-    r.mean = a.mean + d * f;
-    r.m2 = a.m2 + b.m2 + d * d * a.n * f;
-    return r;
-}
-
-// every thread gets the moments of the whole row; sm holds one entry per warp
-__device__ __forceinline__ Moments block_moments(Moments v, Moments *sm) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        Moments u;
-        u.n = __shfl_xor_sync(0xffffffffu, v.n, o);
-        u.mean = __shfl_xor_sync(0xffffffffu, v.mean, o);
-        u.m2 = __shfl_xor_sync(0xffffffffu, v.m2, o);
-        v = merge(v, u);
-    }
-    const int warps = blockDim.x >> 5;
-    __syncthreads();  // sm may still be read from the previous call
-    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = v;
-    __syncthreads();
-    Moments t = sm[0];
-    for (int w = 1; w < warps; w++) t = merge(t, sm[w]);
-    return t;
-}
 
 // Sums of two numbers over the block; every thread gets them.  sm holds two numbers per warp (32 pairs) and must not be the buffer of the
 // call before (calls take turns between two), so one barrier per call is enough.
@@ -114,12 +82,11 @@ __device__ __forceinline__ void store_vec(T *p, const float (&v)[V]) {
 
 // grid = rows.  NV groups of V elements per thread live in registers between the passes (NV * V * blockDim.x >= W).
 // FEW: a decode step, whose time is the chain of dependent steps: the weights are requested in front of the wait for the preceding kernel
-// when they are known not to come from it, the expert rows are requested together, and the statistics take the shorter chain.
-// For many rows that would only cost registers.
-template <typename T, int V, int NV, bool FEW>
-__global__ void __launch_bounds__(NV == 1 ? 256 : FEW ? 512 : 1024) norm_step_kernel(const NormStep p) {
+// when they are known not to come from it, and all expert rows together.  Many rows are bound by how many of them an SM has on their
+// way: 256 threads per row of up to 4096 elements and at most 64 registers, four rows per SM (two of 512 threads before).
+template <typename T, int V, int NV, bool FEW, int THREADS>
+__global__ void __launch_bounds__(THREADS, !FEW && THREADS == 256 && V == 4 ? 4 : 1) norm_step_kernel(const NormStep p) {
     __shared__ float2 sm[2][32];
-    __shared__ Moments sm_m[32];
     const int row = blockIdx.x, W = p.W;
     const int step = blockDim.x * V, i0 = threadIdx.x * V;
     constexpr bool EARLY = FEW;  // weights of both norms in registers
@@ -145,36 +112,6 @@ __global__ void __launch_bounds__(NV == 1 ? 256 : FEW ? 512 : 1024) norm_step_ke
     // mean (0 for a norm by root mean square) and reciprocal deviation of the row.  The deviations are taken around the mean of the whole
     // row, and what rounding left of their own mean corrects both.
     auto norm_of = [&](const float (&v)[NV][V]) {
-        if constexpr (!FEW) {
-            Moments m = {0.f, 0.f, 0.f};
-            float s = 0.f;
-            int n = 0;
-#pragma unroll
-            for (int j = 0; j < NV; j++)
-                if (i0 + j * step < W) {
-#pragma unroll
-                    for (int e = 0; e < V; e++) s += v[j][e];
-                    n += V;
-                }
-            m.n = (float)n;
-            m.mean = n ? s / (float)n : 0.f;
-#pragma unroll
-            for (int j = 0; j < NV; j++)
-                if (i0 + j * step < W) {
-#pragma unroll
-                    for (int e = 0; e < V; e++) {
-                        const float d = v[j][e] - m.mean;
-                        m.m2 += d * d;
-                    }
-                }
-            m = block_moments(m, sm_m);
-            float q = m.m2 / (float)W;
-            if (p.rms) {  // nothing is taken off, and mean(v^2) = var + mean^2
-                q += m.mean * m.mean;
-                m.mean = 0.f;
-            }
-            return make_float2(m.mean, 1.0f / sqrtf(q + p.eps));
-        }
         float s = 0.f, q = 0.f, mean = 0.f;
 #pragma unroll
         for (int pass = 0; pass < 2; pass++) {
@@ -231,7 +168,7 @@ __global__ void __launch_bounds__(NV == 1 ? 256 : FEW ? 512 : 1024) norm_step_ke
 #pragma unroll
                     for (int k = 0; k < V; k++) sv[j][k] = 0.f;
                 // rows in flight together: one after the other each would cost a trip to L2
-                constexpr int U = FEW ? 8 : 1;
+                constexpr int U = FEW ? 8 : NV <= 4 ? 2 : 1;
                 for (int s0 = 0; s0 < p.top; s0 += U) {
                     T t[U][NV][V];
                     float g[U];
@@ -313,26 +250,34 @@ __global__ void __launch_bounds__(NV == 1 ? 256 : FEW ? 512 : 1024) norm_step_ke
 template <typename T, int V>
 static int run_norm(cudaStream_t st, const NormStep &p, int rows) {
     const int groups = (p.W + V - 1) / V;
+#define RUN(NV, FEW, THREADS) MYNN_CUDA_OK(launch_dependent(norm_step_kernel<T, V, NV, FEW, THREADS>, dim3(rows), dim3(threads), 0, st, p))
     // one wave of CTAs at most, rows of up to 4096 elements: measured inside a decode step of one row of 2048 (two norms, eight expert rows)
-    if (rows <= 148 && V == 4 && groups <= 1024) {
-        const int nv = groups <= 256 ? 1 : 2, threads = ((groups + nv - 1) / nv + 31) / 32 * 32;
-        if (nv == 1) MYNN_CUDA_OK(launch_dependent(norm_step_kernel<T, 4, 1, true>, dim3(rows), dim3(threads), 0, st, p));
-        else MYNN_CUDA_OK(launch_dependent(norm_step_kernel<T, 4, 2, true>, dim3(rows), dim3(threads), 0, st, p));
-        MYNN_LAUNCH_OK("norm_step_kernel");
-        return MYNN_OK;
-    }
-    const int nv = groups <= 256 ? 1 : groups <= 2048 ? 2 : groups <= 4096 ? 4 : groups <= 8192 ? 8 : V == 1 && groups <= 32768 ? 32 : 0;
+    const bool few = rows <= 148 && V == 4 && groups <= 1024;
+    const int nv = few ? (groups <= 256 ? 1 : 2) : V == 4 && groups <= 1024 ? (groups <= 256 ? 1 : groups <= 512 ? 2 : 4)
+                   : groups <= 2048 ? 2 : groups <= 4096 ? 4 : groups <= 8192 ? 8 : V == 1 && groups <= 32768 ? 32 : 0;
     if (!nv) return fail(MYNN_E_UNSUPPORTED, "layer_norm: rows of %d elements", p.W);
     const int threads = ((groups + nv - 1) / nv + 31) / 32 * 32;
-    switch (nv) {
-        case 1: MYNN_CUDA_OK(launch_dependent(norm_step_kernel<T, V, 1, false>, dim3(rows), dim3(threads), 0, st, p)); break;
-        case 2: MYNN_CUDA_OK(launch_dependent(norm_step_kernel<T, V, 2, false>, dim3(rows), dim3(threads), 0, st, p)); break;
-        case 4: MYNN_CUDA_OK(launch_dependent(norm_step_kernel<T, V, 4, false>, dim3(rows), dim3(threads), 0, st, p)); break;
-        case 8: MYNN_CUDA_OK(launch_dependent(norm_step_kernel<T, V, 8, false>, dim3(rows), dim3(threads), 0, st, p)); break;
-        default:
-            if constexpr (V == 1) MYNN_CUDA_OK(launch_dependent(norm_step_kernel<T, V, 32, false>, dim3(rows), dim3(threads), 0, st, p));
-            break;
+    if constexpr (V == 4) {
+        if (few) {
+            if (nv == 1) RUN(1, true, 256);
+            else RUN(2, true, 512);
+        } else if (groups <= 1024) {
+            if (nv == 1) RUN(1, false, 256);
+            else if (nv == 2) RUN(2, false, 256);
+            else RUN(4, false, 256);
+        }
     }
+    if (!few && (V != 4 || groups > 1024)) {
+        switch (nv) {
+            case 2: RUN(2, false, 1024); break;
+            case 4: RUN(4, false, 1024); break;
+            case 8: RUN(8, false, 1024); break;
+            default:
+                if constexpr (V == 1) RUN(32, false, 1024);
+                break;
+        }
+    }
+#undef RUN
     MYNN_LAUNCH_OK("norm_step_kernel");
     return MYNN_OK;
 }

@@ -4,7 +4,7 @@
 //   dense_stream_kernel   16-bit, up to a few dozen rows (decode): the weights are read once, straight from global memory into
 //                         mma.m16n8k16 fragments.  The contraction index is permuted so that the 16 bytes a lane loads are two
 //                         k16 fragments of its weight row (the activations use the same permutation), so nothing passes
-//                         through shared memory before the reduction.  A CTA owns 16 or 32 weight rows, its eight warps deal out
+//                         through shared memory before the reduction.  A CTA owns 16 or 32 weight rows, its eight or sixteen warps deal out
 //                         the contraction, and the partial sums meet in shared memory once.
 //   dense_gemm_tc.cu      16-bit, many rows (prefill): tcgen05, TMA, accumulators in tensor memory.
 //   dense_tile_kernel     any dtype and size: 64 x 64 tiles on the FP32 units (true 32-bit products for f32 models).
@@ -121,12 +121,15 @@ __global__ void __launch_bounds__(256) dense_tile_kernel(const GemmView g) {
 }
 
 // ---- 16-bit weights, few rows ----------------------------------------------------------------------------------------
-// grid (ceil(N / (16 RT)), groups), 256 threads.  RT: 16-row weight tiles per warp (with GLU: one gate and one up tile, RT == 1).
+// grid (ceil(N / (16 RT)), groups).  RT: 16-row weight tiles per warp (with GLU: one gate and one up tile, RT == 1).
 // MT: groups of 8 activation rows taken at a time; a group with more rows than 8 MT passes over its weights again (from L2).
-constexpr int kStreamWarps = 8;
+// What bounds it is how many bytes an SM keeps on their way: 32 KB with two CTAs of eight warps.  A grid that leaves each SM one CTA (MT == 1)
+// therefore takes SOLO, sixteen warps per CTA (2048 x 4096 inside a step of one row: 5.0 -> 4.2 us).  Four CTAs of eight warps with half as
+// much in flight each fill the waves of 512 CTAs better and were slower all the same (gate/up of eight experts: 14.4 -> 18.3 us).
 constexpr unsigned kPrefetchCtas = 3 * 148;
-template <typename T, typename O, int MT, int RT, bool GLU>
-__global__ void __launch_bounds__(kStreamWarps * 32, MT * RT * (GLU ? 2 : 1) <= 4 ? 2 : 1) dense_stream_kernel(const GemmView g) {
+template <typename T, typename O, int MT, int RT, bool GLU, bool SOLO>
+__global__ void __launch_bounds__(SOLO ? 512 : 256, !SOLO && MT * RT * (GLU ? 2 : 1) <= 4 ? 2 : 1) dense_stream_kernel(const GemmView g) {
+    constexpr int kStreamWarps = SOLO ? 16 : 8;
     constexpr int WT = GLU ? 2 : RT;  // weight tiles of a warp
     constexpr int U = WT == 1 ? 4 : 2;  // 32-element steps in flight
     __shared__ float red[kStreamWarps][WT * 16][MT * 8 + 1];
@@ -144,8 +147,14 @@ __global__ void __launch_bounds__(kStreamWarps * 32, MT * RT * (GLU ? 2 : 1) <= 
         }
     }
     pdl_wait();
-    int e, r0, cnt;
-    if (!group_rows(g, blockIdx.y, e, r0, cnt)) return;
+    int e = 0, r0 = 0, cnt = g.M;
+    if (g.off) {
+        const int used = *g.n_active;
+        e = g.active[blockIdx.y];  // read beside the count: one trip less in front of the weights
+        if ((int)blockIdx.y >= used) return;
+        r0 = g.off[e];
+        cnt = g.off[e + 1] - r0;
+    }
     const T *act = reinterpret_cast<const T *>(g.act) + z * g.act_stride, *w = reinterpret_cast<const T *>(g.w) + (size_t)(e + z) * (GLU ? 2 : 1) * g.N * g.K;
     const T *wp[WT][2];  // this lane's two rows of every tile; rows past N repeat the last one and are not stored
 #pragma unroll
@@ -228,23 +237,30 @@ static int run_stream(cudaStream_t st, const GemmView &v, int rows, int groups, 
     const int mt = rows <= 8 ? 1 : rows <= 16 ? 2 : 4;
     const bool wide = !glu && (v.batch > 1 ? v.N * (long long)v.batch >= 32 * 148 * 2 : (mt > 1 || v.N >= 16 * 148 * 4) && v.N >= 32 * 100);
     const dim3 grid((v.N + (wide ? 31 : 15)) / (wide ? 32 : 16), groups);
+    const bool solo = mt == 1 && !wide && (long long)grid.x * grid.y <= 148;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
-    cfg.blockDim = dim3(kStreamWarps * 32);
+    cfg.blockDim = dim3(solo ? 512 : 256);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // may start (and fetch weights) while its predecessor drains
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-#define RUN(MT)                                                                                            \
-    {                                                                                                      \
-        if (glu) MYNN_CUDA_OK(cudaLaunchKernelEx(&cfg, dense_stream_kernel<T, O, MT, 1, true>, v));        \
-        else if (wide) MYNN_CUDA_OK(cudaLaunchKernelEx(&cfg, dense_stream_kernel<T, O, MT, 2, false>, v)); \
-        else MYNN_CUDA_OK(cudaLaunchKernelEx(&cfg, dense_stream_kernel<T, O, MT, 1, false>, v));           \
+#define GO(MT, RT, GLU, SOLO) MYNN_CUDA_OK(cudaLaunchKernelEx(&cfg, dense_stream_kernel<T, O, MT, RT, GLU, SOLO>, v))
+#define RUN(MT)                                 \
+    {                                           \
+        if (glu) GO(MT, 1, true, false);        \
+        else if (wide) GO(MT, 2, false, false); \
+        else GO(MT, 1, false, false);           \
     }
+    if (solo) {
+        if (glu) GO(1, 1, true, true);
+        else GO(1, 1, false, true);
+    } else
     if (mt == 1) RUN(1) else if (mt == 2) RUN(2) else RUN(4)
 #undef RUN
+#undef GO
     MYNN_LAUNCH_OK("dense_stream_kernel");
     return MYNN_OK;
 }

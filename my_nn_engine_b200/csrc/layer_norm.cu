@@ -102,7 +102,9 @@ __global__ void __launch_bounds__(THREADS, !FEW && THREADS == 256 && V == 4 ? 4 
                 if (src[q] && i0 + j * step < W) load_vec<float, V>(src[q] + i0 + j * step, we[q][j]);
             }
     };
-    pdl_trigger();
+    // Few rows: the product behind starts fetching its weights when it becomes resident, and this kernel's loads would queue behind them; it
+    // is let go once they are here (combining norm of a step of one row 12 -> 6 us, the product behind unchanged).
+    if (!FEW) pdl_trigger();
     if (!p.fixed_weights) pdl_wait();
     if constexpr (EARLY) get_weights();
     pdl_wait();
@@ -202,6 +204,7 @@ __global__ void __launch_bounds__(THREADS, !FEW && THREADS == 256 && V == 4 ? 4 
                     if (i < W) load_vec<T, V>(sub + (size_t)row * W + i, sv[j]);
                 }
             }
+            if (FEW) pdl_trigger();
             float2 m = make_float2(0.f, 1.f);
             if (p.w1) m = norm_of(sv);
 #pragma unroll

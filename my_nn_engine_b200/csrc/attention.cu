@@ -47,8 +47,9 @@ __device__ int g_ring_status;  // 31: a wait for a tile ran out of time (read an
 MYNN_DEFINE_WAIT_BUDGET_SETTER(attention_decode)
 
 // WIN: a sliding window over a ring cache and a score soft cap (DecodeParams::window, ring_cache, softcap).
-template <typename T, int D, bool RING, bool WIN>
-__global__ void __launch_bounds__(kAttnWarps * 32, RING ? 2 : 4)
+// W: warps per CTA.
+template <typename T, int D, bool RING, bool WIN, int W>
+__global__ void __launch_bounds__(W * 32, W > kAttnWarps ? 1 : RING ? 2 : 4)
 attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const DecodeParams p) {
     constexpr int KS = D / 16;   // k16 steps of QK^T
     constexpr int KCH = D / 32;  // 16-byte K chunks per lane per row
@@ -62,8 +63,8 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     active = max(0, WIN && p.ring_cache ? active : min(active, p.cache_seq));
     // rows [lo, active) are seen; the walk starts at the 16-row tile that holds lo (0 without a window)
     const int lo = WIN ? max(active > 0 ? first_visible(active - 1, p.window, p.chunk) : 0, p.ring_cache ? active - p.cache_seq : 0) : 0, walk0 = lo & ~15;
-    // whole rounds of the CTA's four warps (64 rows): a split that ends inside a round leaves some warps a tile short
-    const int rows_per_split = (((active - walk0 + p.splits - 1) / p.splits) + 16 * kAttnWarps - 1) / (16 * kAttnWarps) * (16 * kAttnWarps);
+    // whole rounds of the CTA's warps (64 rows of four): a split that ends inside a round leaves some warps a tile short
+    const int rows_per_split = (((active - walk0 + p.splits - 1) / p.splits) + 16 * W - 1) / (16 * W) * (16 * W);
     const int row_beg = walk0 + split * rows_per_split;
     const int row_end = min(row_beg + rows_per_split, active);
 
@@ -82,18 +83,18 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     constexpr int NB = D / 64;                      // 128-byte boxes per K (and per V) row
     constexpr uint32_t kBox = 16 * 128;             // one box: 16 rows x 128 bytes
     constexpr uint32_t kTile = 2 * NB * kBox;       // K boxes, then V boxes
-    __shared__ uint64_t full[RING ? kAttnWarps : 1][kRingDepth];
+    __shared__ uint64_t full[RING ? W : 1][kRingDepth];
     __shared__ int abort_flag;
     uint8_t *ring = ring_raw + (size_t)warp * kRingDepth * kTile;
     const int first = row_beg + 16 * warp;
-    const int ntile = first < cache_end ? (cache_end - first + 16 * kAttnWarps - 1) / (16 * kAttnWarps) : 0;
+    const int ntile = first < cache_end ? (cache_end - first + 16 * W - 1) / (16 * W) : 0;
     const int y0 = (b * p.Hkv + kvh) * p.cache_seq;  // first tensor row of this (batch, kv head)
     auto slot = [&](int row) { return WIN && p.ring_cache ? row % p.cache_seq : row; };  // a 16-row tile never wraps: both are multiples of 16
     auto issue = [&](int j) {  // lane 0: tile j of this warp into stage j % depth
         if constexpr (RING) {
             const int s = j % kRingDepth;
             uint8_t *st = ring + (size_t)s * kTile;
-            const int y = y0 + slot(first + 16 * kAttnWarps * j);
+            const int y = y0 + slot(first + 16 * W * j);
             mbar_expect_tx(&full[warp][s], kTile);
 #pragma unroll
             for (int hf = 0; hf < NB; hf++) {
@@ -114,12 +115,32 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         // fused append no tile does: the new row never comes from the cache)
         int j = 0;
         if (lane == 0 && p.settled)
-            for (; j < min(ntile, kRingDepth) && (fused || first + 16 * kAttnWarps * j + 16 < active); j++) issue(j);
+            for (; j < min(ntile, kRingDepth) && (fused || first + 16 * W * j + 16 < active); j++) issue(j);
         pdl_wait();
         if (lane == 0)
             for (; j < min(ntile, kRingDepth); j++) issue(j);
     } else {
         pdl_wait();
+    }
+    // Wide CTAs give the new row to the warp with the fewest tiles and fetch it beside the query (four warps, several CTAs per SM: the
+    // registers are worth more).  Up to 64 rows, where the other warps have nothing to do, it stays with warp 0: the same sums in the
+    // same order as with four warps.
+    const bool takes_new = fused && warp == (W > kAttnWarps && row_end - row_beg > 16 * kAttnWarps ? W - 1 : 0) && new_row >= row_beg && new_row < row_end;
+    uint4 new_k[KCH] = {}, new_v[VH] = {};
+    auto load_new = [&]() {
+        if (g == 0) {
+            const T *kraw = reinterpret_cast<const T *>(p.fused_k) + (size_t)b * p.qkv_stride + (size_t)kvh * D;
+#pragma unroll
+            for (int i = 0; i < KCH; i++) new_k[i] = *reinterpret_cast<const uint4 *>(kraw + 8 * t + 32 * i);
+        }
+        if (t == 0) {
+            const T *vraw = reinterpret_cast<const T *>(p.fused_v) + (size_t)b * p.qkv_stride + (size_t)kvh * D;
+#pragma unroll
+            for (int h = 0; h < VH; h++) new_v[h] = *reinterpret_cast<const uint4 *>(vraw + 8 * g + 64 * h);
+        }
+    };
+    if constexpr (W > kAttnWarps) {
+        if (takes_new) load_new();
     }
     // x rotated against its partner xp (the element half a head away): low half x c - xp s, high half x c + xp s, rounded to
     // the storage type as the stand-alone RoPE kernel rounds it
@@ -238,7 +259,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     if constexpr (RING) {
         for (int j = 0; j < ntile; j++) {
             const int s = j % kRingDepth;
-            const int base = first + 16 * kAttnWarps * j;
+            const int base = first + 16 * W * j;
             int ok_i = 1;
             if (lane == 0) ok_i = mbar_wait_spin(&full[warp][s], (j / kRingDepth) & 1, &abort_flag) ? 1 : 0;
             if (!__shfl_sync(0xffffffffu, ok_i, 0)) {  // the copy never arrived: report it, leave the rows out
@@ -278,7 +299,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
             tile(kr, vr, base, cache_end);
         }
     } else {
-    for (int base = row_beg + 16 * warp; base < cache_end; base += 16 * kAttnWarps) {
+    for (int base = row_beg + 16 * warp; base < cache_end; base += 16 * W) {
         // ---- issue all loads of this tile (rows past the end are clamped to a valid row and masked in the tile) ----
         uint4 kr[2][KCH], vr[4][VH];
 #pragma unroll
@@ -297,7 +318,8 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         tile(kr, vr, base, cache_end);
     }
     }
-    if (fused && warp == 0 && new_row >= row_beg && new_row < row_end) {
+    if (takes_new) {
+        if constexpr (W <= kAttnWarps) load_new();
         // The new row of this (batch, kv head): rotate the key, store key and value into the cache for the steps to come, and
         // run them through one more tile in which only row 0 counts.  K row 0 of the tile lives in lanes g == 0 (chunks
         // 8t + 32i), V row 0 in lanes t == 0 (chunks 8g + 64h); everything else is zero.
@@ -312,10 +334,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
             for (int h = 0; h < VH; h++) vr[r][h] = make_uint4(0u, 0u, 0u, 0u);
         T *kcache = const_cast<T *>(kbase) + (size_t)new_row * D, *vcache = const_cast<T *>(vbase) + (size_t)new_row * D;
         if (g == 0) {
-            const T *kraw = reinterpret_cast<const T *>(p.fused_k) + (size_t)b * p.qkv_stride + (size_t)kvh * D;
-            uint4 raw[KCH];
-#pragma unroll
-            for (int i = 0; i < KCH; i++) raw[i] = *reinterpret_cast<const uint4 *>(kraw + 8 * t + 32 * i);
+            const uint4(&raw)[KCH] = new_k;
 #pragma unroll
             for (int i = 0; i < KCH; i++) {
                 const int d0 = 8 * t + 32 * i;
@@ -327,10 +346,9 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
             }
         }
         if (t == 0) {
-            const T *vraw = reinterpret_cast<const T *>(p.fused_v) + (size_t)b * p.qkv_stride + (size_t)kvh * D;
 #pragma unroll
             for (int h = 0; h < VH; h++) {
-                vr[0][h] = *reinterpret_cast<const uint4 *>(vraw + 8 * g + 64 * h);
+                vr[0][h] = new_v[h];
                 *reinterpret_cast<uint4 *>(vcache + 8 * g + 64 * h) = vr[0][h];
             }
         }
@@ -340,9 +358,9 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     if constexpr (RING) {
         // the warps' staging rows for the merge reuse each warp's own ring (all of its copies have landed and been read)
         __syncwarp();
-        decode_tail<T, D, VH * 4, Map16, true>(p, o, m_run, l_run, reinterpret_cast<float *>(ring_raw), (int)(kRingDepth * kTile / 4));
+        decode_tail<T, D, VH * 4, Map16, true, W>(p, o, m_run, l_run, reinterpret_cast<float *>(ring_raw), (int)(kRingDepth * kTile / 4));
     } else {
-        decode_tail<T, D, VH * 4, Map16>(p, o, m_run, l_run);
+        decode_tail<T, D, VH * 4, Map16, false, W>(p, o, m_run, l_run);
     }
 }
 
@@ -472,6 +490,30 @@ static bool decode_ring_possible(int B, int Hkv, int cache_seq) {
 // resident CTAs per SM of the decode kernel: the ring form at head_dim 128 holds 96 KB of tiles per CTA
 static int decode_ctas_per_sm(bool ring, int D) { return ring && D == 128 ? 2 : kAttnCtasPerSm; }
 
+// Few (batch, kv head) pairs leave SMs without a CTA, and then the time is the number of rounds its warps take one after the other (0.85 us
+// each) plus, with splits, the merge through L2 (2.5 us).  Up to half as many pairs as SMs take CTAs of twice (head_dim 128; registers) or
+// four times the warps (head_dim 64), whose round is as many times longer, so that up to 512 / 1024 rows need no split.  A model's steps
+// do; the operator by itself keeps four warps, with which its ring and its direct form give the same bits.
+constexpr int decode_wide_warps(int D) { return D == 64 ? 16 : 8; }
+static void decode_plan(DecodeParams &p, bool ring, bool step, int B, int D, int rows_bound) {
+    p.wide = step && ring && 2 * B * p.Hkv <= 148;
+    p.splits = p.wide ? decode_splits(B, p.Hkv, rows_bound, 16, 1, decode_wide_warps(D)) : decode_splits(B, p.Hkv, rows_bound, 16, decode_ctas_per_sm(ring, D));
+}
+
+template <typename T, int D, bool WIN, int W>
+static int launch_decode_ring(cudaStream_t st, const DecodeParams &p, int B, const CUtensorMap &mk, const CUtensorMap &mv) {
+    constexpr size_t smem = (size_t)W * kRingDepth * 2 * (D / 64) * 16 * 128;
+    auto kern = attention_decode_kernel<T, D, true, WIN, W>;
+    static bool attr_set = false;
+    if (!attr_set) {  // with the kernel's static shared memory every head_dim is past the 48 KB that need no opt-in
+        MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        attr_set = true;
+    }
+    MYNN_CUDA_OK(launch_dependent(kern, dim3(p.splits, p.Hkv, B), dim3(W * 32), smem, st, mk, mv, p));
+    MYNN_LAUNCH_OK("attention_decode_kernel");
+    return MYNN_OK;
+}
+
 template <typename T, int D, bool WIN = false>
 static int launch_decode(cudaStream_t st, const DecodeParams &p, int B, bool ring) {
     CUtensorMap mk, mv;
@@ -482,17 +524,10 @@ static int launch_decode(cudaStream_t st, const DecodeParams &p, int B, bool rin
         const uint64_t rows = (uint64_t)B * p.Hkv * p.cache_seq, row_bytes = (uint64_t)D * sizeof(T);
         if (int rc = make_map(&mk, p.k, rows, row_bytes, row_bytes, 16)) return rc;
         if (int rc = make_map(&mv, p.v, rows, row_bytes, row_bytes, 16)) return rc;
-        constexpr size_t smem = (size_t)kAttnWarps * kRingDepth * 2 * (D / 64) * 16 * 128;
-        auto kern = attention_decode_kernel<T, D, true, WIN>;
-        static bool attr_set = false;
-        if (!attr_set) {  // with the kernel's static shared memory every head_dim is past the 48 KB that need no opt-in
-            MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            attr_set = true;
-        }
-        MYNN_CUDA_OK(launch_dependent(kern, dim3(p.splits, p.Hkv, B), dim3(kAttnWarps * 32), smem, st, mk, mv, p));
-    } else {
-        MYNN_CUDA_OK(launch_pdl(attention_decode_kernel<T, D, false, WIN>, dim3(p.splits, p.Hkv, B), dim3(kAttnWarps * 32), 0, st, mk, mv, p));
+        return p.wide ? launch_decode_ring<T, D, WIN, decode_wide_warps(D)>(st, p, B, mk, mv)
+                      : launch_decode_ring<T, D, WIN, kAttnWarps>(st, p, B, mk, mv);
     }
+    MYNN_CUDA_OK(launch_pdl(attention_decode_kernel<T, D, false, WIN, kAttnWarps>, dim3(p.splits, p.Hkv, B), dim3(kAttnWarps * 32), 0, st, mk, mv, p));
     MYNN_LAUNCH_OK("attention_decode_kernel");
     return MYNN_OK;
 }
@@ -580,7 +615,7 @@ bool mynn::attention_decode_fast_path(int Sq, int D, int Hq, int Hkv, int dtype,
 int mynn::launch_attention(cudaStream_t st, void *out, const void *q, const void *k, const void *v, float scale, int B,
                            int Hq, int Hkv, int Sq, int D, int cache_seq_len, int active_seq_kv,
                            const int32_t *active_seq_kv_dev, int is_causal, int dtype, void *workspace,
-                           size_t workspace_bytes, int out_bshd, int8_t *limbs_out, float *ascale_out, const AttentionFuse *fuse, int *status_word) {
+                           size_t workspace_bytes, int out_bshd, int8_t *limbs_out, float *ascale_out, const AttentionFuse *fuse, int *status_word, bool step) {
     if (B < 0 || Hq <= 0 || Hkv <= 0 || Sq < 0 || D <= 0 || cache_seq_len < 0 || active_seq_kv < 0)
         return fail(MYNN_E_ARG, "attention: bad shape");
     if (Hq % Hkv != 0) return fail(MYNN_E_ARG, "attention: %d query heads are not a multiple of %d kv heads", Hq, Hkv);
@@ -618,7 +653,7 @@ int mynn::launch_attention(cudaStream_t st, void *out, const void *q, const void
     p.active_dev = active_seq_kv_dev;
     const int rows_bound = active_seq_kv_dev ? cache_seq_len : (active_seq_kv < cache_seq_len ? active_seq_kv : cache_seq_len);
     const bool ring = decode_ring_possible(B, Hkv, cache_seq_len);
-    p.splits = decode_splits(B, Hkv, rows_bound, 16, decode_ctas_per_sm(ring, D));
+    decode_plan(p, ring, fuse != nullptr || step, B, D, rows_bound);
     p.k_scale = nullptr;
     p.v_scale = nullptr;
     p.limbs = limbs_out;
@@ -663,7 +698,7 @@ int mynn::launch_window_attention_decode(cudaStream_t st, int dtype, const Windo
     if (w.window > 0) rows_bound = std::min(rows_bound, w.window + 15);
     if (w.chunk > 0) rows_bound = std::min(rows_bound, w.chunk + 15);
     const bool ring = decode_ring_possible(w.B, w.Hkv, w.cache_rows);
-    p.splits = decode_splits(w.B, w.Hkv, rows_bound, 16, decode_ctas_per_sm(ring, w.D));
+    decode_plan(p, ring, true, w.B, w.D, rows_bound);
     p.k_scale = p.v_scale = nullptr;
     p.limbs = nullptr;
     p.ascale = nullptr;

@@ -120,12 +120,13 @@ struct DecodeParams {
     // Of what the kernel reads, the kernels right in front of it write q and the newest key and value rows only: cached rows, positions and
     // the active length may be read while they still run.
     int settled = 0;
+    int wide = 0;           // host side: CTAs of more than four warps
     int *status = nullptr;  // ring kernel: where a timed-out wait is recorded (null: the library's own word, see attention_check)
 };
 
 // Called by every CTA that has stored final outputs of (batch b, one kv head): the last of the Hkv to arrive converts the
 // whole row to limbs with the arithmetic of the limb pre-pass (23-bit fixed point, power-of-two row scale).
-template <typename T, int D>
+template <typename T, int D, int W>
 __device__ __forceinline__ void decode_row_limbs(const DecodeParams &p, int b, unsigned *sm_flag, float *sm_red) {
     if (p.limbs == nullptr) return;
     __threadfence();
@@ -138,7 +139,7 @@ __device__ __forceinline__ void decode_row_limbs(const DecodeParams &p, int b, u
     const T *row = reinterpret_cast<const T *>(p.out) + (size_t)b * K;
     // up to 8 x 4 elements per thread are fetched in one go (one L2 round trip) and kept for the second pass; longer rows
     // are read again
-    constexpr int kKeep = 8, kStride = 4 * kAttnWarps * 32;
+    constexpr int kKeep = 8, kStride = 4 * W * 32;
     uint2 raw[kKeep];
     float mx = 0.f;
     bool bad = false;
@@ -166,7 +167,7 @@ __device__ __forceinline__ void decode_row_limbs(const DecodeParams &p, int b, u
     __syncthreads();
     float t = sm_red[0];
 #pragma unroll
-    for (int w = 1; w < kAttnWarps; w++) t = fmaxf(t, sm_red[w]);
+    for (int w = 1; w < W; w++) t = fmaxf(t, sm_red[w]);
     int e2 = 0;
     if (t > 0.f) frexpf(t, &e2);
     const float sc1 = t > 0.f ? ldexpf(1.0f, 22 - e2) : 1.0f;
@@ -209,7 +210,7 @@ __device__ __forceinline__ void decode_row_limbs(const DecodeParams &p, int b, u
 // (batch, kv head) pair to arrive (atomic ticket, no spinning) combines the splits and writes the output.
 // ext != nullptr: the per-warp output staging rows live in caller-provided shared memory, warp w's [8][D] floats at
 // ext + w * ext_stride (the ring kernel hands every warp a piece of its own, by then idle, ring).
-template <typename T, int D, int NACC, typename DMap, bool EXT = false>
+template <typename T, int D, int NACC, typename DMap, bool EXT = false, int W = kAttnWarps>
 __device__ __forceinline__ void decode_tail(const DecodeParams &p, const float (&o)[NACC][4], float m_run, float l_run,
                                             float *ext = nullptr, int ext_stride = 0) {
     float *so_base;
@@ -218,13 +219,13 @@ __device__ __forceinline__ void decode_tail(const DecodeParams &p, const float (
         so_base = ext;
         so_stride = ext_stride;
     } else {
-        __shared__ float sm_o[kAttnWarps][8][D];
+        __shared__ float sm_o[W][8][D];
         so_base = &sm_o[0][0][0];
         so_stride = 8 * D;
     }
-    __shared__ float sm_m[kAttnWarps][8], sm_l[kAttnWarps][8];
+    __shared__ float sm_m[W][8], sm_l[W][8];
     __shared__ unsigned sm_last, sm_row_last;
-    __shared__ float sm_red[kAttnWarps];
+    __shared__ float sm_red[W];
     const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int G = p.G;
@@ -252,11 +253,11 @@ __device__ __forceinline__ void decode_tail(const DecodeParams &p, const float (
         const int hd = idx / D, d = idx - hd * D;
         float mx = -INFINITY;
 #pragma unroll
-        for (int w = 0; w < kAttnWarps; w++) mx = fmaxf(mx, sm_m[w][hd]);
+        for (int w = 0; w < W; w++) mx = fmaxf(mx, sm_m[w][hd]);
         float L = 0.f, O = 0.f;
         if (mx > -INFINITY) {
 #pragma unroll
-            for (int w = 0; w < kAttnWarps; w++) {
+            for (int w = 0; w < W; w++) {
                 const float f = __expf(sm_m[w][hd] - mx);
                 L += sm_l[w][hd] * f;
                 O += so_base[(size_t)w * so_stride + hd * D + d] * f;
@@ -274,7 +275,7 @@ __device__ __forceinline__ void decode_tail(const DecodeParams &p, const float (
         }
     }
     if (p.splits == 1) {
-        decode_row_limbs<T, D>(p, b, &sm_row_last, sm_red);
+        decode_row_limbs<T, D, W>(p, b, &sm_row_last, sm_red);
         return;
     }
 
@@ -318,7 +319,7 @@ __device__ __forceinline__ void decode_tail(const DecodeParams &p, const float (
         outp[(size_t)hd * D + d] = from_f32<T>(O / L);
     }
     if (threadIdx.x == 0) p.ws_ticket[pair] = 0u;
-    decode_row_limbs<T, D>(p, b, &sm_row_last, sm_red);
+    decode_row_limbs<T, D, W>(p, b, &sm_row_last, sm_red);
 }
 
 // How many CTAs share the rows of one (batch, kv head) pair.  All CTAs of a launch last equally long, so the grid should fit
@@ -327,9 +328,9 @@ __device__ __forceinline__ void decode_tail(const DecodeParams &p, const float (
 // more CTA), so a split gets at least four tiles per warp, and more than eight splits are only used when a split would
 // otherwise be longer than 32 tiles per warp.  (Measured, 2048 rows, 32 pairs: 1 / 2 / 4 / 8 / 16 / 32 splits = 30 / 21 / 15 /
 // 16 / 22 / 33 us; 256 rows, 4 pairs: 1 / 2 / 4 splits = 4.8 / 7.4 / 7.2 us.)
-inline int decode_splits(int B, int Hkv, int rows_bound, int tile_rows = 16, int ctas_per_sm = kAttnCtasPerSm) {
+inline int decode_splits(int B, int Hkv, int rows_bound, int tile_rows = 16, int ctas_per_sm = kAttnCtasPerSm, int warps = kAttnWarps) {
     const int pairs = B * Hkv;
-    const int round = tile_rows * kAttnWarps;  // rows the four warps of a CTA take at a time
+    const int round = tile_rows * warps;  // rows the warps of a CTA take at a time
     int s = (ctas_per_sm * 148) / pairs;
     int cap = rows_bound / (4 * round);
     if (cap < 1) cap = 1;

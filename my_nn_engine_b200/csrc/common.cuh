@@ -91,15 +91,13 @@ __device__ __forceinline__ float warp_max(float v) {
 }
 
 // ---- programmatic dependent launch -----------------------------------------------------------------------------
-// Only the DequantMatMul kernels are launched with the programmatic-stream-serialization attribute: they have work that
-// does not depend on their predecessor (barrier set-up, streaming the first weight tiles) and order themselves with
-// pdl_wait() before they touch anything an earlier kernel produces.  The other kernels of the decode chain are plain
-// launches; their pdl_trigger() / pdl_wait() are no-ops there and only matter when such a kernel is the predecessor of a
-// DequantMatMul (pdl_trigger() lets that kernel be scheduled early).  Giving every kernel of the chain the attribute was
-// measured three times and rejected: without an early trigger in the GEMM it changed nothing; with a trigger at the GEMM's start
-// the kernels two and three places ahead became resident early and took registers and shared memory from the running kernel
-// (step 4.63 -> 5.31 ms); with a trigger after the GEMM's main loop the gaps stayed as they were (the glue kernels' own run
-// time, not their launch, fills them) and the o_proj CTAs that became resident under the attention kernel slowed it by 5-40 %.
+// Most kernels of a step are launched with the programmatic-stream-serialization attribute (launch_dependent): they may become resident
+// while the kernel in front still runs, do what does not depend on it (barrier set-up, weights, settled state and caches), and order
+// themselves with pdl_wait() before they touch anything that an earlier kernel of the step writes.  pdl_wait() returns when the grid in front
+// has completed and is visible; since every kernel of a chain waits, that covers all before it.  pdl_trigger() says when the next kernel may
+// become resident: at the start where this kernel leaves room beside it (lean products leave eight SMs to the row kernels), not before the
+// end in the tcgen05 products.  (There a trigger at the start made the kernels two and three places ahead take registers and shared memory
+// from the running one, step of batch 32 4.63 -> 5.31 ms, and one behind the main loop moved nothing.)
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -110,7 +108,7 @@ extern int g_fuse_rope;                  // see MYNN_OPT_FUSE_ROPE
 extern int g_decode_ring;                // see MYNN_OPT_DECODE_RING
 extern std::atomic<int> g_inject_stall;  // see MYNN_OPT_INJECT_STALL; consumed by the next launch it applies to
 
-// A plain launch through cudaLaunchKernelEx (no attributes); the name says which kernels belong to the decode chain.
+// A plain launch through cudaLaunchKernelEx (no attributes): everything in front has completed when it starts.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg = {};

@@ -1,6 +1,6 @@
-// Lean DequantMatMul for one to four activation rows over small weight matrices (the GEMV of batch-1 decode).
+// Lean DequantMatMul for one to five activation rows (the products of a decode step of a few sequences).
 //
-//   out[m,n] = scale[n] * sum_k act[m,k] * wq[n,k],   M <= 4, wq [N,K] int8 of at most a few tens of MB
+//   out[m,n] = scale[n] * sum_k act[m,k] * wq[n,k],   M <= 5, wq [N,K] int8
 //
 // A matrix of 10-30 MB streams from HBM in 2-5 us, so everything that is fixed cost in the tcgen05 kernel (tensor-memory
 // allocation, tensor maps, mbarrier ring, a separate limb pre-pass launch, 128-row tiles that leave SMs idle) would dominate.
@@ -12,7 +12,7 @@
 //     the preceding kernel drains;
 //   * the activation row(s) are the same three signed 8-bit limbs of a 23-bit fixed-point value the tensor-core kernel uses, either read
 //     from the workspace, where a fused producer left them, or computed here in shared memory (no extra launch).  Three limbs of up to
-//     four rows are the columns of mma.m16n8k32 (int8, exact int32 sums).  The contraction index is permuted so that the 16 bytes a lane
+//     five rows are the columns of mma.m16n8k32 (int8, exact int32 sums).  The contraction index is permuted so that the 16 bytes a lane
 //     loads are its fragments of two MMAs, for weights and limbs alike; a warp needs its own piece of the limbs only;
 //   * the warps' int32 sums meet in shared memory once, limbs recombined in int64, the same two roundings as the tensor-core kernel:
 //     the outputs are bit-identical to that kernel's, whichever of the two a shape is dispatched to.
@@ -28,6 +28,7 @@
 namespace mynn {
 
 constexpr int kLeanThreads = 512;
+constexpr int kLeanMaxRows = 5;
 constexpr int kLeanWarps = kLeanThreads / 32;
 constexpr int kLeanTiles = 8;                       // row tiles whose partial sums are kept at a time
 constexpr int kLeanFreeSms = 8;
@@ -51,66 +52,123 @@ __device__ __forceinline__ uint4 ldg_stream_16(const void *p) {
     return v;
 }
 
-// One activation row -> limbs in shared memory (and, from CTA 0, in the workspace), with the arithmetic of the limb pre-pass
-// of the tensor-core kernel: |a| * 2^(22-e) rounded to an integer below 2^22, split into three signed bytes.  Rows of up to
-// 8 elements per thread stay in registers between the two passes.
-template <typename ActT>
-__device__ __forceinline__ void row_to_limbs(const ActT *row, int K, int pitch, int8_t *l_s, int8_t *l_g, float *ascale_s, float *ascale_g,
-                                             float *red) {
-    constexpr int kKeep = 8;
-    float keep[kKeep];
-    float mx = 0.f;
-    bool bad = false;
+template <typename T>
+__device__ __forceinline__ void lean_unpack(const uint4 &raw, float (&v)[8]) {
+    const T *e = reinterpret_cast<const T *>(&raw);
 #pragma unroll
-    for (int u = 0; u < kKeep; u++) {
-        const int i = threadIdx.x + u * kLeanThreads;
-        keep[u] = i < K ? to_f32<ActT>(row[i]) : 0.f;
-        bad |= !(fabsf(keep[u]) <= 3.0e38f);
-        mx = fmaxf(mx, fabsf(keep[u]));
-    }
-    for (int i = threadIdx.x + kKeep * kLeanThreads; i < K; i += kLeanThreads) {
-        const float a = to_f32<ActT>(row[i]);
-        bad |= !(fabsf(a) <= 3.0e38f);
-        mx = fmaxf(mx, fabsf(a));
-    }
-    mx = warp_max(mx);
-    const unsigned anybad = __syncthreads_or(bad);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
-    __syncthreads();
-    float t = red[0];
+    for (int j = 0; j < 8; j++) v[j] = to_f32<T>(e[j]);
+}
+
+// The activation rows as limbs in shared memory (and from CTA 0 in the workspace), with the arithmetic of the limb pre-pass of
+// the tensor-core kernel: |a| * 2^(22-e) rounded to an integer below 2^22, split into three signed bytes.  Every CTA does this for
+// itself: all rows at once, eight elements per thread and round, two barriers and no launch in between.  (The norm or the SiLU product in
+// front taken inside as well cost as much as the launch it saved at one row and more at three: 10.2 us for norm and gate/up against 3.0 + 6.0.)
+template <typename ActT, int M, int NB>
+__device__ __forceinline__ void lean_rows_to_limbs(const LeanParams &p, int pitch, int8_t *sm_limbs, float *sm_ascale, unsigned *sm_max) {
+    constexpr int ROUNDS = (M * NB * 128 + kLeanThreads - 1) / kLeanThreads;
+    constexpr bool HALF = sizeof(ActT) == 2;  // 16-bit rows stay in registers between the passes
+    const int per = p.K >> 3, total = M * per, lane = threadIdx.x & 31;
+    const bool even = per % 32 == 0;  // a warp's chunks belong to one row
+    const ActT *act = reinterpret_cast<const ActT *>(p.act);
+    const bool vec = (uintptr_t)act % 16 == 0;
+    uint4 keep[HALF ? ROUNDS : 1];
+    auto fetch = [&](const ActT *src, float (&v)[8], uint4 &raw) {
+        if constexpr (HALF) {
+            if (vec) {
+                raw = __ldcg(reinterpret_cast<const uint4 *>(src));
+            } else {
+                __align__(16) ActT e[8];
 #pragma unroll
-    for (int w = 1; w < kLeanThreads / 32; w++) t = fmaxf(t, red[w]);
-    int e = 0;
-    if (t > 0.f) frexpf(t, &e);
-    const float sc1 = t > 0.f ? ldexpf(1.0f, 22 - e) : 1.0f;
-    const float sc = anybad ? 0.f : sc1;
-    if (threadIdx.x == 0) {
-        const float as = anybad ? __int_as_float(0x7fc00000) : 1.0f / sc1;  // a non-finite input row gives NaN outputs
-        *ascale_s = as;
-        if (ascale_g) *ascale_g = as;
-    }
-    auto emit = [&](float a, int i) {
-        int A = sc == 0.f ? 0 : __float2int_rn(a * sc);
-        const int d0 = (int)(int8_t)(A & 0xFF);
-        A = (A - d0) >> 8;
-        const int d1 = (int)(int8_t)(A & 0xFF);
-        A = (A - d1) >> 8;
-        l_s[i] = (int8_t)d0;
-        l_s[pitch + i] = (int8_t)d1;
-        l_s[2 * pitch + i] = (int8_t)A;
-        if (l_g) {
-            l_g[i] = (int8_t)d0;
-            l_g[K + i] = (int8_t)d1;
-            l_g[2 * (size_t)K + i] = (int8_t)A;
+                for (int j = 0; j < 8; j++) e[j] = src[j];
+                raw = *reinterpret_cast<const uint4 *>(e);
+            }
+            lean_unpack<ActT>(raw, v);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; j++) v[j] = to_f32<ActT>(src[j]);
         }
     };
+    auto chunk = [&](int k, int &m, int &c) {
+        const int i = threadIdx.x + k * kLeanThreads;
+        m = min(i / per, M - 1);
+        c = i - m * per;
+        return i < total;
+    };
 #pragma unroll
-    for (int u = 0; u < kKeep; u++) {
-        const int i = threadIdx.x + u * kLeanThreads;
-        if (i < K) emit(keep[u], i);
+    for (int k = 0; k < ROUNDS; k++) {  // all loads first
+        int m, c;
+        const bool in = chunk(k, m, c);
+        if constexpr (HALF) {
+            keep[k] = make_uint4(0u, 0u, 0u, 0u);
+            float v[8];
+            if (in) fetch(act + (size_t)m * p.K + 8 * c, v, keep[k]);
+        }
     }
-    for (int i = threadIdx.x + kKeep * kLeanThreads; i < K; i += kLeanThreads) emit(to_f32<ActT>(row[i]), i);
-    __syncthreads();  // red is reused by the next row
+#pragma unroll
+    for (int k = 0; k < ROUNDS; k++) {
+        int m, c;
+        const bool in = chunk(k, m, c);
+        float v[8];
+        if constexpr (HALF) {
+            lean_unpack<ActT>(keep[k], v);
+        } else {
+            uint4 none;
+#pragma unroll
+            for (int j = 0; j < 8; j++) v[j] = 0.f;
+            if (in) fetch(act + (size_t)m * p.K + 8 * c, v, none);
+        }
+        unsigned mx = 0u;  // magnitudes as integers: infinities and NaN above every number
+#pragma unroll
+        for (int j = 0; j < 8; j++) mx = max(mx, __float_as_uint(v[j]) & 0x7fffffffu);
+        if (!in) mx = 0u;
+        if (even) {
+            mx = __reduce_max_sync(0xffffffffu, mx);
+            if (lane == 0 && mx) atomicMax(&sm_max[m], mx);
+        } else if (mx) {
+            atomicMax(&sm_max[m], mx);
+        }
+    }
+    __syncthreads();
+    const bool publish = blockIdx.x == 0;
+#pragma unroll
+    for (int k = 0; k < ROUNDS; k++) {
+        int m, c;
+        if (!chunk(k, m, c)) break;
+        const float t = __uint_as_float(sm_max[m]);
+        const bool bad = !(t <= 3.0e38f);
+        int e = 0;
+        if (t > 0.f && !bad) frexpf(t, &e);
+        const float sc = bad ? 0.f : t > 0.f ? ldexpf(1.0f, 22 - e) : 1.0f;
+        if (c == 0) {
+            const float as = bad ? __int_as_float(0x7fc00000) : 1.0f / sc;  // a non-finite input row gives NaN outputs
+            sm_ascale[m] = as;
+            if (publish) p.ascale_g[m] = as;
+        }
+        float v[8];
+        if constexpr (HALF) {
+            lean_unpack<ActT>(keep[k], v);
+        } else {
+            uint4 none;
+            fetch(act + (size_t)m * p.K + 8 * c, v, none);
+        }
+        uint32_t l[3][2] = {};
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            int A = bad ? 0 : __float2int_rn(v[j] * sc);
+            const int d0 = (int)(int8_t)(A & 0xFF);
+            A = (A - d0) >> 8;
+            const int d1 = (int)(int8_t)(A & 0xFF);
+            A = (A - d1) >> 8;
+            l[0][j >> 2] |= (uint32_t)(d0 & 0xFF) << (8 * (j & 3));
+            l[1][j >> 2] |= (uint32_t)(d1 & 0xFF) << (8 * (j & 3));
+            l[2][j >> 2] |= (uint32_t)(A & 0xFF) << (8 * (j & 3));
+        }
+#pragma unroll
+        for (int x = 0; x < 3; x++) {
+            *reinterpret_cast<uint2 *>(sm_limbs + (size_t)(3 * m + x) * pitch + 8 * c) = make_uint2(l[x][0], l[x][1]);
+            if (publish) *reinterpret_cast<uint2 *>(p.limbs_g + (size_t)(3 * m + x) * p.K + 8 * c) = make_uint2(l[x][0], l[x][1]);
+        }
+    }
 }
 
 __device__ __forceinline__ void mma_i8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -121,18 +179,18 @@ __device__ __forceinline__ void mma_i8(int (&c)[4], uint32_t a0, uint32_t a1, ui
 
 // One CTA per SM owns a contiguous range of weight rows, so that the whole grid is one balanced wave.  A warp owns NB blocks of 64 along K
 // (K <= 1024 NB) of all of them; TG tiles of 16 rows are in flight (2 NB TG <= 20 loads per lane, issued before anything else happens).
-// K % 16 == 0; wq and limbs 16-byte aligned.  Dynamic shared memory: limbs [3 M][pitch] (only with act), partial sums [warp][3 M][kLeanPitch].
-template <typename OutT, int M, int NB, int TG>
+// K % 16 == 0; wq and limbs 16-byte aligned.  Dynamic shared memory: limbs [3 M][pitch] (ACT), partial sums [warp][3 M][kLeanPitch].
+template <typename OutT, int M, int NB, int TG, bool ACT>
 __global__ void __launch_bounds__(kLeanThreads, 1) gemv_lean_kernel(const LeanParams p) {
     extern __shared__ __align__(16) int8_t sm_dyn[];
-    __shared__ float sm_ascale[4];
-    __shared__ float red[kLeanWarps];
+    __shared__ float sm_ascale[8];
+    __shared__ unsigned sm_max[8];
     constexpr int C = 3 * M, NT = (C + 7) / 8;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, t = lane & 3;
     const int K = p.K, chunks = K >> 4, pitch = lean_limb_pitch(K);
     const int row0 = blockIdx.x * p.rows_per_cta, rows = min(p.rows_per_cta, p.N - row0), tiles = (rows + 15) >> 4;
     int8_t *sm_limbs = sm_dyn;
-    int *sm_sum = reinterpret_cast<int *>(sm_dyn + (p.act ? (size_t)C * pitch : 0));
+    int *sm_sum = reinterpret_cast<int *>(sm_dyn + (ACT ? (size_t)C * pitch : 0));
     const OutT *scale_p = reinterpret_cast<const OutT *>(p.scale);
     const OutT *resid_p = reinterpret_cast<const OutT *>(p.resid);
     OutT *out_p = reinterpret_cast<OutT *>(p.out);
@@ -159,24 +217,19 @@ __global__ void __launch_bounds__(kLeanThreads, 1) gemv_lean_kernel(const LeanPa
     const int pass_rows = min(rows, 16 * kLeanTiles), my_m = threadIdx.x / pass_rows, my_r = threadIdx.x - my_m * pass_rows;
     float wscale_first = 0.f, resv_first = 0.f;
     if (my_m < M) wscale_first = to_f32<OutT>(scale_p[row0 + my_r]);
+    if constexpr (ACT) {
+        if (threadIdx.x < 8) sm_max[threadIdx.x] = 0u;
+        __syncthreads();
+    }
     pdl_trigger();
     pdl_wait();
     if (my_m < M && resid_p) resv_first = to_f32<OutT>(resid_p[(size_t)my_m * p.N + row0 + my_r]);
     // limbs of this warp's piece of K: column gq (and gq + 8) of the MMAs is limb row gq (gq + 8) = 3 m + l
     uint4 b[NT][NB];
-    if (p.act != nullptr) {
-        int8_t *lg = blockIdx.x == 0 ? p.limbs_g : nullptr;
-        float *ag = blockIdx.x == 0 ? p.ascale_g : nullptr;
-#pragma unroll 1
-        for (int m = 0; m < M; m++) {
-            int8_t *ls = sm_limbs + (size_t)m * 3 * pitch;
-            if (p.act_dtype == MYNN_F32)
-                row_to_limbs<float>((const float *)p.act + (size_t)m * K, K, pitch, ls, lg ? lg + (size_t)m * 3 * K : nullptr, &sm_ascale[m], ag ? ag + m : nullptr, red);
-            else if (p.act_dtype == MYNN_BF16)
-                row_to_limbs<__nv_bfloat16>((const __nv_bfloat16 *)p.act + (size_t)m * K, K, pitch, ls, lg ? lg + (size_t)m * 3 * K : nullptr, &sm_ascale[m], ag ? ag + m : nullptr, red);
-            else
-                row_to_limbs<__half>((const __half *)p.act + (size_t)m * K, K, pitch, ls, lg ? lg + (size_t)m * 3 * K : nullptr, &sm_ascale[m], ag ? ag + m : nullptr, red);
-        }
+    if constexpr (ACT) {
+        if (p.act_dtype == MYNN_F32) lean_rows_to_limbs<float, M, NB>(p, pitch, sm_limbs, sm_ascale, sm_max);
+        else if (p.act_dtype == MYNN_BF16) lean_rows_to_limbs<__nv_bfloat16, M, NB>(p, pitch, sm_limbs, sm_ascale, sm_max);
+        else lean_rows_to_limbs<__half, M, NB>(p, pitch, sm_limbs, sm_ascale, sm_max);
         __syncthreads();
 #pragma unroll
         for (int n = 0; n < NT; n++)
@@ -251,21 +304,24 @@ __global__ void __launch_bounds__(kLeanThreads, 1) gemv_lean_kernel(const LeanPa
     }
 }
 
+constexpr int kLeanMaxSmem = 226 * 1024;
+static size_t lean_smem(bool act, int M, int K) { return (act ? (size_t)3 * M * lean_limb_pitch(K) : 0) + (size_t)kLeanWarps * 3 * M * kLeanPitch * sizeof(int); }
+
+// Up to two rows any matrix that was measured (28672 x 4096 as an operator at one row: 20 us against 25 us with the tcgen05 kernel and its
+// pre-pass; a Llama-3-8B step of two sequences 2554 -> 2331 us).  Three to five rows fill two column tiles and the finish has that much more to
+// do: up to 32 MB (Llama-3-8B at five rows: norm and qkv 10.4 -> 8.8 us), above that the tcgen05 kernel (gate/up at five rows 19 us, 36 us
+// here).
 bool gemv_lean_supported(int M, int N, int K, const void *wq) {
-    // small matrices only: larger ones amortise the tensor-core kernel's set-up and stream faster there
-    return M >= 1 && M <= 4 && K >= 16 && K % 16 == 0 && K <= 6144 && (size_t)3 * M * K <= 96 * 1024 && (size_t)N * K <= ((size_t)32 << 20) &&
-           ((uintptr_t)wq % 16) == 0;
+    return M >= 1 && M <= kLeanMaxRows && K >= 16 && K % 16 == 0 && K <= 6144 && (size_t)N * K <= ((size_t)(M <= 2 ? 160 : 32) << 20) && ((uintptr_t)wq % 16) == 0;
 }
 
-template <typename OutT, int M, int NB, int TG>
+template <typename OutT, int M, int NB, int TG, bool ACT>
 static int launch_lean(cudaStream_t st, LeanParams p) {
-    const size_t smem = (p.act ? (size_t)3 * M * lean_limb_pitch(p.K) : 0) + (size_t)kLeanWarps * 3 * M * kLeanPitch * sizeof(int);
-    auto kern = gemv_lean_kernel<OutT, M, NB, TG>;
+    const size_t smem = lean_smem(ACT, M, p.K);
+    auto kern = gemv_lean_kernel<OutT, M, NB, TG, ACT>;
     static bool attr_set = false;
-    if (!attr_set) {  // the most this form can need
-        constexpr int most = 3 * M * (1024 * NB + 64) + kLeanWarps * 3 * M * kLeanPitch * (int)sizeof(int);
-        static_assert(most <= 227 * 1024, "shared memory of a CTA");
-        MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    if (!attr_set) {
+        MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kLeanMaxSmem));
         attr_set = true;
     }
     static int sms = 0;
@@ -293,6 +349,25 @@ static int launch_lean(cudaStream_t st, LeanParams p) {
     return MYNN_OK;
 }
 
+// blocks of 64 per warp (K <= 1024 / 2048 / 4096 / 6144) and row tiles in flight
+template <typename OutT, int M, bool ACT>
+static int launch_by_k(cudaStream_t st, const LeanParams &p) {
+    if (p.K <= 1024) return launch_lean<OutT, M, 1, 8, ACT>(st, p);
+    if (p.K <= 2048) return launch_lean<OutT, M, 2, 5, ACT>(st, p);
+    if (p.K <= 4096) return launch_lean<OutT, M, 4, 2, ACT>(st, p);
+    return launch_lean<OutT, M, 6, 1, ACT>(st, p);
+}
+template <typename OutT>
+static int launch_by_rows(cudaStream_t st, const LeanParams &p, int M) {
+    switch (M) {
+        case 1: return p.act ? launch_by_k<OutT, 1, true>(st, p) : launch_by_k<OutT, 1, false>(st, p);
+        case 2: return p.act ? launch_by_k<OutT, 2, true>(st, p) : launch_by_k<OutT, 2, false>(st, p);
+        case 3: return launch_by_k<OutT, 3, false>(st, p);
+        case 4: return launch_by_k<OutT, 4, false>(st, p);
+        default: return launch_by_k<OutT, 5, false>(st, p);
+    }
+}
+
 // Same contract as i8_gemm_launch: `workspace` holds status word, row scales and the limb matrix; act == nullptr means a fused
 // producer (or the previous call) left the limbs there.
 int gemv_lean_launch(cudaStream_t st, void *out, const void *act, const int8_t *wq, const void *scale, const void *resid, int M, int N,
@@ -300,7 +375,12 @@ int gemv_lean_launch(cudaStream_t st, void *out, const void *act, const int8_t *
     const size_t need = i8_gemm_workspace_bytes(M, K);
     if (!workspace || workspace_bytes < need || (uintptr_t)workspace % 256)
         return fail(MYNN_E_ARG, "dequant_matmul: workspace of %zu bytes (256-byte aligned) needed", need);
-    LeanParams p;
+    // Every CTA makes the limbs of one or two rows itself; of more, a kernel in front does (three rows of 2048: 5.0 us inside, 2.2 + 2.3 so).
+    if (act && M > 2) {
+        if (int rc = launch_act_limbs(st, act, M, K, act_dtype, (int8_t *)workspace + 512, (float *)((char *)workspace + 256))) return rc;
+        act = nullptr;
+    }
+    LeanParams p = {};
     p.out = out;
     p.act = act;
     p.wq = wq;
@@ -311,25 +391,9 @@ int gemv_lean_launch(cudaStream_t st, void *out, const void *act, const int8_t *
     p.N = N;
     p.K = K;
     p.act_dtype = act_dtype;
-    p.rows_per_cta = 0;
-    // blocks of 64 per warp (K <= 1024 / 2048 / 4096 / 6144) and row tiles in flight
-#define BY_K(OT, MV)                                        \
-    if (K <= 1024) return launch_lean<OT, MV, 1, 8>(st, p); \
-    if (K <= 2048) return launch_lean<OT, MV, 2, 5>(st, p); \
-    if (K <= 4096) return launch_lean<OT, MV, 4, 2>(st, p); \
-    return launch_lean<OT, MV, 6, 1>(st, p);
-#define GO(OT)               \
-    switch (M) {             \
-        case 1: BY_K(OT, 1)  \
-        case 2: BY_K(OT, 2)  \
-        case 3: BY_K(OT, 3)  \
-        default: BY_K(OT, 4) \
-    }
-    if (out_dtype == MYNN_BF16) GO(__nv_bfloat16)
-    if (out_dtype == MYNN_F16) GO(__half)
-    GO(float)
-#undef GO
-#undef BY_K
+    if (out_dtype == MYNN_BF16) return launch_by_rows<__nv_bfloat16>(st, p, M);
+    if (out_dtype == MYNN_F16) return launch_by_rows<__half>(st, p, M);
+    return launch_by_rows<float>(st, p, M);
 }
 
 }  // namespace mynn

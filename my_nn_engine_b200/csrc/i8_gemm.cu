@@ -408,15 +408,9 @@ __global__ void __launch_bounds__(256) act_to_limbs_kernel(int8_t *limbs, float 
     for (int j = 0; j < kMaxPer; j++) {
         const int gi = threadIdx.x + j * 256;
         if (gi < groups) {
-            if constexpr (sizeof(ActT) == 2) {
-                const uint2 raw = *reinterpret_cast<const uint2 *>(row + 4 * gi);
-                const ActT *e = reinterpret_cast<const ActT *>(&raw);
+            // element by element: this form takes the rows that are not aligned for act_limbs_row_kernel
 #pragma unroll
-                for (int i = 0; i < 4; i++) v[j][i] = to_f32<ActT>(e[i]);
-            } else {
-                const float4 raw = *reinterpret_cast<const float4 *>(row + 4 * gi);
-                v[j][0] = raw.x; v[j][1] = raw.y; v[j][2] = raw.z; v[j][3] = raw.w;
-            }
+            for (int i = 0; i < 4; i++) v[j][i] = to_f32<ActT>(row[4 * gi + i]);
 #pragma unroll
             for (int i = 0; i < 4; i++) {
                 bad |= !(fabsf(v[j][i]) <= 3.0e38f);
@@ -899,6 +893,29 @@ static int launch_i8(cudaStream_t st, const CUtensorMap &mw, const CUtensorMap &
     return MYNN_OK;
 }
 
+// Activation rows -> limbs [3 M][K] and row scales.
+int launch_act_limbs(cudaStream_t st, const void *act, int M, int K, int act_dtype, int8_t *limbs, float *ascale) {
+    const bool row_kernel = K % 8 == 0 && (size_t)K * 4 <= 200 * 1024 && ((uintptr_t)act % 16) == 0;
+    const size_t smem = (size_t)K * 4;
+#define PREP(T)                                                                                                          \
+    if (row_kernel) {                                                                                                    \
+        auto kern = act_limbs_row_kernel<T>;                                                                             \
+        if (smem > 48 * 1024) MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+        MYNN_CUDA_OK(launch_dependent(kern, dim3(M), dim3(kRowThreads), smem, st, limbs, ascale, (const T *)act, K));    \
+    } else {                                                                                                             \
+        MYNN_CUDA_OK(launch_pdl(act_to_limbs_kernel<T>, dim3(M), dim3(256), 0, st, limbs, ascale, (const T *)act, K));   \
+    }
+    switch (act_dtype) {
+        case MYNN_BF16: PREP(__nv_bfloat16) break;
+        case MYNN_F16: PREP(__half) break;
+        case MYNN_F32: PREP(float) break;
+        default: return fail(MYNN_E_ARG, "dequant_matmul: bad activation dtype %d", act_dtype);
+    }
+#undef PREP
+    MYNN_LAUNCH_OK("act_to_limbs_kernel");
+    return MYNN_OK;
+}
+
 int i8_gemm_launch(cudaStream_t st, void *out, const void *act, const int8_t *wq, const void *scale, const void *resid,
                    int M, int N, int K, int act_dtype, int out_dtype, void *workspace, size_t workspace_bytes) {
     return i8_gemm_launch_tp(st, out, act, wq, scale, resid, M, N, K, act_dtype, out_dtype, workspace, workspace_bytes, nullptr, nullptr,
@@ -923,26 +940,8 @@ int i8_gemm_launch_tp(cudaStream_t st, void *out, const void *act, const int8_t 
     float *ascale = limbs_ext ? const_cast<float *>(ascale_ext) : (float *)((char *)workspace + 256);
     int8_t *limbs = limbs_ext ? const_cast<int8_t *>(limbs_ext) : (int8_t *)workspace + 512;
     // limb rows 3M..NC-1 are padding: whatever they hold only reaches accumulator columns that are never read
-    if (act != nullptr) {  // act == nullptr: a fused producer has already left limbs and row scales in the workspace
-        const bool row_kernel = K % 8 == 0 && (size_t)K * 4 <= 200 * 1024 && ((uintptr_t)act % 16) == 0;
-        const size_t smem = (size_t)K * 4;
-#define PREP(T)                                                                                                          \
-    if (row_kernel) {                                                                                                    \
-        auto kern = act_limbs_row_kernel<T>;                                                                             \
-        if (smem > 48 * 1024) MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-        MYNN_CUDA_OK(launch_dependent(kern, dim3(M), dim3(kRowThreads), smem, st, limbs, ascale, (const T *)act, K));          \
-    } else {                                                                                                             \
-        MYNN_CUDA_OK(launch_pdl(act_to_limbs_kernel<T>, dim3(M), dim3(256), 0, st, limbs, ascale, (const T *)act, K));   \
-    }
-        switch (act_dtype) {
-            case MYNN_BF16: PREP(__nv_bfloat16) break;
-            case MYNN_F16: PREP(__half) break;
-            case MYNN_F32: PREP(float) break;
-            default: return fail(MYNN_E_ARG, "dequant_matmul: bad activation dtype %d", act_dtype);
-        }
-#undef PREP
-        MYNN_LAUNCH_OK("act_to_limbs_kernel");
-    }
+    if (act != nullptr)  // act == nullptr: a fused producer has already left limbs and row scales in the workspace
+        if (int rc = launch_act_limbs(st, act, M, K, act_dtype, limbs, ascale)) return rc;
     CUtensorMap mw, ma;
     int rc = make_map(&mw, wq, (uint64_t)N, (uint64_t)K, (uint64_t)K, kTileRows);
     if (rc) return rc;

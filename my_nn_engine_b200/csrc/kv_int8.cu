@@ -205,7 +205,7 @@ attention_decode_q8_kernel(const __grid_constant__ CUtensorMap map_k, const __gr
     __shared__ float sm_qinv[8];
 
     pdl_trigger();
-    pdl_wait();
+    if (!p.settled) pdl_wait();  // else only q and the newest kv row come from the preceding kernels
     const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int G = p.G;
@@ -222,6 +222,47 @@ attention_decode_q8_kernel(const __grid_constant__ CUtensorMap map_k, const __gr
     const T *ksc = reinterpret_cast<const T *>(p.k_scale) + head;
     const T *vsc = reinterpret_cast<const T *>(p.v_scale) + head;
     const bool packed_scales = (p.cache_seq & 1) == 0 && ((reinterpret_cast<uintptr_t>(p.k_scale) | reinterpret_cast<uintptr_t>(p.v_scale)) & 3) == 0;
+
+    // ring state (RING only)
+    extern __shared__ __align__(1024) uint8_t ring_raw[];
+    constexpr uint32_t kBox = 32 * 128, kTile = 2 * kBox;
+    __shared__ uint64_t full[RING ? kAttnWarps : 1][kQ8RingDepth];
+    __shared__ __align__(16) T sm_sc[RING ? kAttnWarps : 1][kQ8RingDepth][2][32];
+    __shared__ int abort_flag;
+    uint8_t *ring = ring_raw + (size_t)warp * kQ8RingDepth * kTile;
+    const int first = row_beg + 32 * warp;
+    const int ntile = first < row_end ? (row_end - first + 32 * kAttnWarps - 1) / (32 * kAttnWarps) : 0;
+    auto issue = [&](int j) {  // lane 0: tile j of this warp into stage j % depth
+        if constexpr (RING) {
+            const int s = j % kQ8RingDepth, base = first + 32 * kAttnWarps * j;
+            uint8_t *st = ring + (size_t)s * kTile;
+            const uint32_t sc_bytes = (uint32_t)min(32, p.cache_seq - base) * (uint32_t)sizeof(T);  // a multiple of 16
+            mbar_expect_tx(&full[warp][s], kTile + 2 * sc_bytes);
+            tma_load_2d(st, &map_k, 0, (int)head + base, &full[warp][s]);
+            tma_load_2d(st + kBox, &map_v, 0, (int)head + base, &full[warp][s]);
+            bulk_load_1d(&sm_sc[warp][s][0][0], ksc + base, sc_bytes, &full[warp][s]);
+            bulk_load_1d(&sm_sc[warp][s][1][0], vsc + base, sc_bytes, &full[warp][s]);
+        }
+    };
+    if constexpr (RING) {
+        if (threadIdx.x == 0) abort_flag = 0;
+        if (lane == 0) {
+#pragma unroll
+            for (int s = 0; s < kQ8RingDepth; s++) mbar_init(&full[warp][s], 1);
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
+        __syncthreads();
+        // The first copies travel while the query becomes limbs; with a settled cache those of tiles without the newest row set out while
+        // the kernels in front still run (5 sequences of 3000 rows: 17.3 us with the ring behind the query).
+        int j = 0;
+        if (lane == 0 && p.settled)
+            for (; j < min(ntile, kQ8RingDepth) && first + 32 * kAttnWarps * j + 32 < active; j++) issue(j);
+        pdl_wait();
+        if (lane == 0)
+            for (; j < min(ntile, kQ8RingDepth); j++) issue(j);
+    } else {
+        pdl_wait();
+    }
 
     // ---- query limbs: 16 threads per head, E elements each ----
     {
@@ -274,39 +315,6 @@ attention_decode_q8_kernel(const __grid_constant__ CUtensorMap map_k, const __gr
         for (int i = 0; i < 4; i++) o[j][i] = 0.f;
     float m_run = -INFINITY, l_run = 0.f;
     const int last = row_end - 1;
-
-    // ring state (RING only)
-    extern __shared__ __align__(1024) uint8_t ring_raw[];
-    constexpr uint32_t kBox = 32 * 128, kTile = 2 * kBox;
-    __shared__ uint64_t full[RING ? kAttnWarps : 1][kQ8RingDepth];
-    __shared__ __align__(16) T sm_sc[RING ? kAttnWarps : 1][kQ8RingDepth][2][32];
-    __shared__ int abort_flag;
-    uint8_t *ring = ring_raw + (size_t)warp * kQ8RingDepth * kTile;
-    const int first = row_beg + 32 * warp;
-    const int ntile = first < row_end ? (row_end - first + 32 * kAttnWarps - 1) / (32 * kAttnWarps) : 0;
-    auto issue = [&](int j) {  // lane 0: tile j of this warp into stage j % depth
-        if constexpr (RING) {
-            const int s = j % kQ8RingDepth, base = first + 32 * kAttnWarps * j;
-            uint8_t *st = ring + (size_t)s * kTile;
-            const uint32_t sc_bytes = (uint32_t)min(32, p.cache_seq - base) * (uint32_t)sizeof(T);  // a multiple of 16
-            mbar_expect_tx(&full[warp][s], kTile + 2 * sc_bytes);
-            tma_load_2d(st, &map_k, 0, (int)head + base, &full[warp][s]);
-            tma_load_2d(st + kBox, &map_v, 0, (int)head + base, &full[warp][s]);
-            bulk_load_1d(&sm_sc[warp][s][0][0], ksc + base, sc_bytes, &full[warp][s]);
-            bulk_load_1d(&sm_sc[warp][s][1][0], vsc + base, sc_bytes, &full[warp][s]);
-        }
-    };
-    if constexpr (RING) {
-        if (threadIdx.x == 0) abort_flag = 0;
-        if (lane == 0) {
-#pragma unroll
-            for (int s = 0; s < kQ8RingDepth; s++) mbar_init(&full[warp][s], 1);
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        }
-        __syncthreads();
-        if (lane == 0)
-            for (int j = 0; j < min(ntile, kQ8RingDepth); j++) issue(j);
-    }
 
     for (int base = first, j = 0; base < row_end; base += 32 * kAttnWarps, j++) {
         uint4 kr[2][2][KCH];
@@ -635,7 +643,7 @@ int launch_dequant_kv_rows(cudaStream_t st, int dtype, void *out, const void *ca
 int launch_attention_q8(cudaStream_t st, void *out, const void *q, const void *k, const void *v, const void *k_scale,
                         const void *v_scale, float scale, int B, int Hq, int Hkv, int Sq, int D, int cache_seq_len,
                         int active_seq_kv, const int32_t *active_seq_kv_dev, int is_causal, int dtype, void *workspace,
-                        size_t workspace_bytes, int out_bshd) {
+                        size_t workspace_bytes, int out_bshd, bool step) {
     if (B < 0 || Hq <= 0 || Hkv <= 0 || Sq < 0 || D <= 0 || cache_seq_len < 0 || active_seq_kv < 0)
         return fail(MYNN_E_ARG, "attention_q8: bad shape");
     if (Hq % Hkv != 0) return fail(MYNN_E_ARG, "attention_q8: %d query heads are not a multiple of %d kv heads", Hq, Hkv);
@@ -669,6 +677,7 @@ int launch_attention_q8(cudaStream_t st, void *out, const void *q, const void *k
     const int rows_bound = active_seq_kv_dev ? cache_seq_len : (active_seq_kv < cache_seq_len ? active_seq_kv : cache_seq_len);
     const bool ring = q8_ring_possible(p, B, D);
     p.splits = decode_splits(B, Hkv, rows_bound, 32, ring ? 2 : kAttnCtasPerSm);
+    p.settled = step;
     if (int rc = decode_bind_workspace(p, B, D, workspace, workspace_bytes)) return rc;
     if (dtype == MYNN_BF16) return D == 64 ? launch_decode_q8<__nv_bfloat16, 64>(st, p, B, ring) : launch_decode_q8<__nv_bfloat16, 128>(st, p, B, ring);
     return D == 64 ? launch_decode_q8<__half, 64>(st, p, B, ring) : launch_decode_q8<__half, 128>(st, p, B, ring);

@@ -176,7 +176,7 @@ static int enqueue_forward(Model &m, cudaStream_t st, int S, int head_rows = 0) 
                                     c.max_seq_len, m.active_dev, 1, dt, m.attn_ws, m.attn_ws_bytes, 1));
             } else {
                 RC(launch_attention_q8(st, m.attn, m.q_rot, L.kc, L.vc, L.ksc, L.vsc, attn_scale, B, m.Hq, m.Hkv, S, D,
-                                       c.max_seq_len, c.max_seq_len, m.active_dev, S > 1, dt, m.attn_ws, m.attn_ws_bytes, 1));
+                                       c.max_seq_len, c.max_seq_len, m.active_dev, S > 1, dt, m.attn_ws, m.attn_ws_bytes, 1, S == 1));
             }
         } else if (c.stream_window > 0) {
             // streaming cache: K is appended unrotated at the slot in past_dev; the live rows are rotated at their
@@ -185,7 +185,7 @@ static int enqueue_forward(Model &m, cudaStream_t st, int S, int head_rows = 0) 
                                      S == 1 ? m.pos0_dev : m.pos_dev, B, S, m.Hq, m.Hkv, D, c.max_seq_len, m.past_dev, 0));
             RC(launch_rope_cache_rows(st, dt, m.k_rot, L.kc, m.cos_t, m.sin_t, m.kvpos_dev, B * m.Hkv, c.max_seq_len, D, 0, m.active_dev));
             RC(launch_attention(st, m.attn, m.q_rot, m.k_rot, L.vc, attn_scale, B, m.Hq, m.Hkv, S, D, c.max_seq_len,
-                                c.max_seq_len, m.active_dev, S > 1, dt, m.attn_ws, m.attn_ws_bytes, 1));
+                                c.max_seq_len, m.active_dev, S > 1, dt, m.attn_ws, m.attn_ws_bytes, 1, nullptr, nullptr, nullptr, nullptr, true));
         } else {
             // decode: the attention kernel also leaves its output rows as the activation limbs of o_proj
             attn_limbs = fused && S == 1 && Nq % 16 == 0 && (size_t)Nq * 4 <= 200 * 1024 &&
@@ -194,11 +194,15 @@ static int enqueue_forward(Model &m, cudaStream_t st, int S, int head_rows = 0) 
             // the projection output is one block whose rows and heads are 16-byte aligned
             const bool fuse_rope = g_fuse_rope && attn_limbs && L.qkv_fused && qs % 8 == 0 && D % 32 == 0 &&
                                    (((uintptr_t)kb | (uintptr_t)vb) % 16) == 0;
+            // A lean o_proj takes the rows as they are: limbs made there, or by a row kernel in front, cost less than a last CTA of the attention
+            // that collects the heads (TinyLlama shapes, one sequence: 3.8 us for product and limbs against 2.2 + 3.5).
+            if (tp == 1 && fuse_rope && gemv_lean_supported(M, H, Nq, L.wo)) attn_limbs = false;
             if (fuse_rope) {
                 const AttentionFuse fz = {kb, vb, qs, m.cos_t, m.sin_t, m.pos0_dev, m.past_dev, 1};  // the inputs' copy lies between two steps
                 RC(launch_attention(st, m.attn, qb, L.kc, L.vc, attn_scale, B, m.Hq, m.Hkv, S, D, c.max_seq_len, c.max_seq_len,
-                                    m.active_dev, 0, dt, m.attn_ws, m.attn_ws_bytes, 1, (int8_t *)m.gemm_ws + 512,
-                                    (float *)((char *)m.gemm_ws + 256), &fz, (int *)m.gemm_ws));
+                                    m.active_dev, 0, dt, m.attn_ws, m.attn_ws_bytes, 1,
+                                    attn_limbs ? (int8_t *)m.gemm_ws + 512 : nullptr, attn_limbs ? (float *)((char *)m.gemm_ws + 256) : nullptr, &fz,
+                                    (int *)m.gemm_ws));
             } else {
                 RC(launch_rope_kv_append(st, dt, m.q_rot, L.kc, L.vc, qb, kb, vb, qs, ks, vs, m.cos_t, m.sin_t,
                                          S == 1 ? m.pos0_dev : m.pos_dev, B, S, m.Hq, m.Hkv, D, c.max_seq_len, m.past_dev));
@@ -206,7 +210,7 @@ static int enqueue_forward(Model &m, cudaStream_t st, int S, int head_rows = 0) 
                 RC(launch_attention(st, m.attn, m.q_rot, L.kc, L.vc, attn_scale, B, m.Hq, m.Hkv, S, D, c.max_seq_len,
                                     c.max_seq_len, m.active_dev, S > 1, dt, m.attn_ws, m.attn_ws_bytes, 1,
                                     attn_limbs ? (int8_t *)m.gemm_ws + 512 : nullptr, attn_limbs ? (float *)((char *)m.gemm_ws + 256) : nullptr,
-                                    nullptr, (int *)m.gemm_ws));
+                                    nullptr, (int *)m.gemm_ws, true));
             }
         }
         if (tp == 1) {

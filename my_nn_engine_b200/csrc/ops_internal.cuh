@@ -34,11 +34,12 @@ int launch_rope_kv_append_q8(cudaStream_t st, int dtype, void *q_out, void *k_ca
                              const int64_t *positions, int B, int S, int Hq, int Hkv, int D, int cache_seq,
                              const int32_t *past_len_dev, int rotate_k = 1);
 
-// Attention over an int8 KV cache (per-token scales), with the output-layout choice of launch_attention.
+// Attention over an int8 KV cache (per-token scales), with the output-layout choice of launch_attention.  step: a decode step of a model (see
+// DecodeParams::settled).
 int launch_attention_q8(cudaStream_t st, void *out, const void *q, const void *k, const void *v, const void *k_scale,
                         const void *v_scale, float scale, int B, int Hq, int Hkv, int Sq, int D, int cache_seq_len,
                         int active_seq_kv, const int32_t *active_seq_kv_dev, int is_causal, int dtype, void *workspace,
-                        size_t workspace_bytes, int out_bshd);
+                        size_t workspace_bytes, int out_bshd, bool step = false);
 
 // out[m, f] = swish(gate[m, f]) * up[m, f] with gate/up rows `in_stride` elements apart.
 int launch_swiglu_strided(cudaStream_t st, int dtype, void *out, const void *gate, const void *up, int M, int F,
@@ -66,7 +67,8 @@ int launch_attention(cudaStream_t st, void *out, const void *q, const void *k, c
                      int Hq, int Hkv, int Sq, int D, int cache_seq_len, int active_seq_kv,
                      const int32_t *active_seq_kv_dev, int is_causal, int dtype, void *workspace,
                      size_t workspace_bytes, int out_bshd, int8_t *limbs_out = nullptr, float *ascale_out = nullptr,
-                     const AttentionFuse *fuse = nullptr, int *status_word = nullptr);
+                     const AttentionFuse *fuse = nullptr, int *status_word = nullptr, bool step = false);
+// step: a decode step of a model (few sequences then take wider CTAs; implied by fuse)
 // status_word: where the ring form of the decode kernel records a timed-out wait (null: the library's own word)
 int attention_decode_take_status(int *status);
 int attention_decode_q8_take_status(int *status);

@@ -1,0 +1,158 @@
+"""Forms that one operator is dispatched to, on both sides of each rule and at the edges of their tiles: integer sums are exact, so forms of
+the int8 products agree to the last bit; the others are compared with float64."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from my_nn_engine_b200 import ops  # noqa: E402
+from oracle import ref_ops as R  # noqa: E402
+from oracle import ref_vebisun as V  # noqa: E402
+
+DT = {"bf16": torch.bfloat16, "f16": torch.float16, "f32": torch.float32}
+
+
+def gen(seed):
+    return torch.Generator(device="cuda").manual_seed(seed)
+
+
+def randn(g, *shape):
+    return torch.randn(*shape, generator=g, device="cuda")
+
+
+def int8(g, *shape):
+    return torch.randint(-127, 128, shape, generator=g, device="cuda", dtype=torch.int32).to(torch.int8)
+
+
+def scales(g, n, dt):
+    return (0.002 + 0.018 * torch.rand(n, generator=g, device="cuda")).to(dt)
+
+
+# ---- DequantMatMul of a few rows: up to five go to the lean kernel, eight to the tcgen05 one ----
+@pytest.mark.parametrize("dt", ["bf16", "f16", "f32"])
+@pytest.mark.parametrize("n,k", [(1, 16), (130, 1040), (2561, 2048), (2100, 4096), (700, 4112), (5000, 6144), (40001, 512), (9000, 4096)])
+def test_lean_product_equals_the_tensor_core_product(dt, n, k):
+    g = gen(n + k)
+    w, s, act = int8(g, n, k), scales(g, n, DT[dt]), randn(g, 8, k).to(DT[dt])
+    act[2] = 0
+    res = randn(g, 8, n).to(DT[dt])
+    want, want_res = ops.dequant_matmul(act, w, s), ops.dequant_matmul_residual(act, w, s, res)
+    for m in (1, 2, 3, 4, 5):
+        assert torch.equal(ops.dequant_matmul(act[:m], w, s), want[:m])
+        assert torch.equal(ops.dequant_matmul_residual(act[:m], w, s, res[:m]), want_res[:m])
+    shifted = torch.empty(3 * k + 1, dtype=DT[dt], device="cuda")[1:].view(3, k)  # rows that no 16-byte load may touch
+    shifted.copy_(act[:3])
+    assert torch.equal(ops.dequant_matmul(shifted, w, s), want[:3])
+    act[1, k // 2] = float("inf")  # spoils its own row alone
+    got = ops.dequant_matmul(act[:4], w, s)
+    assert torch.isnan(got[1]).all() and torch.equal(got[[0, 2, 3]], want[[0, 2, 3]])
+
+
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("hidden,ffn", [(256, 704), (512, 1040), (384, 512)])
+def test_small_batches_step_like_a_large_one(dt, hidden, ffn):
+    """A first token attends to itself alone, so a step of one to five sequences (lean products, limbs of the
+    attention's rows made inside) and of eight (tcgen05 products) have to agree to the last bit."""
+    from my_nn_engine_b200.decoder import DecoderModel
+    from my_nn_engine_b200.quantize import random_llama_state
+    cfg = dict(hidden_size=hidden, num_hidden_layers=2, num_attention_heads=hidden // 64, num_key_value_heads=2, head_dim=64, intermediate_size=ffn, vocab_size=500,
+               rms_norm_eps=1e-5, rope_theta=1e4)
+    state, tokens, rows = random_llama_state(cfg, seed=3), np.arange(8) * 61 % 500, {}
+    for batch in (1, 2, 3, 5, 8):
+        model = DecoderModel(cfg, state, dtype=dt, max_seq_len=32, batch=batch)
+        rows[batch] = model.step(tokens[:batch], 0).clone()
+        model.close()
+    for batch in (1, 2, 3, 5):
+        assert torch.equal(rows[batch], rows[8][:batch])
+
+
+# ---- products of many int8 rows: tile widths, ragged last tiles ----
+@pytest.mark.parametrize("m,n,k", [(257, 3001, 1040), (520, 128, 2064), (777, 14336, 256), (2047, 640, 512), (1500, 5632, 128), (40, 130, 16)])
+def test_w8a8_product_is_exact(m, n, k):
+    g = gen(m)
+    a, w, sa, sw = int8(g, m, k), int8(g, n, k), scales(g, m, torch.bfloat16), scales(g, n, torch.bfloat16)
+    want = ((a.double() @ w.double().t()).float() * sa.float()[:, None] * sw.float()).bfloat16()
+    assert torch.equal(ops.quantized_matmul(a, sa, w, sw), want)
+
+
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("m,n,k", [(33, 130, 48), (333, 2560, 2048), (777, 3001, 2064), (2047, 1000, 512)])
+def test_prompt_product_rounds_like_float64(dt, m, n, k):
+    """Two limbs hold 15 bits of the row maximum, so the error of a sum of k random terms stays near sqrt(k) 2^-16 max|a| |w|, far below the
+    rounding of the result; a non-finite row spoils itself alone."""
+    g = gen(m + 1)
+    w, s, act = int8(g, n, k), scales(g, n, DT[dt]), randn(g, m, k).to(DT[dt])
+    act[m // 2] = 0
+    act[m - 1, 3] = float("nan")
+    got, want = ops.dequant_matmul(act, w, s), act.double() @ w.double().t() * s.double()
+    assert torch.isnan(got[m - 1]).all()
+    ulp = 2.0 ** (-7 if dt == "bf16" else -10)
+    assert (got[:-1].double() - want[:-1]).abs().max() <= ulp * want[:-1].abs().max()
+
+
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("rows,inner", [(3, 8), (5, 2056), (2, 8192), (2, 8200), (300, 4096)])
+def test_dynamic_quantisation_of_rows(dt, rows, inner):
+    x = randn(gen(inner), rows, inner).to(DT[dt]) * 3
+    want, want_s, _ = R.dynamic_quantize_linear(x.float().cpu().numpy(), True, True, dt)
+    y, s, zp = ops.dynamic_quantize_linear(x)
+    assert np.array_equal(y.cpu().numpy(), want) and np.array_equal(s.float().cpu().numpy(), want_s) and not zp.any()
+
+
+# ---- decode attention: wide CTAs up to 74 (sequence, kv head) pairs, four warps above; rounds of 64 to 256 rows, splits ----
+@pytest.mark.parametrize("b,hkv,d", [(1, 1, 64), (37, 2, 64), (38, 2, 64), (9, 8, 128), (10, 8, 128)])
+@pytest.mark.parametrize("active", [1, 16, 255, 257, 1025, 2300])
+def test_decode_attention_rows(b, hkv, d, active):
+    g, G = gen(active), 3
+    q, k, v = (randn(g, b, h, n, d).bfloat16() for h, n in ((G * hkv, 1), (hkv, 2304), (hkv, 2304)))
+    out = ops.window_attention(q, k, v, d ** -0.5, active, 0, 0.0).view_as(q)
+    ops.attention_check()
+    kk, vv = (t[:, :, :active].double().repeat_interleave(G, 1) for t in (k, v))
+    want = torch.softmax((q.double() @ kk.transpose(2, 3)) * d ** -0.5, -1) @ vv
+    # the weights are split into two 16-bit parts, so the rounding of the result to bf16 (2^-9) is what remains
+    assert (out.double() - want).abs().max() <= 2.0 ** -8 * want.abs().max()
+
+
+# ---- norms: few rows, many rows, widths around the number of groups per thread ----
+@pytest.mark.parametrize("rows", [1, 148, 149])
+@pytest.mark.parametrize("W", [4, 1024, 1028, 2052, 4096, 4100, 8192, 8196])
+def test_norms_of_few_and_many_rows(rows, W):
+    g = gen(W)
+    x, w, b = randn(g, rows, W) * 3 + 40.0, randn(g, W), randn(g, W)  # a mean that is large against the deviations
+    xd = x.double()
+    ln = (xd - xd.mean(1, keepdim=True)) / torch.sqrt(xd.var(1, unbiased=False, keepdim=True) + 1e-5) * w + b
+    out = ops.layer_norm(x, w, b, 1e-5, torch.float32)
+    assert (out.double() - ln).abs().max() <= 3e-5 * ln.abs().max()  # 40 / 3 * 2^-24 of the mean, times the largest weight
+    sub, y = randn(g, rows, W).bfloat16(), x.clone()
+    out = ops.residual_rms_norm(y, sub, w, 1e-5)
+    s = xd + sub.double()
+    rms = s / torch.sqrt((s * s).mean(1, keepdim=True) + 1e-5) * w
+    assert (y.double() - s).abs().max() <= 1e-6 * s.abs().max()
+    assert (out.double() - rms).abs().max() <= 2.0 ** -8 * rms.abs().max()
+
+
+# ---- expert choice: logits per lane 2, 8, 32; one CTA up to 64 tokens ----
+@pytest.mark.parametrize("M", [1, 64, 65])
+@pytest.mark.parametrize("E,top,groups,keep", [(64, 8, 8, 4), (65, 3, 5, 2), (256, 32, 64, 40), (264, 4, 33, 3), (1024, 8, 64, 5)])
+def test_expert_choice(M, E, top, groups, keep):
+    z = randn(gen(E + M), M, E)
+    z[0, :4] = z[0].max() + 1.0  # equal scores go to the lower expert
+    z[0, E // 2] = -0.0
+    r = ops.MoeRouting(z, top, groups, keep)
+    rows, chosen, weights = r.rows().cpu().numpy().reshape(-1), r.chosen.cpu().numpy(), r.weights.double().cpu().numpy()
+    for t in range(M):
+        e, w = V.route(z[t].double().cpu().numpy(), top, groups, keep)
+        assert chosen[t].tolist() == list(e) and np.abs(weights[t] - w).max() <= 3e-6 * w.max()
+    order = np.empty(M * top, int)
+    order[rows] = chosen.reshape(-1)  # a permutation, ordered by expert
+    assert sorted(rows.tolist()) == list(range(M * top)) and (np.diff(order) >= 0).all()
+
+
+# ---- products over unquantised weights: sixteen warps up to 148 CTAs, blocks of row tiles ----
+@pytest.mark.parametrize("M,N,K", [(1, 2368, 264), (8, 2384, 264), (5, 40, 4104), (3, 2050, 72), (3300, 300, 8192)])
+def test_dense_products(M, N, K):
+    g = gen(N)
+    act, w, status = randn(g, M, K).bfloat16(), randn(g, N, K).bfloat16(), torch.zeros(1, dtype=torch.int32, device="cuda")
+    want = act.double() @ w.double().t()
+    assert (ops.dense_matmul(act, w, status=status).double() - want).abs().max() <= 2.0 ** -8 * want.abs().max()

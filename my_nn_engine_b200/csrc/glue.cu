@@ -253,15 +253,14 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 rope_kv_append_vec_kernel(T *q_out, T *k_cache, T *v_cache, const T *q, const T *k, const T *v, long long q_stride,
                           long long k_stride, long long v_stride, const T *cos_t, const T *sin_t, const int64_t *positions,
-                          long long units, int S, int Hq, int Hkv, int D, int cache_seq, const int32_t *past_len_dev, int rotate_k) {
+                          unsigned units, int S, int Hq, int Hkv, int D, int cache_seq, const int32_t *past_len_dev, int rotate_k) {
     pdl_trigger();
     pdl_wait();
-    const long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned u = blockIdx.x * blockDim.x + threadIdx.x;  // 32 bits: three divisions of 64 bits took longer than the rotation
     if (u >= units) return;
-    const int half = D >> 1, groups = half >> 3, slots = Hq + 2 * Hkv;
-    const int g = (int)(u % groups), slot = (int)((u / groups) % slots);
-    const int row = (int)(u / ((long long)groups * slots)), b = row / S, s = row - b * S;
-    const int j0 = 8 * g;
+    const unsigned half = D >> 1, groups = half >> 3, slots = Hq + 2 * Hkv;
+    const unsigned head = u / groups;
+    const int j0 = 8 * (int)(u - head * groups), row = (int)(head / slots), slot = (int)(head - row * slots), b = row / S, s = row - b * S;
     const int cache_row = *past_len_dev + s;
     const bool in_cache = cache_row >= 0 && cache_row < cache_seq;
     const bool is_q = slot < Hq, is_k = !is_q && slot < Hq + Hkv;
@@ -301,6 +300,7 @@ int launch_rope_kv_append(cudaStream_t st, int dtype, void *q_out, void *k_cache
                           int Hkv, int D, int cache_seq, const int32_t *past_len_dev, int rotate_k) {
     if (B * S == 0) return MYNN_OK;
     const bool vec = dtype != MYNN_F32 && D % 16 == 0 && q_stride % 8 == 0 && k_stride % 8 == 0 && v_stride % 8 == 0 &&
+                     (long long)B * S * (Hq + 2 * Hkv) * (D / 16) < (1ll << 32) - 256 &&
                      (((uintptr_t)q_out | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)q | (uintptr_t)k | (uintptr_t)v |
                        (uintptr_t)cos_t | (uintptr_t)sin_t) % 16) == 0;
     if (vec) {
@@ -310,12 +310,12 @@ int launch_rope_kv_append(cudaStream_t st, int dtype, void *q_out, void *k_cache
             using T = __nv_bfloat16;
             MYNN_CUDA_OK(launch_dependent(rope_kv_append_vec_kernel<T>, dim3(blocks), dim3(256), 0, st, (T *)q_out, (T *)k_cache, (T *)v_cache,
                                     (const T *)q, (const T *)k, (const T *)v, q_stride, k_stride, v_stride, (const T *)cos_t,
-                                    (const T *)sin_t, positions, units, S, Hq, Hkv, D, cache_seq, past_len_dev, rotate_k));
+                                    (const T *)sin_t, positions, (unsigned)units, S, Hq, Hkv, D, cache_seq, past_len_dev, rotate_k));
         } else {
             using T = __half;
             MYNN_CUDA_OK(launch_dependent(rope_kv_append_vec_kernel<T>, dim3(blocks), dim3(256), 0, st, (T *)q_out, (T *)k_cache, (T *)v_cache,
                                     (const T *)q, (const T *)k, (const T *)v, q_stride, k_stride, v_stride, (const T *)cos_t,
-                                    (const T *)sin_t, positions, units, S, Hq, Hkv, D, cache_seq, past_len_dev, rotate_k));
+                                    (const T *)sin_t, positions, (unsigned)units, S, Hq, Hkv, D, cache_seq, past_len_dev, rotate_k));
         }
         MYNN_LAUNCH_OK("rope_kv_append_vec_kernel");
         return MYNN_OK;

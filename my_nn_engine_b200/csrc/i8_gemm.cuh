@@ -42,7 +42,7 @@ int i8_prefill_launch(cudaStream_t st, void *out, const void *act, const int8_t 
 // Fused producers for the prefill kernel (rows > 32): leave two limbs per element + row scales in `workspace`; the following
 // i8_prefill_launch is called with act == nullptr.  prefill_fused_supported: 16-bit dtype, K % 16 == 0, 16-byte aligned inputs.
 bool prefill_fused_supported(int dtype, int K, const void *a, const void *b);
-int launch_rms_norm_limbs2(cudaStream_t st, int dtype, void *workspace, size_t workspace_bytes, const void *x, const void *w, float eps,
+int launch_rms_norm_limbs2(cudaStream_t st, int dtype, void *workspace, size_t workspace_bytes, void *x, const void *add, const void *w, float eps,
                            int rows, int D);
 int launch_swiglu_limbs2(cudaStream_t st, int dtype, void *workspace, size_t workspace_bytes, const void *gate, const void *up, int rows,
                          int F, long long in_stride);

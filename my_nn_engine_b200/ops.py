@@ -8,6 +8,7 @@ tensors and the call raises otherwise.
 from __future__ import annotations
 
 import ctypes
+import functools
 
 import torch
 
@@ -34,16 +35,22 @@ def _ptr(t):
 
 
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream of the current device, without building a Stream object (a call of a small operator is bound by its host time)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 _gemm_ws: dict = {}
 
 
+@functools.lru_cache(maxsize=4096)
+def _gemm_ws_bytes(m, n, k):
+    return ffi.lib().mynn_b200_dequant_matmul_workspace_bytes(m, n, k)
+
+
 def dequant_matmul_workspace(m, n, k, device):
     """Zero-initialised scratch for DequantMatMul (the operator's WORKSPACE slot), cached per device and stream."""
-    need = ffi.lib().mynn_b200_dequant_matmul_workspace_bytes(m, n, k)
-    key = (str(device), torch.cuda.current_stream().cuda_stream)
+    need = _gemm_ws_bytes(m, n, k)
+    key = (device if isinstance(device, torch.device) else torch.device(device), _stream())
     ws = _gemm_ws.get(key)
     if ws is None or ws.numel() < need:
         ws = torch.zeros(max(need, 512), dtype=torch.uint8, device=device)

@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(SOLO ? 512 : 256, !SOLO && MT * RT * (GLU ? 2 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, t = lane & 3;
     pdl_trigger();
     const int n0 = blockIdx.x * 16 * (GLU ? 1 : RT), z = g.batch > 1 ? blockIdx.y : 0;
-    if (!g.off && gridDim.x <= kPrefetchCtas) {
+    if (!g.off && (gridDim.x <= kPrefetchCtas || blockIdx.x < 2 * 148)) {
         // launched as a programmatic dependent: the weights of this CTA travel to L2 while the kernel in front of it still runs
         // (a CTA of a later wave starts long after that, for it the prefetch would only be one more request)
         const size_t line = 128 / sizeof(T), total = (size_t)min(16 * (GLU ? 1 : RT), g.N - n0) * g.K;
@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(SOLO ? 512 : 256, !SOLO && MT * RT * (GLU ? 2 
 template <typename T, typename O>
 static int run_stream(cudaStream_t st, const GemmView &v, int rows, int groups, int glu) {
     const int mt = rows <= 8 ? 1 : rows <= 16 ? 2 : 4;
-    const bool wide = !glu && (v.batch > 1 ? v.N * (long long)v.batch >= 32 * 148 * 2 : (mt > 1 || v.N >= 16 * 148 * 4) && v.N >= 32 * 100);
+    const bool wide = !glu && (v.batch > 1 ? v.N * (long long)v.batch >= 32 * 148 * 2 : (mt > 1 || v.N > 16 * (int)kPrefetchCtas) && v.N >= 32 * 100);
     const dim3 grid((v.N + (wide ? 31 : 15)) / (wide ? 32 : 16), groups);
     const bool solo = mt == 1 && !wide && (long long)grid.x * grid.y <= 148;
     cudaLaunchConfig_t cfg = {};

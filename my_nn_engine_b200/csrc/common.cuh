@@ -95,9 +95,9 @@ __device__ __forceinline__ float warp_max(float v) {
 // while the kernel in front still runs, do what does not depend on it (barrier set-up, weights, settled state and caches), and order
 // themselves with pdl_wait() before they touch anything that an earlier kernel of the step writes.  pdl_wait() returns when the grid in front
 // has completed and is visible; since every kernel of a chain waits, that covers all before it.  pdl_trigger() says when the next kernel may
-// become resident: at the start where this kernel leaves room beside it (lean products leave eight SMs to the row kernels), not before the
-// end in the tcgen05 products.  (There a trigger at the start made the kernels two and three places ahead take registers and shared memory
-// from the running one, step of batch 32 4.63 -> 5.31 ms, and one behind the main loop moved nothing.)
+// become resident: at the start where this kernel leaves room beside it (lean products leave eight SMs to the row kernels), when the
+// accumulators are complete in the tcgen05 products (step of batch 32: 3.98 -> 3.85 ms; a trigger at their start made the kernels two and three
+// places ahead take registers and shared memory from the running one, 4.63 -> 5.31 ms), when its own loads are here in the norms of few rows.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

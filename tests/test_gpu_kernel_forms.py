@@ -41,9 +41,10 @@ def test_lean_product_equals_the_tensor_core_product(dt, n, k):
     for m in (1, 2, 3, 4, 5):
         assert torch.equal(ops.dequant_matmul(act[:m], w, s), want[:m])
         assert torch.equal(ops.dequant_matmul_residual(act[:m], w, s, res[:m]), want_res[:m])
-    shifted = torch.empty(3 * k + 1, dtype=DT[dt], device="cuda")[1:].view(3, k)  # rows that no 16-byte load may touch
-    shifted.copy_(act[:3])
-    assert torch.equal(ops.dequant_matmul(shifted, w, s), want[:3])
+    for m in (1, 3, 8):
+        shifted = torch.empty(m * k + 1, dtype=DT[dt], device="cuda")[1:].view(m, k)  # rows that no wider load may touch
+        shifted.copy_(act[:m])
+        assert torch.equal(ops.dequant_matmul(shifted, w, s), want[:m])
     act[1, k // 2] = float("inf")  # spoils its own row alone
     got = ops.dequant_matmul(act[:4], w, s)
     assert torch.isnan(got[1]).all() and torch.equal(got[[0, 2, 3]], want[[0, 2, 3]])

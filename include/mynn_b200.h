@@ -84,7 +84,8 @@ int mynn_b200_compiled_arch(void);
  * [N,K] problems of up to 32 rows with K % 16 == 0 run on the tcgen05 int8 tensor-core kernel (exact int32
  * accumulation of 23-bit fixed-point activations).  With workspace == NULL, or for other shapes, kernels that need no
  * scratch are used (mma.sync streaming kernel for K % 64 == 0, N % 16 == 0, M <= 32; a generic kernel otherwise).
- * Calls that share a workspace must be ordered on one stream. */
+ * Calls that share a workspace must be ordered on one stream.  Any operand, wq and scale too, may be the output of the
+ * call right in front on that stream. */
 size_t mynn_b200_dequant_matmul_workspace_bytes(int M, int N, int K);
 int mynn_b200_dequant_matmul(void *stream, void *out, const void *act, const int8_t *wq, const void *scale, int M,
                              int N, int K, int act_dtype, int out_dtype, int w_layout, void *workspace,

@@ -92,13 +92,18 @@ __device__ __forceinline__ float warp_max(float v) {
 
 // ---- programmatic dependent launch -----------------------------------------------------------------------------
 // Most kernels of a step are launched with the programmatic-stream-serialization attribute (launch_dependent): they may become resident
-// while the kernel in front still runs, do what does not depend on it (barrier set-up, weights, settled state and caches), and order
-// themselves with pdl_wait() before they touch anything that an earlier kernel of the step writes.  pdl_wait() returns when the grid in front
-// has completed and is visible; since every kernel of a chain waits, that covers all before it.  pdl_trigger() says when the next kernel may
-// become resident: at the start where this kernel leaves room beside it (lean products leave eight SMs to the row kernels), when the
+// while the kernel in front still runs.  A dependent writes nothing before pdl_wait(), and before it reads only what no kernel since the last
+// full barrier on its stream (a copy, a synchronisation) writes.  A model's step begins with the copy of its inputs, so its weights,
+// positions and the state that earlier steps left may be read early; an operator's caller may have made any operand with the kernel right in
+// front, so the operators read nothing early: each early read stands behind a flag that only a model's step sets (settled,
+// fixed_weights).  A prefetch into L2 is no read.  What the kernel in front triggers, and when, makes no difference to this.
+// pdl_wait() returns when the grid in front has completed and is visible; since the kernels of a chain wait, that covers all before it.  The
+// one that does not, tp_reduce_norm_limbs_kernel, polls for each word it takes from the grid in front.
+// pdl_trigger() says when the next kernel may become resident: at the start where this kernel leaves room beside it (lean products leave eight SMs to the row kernels), when the
 // accumulators are complete in the tcgen05 products (step of batch 32: 3.98 -> 3.85 ms; a trigger at their start made the kernels two and three
 // places ahead take registers and shared memory from the running one, 4.63 -> 5.31 ms), when its own loads are here in the norms of few rows.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Library options (mynn_b200_set_option).

@@ -472,18 +472,16 @@ static int dequant_matmul_typed(cudaStream_t st, OutT *out, const ActT *act, con
     return MYNN_OK;
 }
 
-static int dequant_matmul_dispatch(void *stream, void *out, const void *act, const int8_t *wq, const void *scale,
-                                   const void *resid, int M, int N, int K, int act_dtype, int out_dtype,
-                                   int w_layout, void *workspace, size_t workspace_bytes) {
+int launch_dequant_matmul(cudaStream_t st, void *out, const void *act, const int8_t *wq, const void *scale, const void *resid, int M, int N,
+                          int K, int act_dtype, int out_dtype, int w_layout, void *workspace, size_t workspace_bytes, bool settled) {
     if (M < 0 || N < 0 || K < 0) return fail(MYNN_E_ARG, "dequant_matmul: negative dimension (M=%d N=%d K=%d)", M, N, K);
     if (w_layout != MYNN_W_NK && w_layout != MYNN_W_KN) return fail(MYNN_E_ARG, "dequant_matmul: bad weight layout %d", w_layout);
     if (!dtype_ok(act_dtype) || !dtype_ok(out_dtype)) return fail(MYNN_E_ARG, "dequant_matmul: bad dtype");
     if (M == 0 || N == 0) return MYNN_OK;
     if (!out || !wq || !scale || (!act && K > 0)) return fail(MYNN_E_ARG, "dequant_matmul: null pointer");
-    cudaStream_t st = (cudaStream_t)stream;
     // With scratch memory the tcgen05 int8 kernel takes every [N,K] problem of up to 32 rows.
     if (workspace && w_layout == MYNN_W_NK && i8_gemm_supported(M, N, K, wq, act_dtype, out_dtype))
-        return i8_gemm_launch(st, out, act, wq, scale, resid, M, N, K, act_dtype, out_dtype, workspace, workspace_bytes);
+        return i8_gemm_launch(st, out, act, wq, scale, resid, M, N, K, act_dtype, out_dtype, workspace, workspace_bytes, settled);
     // More rows: the prefill kernel (two activation limbs, 128 x 128-token tiles) if the scratch is large enough.
     if (workspace && w_layout == MYNN_W_NK && i8_prefill_supported(M, N, K, wq, act_dtype, out_dtype) &&
         workspace_bytes >= i8_prefill_workspace_bytes(M, K))
@@ -512,15 +510,15 @@ extern "C" size_t mynn_b200_dequant_matmul_workspace_bytes(int M, int N, int K) 
 extern "C" int mynn_b200_dequant_matmul(void *stream, void *out, const void *act, const int8_t *wq, const void *scale,
                                         int M, int N, int K, int act_dtype, int out_dtype, int w_layout,
                                         void *workspace, size_t workspace_bytes) {
-    return mynn::dequant_matmul_dispatch(stream, out, act, wq, scale, nullptr, M, N, K, act_dtype, out_dtype, w_layout,
-                                         workspace, workspace_bytes);
+    return mynn::launch_dequant_matmul((cudaStream_t)stream, out, act, wq, scale, nullptr, M, N, K, act_dtype, out_dtype, w_layout, workspace,
+                                       workspace_bytes, false);
 }
 
 extern "C" int mynn_b200_dequant_matmul_residual(void *stream, void *out, const void *act, const int8_t *wq,
                                                  const void *scale, const void *residual, int M, int N, int K,
                                                  int dtype, void *workspace, size_t workspace_bytes) {
-    return mynn::dequant_matmul_dispatch(stream, out, act, wq, scale, residual, M, N, K, dtype, dtype, MYNN_W_NK,
-                                         workspace, workspace_bytes);
+    return mynn::launch_dequant_matmul((cudaStream_t)stream, out, act, wq, scale, residual, M, N, K, dtype, dtype, MYNN_W_NK, workspace,
+                                       workspace_bytes, false);
 }
 
 // DequantMatMul for activations that the PREVIOUS call on this workspace already converted: several weight matrices
@@ -533,7 +531,7 @@ extern "C" int mynn_b200_dequant_matmul_same_act(void *stream, void *out, const 
     if (!dtype_ok(act_dtype) || !dtype_ok(out_dtype)) return fail(MYNN_E_ARG, "dequant_matmul_same_act: bad dtype");
     if (!workspace || !i8_gemm_supported(M, N, K, wq, act_dtype, out_dtype))
         return fail(MYNN_E_UNSUPPORTED, "dequant_matmul_same_act: needs the tensor-core path (a workspace, at most %d rows, K %% 16 == 0, 16-byte aligned weights)", kI8MaxRows);
-    return i8_gemm_launch((cudaStream_t)stream, out, nullptr, wq, scale, nullptr, M, N, K, act_dtype, out_dtype, workspace, workspace_bytes);
+    return i8_gemm_launch((cudaStream_t)stream, out, nullptr, wq, scale, nullptr, M, N, K, act_dtype, out_dtype, workspace, workspace_bytes, false);
 }
 
 // Reads the status word of a DequantMatMul workspace after synchronising the stream: non-zero means a pipeline

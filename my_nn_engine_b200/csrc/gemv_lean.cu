@@ -8,8 +8,8 @@
 // warp per row, one 16-byte load in flight per lane):
 //   * one CTA per SM with an equal share of the rows, so the grid is a single balanced wave.  Its rows are tiles of 16; the sixteen warps
 //     deal out the contraction, so that every warp has the same piece of every row, and each lane issues all its 128-bit loads (up to 20)
-//     before it touches anything else, and before the programmatic-dependent-launch wait: the weights are in flight while
-//     the preceding kernel drains;
+//     before it touches anything else and, where the weights are settled (i8_gemm.cuh), before the programmatic-dependent-launch wait: they
+//     are in flight while the preceding kernel drains;
 //   * the activation row(s) are the same three signed 8-bit limbs of a 23-bit fixed-point value the tensor-core kernel uses, either read
 //     from the workspace, where a fused producer left them, or computed here in shared memory (no extra launch).  Three limbs of up to
 //     five rows are the columns of mma.m16n8k32 (int8, exact int32 sums).  The contraction index is permuted so that the 16 bytes a lane
@@ -44,11 +44,13 @@ struct LeanParams {
     int8_t *limbs_g;        // workspace limb matrix [(3m + l)][K]; read when act == null, written by CTA 0 otherwise
     float *ascale_g;        // [M] row scales
     int N, K, act_dtype, rows_per_cta;
+    int settled;            // wq and scale may be read while the kernels in front still run
 };
 
+// not ld.global.nc: weights that are not settled may have been written during the lifetime of this grid
 __device__ __forceinline__ uint4 ldg_stream_16(const void *p) {
     uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
 
@@ -209,7 +211,16 @@ __global__ void __launch_bounds__(kLeanThreads, 1) gemv_lean_kernel(const LeanPa
             }
         }
     };
-    // the first tiles of weights and the row scale of this thread's output depend on nothing an earlier kernel writes
+    // settled: the first tiles of weights and the row scale of this thread's output depend on nothing an earlier kernel writes; else the
+    // weights only travel to L2 ahead of the wait
+    if (!p.settled) {
+        if (t == 0)
+            for (int row = gq; row < min(rows, 16 * TG); row += 8)
+#pragma unroll
+                for (int j = 0; j < NB; j++)
+                    if (c0 + 4 * j < chunks) prefetch_l2(p.wq + (size_t)(row0 + row) * K + 16 * (size_t)(c0 + 4 * j));
+        pdl_wait();
+    }
 #pragma unroll
     for (int i = 0; i < TG; i++)
         if (i < tiles) load_tile(w[i], i);
@@ -371,7 +382,7 @@ static int launch_by_rows(cudaStream_t st, const LeanParams &p, int M) {
 // Same contract as i8_gemm_launch: `workspace` holds status word, row scales and the limb matrix; act == nullptr means a fused
 // producer (or the previous call) left the limbs there.
 int gemv_lean_launch(cudaStream_t st, void *out, const void *act, const int8_t *wq, const void *scale, const void *resid, int M, int N,
-                     int K, int act_dtype, int out_dtype, void *workspace, size_t workspace_bytes) {
+                     int K, int act_dtype, int out_dtype, void *workspace, size_t workspace_bytes, bool settled) {
     const size_t need = i8_gemm_workspace_bytes(M, K);
     if (!workspace || workspace_bytes < need || (uintptr_t)workspace % 256)
         return fail(MYNN_E_ARG, "dequant_matmul: workspace of %zu bytes (256-byte aligned) needed", need);
@@ -391,6 +402,7 @@ int gemv_lean_launch(cudaStream_t st, void *out, const void *act, const int8_t *
     p.N = N;
     p.K = K;
     p.act_dtype = act_dtype;
+    p.settled = settled;
     if (out_dtype == MYNN_BF16) return launch_by_rows<__nv_bfloat16>(st, p, M);
     if (out_dtype == MYNN_F16) return launch_by_rows<__half>(st, p, M);
     return launch_by_rows<float>(st, p, M);

@@ -48,10 +48,12 @@ struct I8GemmParams {
     void *out;
     const void *scale, *resid;
     const float *ascale;  // [M] activation row scales 2^(e-22)
+    const int8_t *wq;
     int M, N, K;
     int *status;          // device int, set non-zero on a timed-out wait
     int stages;           // pipeline depth: kStages or kMaxStages
     I8Tp tp;              // tensor-parallel form: the outputs are delivered to every rank as partial sums (mode 0: off)
+    int settled;          // the weights may be read while the kernels in front still run (i8_gemm.cuh)
     int skip_last_stage;  // test aid (MYNN_OPT_INJECT_STALL): the producer leaves out the last k block, so a bounded wait expires
 #ifdef MYNN_TUNING
     unsigned long long *timing;  // 8 timestamps (ns) of CTA (0,0), or null
@@ -140,8 +142,9 @@ i8_stream_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         if (lane == 0) {
             asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
             asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
-            // The weights do not depend on the preceding kernel: start streaming them at once, and only then wait
+            // Settled weights do not depend on the kernels in front: start streaming them at once, and only then wait
             // (programmatic dependent launch) for the grid that writes the activation limbs.
+            if (!p.settled) pdl_wait();
             const int nload = nkb - ((p.skip_last_stage & 1) ? 1 : 0);  // normally every k block
             const int pre = min(nload, stages);
             for (int i = 0; i < pre; i++) {
@@ -227,6 +230,12 @@ i8_stream_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     float wscale = 0.f, res_r[RPC > kOwnMax ? RPC : kOwnMax];  // one array: the two forms never run together
     bool have_acc = false;
     if (warp >= 2) {
+        if (!p.settled) {  // the stages that the producer fills first travel to L2 while the kernel in front still runs
+            for (int i = et; i < min(nkb, stages) * kTileRows; i += kEpiThreads) {
+                const int row = row0 + i % kTileRows, k = (kb_beg + i / kTileRows) * kBlockK;
+                if (row < p.N) prefetch_l2(p.wq + (size_t)row * p.K + k);
+            }
+        }
         asm volatile("griddepcontrol.wait;" ::: "memory");  // row scales and the residual come from earlier grids
         // everything the finish needs from global memory is requested before waiting for the accumulators
         if (et < 32) sh_ascale[et] = et < p.M ? p.ascale[et] : 0.f;
@@ -916,18 +925,18 @@ int launch_act_limbs(cudaStream_t st, const void *act, int M, int K, int act_dty
 }
 
 int i8_gemm_launch(cudaStream_t st, void *out, const void *act, const int8_t *wq, const void *scale, const void *resid,
-                   int M, int N, int K, int act_dtype, int out_dtype, void *workspace, size_t workspace_bytes) {
-    return i8_gemm_launch_tp(st, out, act, wq, scale, resid, M, N, K, act_dtype, out_dtype, workspace, workspace_bytes, nullptr, nullptr,
+                   int M, int N, int K, int act_dtype, int out_dtype, void *workspace, size_t workspace_bytes, bool settled) {
+    return i8_gemm_launch_tp(st, out, act, wq, scale, resid, M, N, K, act_dtype, out_dtype, workspace, workspace_bytes, settled, nullptr, nullptr,
                              nullptr);
 }
 
 // tp: tensor-parallel form of the launch or null.  limbs_ext / ascale_ext: activation limbs that live outside the workspace
 // (the workspace then only carries the status word).
 int i8_gemm_launch_tp(cudaStream_t st, void *out, const void *act, const int8_t *wq, const void *scale, const void *resid,
-                      int M, int N, int K, int act_dtype, int out_dtype, void *workspace, size_t workspace_bytes, const I8Tp *tp,
-                      const int8_t *limbs_ext, const float *ascale_ext) {
+                      int M, int N, int K, int act_dtype, int out_dtype, void *workspace, size_t workspace_bytes, bool settled,
+                      const I8Tp *tp, const int8_t *limbs_ext, const float *ascale_ext) {
     if (!tp && !limbs_ext && gemv_lean_supported(M, N, K, wq))  // a few rows over a small matrix: no tensor-core set-up to amortise
-        return gemv_lean_launch(st, out, act, wq, scale, resid, M, N, K, act_dtype, out_dtype, workspace, workspace_bytes);
+        return gemv_lean_launch(st, out, act, wq, scale, resid, M, N, K, act_dtype, out_dtype, workspace, workspace_bytes, settled);
     const size_t need = limbs_ext ? 256 : i8_gemm_workspace_bytes(M, K);
     if (!workspace || workspace_bytes < need)
         return fail(MYNN_E_ARG, "dequant_matmul: workspace of %zu bytes needed, %zu given", need, workspace ? workspace_bytes : (size_t)0);
@@ -951,12 +960,14 @@ int i8_gemm_launch_tp(cudaStream_t st, void *out, const void *act, const int8_t 
     p.scale = scale;
     p.resid = resid;
     p.ascale = ascale;
+    p.wq = wq;
     p.M = M;
     p.N = N;
     p.K = K;
     p.status = status;
     if (tp) p.tp = *tp;
     else memset(&p.tp, 0, sizeof p.tp);
+    p.settled = settled;
     p.skip_last_stage = 0;
     {
         int want = 1;

@@ -34,26 +34,22 @@ static mynn_b200_model_config g_cfg;
 static bool g_cfg_set = false, g_cfg_blocks = false;
 static int g_status = MYNN_OK;
 
-// DequantMatMul over any number of rows: the streaming kernel takes up to 32 rows per pass.
+// DequantMatMul over any number of rows: the streaming kernel takes up to 32 rows per pass.  A model's weights are settled: no kernel of a
+// step writes them, and a copy of the step's inputs lies between whatever ran before and the step.
 static int gemm(cudaStream_t st, const Model &m, void *out, const void *act, const int8_t *w, const void *scale,
                 const void *resid, int M, int N, int K, int out_dtype) {
     const int dt = m.c.dtype;
     const size_t esz = dtype_size(dt), osz = dtype_size(out_dtype);
     if (M > 32 && m.gemm_ws && m.gemm_ws_bytes >= mynn_b200_dequant_matmul_workspace_bytes(M, N, K)) {
         // prefill: one launch of the large-tile tensor-core kernel over all rows
-        if (resid) return mynn_b200_dequant_matmul_residual(st, out, act, w, scale, resid, M, N, K, dt, m.gemm_ws, m.gemm_ws_bytes);
-        return mynn_b200_dequant_matmul(st, out, act, w, scale, M, N, K, dt, out_dtype, MYNN_W_NK, m.gemm_ws, m.gemm_ws_bytes);
+        return launch_dequant_matmul(st, out, act, w, scale, resid, M, N, K, dt, resid ? dt : out_dtype, MYNN_W_NK, m.gemm_ws, m.gemm_ws_bytes, true);
     }
     for (int m0 = 0; m0 < M; m0 += 32) {
         const int mm = M - m0 < 32 ? M - m0 : 32;
         char *o = (char *)out + (size_t)m0 * N * osz;
         const char *a = (const char *)act + (size_t)m0 * K * esz;
-        if (resid) {
-            RC(mynn_b200_dequant_matmul_residual(st, o, a, w, scale, (const char *)resid + (size_t)m0 * N * osz, mm, N, K, dt,
-                                                 m.gemm_ws, m.gemm_ws_bytes));
-        } else {
-            RC(mynn_b200_dequant_matmul(st, o, a, w, scale, mm, N, K, dt, out_dtype, MYNN_W_NK, m.gemm_ws, m.gemm_ws_bytes));
-        }
+        const char *r = resid ? (const char *)resid + (size_t)m0 * N * osz : nullptr;
+        RC(launch_dequant_matmul(st, o, a, w, scale, r, mm, N, K, dt, resid ? dt : out_dtype, MYNN_W_NK, m.gemm_ws, m.gemm_ws_bytes, true));
     }
     return MYNN_OK;
 }
@@ -61,7 +57,7 @@ static int gemm(cudaStream_t st, const Model &m, void *out, const void *act, con
 // DequantMatMul whose activations a fused producer has already left as limbs in the GEMM workspace.
 static int gemm_prequant(cudaStream_t st, const Model &m, void *out, const int8_t *w, const void *scale, const void *resid,
                          int M, int N, int K, int out_dtype) {
-    return i8_gemm_launch(st, out, nullptr, w, scale, resid, M, N, K, m.c.dtype, out_dtype, m.gemm_ws, m.gemm_ws_bytes);
+    return i8_gemm_launch(st, out, nullptr, w, scale, resid, M, N, K, m.c.dtype, out_dtype, m.gemm_ws, m.gemm_ws_bytes, true);
 }
 
 // The same for more than 32 rows: two limbs per element in the layout of the prefill kernel.
@@ -102,7 +98,7 @@ static int enqueue_forward(Model &m, cudaStream_t st, int S, int head_rows = 0) 
     auto push = [&](int buf, const void *act, const int8_t *w, const void *scale, int K) -> int {  // row-parallel product
         int skip = 0, want = 2;
         if (g_inject_stall.compare_exchange_strong(want, 0)) skip = 1;  // test aid: this launch delivers nothing
-        return launch_tp_gemm_push(st, m.tp, buf, act, w, (const float *)scale, M, H, K, dt, m.gemm_ws, m.gemm_ws_bytes, skip);
+        return launch_tp_gemm_push(st, m.tp, buf, act, w, (const float *)scale, M, H, K, dt, m.gemm_ws, m.gemm_ws_bytes, true, skip);
     };
     auto reduce = [&](int buf, const void *w) -> int {  // fused reduction of the partial sums in buffer `buf`
         reduced_limbs = w != nullptr;

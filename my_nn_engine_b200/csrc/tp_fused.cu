@@ -183,7 +183,7 @@ tp_reduce_norm_limbs_kernel(int8_t *limbs, float *ascale, T *x, const T *w, floa
 }
 
 int launch_tp_gemm_push(cudaStream_t st, const TpPeers &peers, int buf, const void *act, const int8_t *wq, const float *scale, int M,
-                        int N, int K, int act_dtype, void *workspace, size_t workspace_bytes, int skip_delivery) {
+                        int N, int K, int act_dtype, void *workspace, size_t workspace_bytes, bool settled, int skip_delivery) {
     if (buf != 0 && buf != 1) return fail(MYNN_E_ARG, "tp push: buffer %d", buf);
     if (M < 1 || M > peers.lay.max_rows || N != peers.lay.hidden)
         return fail(MYNN_E_ARG, "tp push: M=%d N=%d do not fit a group of %d rows x %d", M, N, peers.lay.max_rows, peers.lay.hidden);
@@ -197,7 +197,7 @@ int launch_tp_gemm_push(cudaStream_t st, const TpPeers &peers, int buf, const vo
     t.max_rows = peers.lay.max_rows;
     for (int r = 0; r < peers.world; r++) t.part[r] = reinterpret_cast<uint32_t *>(peers.blocks[r] + peers.lay.part_off[buf]);
     t.skip = skip_delivery;
-    return i8_gemm_launch_tp(st, nullptr, act, wq, scale, nullptr, M, N, K, act_dtype, MYNN_F32, workspace, workspace_bytes, &t, nullptr, nullptr);
+    return i8_gemm_launch_tp(st, nullptr, act, wq, scale, nullptr, M, N, K, act_dtype, MYNN_F32, workspace, workspace_bytes, settled, &t, nullptr, nullptr);
 }
 
 int launch_tp_reduce_norm_limbs(cudaStream_t st, int dtype, const TpPeers &peers, int buf, void *workspace, size_t workspace_bytes,
@@ -282,7 +282,7 @@ extern "C" int mynn_b200_tp_dequant_matmul_push(void *stream, const mynn_b200_tp
     if (!dtype_ok(act_dtype)) return fail(MYNN_E_ARG, "tp_dequant_matmul_push: bad dtype %d", act_dtype);
     int skip = 0, want = 2;
     if (g_inject_stall.compare_exchange_strong(want, 0)) skip = 1;
-    return launch_tp_gemm_push((cudaStream_t)stream, peers, buffer, act, wq, scale, M, peers.lay.hidden, K, act_dtype, workspace, workspace_bytes, skip);
+    return launch_tp_gemm_push((cudaStream_t)stream, peers, buffer, act, wq, scale, M, peers.lay.hidden, K, act_dtype, workspace, workspace_bytes, false, skip);
 }
 
 extern "C" int mynn_b200_tp_reduce_norm(void *stream, const mynn_b200_tp_group *group, int buffer, void *x, const void *weight, float eps,

@@ -61,9 +61,9 @@ struct I8Tp {
 };
 
 // Row-parallel DequantMatMul whose f32 outputs go to every rank as partial sums.  act == nullptr: limbs already in
-// `workspace`.  skip_delivery (test aid): run the product but deliver nothing.
+// `workspace`.  settled: see i8_gemm.cuh.  skip_delivery (test aid): run the product but deliver nothing.
 int launch_tp_gemm_push(cudaStream_t st, const TpPeers &peers, int buf, const void *act, const int8_t *wq, const float *scale, int M,
-                        int N, int K, int act_dtype, void *workspace, size_t workspace_bytes, int skip_delivery);
+                        int N, int K, int act_dtype, void *workspace, size_t workspace_bytes, bool settled, int skip_delivery);
 // sum over ranks of the partial rows -> x = round(x + round(sum)); if w != null: y = round(RMSNorm(x) * w) -> limbs + row
 // scales in `workspace` (the DequantMatMul workspace of the product that follows).  after_push: the kernel in front of this
 // one on the stream is the delivering DequantMatMul of the same reduction (the two may then overlap).

@@ -1,0 +1,76 @@
+"""Operators queued one behind the other without a host synchronisation: what one writes is what the next reads, whichever operand it is."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from my_nn_engine_b200 import ffi, ops  # noqa: E402
+
+DT = {"bf16": torch.bfloat16, "f16": torch.float16}
+
+
+def randn(seed, *shape):
+    return torch.randn(*shape, generator=torch.Generator(device="cuda").manual_seed(seed), device="cuda")
+
+
+def quantise_into(q, s, zp, w):
+    ffi.check(ffi.lib().mynn_b200_dynamic_quantize_linear(ops._stream(), q.data_ptr(), s.data_ptr(), zp.data_ptr(), w.data_ptr(), *w.shape, 1, 1, ops._dt(w)))
+
+
+# rows of W: fewer than SMs, a ragged last wave, many waves; k of every form of the products and, at 8208, past the quantiser for short rows
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("n,k", [(64, 2048), (1000, 512), (1000, 8192), (1000, 8208), (5632, 2048), (20000, 4096)])
+def test_weights_quantised_right_in_front_of_the_product(dt, n, k):
+    """DynamicQuantizeLinear makes int8 rows and one scale per row, which is what DequantMatMul takes as weights.  One launch after the other,
+    with work in front so that the host is ahead, and replayed from a graph, the product has the bits of the synchronised sequence."""
+    w, other = randn(n, n, k).to(DT[dt]), randn(n + 1, n, k).to(DT[dt])
+    acts = [randn(m, m, k).to(DT[dt]) for m in (1, 2, 3, 5, 8, 32, 40)]
+    res = [randn(n + a.shape[0], a.shape[0], n).to(DT[dt]) for a in acts]
+    q, s, zp = ops.dynamic_quantize_linear(w)
+    torch.cuda.synchronize()
+    want = [(ops.dequant_matmul(a, q, s), ops.dequant_matmul_residual(a, q, s, r)) for a, r in zip(acts, res)]
+    torch.cuda.synchronize()
+    busy = randn(0, 4096, 4096)
+
+    def once():
+        got = []
+        for a, r in zip(acts, res):
+            quantise_into(q, s, zp, other)  # stale weights and scales for the next two
+            quantise_into(q, s, zp, w)
+            x = ops.dequant_matmul(a, q, s)
+            quantise_into(q, s, zp, other)
+            quantise_into(q, s, zp, w)
+            got.append((x, ops.dequant_matmul_residual(a, q, s, r)))
+        return got
+
+    for _ in range(3):
+        busy @ busy
+        for (x, y), (x0, y0) in zip(once(), want):
+            assert torch.equal(x, x0) and torch.equal(y, y0)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = once()
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    for (x, y), (x0, y0) in zip(got, want):
+        assert torch.equal(x, x0) and torch.equal(y, y0)
+
+
+@pytest.mark.parametrize("m", [1, 3, 8, 32])
+def test_second_matrix_quantised_right_in_front_of_its_product(m):
+    """dequant_matmul_same_act: the activations' limbs come from the call before, the weights from the kernel right in front."""
+    n, k = 1500, 2048
+    a, w1, w2 = randn(1, m, k).bfloat16(), randn(2, n, k).bfloat16(), randn(3, n, k).bfloat16()
+    q1, s1, _ = ops.dynamic_quantize_linear(w1)
+    q2, s2, zp = ops.dynamic_quantize_linear(w2)
+    torch.cuda.synchronize()
+    want = ops.dequant_matmul(a, q2, s2)
+    torch.cuda.synchronize()
+    busy = randn(0, 4096, 4096)
+    for _ in range(5):
+        busy @ busy
+        ops.dequant_matmul(a, q1, s1)
+        quantise_into(q2, s2, zp, w1)
+        quantise_into(q2, s2, zp, w2)
+        assert torch.equal(ops.dequant_matmul_same_act(a, q2, s2), want)

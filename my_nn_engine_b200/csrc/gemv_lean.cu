@@ -214,11 +214,9 @@ __global__ void __launch_bounds__(kLeanThreads, 1) gemv_lean_kernel(const LeanPa
     // settled: the first tiles of weights and the row scale of this thread's output depend on nothing an earlier kernel writes; else the
     // weights only travel to L2 ahead of the wait
     if (!p.settled) {
-        if (t == 0)
-            for (int row = gq; row < min(rows, 16 * TG); row += 8)
-#pragma unroll
-                for (int j = 0; j < NB; j++)
-                    if (c0 + 4 * j < chunks) prefetch_l2(p.wq + (size_t)(row0 + row) * K + 16 * (size_t)(c0 + 4 * j));
+        const int8_t *w0 = p.wq + (size_t)row0 * K;
+#pragma unroll 1
+        for (int i = 128 * threadIdx.x; i < min(rows, 16 * TG) * K; i += 128 * kLeanThreads) prefetch_l2(w0 + i);
         pdl_wait();
     }
 #pragma unroll

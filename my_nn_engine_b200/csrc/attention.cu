@@ -55,7 +55,8 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     constexpr int KCH = D / 32;  // 16-byte K chunks per lane per row
     constexpr int VH = D / 64;   // 16-byte V chunks per lane per row
     pdl_trigger();
-    if (!p.settled) pdl_wait();  // else only q and the newest kv row come from the preceding kernels
+    const bool settled = p.appended != nullptr;
+    if (!settled) pdl_wait();  // else only q and one kv row come from the preceding kernels
     const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int G = p.G;
@@ -111,11 +112,13 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
         __syncthreads();
-        // with a settled cache the tiles that do not hold the newest row set out while the projection in front still runs (with the
-        // fused append no tile does: the new row never comes from the cache)
+        // with a settled cache the tiles that do not hold the row being written set out while the projection in front still runs (with the
+        // fused append no tile counts: that row never comes from the cache)
         int j = 0;
-        if (lane == 0 && p.settled)
-            for (; j < min(ntile, kRingDepth) && (fused || first + 16 * W * j + 16 < active); j++) issue(j);
+        if (lane == 0 && settled) {
+            const int written = fused ? 0 : slot(*p.appended);
+            for (; j < min(ntile, kRingDepth) && (fused || (unsigned)(written - slot(first + 16 * W * j)) >= 16u); j++) issue(j);
+        }
         pdl_wait();
         if (lane == 0)
             for (; j < min(ntile, kRingDepth); j++) issue(j);
@@ -670,7 +673,7 @@ int mynn::launch_attention(cudaStream_t st, void *out, const void *q, const void
         p.sin_t = fuse->sin_t;
         p.fused_pos = fuse->pos;
         p.fused_row = fuse->row;
-        p.settled = fuse->settled;
+        p.appended = fuse->row;
     }
     if (int rc = decode_bind_workspace(p, B, D, workspace, workspace_bytes)) return rc;
     if (dtype == MYNN_BF16) return D == 64 ? launch_decode<__nv_bfloat16, 64>(st, p, B, ring) : launch_decode<__nv_bfloat16, 128>(st, p, B, ring);
@@ -707,7 +710,7 @@ int mynn::launch_window_attention_decode(cudaStream_t st, int dtype, const Windo
     p.chunk = w.chunk;
     p.ring_cache = 1;
     p.softcap = w.softcap;
-    p.settled = w.settled;
+    p.appended = w.appended;
     if (int rc = decode_bind_workspace(p, w.B, w.D, w.workspace, w.workspace_bytes)) return rc;
     if (dtype == MYNN_BF16) return w.D == 64 ? launch_decode<__nv_bfloat16, 64, true>(st, p, w.B, ring) : launch_decode<__nv_bfloat16, 128, true>(st, p, w.B, ring);
     return w.D == 64 ? launch_decode<__half, 64, true>(st, p, w.B, ring) : launch_decode<__half, 128, true>(st, p, w.B, ring);

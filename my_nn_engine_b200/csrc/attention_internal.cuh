@@ -117,9 +117,10 @@ struct DecodeParams {
     int window = 0, ring_cache = 0;
     int chunk = 0;  // and none before the query's own chunk of that many positions (counted from position 0)
     float softcap = 0.f;
-    // Of what the kernel reads, the kernels right in front of it write q and the newest key and value rows only: cached rows, positions and
-    // the active length may be read while they still run.
-    int settled = 0;
+    // A step of a model: of what the kernel reads, the kernels of the step in front of it write q and the key and value rows at position
+    // *appended (device; any position, not only the last visible one) only.  The other cached rows, positions and the active length may be
+    // read while they still run.  Null: nothing may.  (With the fused append the kernel writes that row itself.)
+    const int32_t *appended = nullptr;
     int wide = 0;           // host side: CTAs of more than four warps
     int *status = nullptr;  // ring kernel: where a timed-out wait is recorded (null: the library's own word, see attention_check)
 };

@@ -338,7 +338,7 @@ static int mix_attention(Model &m, cudaStream_t st, const BlockLayer &L, const B
     at.active = m.active_dev;
     at.workspace = m.attn_ws;
     at.workspace_bytes = m.attn_ws_bytes;
-    at.settled = 1;
+    at.appended = m.past_dev;
     at.status_word = (int *)m.gemm_ws;
     return launch_window_attention(st, dt, at);
 }

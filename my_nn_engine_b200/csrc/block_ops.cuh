@@ -83,7 +83,7 @@ struct WindowAttention {
     const int32_t *active = nullptr;   // device: positions written so far, the new rows included
     void *workspace = nullptr;
     size_t workspace_bytes = 0;
-    int settled = 0;                   // decode: the kernels right in front write q and the newest key and value rows, nothing else read here
+    const int32_t *appended = nullptr; // decode steps of a model, see DecodeParams
     int *status_word = nullptr;
 };
 int launch_window_attention(cudaStream_t st, int dtype, const WindowAttention &p);

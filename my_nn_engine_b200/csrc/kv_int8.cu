@@ -205,7 +205,8 @@ attention_decode_q8_kernel(const __grid_constant__ CUtensorMap map_k, const __gr
     __shared__ float sm_qinv[8];
 
     pdl_trigger();
-    if (!p.settled) pdl_wait();  // else only q and the newest kv row come from the preceding kernels
+    const bool settled = p.appended != nullptr;
+    if (!settled) pdl_wait();  // else only q and one kv row come from the preceding kernels
     const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int G = p.G;
@@ -252,11 +253,13 @@ attention_decode_q8_kernel(const __grid_constant__ CUtensorMap map_k, const __gr
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
         __syncthreads();
-        // The first copies travel while the query becomes limbs; with a settled cache those of tiles without the newest row set out while
-        // the kernels in front still run (5 sequences of 3000 rows: 17.3 us with the ring behind the query).
+        // The first copies travel while the query becomes limbs; with a settled cache those of tiles without the row being written
+        // set out while the kernels in front still run (5 sequences of 3000 rows: 17.3 us with the ring behind the query).
         int j = 0;
-        if (lane == 0 && p.settled)
-            for (; j < min(ntile, kQ8RingDepth) && first + 32 * kAttnWarps * j + 32 < active; j++) issue(j);
+        if (lane == 0 && settled) {
+            const int written = *p.appended;
+            for (; j < min(ntile, kQ8RingDepth) && (unsigned)(written - first - 32 * kAttnWarps * j) >= 32u; j++) issue(j);
+        }
         pdl_wait();
         if (lane == 0)
             for (; j < min(ntile, kQ8RingDepth); j++) issue(j);
@@ -643,7 +646,7 @@ int launch_dequant_kv_rows(cudaStream_t st, int dtype, void *out, const void *ca
 int launch_attention_q8(cudaStream_t st, void *out, const void *q, const void *k, const void *v, const void *k_scale,
                         const void *v_scale, float scale, int B, int Hq, int Hkv, int Sq, int D, int cache_seq_len,
                         int active_seq_kv, const int32_t *active_seq_kv_dev, int is_causal, int dtype, void *workspace,
-                        size_t workspace_bytes, int out_bshd, bool step) {
+                        size_t workspace_bytes, int out_bshd, const int32_t *appended) {
     if (B < 0 || Hq <= 0 || Hkv <= 0 || Sq < 0 || D <= 0 || cache_seq_len < 0 || active_seq_kv < 0)
         return fail(MYNN_E_ARG, "attention_q8: bad shape");
     if (Hq % Hkv != 0) return fail(MYNN_E_ARG, "attention_q8: %d query heads are not a multiple of %d kv heads", Hq, Hkv);
@@ -677,7 +680,7 @@ int launch_attention_q8(cudaStream_t st, void *out, const void *q, const void *k
     const int rows_bound = active_seq_kv_dev ? cache_seq_len : (active_seq_kv < cache_seq_len ? active_seq_kv : cache_seq_len);
     const bool ring = q8_ring_possible(p, B, D);
     p.splits = decode_splits(B, Hkv, rows_bound, 32, ring ? 2 : kAttnCtasPerSm);
-    p.settled = step;
+    p.appended = appended;
     if (int rc = decode_bind_workspace(p, B, D, workspace, workspace_bytes)) return rc;
     if (dtype == MYNN_BF16) return D == 64 ? launch_decode_q8<__nv_bfloat16, 64>(st, p, B, ring) : launch_decode_q8<__nv_bfloat16, 128>(st, p, B, ring);
     return D == 64 ? launch_decode_q8<__half, 64>(st, p, B, ring) : launch_decode_q8<__half, 128>(st, p, B, ring);

@@ -172,7 +172,7 @@ static int enqueue_forward(Model &m, cudaStream_t st, int S, int head_rows = 0) 
                                     c.max_seq_len, m.active_dev, 1, dt, m.attn_ws, m.attn_ws_bytes, 1));
             } else {
                 RC(launch_attention_q8(st, m.attn, m.q_rot, L.kc, L.vc, L.ksc, L.vsc, attn_scale, B, m.Hq, m.Hkv, S, D,
-                                       c.max_seq_len, c.max_seq_len, m.active_dev, S > 1, dt, m.attn_ws, m.attn_ws_bytes, 1, S == 1));
+                                       c.max_seq_len, c.max_seq_len, m.active_dev, S > 1, dt, m.attn_ws, m.attn_ws_bytes, 1, S == 1 ? m.past_dev : nullptr));
             }
         } else if (c.stream_window > 0) {
             // streaming cache: K is appended unrotated at the slot in past_dev; the live rows are rotated at their
@@ -194,7 +194,7 @@ static int enqueue_forward(Model &m, cudaStream_t st, int S, int head_rows = 0) 
             // that collects the heads (TinyLlama shapes, one sequence: 3.8 us for product and limbs against 2.2 + 3.5).
             if (tp == 1 && fuse_rope && gemv_lean_supported(M, H, Nq, L.wo)) attn_limbs = false;
             if (fuse_rope) {
-                const AttentionFuse fz = {kb, vb, qs, m.cos_t, m.sin_t, m.pos0_dev, m.past_dev, 1};  // the inputs' copy lies between two steps
+                const AttentionFuse fz = {kb, vb, qs, m.cos_t, m.sin_t, m.pos0_dev, m.past_dev};
                 RC(launch_attention(st, m.attn, qb, L.kc, L.vc, attn_scale, B, m.Hq, m.Hkv, S, D, c.max_seq_len, c.max_seq_len,
                                     m.active_dev, 0, dt, m.attn_ws, m.attn_ws_bytes, 1,
                                     attn_limbs ? (int8_t *)m.gemm_ws + 512 : nullptr, attn_limbs ? (float *)((char *)m.gemm_ws + 256) : nullptr, &fz,

@@ -34,12 +34,11 @@ int launch_rope_kv_append_q8(cudaStream_t st, int dtype, void *q_out, void *k_ca
                              const int64_t *positions, int B, int S, int Hq, int Hkv, int D, int cache_seq,
                              const int32_t *past_len_dev, int rotate_k = 1);
 
-// Attention over an int8 KV cache (per-token scales), with the output-layout choice of launch_attention.  step: a decode step of a model (see
-// DecodeParams::settled).
+// Attention over an int8 KV cache (per-token scales), with the output-layout choice of launch_attention.  appended: see DecodeParams.
 int launch_attention_q8(cudaStream_t st, void *out, const void *q, const void *k, const void *v, const void *k_scale,
                         const void *v_scale, float scale, int B, int Hq, int Hkv, int Sq, int D, int cache_seq_len,
                         int active_seq_kv, const int32_t *active_seq_kv_dev, int is_causal, int dtype, void *workspace,
-                        size_t workspace_bytes, int out_bshd, bool step = false);
+                        size_t workspace_bytes, int out_bshd, const int32_t *appended = nullptr);
 
 // out[m, f] = swish(gate[m, f]) * up[m, f] with gate/up rows `in_stride` elements apart.
 int launch_swiglu_strided(cudaStream_t st, int dtype, void *out, const void *gate, const void *up, int M, int F,
@@ -61,7 +60,6 @@ struct AttentionFuse {
     const void *cos_t, *sin_t;
     const int64_t *pos;
     const int32_t *row;
-    int settled;  // see DecodeParams
 };
 int launch_attention(cudaStream_t st, void *out, const void *q, const void *k, const void *v, float scale, int B,
                      int Hq, int Hkv, int Sq, int D, int cache_seq_len, int active_seq_kv,

@@ -74,3 +74,28 @@ def test_second_matrix_quantised_right_in_front_of_its_product(m):
         quantise_into(q2, s2, zp, w1)
         quantise_into(q2, s2, zp, w2)
         assert torch.equal(ops.dequant_matmul_same_act(a, q2, s2), want)
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(4, 2, 64), (4, 1, 128)])
+def test_int8_cache_row_rewritten_below_the_last_visible_one(heads, kv_heads, head_dim):
+    """A step may write a row in the middle of the rows it attends to (past_len below active_seq_kv - 1).  The row holds something else before
+    the first pass and its own bytes before the second, so the two agree only if the attention takes the row that the step wrote."""
+    from my_nn_engine_b200.decoder import DecoderModel
+    from my_nn_engine_b200.quantize import random_llama_state
+    cfg = dict(hidden_size=heads * head_dim, num_hidden_layers=3, num_attention_heads=heads, num_key_value_heads=kv_heads, head_dim=head_dim, intermediate_size=512,
+               vocab_size=300, rms_norm_eps=1e-5, rope_theta=1e4)
+    model = DecoderModel(cfg, random_llama_state(cfg, seed=1), dtype="bf16", max_seq_len=2048, batch=2, kv_int8=True)
+    for i in range(3):
+        for cache, scale in ((model.k_cache[i], model.k_scale[i]), (model.v_cache[i], model.v_scale[i])):
+            cache.copy_((randn(i, *cache.shape) * 40).clamp(-127, 127).to(torch.int8))
+            scale.fill_(0.02)
+    for past in (0, 31, 32, 700, 1023, 1030, 1999):
+        for i in range(3):
+            for cache, scale in ((model.k_cache[i], model.k_scale[i]), (model.v_cache[i], model.v_scale[i])):
+                cache[:, :, past] = 127
+                scale[:, :, past] = 3.0
+        torch.cuda.synchronize()
+        first = model.step([5, 7], past, 2000).clone()
+        for _ in range(3):
+            assert torch.equal(model.step([5, 7], past, 2000), first)
+    model.close()

@@ -507,11 +507,8 @@ template <typename T, int D, bool WIN, int W>
 static int launch_decode_ring(cudaStream_t st, const DecodeParams &p, int B, const CUtensorMap &mk, const CUtensorMap &mv) {
     constexpr size_t smem = (size_t)W * kRingDepth * 2 * (D / 64) * 16 * 128;
     auto kern = attention_decode_kernel<T, D, true, WIN, W>;
-    static bool attr_set = false;
-    if (!attr_set) {  // with the kernel's static shared memory every head_dim is past the 48 KB that need no opt-in
-        MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr_set = true;
-    }
+    static SmemLimit limit;  // with the kernel's static shared memory every head_dim is past the 48 KB that need no opt-in
+    MYNN_CUDA_OK(limit.raise((const void *)kern, smem));
     MYNN_CUDA_OK(launch_dependent(kern, dim3(p.splits, p.Hkv, B), dim3(W * 32), smem, st, mk, mv, p));
     MYNN_LAUNCH_OK("attention_decode_kernel");
     return MYNN_OK;

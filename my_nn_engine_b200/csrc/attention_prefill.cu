@@ -230,11 +230,8 @@ template <typename T, int D>
 static int launch_pfa(cudaStream_t st, const PrefillAttnParams &p, int B) {
     const size_t smem = (size_t)kPfaRows * D * 2 + 4 * (size_t)kPfaCols * D * 2;
     auto kern = attention_prefill_kernel<T, D>;
-    static bool attr_set = false;
-    if (!attr_set) {
-        MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr_set = true;
-    }
+    static SmemLimit limit;
+    MYNN_CUDA_OK(limit.raise((const void *)kern, smem));
     kern<<<dim3((p.Sq + kPfaRows - 1) / kPfaRows, p.Hq, B), kPfaThreads, smem, st>>>(p);
     MYNN_LAUNCH_OK("attention_prefill_kernel");
     return MYNN_OK;

@@ -778,11 +778,8 @@ template <typename T, int D, bool WIN>
 static int launch_tc(cudaStream_t st, const CUtensorMap &mq, const CUtensorMap &mk, const CUtensorMap &mv, const TcAttnParams &p, int B) {
     constexpr size_t smem = (size_t)(D / 64) * kTcSlab * (1 + 4) + 2 * kTcSlab + 1024;  // Q, 2 x (K, V), P, alignment slack
     auto kern = attention_prefill_tc_kernel<T, D, WIN>;
-    static bool attr_set = false;
-    if (!attr_set) {
-        MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr_set = true;
-    }
+    static SmemLimit limit;
+    MYNN_CUDA_OK(limit.raise((const void *)kern, smem));
     TcAttnParams q = p;
     q.n_qt = (p.Sq + kTcRows - 1) / kTcRows;
     q.heads_per_grid = p.Hq;
@@ -796,11 +793,8 @@ template <typename T, int D, bool WIN>
 static int launch_tc2(cudaStream_t st, const CUtensorMap &mq, const CUtensorMap &mk, const CUtensorMap &mv, const TcAttnParams &p, int B) {
     constexpr size_t smem = (size_t)(D / 64) * kTcSlab * 6 + 1024;  // 2 x Q, 2 x K, 2 x V, alignment slack
     auto kern = attention_prefill_tc2_kernel<T, D, WIN>;
-    static bool attr_set = false;
-    if (!attr_set) {
-        MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr_set = true;
-    }
+    static SmemLimit limit;
+    MYNN_CUDA_OK(limit.raise((const void *)kern, smem));
     TcAttnParams q = p;
     q.n_qt = (p.Sq + kTcRows - 1) / kTcRows;
     q.heads_per_grid = p.Hq / 2;

@@ -12,6 +12,7 @@
 #include <cstdio>
 
 #include "../../include/mynn_b200.h"
+#include "smem_limit.h"
 
 namespace mynn {
 

@@ -274,11 +274,8 @@ template <typename T, typename O, bool GLU>
 static int launch_dg(cudaStream_t st, const CUtensorMap &ma, const CUtensorMap &mw, const DgParams &p, long long tiles_bound) {
     constexpr size_t smem = (size_t)kDgStages * kDgStageBytes + 1024;
     auto kern = dense_gemm_tc_kernel<T, O, GLU>;
-    static bool attr_set = false;
-    if (!attr_set) {
-        MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr_set = true;
-    }
+    static SmemLimit limit;
+    MYNN_CUDA_OK(limit.raise((const void *)kern, smem));
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -328,11 +328,8 @@ template <typename OutT, int M, int NB, int TG, bool ACT>
 static int launch_lean(cudaStream_t st, LeanParams p) {
     const size_t smem = lean_smem(ACT, M, p.K);
     auto kern = gemv_lean_kernel<OutT, M, NB, TG, ACT>;
-    static bool attr_set = false;
-    if (!attr_set) {
-        MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kLeanMaxSmem));
-        attr_set = true;
-    }
+    static SmemLimit limit;
+    MYNN_CUDA_OK(limit.raise((const void *)kern, kLeanMaxSmem));
     static int sms = 0;
     if (sms == 0) {
         int dev = 0;

@@ -877,11 +877,8 @@ static int launch_i8(cudaStream_t st, const CUtensorMap &mw, const CUtensorMap &
     constexpr uint32_t kStageBytes = kTileRows * kBlockK + ((NC * kBlockK + 1023) / 1024) * 1024;
     const size_t smem = (size_t)p.stages * kStageBytes + 1024;
     auto kern = i8_stream_gemm_kernel<OutT, NC>;
-    static bool attr_set = false;
-    if (!attr_set) {
-        MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kMaxStages * kStageBytes + 1024)));
-        attr_set = true;
-    }
+    static SmemLimit limit;
+    MYNN_CUDA_OK(limit.raise((const void *)kern, kMaxStages * kStageBytes + 1024));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((p.N + kTileRows - 1) / kTileRows, S, 1);
     cfg.blockDim = dim3(kGemmThreads, 1, 1);

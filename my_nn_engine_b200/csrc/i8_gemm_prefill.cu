@@ -517,11 +517,8 @@ template <typename OutT, int LIMBS>
 static int launch_pf(cudaStream_t st, const CUtensorMap &mw, const CUtensorMap &ma, const PfParams &p) {
     const size_t smem = (size_t)kPfStages * kPfStageBytes + 1024;
     auto kern = i8_prefill_gemm_kernel<OutT, LIMBS>;
-    static bool attr_set = false;
-    if (!attr_set) {
-        MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr_set = true;
-    }
+    static SmemLimit limit;
+    MYNN_CUDA_OK(limit.raise((const void *)kern, smem));
     const int tiles = p.w_tiles * p.t_tiles, sms = pf_sms();
     MYNN_CUDA_OK(launch_dependent(kern, dim3(tiles < sms ? tiles : sms), dim3(kPfThreads), smem, st, mw, ma, p));
     MYNN_LAUNCH_OK("i8_prefill_gemm_kernel");

@@ -589,11 +589,8 @@ static int launch_decode_q8(cudaStream_t st, const DecodeParams &p, int B, bool 
             if (int rc = make_map(&mv, p.v, rows, D, D, 32)) return rc;
             constexpr size_t smem = (size_t)kAttnWarps * kQ8RingDepth * 2 * 32 * 128;
             auto kern = attention_decode_q8_kernel<T, D, true>;
-            static bool attr_set = false;
-            if (!attr_set) {
-                MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-                attr_set = true;
-            }
+            static SmemLimit limit;
+            MYNN_CUDA_OK(limit.raise((const void *)kern, smem));
             MYNN_CUDA_OK(launch_dependent(kern, dim3(p.splits, p.Hkv, B), dim3(kAttnWarps * 32), smem, st, mk, mv, p));
             MYNN_LAUNCH_OK("attention_decode_q8_kernel");
             return MYNN_OK;

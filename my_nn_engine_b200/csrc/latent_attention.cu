@@ -395,11 +395,8 @@ static int run_latent(cudaStream_t st, const LatParams &l, int queries) {
     constexpr size_t smem = sizeof(LatSmem<T, R, MT>);
     static_assert(smem <= 227 * 1024, "shared memory of a CTA");
     auto kern = latent_attention_kernel<T, R, MT>;
-    static bool attr_set = false;
-    if (!attr_set) {
-        MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr_set = true;
-    }
+    static SmemLimit limit;
+    MYNN_CUDA_OK(limit.raise((const void *)kern, smem));
     MYNN_CUDA_OK(launch_dependent(kern, dim3(l.splits, queries, l.groups), dim3(lat_warps(R) * 32), smem, st, l));
     MYNN_LAUNCH_OK("latent_attention_kernel");
     if (l.splits > 1) {

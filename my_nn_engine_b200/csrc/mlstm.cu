@@ -578,11 +578,8 @@ static int run_chunk_pass(cudaStream_t st, const MlstmStep &p, const ChunkWs &w)
     constexpr size_t smem = sizeof(ChunkSmem<T, KD, OUT>);
     static_assert(smem <= 227 * 1024, "shared memory of a CTA");
     auto kern = mlstm_chunk_kernel<T, KD, OUT>;
-    static bool attr_set = false;
-    if (!attr_set) {
-        MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr_set = true;
-    }
+    static SmemLimit limit;
+    MYNN_CUDA_OK(limit.raise((const void *)kern, smem));
     kern<<<dim3((p.E + kChunkCols - 1) / kChunkCols, p.H, p.B * (OUT ? w.segments : w.segments - 1)), kChunkThreads, smem, st>>>(p, w);
     MYNN_LAUNCH_OK("mlstm_chunk_kernel");
     return MYNN_OK;

@@ -431,11 +431,8 @@ static int run_mt(cudaStream_t st, const MlstmStep &p, const ChunkWs &w) {
     constexpr size_t smem = MtLayout<KD, OUT>::kBytes + 1024;
     static_assert(smem + 10 * 1024 <= 227 * 1024, "shared memory of a CTA");
     auto kern = mlstm_tc_kernel<T, KD, OUT>;
-    static bool attr_set = false;
-    if (!attr_set) {
-        MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr_set = true;
-    }
+    static SmemLimit limit;
+    MYNN_CUDA_OK(limit.raise((const void *)kern, smem));
     CUtensorMap map;
     const uint64_t row = (uint64_t)2 * p.H * (p.D + p.E) * 2;
     if (int rc = make_map(&map, p.proj, (uint64_t)p.B * p.S, row, row, kChunk)) return rc;
@@ -448,11 +445,8 @@ template <typename T, int KD>
 static int run_prepare(cudaStream_t st, const MlstmStep &p, const ChunkWs &w) {
     constexpr size_t smem = 2 * (KD / 64) * kMtSlab + 1024;
     auto kern = mlstm_prepare_kernel<T, KD>;
-    static bool attr_set = false;
-    if (!attr_set) {
-        MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr_set = true;
-    }
+    static SmemLimit limit;
+    MYNN_CUDA_OK(limit.raise((const void *)kern, smem));
     kern<<<dim3(w.chunks, p.H, p.B), 256, smem, st>>>(p, w);
     MYNN_LAUNCH_OK("mlstm_prepare_kernel");
     return MYNN_OK;

@@ -34,9 +34,15 @@ def _ptr(t):
     return t.data_ptr()
 
 
+# torch's own short way to the current stream, where this build of it has one
+_raw_stream, _device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+
+
 def _stream():
     """The current stream of the current device, without building a Stream object (a call of a small operator is bound by its host time)."""
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    if _raw_stream is None or _device is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_device())
 
 
 _gemm_ws: dict = {}

@@ -539,7 +539,8 @@ int mynn_b200_moe_matmul(void *stream, void *out, const void *act, const void *w
                          int K, int experts, int top, int gather, int glu, int dtype, int out_dtype, int32_t *status);
 
 /* How many CTAs the 16-bit decode attention kernel lets share the kv rows of one (batch, kv head) pair, given an upper bound
- * of the rows and the number of CTAs of that kernel an SM holds (2 for the ring form at head_dim 128, else 4).  Pure host
+ * of the rows and the number of CTAs of that kernel an SM holds (2 for the ring form at head_dim 128, else 4).  This is the
+ * operator's plan; a model's step of few pairs takes CTAs of more warps and fewer of them.  Pure host
  * arithmetic, exported so that an integrator can see what mynn_b200_attention_workspace_bytes is sized for. */
 int mynn_b200_attention_decode_splits(int B, int Hkv, int rows_bound, int ctas_per_sm);
 

@@ -157,3 +157,41 @@ def test_dense_products(M, N, K):
     act, w, status = randn(g, M, K).bfloat16(), randn(g, N, K).bfloat16(), torch.zeros(1, dtype=torch.int32, device="cuda")
     want = act.double() @ w.double().t()
     assert (ops.dense_matmul(act, w, status=status).double() - want).abs().max() <= 2.0 ** -8 * want.abs().max()
+
+
+# ---- decode attention that rotates and appends the new row itself: wide CTAs, several splits, the new row around their borders ----
+@pytest.mark.parametrize("head_dim,kv_heads,batch", [(64, 1, 1), (64, 2, 3), (128, 1, 1), (128, 2, 2)])
+def test_fused_append_over_a_long_cache(head_dim, kv_heads, batch):
+    """Against the rotation and append in front of the attention, over caches whose rows are given.  Few pairs and 4096 rows: eight warps (head_dim
+    128) and sixteen (64), eight and four splits of 4096 rows, rounds of 128 and 256; the contexts put the new row on both sides of warp, round and split borders."""
+    from my_nn_engine_b200 import ffi
+    from my_nn_engine_b200.decoder import DecoderModel
+    from my_nn_engine_b200.quantize import random_llama_state
+    cfg = dict(hidden_size=256, num_hidden_layers=1, num_attention_heads=4 * kv_heads, num_key_value_heads=kv_heads, head_dim=head_dim, intermediate_size=256,
+               vocab_size=300, rms_norm_eps=1e-5, rope_theta=1e4)
+    state, g = random_llama_state(cfg, seed=2), gen(head_dim)
+    shape = (batch, kv_heads, 4096, head_dim)
+    k, v = randn(g, *shape).bfloat16(), randn(g, *shape).bfloat16()
+    edges = [0, 15, 16, 63, 64, 65, 127, 128, 255, 256, 257, 511, 512, 1023, 1024, 1025, 1151, 1152, 2047, 2048, 2049, 4080, 4094]
+    runs = []
+    try:
+        for fuse in (0, 1):
+            ffi.set_option(ffi.OPT_FUSE_ROPE, fuse)
+            model = DecoderModel(cfg, state, dtype="bf16", max_seq_len=4096, batch=batch)
+            rows = []
+            for past in edges:
+                model.k_cache[0].copy_(k), model.v_cache[0].copy_(v)
+                torch.cuda.synchronize()
+                rows.append(model.step(np.arange(batch) + past % 200, past).float().clone())
+                rows.append((model.k_cache[0].clone(), model.v_cache[0].clone()))
+            runs.append(rows)
+            model.close()
+    finally:
+        ffi.set_option(ffi.OPT_FUSE_ROPE, 1)
+    for i, past in enumerate(edges):
+        # one layer: the appended rows are the same bits; the softmax sums in another order, and what a rounding of the attention to bf16 does to
+        # the logits stays within a few of theirs
+        (a, b), (ca, cb) = (r[2 * i] for r in runs), (r[2 * i + 1] for r in runs)
+        assert torch.equal(ca[0], cb[0]) and torch.equal(ca[1], cb[1]), past
+        assert not torch.equal(ca[0][:, :, past], k[:, :, past]) and torch.equal(ca[0][:, :, past + 1:], k[:, :, past + 1:])
+        assert (a - b).abs().max() <= 8 * 2.0 ** -7 * a.abs().max(), past

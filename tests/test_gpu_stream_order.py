@@ -99,3 +99,46 @@ def test_int8_cache_row_rewritten_below_the_last_visible_one(heads, kv_heads, he
         for _ in range(3):
             assert torch.equal(model.step([5, 7], past, 2000), first)
     model.close()
+
+
+def llama(kv_int8, use_graph):
+    from my_nn_engine_b200.decoder import DecoderModel
+    from my_nn_engine_b200.quantize import random_llama_state
+    cfg = dict(hidden_size=256, num_hidden_layers=4, num_attention_heads=2, num_key_value_heads=1, head_dim=128, intermediate_size=512, vocab_size=300,
+               rms_norm_eps=1e-5, rope_theta=1e4)
+    state = random_llama_state(cfg, seed=1)
+    return 300, lambda: DecoderModel(cfg, state, dtype="bf16", max_seq_len=512, batch=2, kv_int8=kv_int8, use_graph=use_graph)
+
+
+def blocks(family, name, use_graph):
+    from my_nn_engine_b200 import fimadra, vebisun
+    from tests import block_models as bm
+    from tests import fimadra_models as fm
+    lib, models = (fimadra, fm) if family == "fimadra" else (vebisun, bm)
+    cfg = getattr(models, name)()
+    state = models.weights(cfg, seed=1)
+    return cfg["vocab"], lambda: lib.build(cfg, state, dtype="bf16", max_seq_len=512, batch=2, use_graph=use_graph)
+
+
+@pytest.mark.parametrize("use_graph", [False, True])
+@pytest.mark.parametrize("make", [lambda g: llama(False, g), lambda g: llama(True, g), lambda g: blocks("vebisun", "even_group", g), lambda g: blocks("vebisun", "odd_group", g),
+                                  lambda g: blocks("fimadra", "chunkwise", g), lambda g: blocks("fimadra", "wide", g)])
+def test_queued_steps_equal_synchronised_ones(make, use_graph):
+    """What a step reads ahead of its kernels (cached rows, memories, conv history, positions) is what the step before it has left, also when
+    the steps are queued one behind the other."""
+    vocab, build = make(use_graph)
+    steps = 300
+    ids = torch.randint(0, vocab, (steps, 2), generator=torch.Generator().manual_seed(3)).cuda()
+    outs, stream = [], torch.cuda.Stream()
+    for synchronise in (True, False):
+        model = build()
+        out = torch.empty(steps, 2, vocab, dtype=model._logits_dtype, device="cuda")
+        torch.cuda.synchronize()
+        for i in range(steps):
+            model.step_device(ids[i], i, out[i], stream.cuda_stream)
+            if synchronise:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        outs.append(out)
+        model.close()
+    assert torch.isfinite(outs[0].float()).all() and torch.equal(outs[0], outs[1])

@@ -495,7 +495,8 @@ static int decode_ctas_per_sm(bool ring, int D) { return ring && D == 128 ? 2 : 
 
 // Few (batch, kv head) pairs leave SMs without a CTA, and then the time is the number of rounds its warps take one after the other (0.85 us
 // each) plus, with splits, the merge through L2 (2.5 us).  Up to half as many pairs as SMs take CTAs of twice (head_dim 128; registers) or
-// four times the warps (head_dim 64), whose round is as many times longer, so that up to 512 / 1024 rows need no split.  A model's steps
+// four times the warps (head_dim 64), whose round is as many times longer, so that fewer than 1024 / 2048 rows (decode_splits: four rounds a split)
+// need no split; rows are those of the cache or window, since the live ones are known on the device only.  A model's steps
 // do; the operator by itself keeps four warps, with which its ring and its direct form give the same bits.
 constexpr int decode_wide_warps(int D) { return D == 64 ? 16 : 8; }
 static void decode_plan(DecodeParams &p, bool ring, bool step, int B, int D, int rows_bound) {
@@ -527,7 +528,7 @@ static int launch_decode(cudaStream_t st, const DecodeParams &p, int B, bool rin
         return p.wide ? launch_decode_ring<T, D, WIN, decode_wide_warps(D)>(st, p, B, mk, mv)
                       : launch_decode_ring<T, D, WIN, kAttnWarps>(st, p, B, mk, mv);
     }
-    MYNN_CUDA_OK(launch_pdl(attention_decode_kernel<T, D, false, WIN, kAttnWarps>, dim3(p.splits, p.Hkv, B), dim3(kAttnWarps * 32), 0, st, mk, mv, p));
+    MYNN_CUDA_OK(launch_plain(attention_decode_kernel<T, D, false, WIN, kAttnWarps>, dim3(p.splits, p.Hkv, B), dim3(kAttnWarps * 32), 0, st, mk, mv, p));
     MYNN_LAUNCH_OK("attention_decode_kernel");
     return MYNN_OK;
 }

@@ -116,7 +116,7 @@ extern std::atomic<int> g_inject_stall;  // see MYNN_OPT_INJECT_STALL; consumed 
 
 // A plain launch through cudaLaunchKernelEx (no attributes): everything in front has completed when it starts.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+inline cudaError_t launch_plain(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -127,7 +127,7 @@ inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, siz
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
-// A launch that may begin while the kernel in front of it drains; the kernel itself waits (pdl_wait) before it touches memory.
+// A launch that may begin while the kernel in front of it drains; what the kernel may do before its pdl_wait stands above.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
     cudaLaunchAttribute attr[1];

@@ -316,10 +316,12 @@ __global__ void __launch_bounds__(kLeanThreads, 1) gemv_lean_kernel(const LeanPa
 constexpr int kLeanMaxSmem = 226 * 1024;
 static size_t lean_smem(bool act, int M, int K) { return (act ? (size_t)3 * M * lean_limb_pitch(K) : 0) + (size_t)kLeanWarps * 3 * M * kLeanPitch * sizeof(int); }
 
-// Up to two rows any matrix that was measured (28672 x 4096 as an operator at one row: 20 us against 25 us with the tcgen05 kernel and its
-// pre-pass; a Llama-3-8B step of two sequences 2554 -> 2331 us).  Three to five rows fill two column tiles and the finish has that much more to
-// do: up to 32 MB (Llama-3-8B at five rows: norm and qkv 10.4 -> 8.8 us), above that the tcgen05 kernel (gate/up at five rows 19 us, 36 us
-// here).
+// Up to two rows all matrices of a layer (28672 x 4096, 112 MB, as an operator at one row: 20.5 us against 23.5 us with the tcgen05 kernel and
+// its pre-pass; Llama-3-8B steps of one and two sequences over 1000 rows 2356 -> 2232 and 2342 -> 2265 us).  The line at 160 MB lies above the
+// largest of them.  What lies beyond are heads of large vocabularies: 128256 x 4096, 501 MB, by itself 79 against 85 us, but nothing in the
+// same two steps (2229 and 2267 us), so it stays where the pre-pass and the tiles are the smaller part.
+// Three to five rows fill two column tiles and the finish has that much more to do: up to 32 MB (Llama-3-8B at five rows: norm and qkv 10.4 ->
+// 8.8 us), above that the tcgen05 kernel (a step of five sequences 2577 us, 3324 us with gate/up and head here; gate/up 19 and 36 us).
 bool gemv_lean_supported(int M, int N, int K, const void *wq) {
     return M >= 1 && M <= kLeanMaxRows && K >= 16 && K % 16 == 0 && K <= 6144 && (size_t)N * K <= ((size_t)(M <= 2 ? 160 : 32) << 20) && ((uintptr_t)wq % 16) == 0;
 }

@@ -322,7 +322,7 @@ int launch_rope_kv_append(cudaStream_t st, int dtype, void *q_out, void *k_cache
     }
     const int threads = D / 2 >= 64 ? 64 : 32;
     MYNN_DISPATCH_DTYPE(dtype, T, {
-        MYNN_CUDA_OK(launch_pdl(rope_kv_append_kernel<T>, dim3(B * S, Hq + 2 * Hkv), dim3(threads), 0, st, (T *)q_out, (T *)k_cache,
+        MYNN_CUDA_OK(launch_plain(rope_kv_append_kernel<T>, dim3(B * S, Hq + 2 * Hkv), dim3(threads), 0, st, (T *)q_out, (T *)k_cache,
                                 (T *)v_cache, (const T *)q, (const T *)k, (const T *)v, q_stride, k_stride, v_stride,
                                 (const T *)cos_t, (const T *)sin_t, positions, S, Hq, Hkv, D, cache_seq, past_len_dev, rotate_k));
     });

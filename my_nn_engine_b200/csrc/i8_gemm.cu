@@ -908,7 +908,7 @@ int launch_act_limbs(cudaStream_t st, const void *act, int M, int K, int act_dty
         if (smem > 48 * 1024) MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
         MYNN_CUDA_OK(launch_dependent(kern, dim3(M), dim3(kRowThreads), smem, st, limbs, ascale, (const T *)act, K));    \
     } else {                                                                                                             \
-        MYNN_CUDA_OK(launch_pdl(act_to_limbs_kernel<T>, dim3(M), dim3(256), 0, st, limbs, ascale, (const T *)act, K));   \
+        MYNN_CUDA_OK(launch_plain(act_to_limbs_kernel<T>, dim3(M), dim3(256), 0, st, limbs, ascale, (const T *)act, K));   \
     }
     switch (act_dtype) {
         case MYNN_BF16: PREP(__nv_bfloat16) break;

@@ -596,7 +596,7 @@ static int launch_decode_q8(cudaStream_t st, const DecodeParams &p, int B, bool 
             return MYNN_OK;
         }
     }
-    MYNN_CUDA_OK(launch_pdl(attention_decode_q8_kernel<T, D, false>, dim3(p.splits, p.Hkv, B), dim3(kAttnWarps * 32), 0, st, mk, mv, p));
+    MYNN_CUDA_OK(launch_plain(attention_decode_q8_kernel<T, D, false>, dim3(p.splits, p.Hkv, B), dim3(kAttnWarps * 32), 0, st, mk, mv, p));
     MYNN_LAUNCH_OK("attention_decode_q8_kernel");
     return MYNN_OK;
 }

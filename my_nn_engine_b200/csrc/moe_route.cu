@@ -65,8 +65,8 @@ __device__ __forceinline__ void warp_argmax(unsigned &key, int &i) {
 
 // The choice for one token by one warp; z: room for its E logits in shared memory.  Slot s: expert in lane s's `e`, weight in `w`.
 // NU: logits per lane (E <= 32 NU), in registers as ordered integers, so that a slot costs two warp reductions: at one token the choice
-// is a chain of `keep + top` of them and nothing else (eight of 64 experts out of four of eight groups: 7.7 us with five shuffle steps of value and index over
-// shared memory, 4.3 us so).
+// is a chain of `keep + top` of them and nothing else (eight of 64 experts out of four of eight groups: 9.1 us for the whole kernel, one after the other in a graph,
+// with five shuffle steps of value and index over shared memory, 5.8 us so).
 template <int NU>
 __device__ __forceinline__ void choose(float *z, const float *src, int E, int top, int groups, int keep, int &e_out, float &w_out) {
     const int lane = threadIdx.x & 31;

@@ -203,7 +203,7 @@ static int launch_streaming_typed(cudaStream_t st, void *out, const void *q, con
                                   const int64_t *kv_position, int out_bshd) {
     const unsigned blocks = (unsigned)((long long)B * Hq * Sq);
 #define GEN(MAXE)                                                                                                                       \
-    MYNN_CUDA_OK(launch_pdl(attention_streaming_kernel<T, TKV, MAXE>, dim3(blocks), dim3(kStreamWarps * 32), 0, st, (T *)out, (const T *)q, \
+    MYNN_CUDA_OK(launch_plain(attention_streaming_kernel<T, TKV, MAXE>, dim3(blocks), dim3(kStreamWarps * 32), 0, st, (T *)out, (const T *)q, \
                             (const TKV *)k, (const TKV *)v, (const T *)k_scale, (const T *)v_scale, scale, Hq, Hkv, Sq, D, cache_seq, active, \
                             active_dev, causal, rs, rw, r0, (const T *)cos_t, (const T *)sin_t, (const long long *)kv_position, out_bshd))
     if (D <= 32) GEN(1);

@@ -127,20 +127,29 @@ inline cudaError_t launch_plain(void (*kern)(KArgs...), dim3 grid, dim3 block, s
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
-// A launch that may begin while the kernel in front of it drains; what the kernel may do before its pdl_wait stands above.
+// A launch that may begin while the kernel in front of it drains; what the kernel may do before its pdl_wait stands above.  Clusters of
+// `cluster` CTAs along x.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
-    cudaLaunchAttribute attr[1];
+inline cudaError_t launch_dependent_cluster(unsigned cluster, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+    return launch_dependent_cluster(1, kern, grid, block, smem, st, args...);
 }
 
 // Dispatch a launcher template over the three storage dtypes.

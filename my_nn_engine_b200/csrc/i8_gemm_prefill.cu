@@ -8,12 +8,19 @@
 // int32 accumulation, [N weight rows] x [2 x tokens] x K, and the int8 pipe runs at twice the bf16 rate, so two limbs
 // cost the same tensor time as one bf16 product.
 //
-// Kernel: persistent CTAs (one per SM), tile = 128 weight rows x up to 128 tokens (256 limb columns), UMMA M=128 N<=256 K=32;
-// warp 0 streams weight and limb tiles by TMA through a 4-stage mbarrier ring (48 KB per stage), warp 1 issues the
-// MMAs into one of two 256-column TMEM accumulators, warps 2-9 drain the other accumulator (tcgen05.ld), recombine
+// Kernel: persistent pairs of CTAs (clusters of two, one CTA per SM), tile = 256 weight rows x up to 128 tokens (256 limb columns), UMMA
+// cta_group::2 M=256 N<=256 K=32.  Each CTA of a pair owns 128 of the weight rows, and brings them and half of the limb rows to its
+// shared memory: 32 KB per 128 of K where a CTA on its own needs 48.  That is what bounds this kernel: an SM gets about 64 bytes per clock from
+// L2 (220 ns per stage of 128 columns, 24 KB, and of 332 ns, 32 KB, at the clock that full tiles leave), and at the int8 rate of 128 x 256 x 32
+// per 128 clocks a CTA alone would take in 96.  Full tiles run at the power cap.
+// 2048 rows: 28672 x 4096 325 -> 272 us (3.54 POP/s), 4096 x 14336 198 -> 166, 6144 x 4096 76 -> 69, 4096 x 4096 52 -> 48; one limb,
+// 777 rows of 14336 x 4096, 48 -> 36.  About half of it came from walking the two issuing loops with whole warps (see elect_one).
+// Warp 0 of both CTAs streams by TMA through a ring of six to nine mbarrier stages, warp 1 of the first issues the MMAs of both into one
+// of two 256-column TMEM accumulators, warps 2-9 of both drain the other accumulator (tcgen05.ld), recombine
 // the limbs, scale, add the optional residual and store -- so the epilogue of one tile overlaps the main loop of the
 // next.  Tiles are walked with the token tile fastest, so concurrently running CTAs share weight tiles in L2.
 // All waits are bounded and report through the workspace status word.
+#include <algorithm>
 #include <type_traits>
 
 #include "common.cuh"
@@ -24,14 +31,14 @@ namespace mynn {
 
 MYNN_DEFINE_WAIT_BUDGET_SETTER(i8_gemm_prefill)
 
-constexpr int kPfRows = 128;      // weight rows per tile (UMMA M)
+constexpr int kPfRows = 128;      // weight rows of one CTA of a pair (half of UMMA M)
 constexpr int kPfCols = 256;      // most accumulator columns per tile (UMMA N): LIMBS columns per activation row
 constexpr int kPfBlockK = 128;
-constexpr int kPfStages = 4;
+constexpr int kPfMaxStages = 9;
 constexpr int kPfEpiWarps = 8;    // two per TMEM lane quadrant
 constexpr int kPfThreads = 64 + 32 * kPfEpiWarps;
-constexpr uint32_t kPfWBytes = kPfRows * kPfBlockK, kPfABytes = kPfCols * kPfBlockK;
-constexpr uint32_t kPfStageBytes = kPfWBytes + kPfABytes;  // 48 KB
+constexpr uint32_t kPfWBytes = kPfRows * kPfBlockK;
+constexpr uint32_t kPfRingBytes = 216 * 1024;  // six stages of 256 columns (32 KB in each CTA), nine of up to 128
 
 // ---- pre-pass: rows -> two int8 limbs + power-of-two row scale ----------------------------------------------------
 // limbs [(2m + l)][K]; with max |row| < 2^e the row is scaled by 2^(14-e), so |A| <= 2^14 and the high limb is within
@@ -234,8 +241,9 @@ struct PfParams {
     const void *ascale_t;   // QuantizedMatMul: lhs scales in the output dtype, element m * ascale_stride
     int ascale_stride;      // 1 = one scale per row, 0 = one scale for the whole tensor
     int M, N, K;
-    int cols;             // accumulator columns per tile, a multiple of 16
-    int w_tiles, t_tiles, t_full;  // t_full: token tiles that have all their rows
+    int stages;           // of the ring
+    int cols;             // accumulator columns per tile, a multiple of 32
+    int w_tiles, t_tiles, t_full;  // weight tiles (of a pair), token tiles, token tiles that have all their rows
     int *status;
 };
 
@@ -252,7 +260,7 @@ __device__ __forceinline__ void pf_place(const PfParams &p, int tile, int &wt, i
     }
 }
 
-// grid = min(#SMs, #tiles) persistent CTAs that walk the tiles with stride gridDim.x.
+// min(#SMs / 2, #tiles) persistent pairs of CTAs that walk the tiles with stride gridDim.x / 2.
 // LIMBS = 2: DequantMatMul, limb rows (2m + l), up to 128 activation rows per tile.
 // LIMBS = 1: QuantizedMatMul (W8A8), the int8 lhs matrix itself is the operand, up to 256 activation rows per tile.
 template <typename OutT, int LIMBS>
@@ -260,99 +268,116 @@ __global__ void __launch_bounds__(kPfThreads, 1)
 i8_prefill_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const PfParams p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    __shared__ uint64_t full_bar[kPfStages], empty_bar[kPfStages], acc_full[2], acc_empty[2];
+    __shared__ uint64_t full_bar[kPfMaxStages], empty_bar[kPfMaxStages], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
     __shared__ __align__(16) float sh_ascale[2][kPfCols / LIMBS];
     __shared__ int sh_go[2];
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_ctarank();
+    const int first_tile = blockIdx.x >> 1, tile_stride = gridDim.x >> 1;
     const int n_tiles = p.w_tiles * p.t_tiles, tok = p.cols / LIMBS;  // tok: activation rows per tile
+    // N of a tile's MMA = the accumulator columns the tile really has (rows past M are zero-filled by TMA and need no tensor time), rounded
+    // up to the instruction's granularity of 32; the first CTA holds the first half of them as B's rows, the second the other
+    const uint32_t stage_bytes = kPfWBytes + (uint32_t)p.cols * (kPfBlockK / 2);
+    auto tile_cols = [&](int tt) { return min(p.cols, (((p.M - tt * tok) * LIMBS + 31) >> 5) << 5); };
     const int kblocks = (p.K + kPfBlockK - 1) / kPfBlockK;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kPfStages; s++) {
+        for (int s = 0; s < p.stages; s++) {
             mbar_init(&full_bar[s], 1);
             mbar_init(&empty_bar[s], 1);
         }
         for (int b = 0; b < 2; b++) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], kPfEpiWarps);  // one arrival per epilogue warp
+            mbar_init(&acc_empty[b], 2 * kPfEpiWarps);  // one arrival per epilogue warp of both CTAs (used in the first CTA)
         }
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 1) tmem_alloc(&tmem_slot, 512);
+    if (warp == 1) tmem_alloc_pair(&tmem_slot, 512);
     tc_fence_before();
     __syncthreads();
+    cluster_sync_all();  // the barriers of both CTAs are set up
     tc_fence_after();
     const uint32_t tmem_base = tmem_slot;
     pdl_wait();  // limbs and row scales come from the pre-pass
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
-        if (lane == 0) {
+        if (elect_one()) {
             asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
             asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
-            int kc = 0;
-            bool ok = true;
-            const uint32_t bytes = kPfWBytes + (uint32_t)p.cols * kPfBlockK;
-            for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-                int wt, tt;
-                pf_place(p, tile, wt, tt);
-                for (int kb = 0; kb < kblocks; kb++, kc++) {
-                    const int s = kc % kPfStages, use = kc / kPfStages;
-                    if (use > 0 && !mbar_wait_spin(&empty_bar[s], (use - 1) & 1, &abort_flag)) {
+        }
+        int s = 0, use = 0;
+        bool ok = true;
+        for (int tile = first_tile; tile < n_tiles && ok; tile += tile_stride) {
+            int wt, tt;
+            pf_place(p, tile, wt, tt);
+            const int w_row = (2 * wt + (int)rank) * kPfRows, a_row = tt * p.cols + (int)rank * (tile_cols(tt) >> 1);
+            for (int kb = 0; kb < kblocks; kb++) {
+                if (use > 0 && !__all_sync(0xffffffffu, mbar_wait_spin(&empty_bar[s], (use - 1) & 1, &abort_flag))) {
+                    if (lane == 0) {
                         atomicExch(&abort_flag, 1);
                         atomicExch(p.status, 11);
-                        ok = false;
-                        break;
                     }
-                    uint8_t *st = smem + s * kPfStageBytes;
-                    mbar_expect_tx(&full_bar[s], bytes);
-                    tma_load_2d(st, &map_w, kb * kPfBlockK, wt * kPfRows, &full_bar[s]);
-                    tma_load_2d(st + kPfWBytes, &map_a, kb * kPfBlockK, tt * p.cols, &full_bar[s]);
+                    ok = false;
+                    break;
                 }
+                uint8_t *st = smem + s * stage_bytes;
+                const uint32_t bar = map_rank(smem_u32(&full_bar[s]), 0);
+                if (elect_one()) {
+                    if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * stage_bytes);  // what both CTAs bring into a stage
+                    tma_load_2d_pair(st, &map_w, kb * kPfBlockK, w_row, bar);
+                    tma_load_2d_pair(st + kPfWBytes, &map_a, kb * kPfBlockK, a_row, bar);
+                }
+                __syncwarp();
+                if (++s == p.stages) s = 0, use++;
             }
         }
-        __syncwarp();
     } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            int kc = 0, it = 0;
+        // ---------------- MMA issuer of the pair ----------------
+        if (rank == 0) {
+            int s = 0, phase = 0, it = 0;
             bool ok = true;
-            for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, it++) {
+            for (int tile = first_tile; tile < n_tiles && ok; tile += tile_stride, it++) {
                 const int buf = it & 1, use = it >> 1;
-                // N of the MMA = the accumulator columns this tile really has (rows past M are zero-filled by TMA and
-                // need no tensor time), rounded up to the instruction's granularity of 16
                 int wt_, tt_;
                 pf_place(p, tile, wt_, tt_);
-                const int cols = min(p.cols, (((p.M - tt_ * tok) * LIMBS + 15) >> 4) << 4);
-                const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(cols >> 3) << 17) | ((uint32_t)(kPfRows >> 4) << 24);
-                if (use > 0 && !mbar_wait_spin(&acc_empty[buf], (use - 1) & 1, &abort_flag)) {  // epilogue has drained it
-                    atomicExch(&abort_flag, 1);
-                    atomicExch(p.status, 12);
+                const int cols = tile_cols(tt_);
+                const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(cols >> 3) << 17) | ((uint32_t)(2 * kPfRows >> 4) << 24);
+                if (use > 0 && !__all_sync(0xffffffffu, mbar_wait_spin(&acc_empty[buf], (use - 1) & 1, &abort_flag))) {  // epilogue has drained it
+                    if (lane == 0) {
+                        atomicExch(&abort_flag, 1);
+                        atomicExch(p.status, 12);
+                    }
                     break;
                 }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + (uint32_t)(buf * kPfCols);
-                for (int kb = 0; kb < kblocks; kb++, kc++) {
-                    const int s = kc % kPfStages;
-                    if (!mbar_wait_spin(&full_bar[s], (kc / kPfStages) & 1, &abort_flag)) {
-                        atomicExch(&abort_flag, 1);
-                        atomicExch(p.status, 13);
+                for (int kb = 0; kb < kblocks; kb++) {
+                    if (!__all_sync(0xffffffffu, mbar_wait_spin(&full_bar[s], phase, &abort_flag))) {
+                        if (lane == 0) {
+                            atomicExch(&abort_flag, 1);
+                            atomicExch(p.status, 13);
+                        }
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t a_addr = smem_u32(smem + s * kPfStageBytes);
+                    const uint32_t a_addr = smem_u32(smem + s * stage_bytes);
                     const uint64_t adesc = make_kmajor_sw128_desc(a_addr), bdesc = make_kmajor_sw128_desc(a_addr + kPfWBytes);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < kPfBlockK / 32; k++)
-                        umma_i8(d_tmem, adesc + (uint64_t)(k * 2), bdesc + (uint64_t)(k * 2), idesc, (kb | k) ? 1u : 0u);
-                    umma_commit(&empty_bar[s]);
+                        for (int k = 0; k < kPfBlockK / 32; k++)
+                            umma_i8_pair(d_tmem, adesc + (uint64_t)(k * 2), bdesc + (uint64_t)(k * 2), idesc, (kb | k) ? 1u : 0u);
+                        umma_commit_pair(&empty_bar[s]);
+                        if (kb == kblocks - 1) umma_commit_pair(&acc_full[buf]);
+                    }
+                    __syncwarp();
+                    if (++s == p.stages) s = 0, phase ^= 1;
                 }
-                if (ok) umma_commit(&acc_full[buf]);
             }
         }
         __syncwarp();
@@ -368,11 +393,11 @@ i8_prefill_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         const OutT *resid_p = reinterpret_cast<const OutT *>(p.resid);
         OutT *out_p = reinterpret_cast<OutT *>(p.out);
         int it = 0;
-        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, it++) {
+        for (int tile = first_tile; tile < n_tiles; tile += tile_stride, it++) {
             int wt, tt;
             pf_place(p, tile, wt, tt);
             const int buf = it & 1, use = it >> 1;
-            const int n = wt * kPfRows + r_local, tok0 = tt * tok, live = min(tok, p.M - tok0);
+            const int n = (2 * wt + (int)rank) * kPfRows + r_local, tok0 = tt * tok, live = min(tok, p.M - tok0);
             const float wscale = n < p.N ? to_f32<OutT>(scale_p[n]) : 0.f;
             for (int i = et; i < tok; i += 32 * kPfEpiWarps) {
                 float a = 0.f;
@@ -457,13 +482,14 @@ i8_prefill_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty[buf]);  // this warp has drained its share of the accumulator
+            if (lane == 0) mbar_arrive_pair(map_rank(smem_u32(&acc_empty[buf]), 0));  // this warp has drained its share of the accumulator
         }
     }
 
     tc_fence_before();
     __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem_base, 512);
+    cluster_sync_all();  // neither CTA leaves while the other's arrivals, copies or MMAs may still reach it
+    if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
 }
 
 // ---- host side ---------------------------------------------------------------------------------------------------
@@ -488,39 +514,40 @@ static int pf_sms() {
     return sms;
 }
 
-// How many columns a tile gets: the width whose slowest CTA has the least to do.  A tile costs its columns plus about 48 more (the weight
-// tile's share of the copies, the hand-over of the accumulator); full tiles are dealt out first, ragged ones behind them.  2048 tokens
-// x 4096 weight rows, two limbs: 512 tiles of 256 are four rounds of 148 CTAs with the last one 46 % full, 576 of 240 are four as well.
-static int pf_columns(int limbs, int M, int w_tiles, int sms) {
+// How many columns a tile gets: the width whose slowest pair has the least to do.  A stage brings 128 weight rows and half of the columns into
+// each SM at about 64 bytes per clock, so a tile costs its columns plus 256 (the tensor core, at two clocks per column, is not slower up to 256
+// columns); full tiles are dealt out first, ragged ones behind them.
+static int pf_columns(int limbs, int M, int w_tiles, int pairs) {
     int best = kPfCols;
     long long best_cost = -1;
-    for (int cols = kPfCols; cols >= 128; cols -= 16) {
+    for (int cols = kPfCols; cols >= 96; cols -= 32) {
         const int tok = cols / limbs, full_t = M / tok, rest = M - full_t * tok;
-        const long long full = (long long)w_tiles * full_t, all = full + (rest ? w_tiles : 0), r = full % sms;
-        const int unit = cols + 48, rest_unit = (rest * limbs + 15) / 16 * 16 + 48;
-        const long long f0 = (full + sms - 1) / sms, c0 = f0 * unit + ((all + sms - 1) / sms - f0) * rest_unit;  // CTA 0
-        const long long f1 = full / sms, c1 = f1 * unit + (all > r ? (all - r + sms - 1) / sms - f1 : 0) * rest_unit;  // the first with one full tile less
+        const long long full = (long long)w_tiles * full_t, all = full + (rest ? w_tiles : 0), r = full % pairs;
+        const int unit = cols + 256, rest_unit = (rest * limbs + 31) / 32 * 32 + 256;
+        const long long f0 = (full + pairs - 1) / pairs, c0 = f0 * unit + ((all + pairs - 1) / pairs - f0) * rest_unit;  // the first pair
+        const long long f1 = full / pairs, c1 = f1 * unit + (all > r ? (all - r + pairs - 1) / pairs - f1 : 0) * rest_unit;  // the first with one full tile less
         const long long cost = c0 > c1 ? c0 : c1;
         if (best_cost < 0 || cost < best_cost) best_cost = cost, best = cols;
     }
     return best;
 }
 static void pf_tiles(PfParams &p, int limbs) {
-    p.w_tiles = (p.N + kPfRows - 1) / kPfRows;
-    p.cols = pf_columns(limbs, p.M, p.w_tiles, pf_sms());
+    p.w_tiles = (p.N + 2 * kPfRows - 1) / (2 * kPfRows);
+    p.cols = pf_columns(limbs, p.M, p.w_tiles, pf_sms() / 2);
     const int tok = p.cols / limbs;
+    p.stages = std::min<int>(kPfMaxStages, kPfRingBytes / (kPfWBytes + p.cols * (kPfBlockK / 2)));
     p.t_full = p.M / tok;
     p.t_tiles = (p.M + tok - 1) / tok;
 }
 
 template <typename OutT, int LIMBS>
 static int launch_pf(cudaStream_t st, const CUtensorMap &mw, const CUtensorMap &ma, const PfParams &p) {
-    const size_t smem = (size_t)kPfStages * kPfStageBytes + 1024;
+    const size_t smem = (size_t)kPfRingBytes + 1024;
     auto kern = i8_prefill_gemm_kernel<OutT, LIMBS>;
     static SmemLimit limit;
     MYNN_CUDA_OK(limit.raise((const void *)kern, smem));
-    const int tiles = p.w_tiles * p.t_tiles, sms = pf_sms();
-    MYNN_CUDA_OK(launch_dependent(kern, dim3(tiles < sms ? tiles : sms), dim3(kPfThreads), smem, st, mw, ma, p));
+    const int tiles = p.w_tiles * p.t_tiles, pairs = pf_sms() / 2;
+    MYNN_CUDA_OK(launch_dependent_cluster(2, kern, dim3(2 * (tiles < pairs ? tiles : pairs)), dim3(kPfThreads), smem, st, mw, ma, p));
     MYNN_LAUNCH_OK("i8_prefill_gemm_kernel");
     return MYNN_OK;
 }
@@ -566,7 +593,7 @@ int i8_prefill_launch(cudaStream_t st, void *out, const void *act, const int8_t 
     CUtensorMap mw, ma;
     int rc = make_map(&mw, wq, (uint64_t)N, (uint64_t)K, (uint64_t)K, kPfRows);
     if (rc) return rc;
-    rc = make_map(&ma, limbs, (uint64_t)2 * M, (uint64_t)K, (uint64_t)K, (uint32_t)p.cols);
+    rc = make_map(&ma, limbs, (uint64_t)2 * M, (uint64_t)K, (uint64_t)K, (uint32_t)p.cols / 2);
     if (rc) return rc;
     if (out_dtype == MYNN_BF16) return launch_pf<__nv_bfloat16, 2>(st, mw, ma, p);
     if (out_dtype == MYNN_F16) return launch_pf<__half, 2>(st, mw, ma, p);
@@ -650,7 +677,7 @@ int i8_w8a8_launch(cudaStream_t st, void *out, const int8_t *lhs, const void *lh
     CUtensorMap mw, ma;
     int rc = make_map(&mw, rhs, (uint64_t)N, (uint64_t)K, (uint64_t)K, kPfRows);
     if (rc) return rc;
-    rc = make_map(&ma, lhs, (uint64_t)M, (uint64_t)K, (uint64_t)K, (uint32_t)p.cols);
+    rc = make_map(&ma, lhs, (uint64_t)M, (uint64_t)K, (uint64_t)K, (uint32_t)p.cols / 2);
     if (rc) return rc;
     if (dtype == MYNN_BF16) return launch_pf<__nv_bfloat16, 1>(st, mw, ma, p);
     if (dtype == MYNN_F16) return launch_pf<__half, 1>(st, mw, ma, p);

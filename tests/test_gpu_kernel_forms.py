@@ -77,6 +77,20 @@ def test_w8a8_product_is_exact(m, n, k):
     assert torch.equal(ops.quantized_matmul(a, sa, w, sw), want)
 
 
+# a pair of CTAs owns 256 weight rows and up to 256 int8 rows: second CTA without rows, with one, tiles of 32 columns and one more, rings of six to nine stages
+@pytest.mark.parametrize("m,n,k", [(33, 1, 16), (32, 128, 144), (95, 129, 1152), (97, 257, 1168), (256, 385, 784), (288, 19200, 128), (1025, 512, 896)])
+def test_int8_products_of_cta_pairs_are_exact(m, n, k):
+    g = gen(m + n)
+    a, w, sa, sw = int8(g, m, k), int8(g, n, k), scales(g, m, torch.bfloat16), scales(g, n, torch.bfloat16)
+    exact = a.double() @ w.double().t()
+    assert torch.equal(ops.quantized_matmul(a, sa, w, sw), (exact.float() * sa.float()[:, None] * sw.float()).bfloat16())
+    if m > 32:  # whole numbers up to 127 are their own limbs, so these sums are exact too; the residual is added behind a rounding of its own
+        res = randn(g, m, n).bfloat16()
+        want = (exact.float() * sw.float()).bfloat16()
+        assert torch.equal(ops.dequant_matmul(a.bfloat16(), w, sw), want)
+        assert torch.equal(ops.dequant_matmul_residual(a.bfloat16(), w, sw, res), (want.float() + res.float()).bfloat16())
+
+
 @pytest.mark.parametrize("dt", ["bf16", "f16"])
 @pytest.mark.parametrize("m,n,k", [(33, 130, 48), (333, 2560, 2048), (777, 3001, 2064), (2047, 1000, 512)])
 def test_prompt_product_rounds_like_float64(dt, m, n, k):

@@ -154,7 +154,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     __shared__ int abort_flag;
     __shared__ float sh_max[2][2][kTcRows];  // [tile parity][column half][row]: the halves of a row exchange their maxima
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     // 1-D grid with the query tile as the slowest index, last tile first: with a causal mask the work of a CTA grows with its
     // query tile, and CTAs are dispatched in index order, so the longest ones of ALL heads start first
     const int per_qt = p.heads_per_grid * p.B;
@@ -236,49 +236,55 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         __syncwarp();
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0 && n_tiles > 0) {
+        if (n_tiles > 0) {  // walked by the whole warp, see elect_one
             constexpr uint32_t ab = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;  // operand format: 0 = f16, 1 = bf16
             // D = f32; A and B 16-bit; M = 128.  S: both operands K-major, N = 128.  O: B (= V) MN-major, N = D.
             const uint32_t idesc_s = (1u << 4) | (ab << 7) | (ab << 10) | ((uint32_t)(kTcCols >> 3) << 17) | ((uint32_t)(kTcRows >> 4) << 24);
             const uint32_t idesc_o = (1u << 4) | (ab << 7) | (ab << 10) | (1u << 16) | ((uint32_t)(D >> 3) << 17) | ((uint32_t)(kTcRows >> 4) << 24);
-            bool ok = mbar_wait(&q_full, 0, &abort_flag);
-            if (!ok) give_up(2);
+            auto wait_all = [&](uint64_t *bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait_spin(bar, parity, &abort_flag)) != 0; };
+            bool ok = wait_all(&q_full, 0);
+            if (!ok && lane == 0) give_up(2);
             auto issue_s = [&](int j) {
                 const int s = j & 1, u = j >> 1;
-                if (!mbar_wait(&k_full[s], u & 1, &abort_flag) || (u >= 1 && !p.p_tmem && !mbar_wait(&s_empty[s], (u - 1) & 1, &abort_flag))) {
-                    give_up(3);
+                if (!wait_all(&k_full[s], u & 1) || (u >= 1 && !p.p_tmem && !wait_all(&s_empty[s], (u - 1) & 1))) {
+                    if (lane == 0) give_up(3);
                     return false;
                 }
                 tc_fence_after();
-                const uint32_t qa = smem_u32(s_q), ka = smem_u32(s_kv + s * kStage);
+                const uint64_t qd = make_kmajor_sw128_desc(smem_u32(s_q)), kd = make_kmajor_sw128_desc(smem_u32(s_kv + s * kStage));
+                if (elect_one()) {
 #pragma unroll
-                for (int ks = 0; ks < D / 16; ks++) {
-                    const uint32_t off = (uint32_t)(ks >> 2) * kTcSlab + (uint32_t)(ks & 3) * 32;
-                    umma_f16(tmem_base + kColS + s * 128, make_kmajor_sw128_desc(qa + off), make_kmajor_sw128_desc(ka + off), idesc_s, ks ? 1u : 0u);
+                    for (int ks = 0; ks < D / 16; ks++) {
+                        const uint64_t off = (uint64_t)(((ks >> 2) * kTcSlab + (ks & 3) * 32) >> 4);
+                        umma_f16(tmem_base + kColS + s * 128, qd + off, kd + off, idesc_s, ks ? 1u : 0u);
+                    }
+                    umma_commit(&s_full[s]);
+                    umma_commit(&k_empty[s]);  // the K buffer may be refilled once these MMAs have read it
                 }
-                umma_commit(&s_full[s]);
-                umma_commit(&k_empty[s]);  // the K buffer may be refilled once these MMAs have read it
+                __syncwarp();
                 return true;
             };
             ok = ok && issue_s(0);
             for (int j = 0; j < n_tiles && ok; j++) {
                 if (j + 1 < n_tiles && !issue_s(j + 1)) break;
                 const int s = j & 1, u = j >> 1;
-                if (!mbar_wait(&p_full, j & 1, &abort_flag) || !mbar_wait(&v_full[s], u & 1, &abort_flag)) {
-                    give_up(4);
+                if (!wait_all(&p_full, j & 1) || !wait_all(&v_full[s], u & 1)) {
+                    if (lane == 0) give_up(4);
                     break;
                 }
                 tc_fence_after();
-                const uint32_t pa = smem_u32(s_p), va = smem_u32(s_kv + s * kStage + kTile);
+                const uint64_t pd = make_kmajor_sw128_desc(smem_u32(s_p)), vd = make_sw128_desc(smem_u32(s_kv + s * kStage + kTile), p.v_lbo, p.v_sbo);
+                if (elect_one()) {
 #pragma unroll
-                for (int kk = 0; kk < kTcCols / 16; kk++) {
-                    const uint32_t aoff = (uint32_t)(kk >> 2) * kTcSlab + (uint32_t)(kk & 3) * 32;
-                    const uint64_t vdesc = make_sw128_desc(va + kk * 16 * 128, p.v_lbo, p.v_sbo);
-                    if (p.p_tmem) umma_f16_ta(tmem_base + kColO, tmem_base + kColS + s * 128 + kk * 8, vdesc, idesc_o, (j | kk) ? 1u : 0u);
-                    else umma_f16(tmem_base + kColO, make_kmajor_sw128_desc(pa + aoff), vdesc, idesc_o, (j | kk) ? 1u : 0u);
+                    for (int kk = 0; kk < kTcCols / 16; kk++) {
+                        const uint64_t poff = (uint64_t)(((kk >> 2) * kTcSlab + (kk & 3) * 32) >> 4), voff = (uint64_t)((kk * 16 * 128) >> 4);
+                        if (p.p_tmem) umma_f16_ta(tmem_base + kColO, tmem_base + kColS + s * 128 + kk * 8, vd + voff, idesc_o, (j | kk) ? 1u : 0u);
+                        else umma_f16(tmem_base + kColO, pd + poff, vd + voff, idesc_o, (j | kk) ? 1u : 0u);
+                    }
+                    umma_commit(&v_empty[s]);  // the V buffer may be refilled once these MMAs have read it
+                    umma_commit(&pv_done);
                 }
-                umma_commit(&v_empty[s]);  // the V buffer may be refilled once these MMAs have read it
-                umma_commit(&pv_done);
+                __syncwarp();
             }
         }
         __syncwarp();
@@ -494,7 +500,7 @@ attention_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int per_qt = p.heads_per_grid * p.B;  // 1-D grid, query tile slowest and last tile first (see the one-head kernel)
     const int qt = p.n_qt - 1 - (int)blockIdx.x / per_qt, h0 = 2 * (((int)blockIdx.x % per_qt) % p.heads_per_grid), b = ((int)blockIdx.x % per_qt) / p.heads_per_grid;
     const int kvh = h0 / (p.Hq / p.Hkv);  // the group size is even: both heads read the same kv head
@@ -566,53 +572,58 @@ attention_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __
         __syncwarp();
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0 && n_tiles > 0) {
+        if (n_tiles > 0) {  // walked by the whole warp, see elect_one
             constexpr uint32_t ab = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
             const uint32_t idesc_s = (1u << 4) | (ab << 7) | (ab << 10) | ((uint32_t)(kTcCols >> 3) << 17) | ((uint32_t)(kTcRows >> 4) << 24);
             const uint32_t idesc_o = (1u << 4) | (ab << 7) | (ab << 10) | (1u << 16) | ((uint32_t)(D >> 3) << 17) | ((uint32_t)(kTcRows >> 4) << 24);
             auto issue_s = [&](int t, int j) {  // S_t(j) = Q_t K_j^T; the caller has waited for K_j
-                const uint32_t qa = smem_u32(s_q + t * kTile), ka = smem_u32(s_k + (j & 1) * kTile);
+                const uint64_t qd = make_kmajor_sw128_desc(smem_u32(s_q + t * kTile)), kd = make_kmajor_sw128_desc(smem_u32(s_k + (j & 1) * kTile));
+                if (elect_one()) {
 #pragma unroll
-                for (int ks = 0; ks < D / 16; ks++) {
-                    const uint32_t off = (uint32_t)(ks >> 2) * kTcSlab + (uint32_t)(ks & 3) * 32;
-                    umma_f16(tmem_base + t * 128, make_kmajor_sw128_desc(qa + off), make_kmajor_sw128_desc(ka + off), idesc_s, ks ? 1u : 0u);
+                    for (int ks = 0; ks < D / 16; ks++) {
+                        const uint64_t off = (uint64_t)(((ks >> 2) * kTcSlab + (ks & 3) * 32) >> 4);
+                        umma_f16(tmem_base + t * 128, qd + off, kd + off, idesc_s, ks ? 1u : 0u);
+                    }
+                    umma_commit(&s_full[t]);
+                    if (t == 1) umma_commit(&k_empty[j & 1]);
                 }
-                umma_commit(&s_full[t]);
+                __syncwarp();
             };
-            bool ok = wait_fast(&q_full, 0) && wait_fast(&k_full[0], 0);
-            if (!ok) give_up(12);
+            auto wait_all = [&](uint64_t *bar, uint32_t parity) { return __all_sync(0xffffffffu, wait_fast(bar, parity)) != 0; };
+            bool ok = wait_all(&q_full, 0) && wait_all(&k_full[0], 0);
+            if (!ok && lane == 0) give_up(12);
             if (ok) {
                 tc_fence_after();
                 issue_s(0, 0);
                 issue_s(1, 0);
-                umma_commit(&k_empty[0]);
             }
             for (int j = 0; j < n_tiles && ok; j++) {
                 const int st = j & 1, u = j >> 1;
 #pragma unroll
                 for (int t = 0; t < 2; t++) {
-                    if (!wait_fast(&p_full[t], j & 1) || (t == 0 && !wait_fast(&v_full[st], u & 1))) {
-                        give_up(13);
+                    if (!wait_all(&p_full[t], j & 1) || (t == 0 && !wait_all(&v_full[st], u & 1))) {
+                        if (lane == 0) give_up(13);
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t va = smem_u32(s_v + st * kTile);
+                    const uint64_t vd = make_sw128_desc(smem_u32(s_v + st * kTile), p.v_lbo, p.v_sbo);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int kk = 0; kk < kTcCols / 16; kk++)
-                        umma_f16_ta(tmem_base + 256 + t * 128, tmem_base + t * 128 + kk * 8, make_sw128_desc(va + kk * 16 * 128, p.v_lbo, p.v_sbo),
-                                    idesc_o, (j | kk) ? 1u : 0u);
-                    umma_commit(&o_done[t]);
-                    if (t == 1) umma_commit(&v_empty[st]);
+                        for (int kk = 0; kk < kTcCols / 16; kk++)
+                            umma_f16_ta(tmem_base + 256 + t * 128, tmem_base + t * 128 + kk * 8, vd + (uint64_t)((kk * 16 * 128) >> 4), idesc_o, (j | kk) ? 1u : 0u);
+                        umma_commit(&o_done[t]);
+                        if (t == 1) umma_commit(&v_empty[st]);
+                    }
+                    __syncwarp();
                     if (j + 1 < n_tiles) {
-                        if (t == 0 && !wait_fast(&k_full[(j + 1) & 1], ((j + 1) >> 1) & 1)) {
-                            give_up(14);
+                        if (t == 0 && !wait_all(&k_full[(j + 1) & 1], ((j + 1) >> 1) & 1)) {
+                            if (lane == 0) give_up(14);
                             ok = false;
                             break;
                         }
                         tc_fence_after();
                         issue_s(t, j + 1);
-                        if (t == 1) umma_commit(&k_empty[(j + 1) & 1]);
                     }
                 }
             }

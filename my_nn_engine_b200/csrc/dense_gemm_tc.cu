@@ -74,7 +74,7 @@ dense_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     __shared__ int abort_flag;
     constexpr int NT = GLU ? kDgCols / 2 : kDgCols;  // outputs per tile
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int kblocks = (p.K + kDgK - 1) / kDgK;
     if (threadIdx.x == 0) {
         for (int s = 0; s < kDgStages; s++) {
@@ -113,24 +113,25 @@ dense_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
-        if (lane == 0) {
+        if (elect_one()) {
             asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
             asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
-            int kc = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
-                int mt, nt;
-                locate(tile, mt, nt);
-                const int e = p.tile_e ? p.tile_e[mt] : 0, row = p.tile_row ? p.tile_row[mt] : dense_row(mt);
-                const int wrow = e * (GLU ? 2 * p.N : p.N) + nt * NT;
-                for (int kb = 0; kb < kblocks; kb++, kc++) {
-                    const int s = kc % kDgStages, use = kc / kDgStages;
-                    if (use > 0 && !mbar_wait_spin(&empty_bar[s], (use - 1) & 1, &abort_flag)) {
-                        give_up(41);
-                        ok = false;
-                        break;
-                    }
-                    uint8_t *st = smem + s * kDgStageBytes;
+        }
+        int s = 0, use = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
+            int mt, nt;
+            locate(tile, mt, nt);
+            const int e = p.tile_e ? p.tile_e[mt] : 0, row = p.tile_row ? p.tile_row[mt] : dense_row(mt);
+            const int wrow = e * (GLU ? 2 * p.N : p.N) + nt * NT;
+            for (int kb = 0; kb < kblocks; kb++) {
+                if (use > 0 && !__all_sync(0xffffffffu, mbar_wait_spin(&empty_bar[s], (use - 1) & 1, &abort_flag))) {
+                    if (lane == 0) give_up(41);
+                    ok = false;
+                    break;
+                }
+                uint8_t *st = smem + s * kDgStageBytes;
+                if (elect_one()) {
                     mbar_expect_tx(&full_bar[s], kDgStageBytes);
                     tma_load_2d(st, &map_a, kb * 128, row, &full_bar[s]);  // byte maps: x counts bytes
                     if constexpr (GLU) {
@@ -140,44 +141,47 @@ dense_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                         tma_load_2d(st + kDgABytes, &map_w, kb * 128, wrow, &full_bar[s]);
                     }
                 }
+                __syncwarp();
+                if (++s == kDgStages) s = 0, use++;
             }
         }
         __syncwarp();
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            constexpr uint32_t ab = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;  // operand format: 0 = f16, 1 = bf16
-            int kc = 0, it = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x, it++) {
-                const int buf = it & 1, use = it >> 1;
-                int mt, nt;
-                locate(tile, mt, nt);
-                // only as many columns as the tile has weight rows (gating needs both halves in place)
-                const int cols = GLU ? kDgCols : min(kDgCols, ((p.N - nt * NT + 15) >> 4) << 4);
-                const uint32_t idesc = (1u << 4) | (ab << 7) | (ab << 10) | ((uint32_t)(cols >> 3) << 17) | ((uint32_t)(kDgRows >> 4) << 24);
-                if (use > 0 && !mbar_wait_spin(&acc_empty[buf], (use - 1) & 1, &abort_flag)) {  // the epilogue has drained it
-                    give_up(42);
+        constexpr uint32_t ab = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;  // operand format: 0 = f16, 1 = bf16
+        int s = 0, phase = 0, it = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x, it++) {
+            const int buf = it & 1, use = it >> 1;
+            int mt, nt;
+            locate(tile, mt, nt);
+            // only as many columns as the tile has weight rows (gating needs both halves in place)
+            const int cols = GLU ? kDgCols : min(kDgCols, ((p.N - nt * NT + 15) >> 4) << 4);
+            const uint32_t idesc = (1u << 4) | (ab << 7) | (ab << 10) | ((uint32_t)(cols >> 3) << 17) | ((uint32_t)(kDgRows >> 4) << 24);
+            if (use > 0 && !__all_sync(0xffffffffu, mbar_wait_spin(&acc_empty[buf], (use - 1) & 1, &abort_flag))) {  // the epilogue has drained it
+                if (lane == 0) give_up(42);
+                break;
+            }
+            tc_fence_after();
+            const uint32_t d_tmem = tmem_base + (uint32_t)(buf * kDgCols);
+            for (int kb = 0; kb < kblocks; kb++) {
+                if (!__all_sync(0xffffffffu, mbar_wait_spin(&full_bar[s], phase, &abort_flag))) {
+                    if (lane == 0) give_up(43);
+                    ok = false;
                     break;
                 }
                 tc_fence_after();
-                const uint32_t d_tmem = tmem_base + (uint32_t)(buf * kDgCols);
-                for (int kb = 0; kb < kblocks; kb++, kc++) {
-                    const int s = kc % kDgStages;
-                    if (!mbar_wait_spin(&full_bar[s], (kc / kDgStages) & 1, &abort_flag)) {
-                        give_up(43);
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t a_addr = smem_u32(smem + s * kDgStageBytes);
-                    const uint64_t adesc = make_kmajor_sw128_desc(a_addr), bdesc = make_kmajor_sw128_desc(a_addr + kDgABytes);
+                const uint32_t a_addr = smem_u32(smem + s * kDgStageBytes);
+                const uint64_t adesc = make_kmajor_sw128_desc(a_addr), bdesc = make_kmajor_sw128_desc(a_addr + kDgABytes);
+                if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < kDgK / 16; k++)
                         umma_f16(d_tmem, adesc + (uint64_t)(k * 2), bdesc + (uint64_t)(k * 2), idesc, (kb | k) ? 1u : 0u);
                     umma_commit(&empty_bar[s]);
+                    if (kb == kblocks - 1) umma_commit(&acc_full[buf]);
                 }
-                if (ok) umma_commit(&acc_full[buf]);
+                __syncwarp();
+                if (++s == kDgStages) s = 0, phase ^= 1;
             }
         }
         __syncwarp();

@@ -110,7 +110,7 @@ i8_stream_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     __shared__ int abort_flag;
     __shared__ float sh_ascale[32];
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int S = gridDim.y;
     MYNN_STAMP(threadIdx.x == 0, 0);
     const int rank = S > 1 ? (int)cluster_ctarank() : 0;
@@ -139,60 +139,75 @@ i8_stream_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
-        if (lane == 0) {
+        if (elect_one()) {
             asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
             asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
-            // Settled weights do not depend on the kernels in front: start streaming them at once, and only then wait
-            // (programmatic dependent launch) for the grid that writes the activation limbs.
-            if (!p.settled) pdl_wait();
-            const int nload = nkb - ((p.skip_last_stage & 1) ? 1 : 0);  // normally every k block
-            const int pre = min(nload, stages);
+        }
+        // Settled weights do not depend on the kernels in front: start streaming them at once, and only then wait
+        // (programmatic dependent launch) for the grid that writes the activation limbs.
+        if (!p.settled) pdl_wait();
+        const int nload = nkb - ((p.skip_last_stage & 1) ? 1 : 0);  // normally every k block
+        const int pre = min(nload, stages);
+        if (elect_one()) {
             for (int i = 0; i < pre; i++) {
                 mbar_expect_tx(&full_bar[i], kWBytes + kABytes);
                 tma_load_2d(smem + i * kStageBytes, &map_w, (kb_beg + i) * kBlockK, row0, &full_bar[i]);
             }
-            asm volatile("griddepcontrol.wait;" ::: "memory");
-            MYNN_STAMP(true, 2);  // predecessor grid complete
+        }
+        __syncwarp();
+        pdl_wait();
+        MYNN_STAMP(lane == 0, 2);  // predecessor grid complete
+        if (elect_one()) {
             for (int i = 0; i < pre; i++)
                 tma_load_2d(smem + i * kStageBytes + kWBytes, &map_a, (kb_beg + i) * kBlockK, 0, &full_bar[i]);
-            for (int i = pre; i < nload; i++) {
-                const int s = i % stages, it = i / stages;
-                if (!mbar_wait_spin(&empty_bar[s], (it - 1) & 1, &abort_flag)) {
+        }
+        __syncwarp();
+        int st = 0, phase = 0;
+        for (int i = pre; i < nload; i++) {
+            if (!__all_sync(0xffffffffu, mbar_wait_spin(&empty_bar[st], phase, &abort_flag))) {
+                if (lane == 0) {
                     atomicExch(&abort_flag, 1);
                     atomicExch(p.status, 1);
-                    break;
                 }
-                uint8_t *st = smem + s * kStageBytes;
-                mbar_expect_tx(&full_bar[s], kWBytes + kABytes);
-                tma_load_2d(st, &map_w, (kb_beg + i) * kBlockK, row0, &full_bar[s]);
-                tma_load_2d(st + kWBytes, &map_a, (kb_beg + i) * kBlockK, 0, &full_bar[s]);
+                break;
             }
+            uint8_t *at = smem + st * kStageBytes;
+            if (elect_one()) {
+                mbar_expect_tx(&full_bar[st], kWBytes + kABytes);
+                tma_load_2d(at, &map_w, (kb_beg + i) * kBlockK, row0, &full_bar[st]);
+                tma_load_2d(at + kWBytes, &map_a, (kb_beg + i) * kBlockK, 0, &full_bar[st]);
+            }
+            __syncwarp();
+            if (++st == stages) st = 0, phase ^= 1;
         }
         __syncwarp();
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            // instruction descriptor: D = S32, A = B = signed int8, both K-major, N = NC, M = 128
-            constexpr uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NC >> 3) << 17) | ((uint32_t)(kTileRows >> 4) << 24);
-            bool ok = true;
-            for (int i = 0; i < nkb && ok; i++) {
-                const int s = i % stages, it = i / stages;
-                if (!mbar_wait_spin(&full_bar[s], it & 1, &abort_flag)) {
+        // instruction descriptor: D = S32, A = B = signed int8, both K-major, N = NC, M = 128
+        constexpr uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NC >> 3) << 17) | ((uint32_t)(kTileRows >> 4) << 24);
+        int st = 0, phase = 0;
+        for (int i = 0; i < nkb; i++) {
+            if (!__all_sync(0xffffffffu, mbar_wait_spin(&full_bar[st], phase, &abort_flag))) {
+                if (lane == 0) {
                     atomicExch(&abort_flag, 1);
                     atomicExch(p.status, 2);
-                    ok = false;
-                    break;
                 }
-                tc_fence_after();
-                const uint32_t a_addr = smem_u32(smem + s * kStageBytes);
-                const uint64_t adesc = make_kmajor_sw128_desc(a_addr), bdesc = make_kmajor_sw128_desc(a_addr + kWBytes);
+                break;
+            }
+            tc_fence_after();
+            const uint32_t a_addr = smem_u32(smem + st * kStageBytes);
+            const uint64_t adesc = make_kmajor_sw128_desc(a_addr), bdesc = make_kmajor_sw128_desc(a_addr + kWBytes);
+            if (elect_one()) {
 #pragma unroll
                 for (int k = 0; k < kBlockK / 32; k++)  // 32 bytes of k per instruction: advance the start address
                     umma_i8(tmem_base, adesc + (uint64_t)(k * 2), bdesc + (uint64_t)(k * 2), idesc, (i | k) ? 1u : 0u);
-                umma_commit(&empty_bar[s]);  // the stage may be refilled once these MMAs have read it
+                umma_commit(&empty_bar[st]);  // the stage may be refilled once these MMAs have read it
             }
-            umma_commit(&accum_bar);  // accumulators complete (also fires when nothing was issued)
+            __syncwarp();
+            if (++st == stages) st = 0, phase ^= 1;
         }
+        __syncwarp();
+        if (elect_one()) umma_commit(&accum_bar);  // accumulators complete (also fires when nothing was issued)
         __syncwarp();
     }
 

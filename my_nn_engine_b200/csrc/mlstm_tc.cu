@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(kMtThreads, 1) mlstm_tc_kernel(const __grid_co
     pdl_wait();
     const int h = blockIdx.y, b = blockIdx.z / (OUT ? w.segments : w.segments - 1), seg = blockIdx.z - b * (OUT ? w.segments : w.segments - 1), pair = b * p.H + h;
     const bool single = w.segments == 1, final_state = OUT && seg == w.segments - 1;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int quad = warp & 3, quarter = warp >> 2, e0 = blockIdx.x * kChunkCols, e = e0 + quad * 32 + lane, d0 = quarter * DQ;
     const float q_scale = 1.0f / sqrtf((float)p.D);
     const int c_beg = seg * w.per, c_end = min(c_beg + w.per, w.chunks);
@@ -306,33 +306,40 @@ __global__ void __launch_bounds__(kMtThreads, 1) mlstm_tc_kernel(const __grid_co
             ok = false;
             break;
         }
-        if (threadIdx.x == 0) {
+        if (warp == 0) {  // the whole warp, see elect_one
             tc_fence_after();
             if constexpr (OUT) {
                 ok = mbar_wait_spin(&p_full, parity, &abort_flag);
+                __syncwarp();
                 constexpr uint32_t idesc = kIdesc | ((uint32_t)(kChunk >> 3) << 17);
                 const uint64_t dq = make_kmajor_sw128_desc(smem_base + L::kQ + off_k);
                 const uint64_t dv = make_sw128_desc(smem_base + L::kV + off_v, kMtSlab, 1024), dp = make_kmajor_sw128_desc(smem_base + L::kP);
+                if (elect_one()) {
 #pragma unroll
-                for (int i = 0; i < 2 * (kChunk / 16); i++) {
-                    const int hp = i / (kChunk / 16), ks = i % (kChunk / 16);
-                    umma_f16(tm + L::kColPv, dv + (uint64_t)((ks * 2048) >> 4), dp + (uint64_t)((hp * kMtSlab + ks * 32) >> 4), idesc | kAmn, i ? 1u : 0u);
-                }
+                    for (int i = 0; i < 2 * (kChunk / 16); i++) {
+                        const int hp = i / (kChunk / 16), ks = i % (kChunk / 16);
+                        umma_f16(tm + L::kColPv, dv + (uint64_t)((ks * 2048) >> 4), dp + (uint64_t)((hp * kMtSlab + ks * 32) >> 4), idesc | kAmn, i ? 1u : 0u);
+                    }
 #pragma unroll
-                for (int i = 0; i < 2 * (KD / 16); i++) {
-                    const int hp = i / (KD / 16), ks = i % (KD / 16);
-                    umma_f16_ta(tm + L::kColInter, tm + (ks / (DQ / 16)) * DQ + hp * (DQ / 2) + (ks % (DQ / 16)) * 8,
-                                dq + (uint64_t)(((ks >> 2) * kMtSlab + (ks & 3) * 32) >> 4), idesc, i ? 1u : 0u);
+                    for (int i = 0; i < 2 * (KD / 16); i++) {
+                        const int hp = i / (KD / 16), ks = i % (KD / 16);
+                        umma_f16_ta(tm + L::kColInter, tm + (ks / (DQ / 16)) * DQ + hp * (DQ / 2) + (ks % (DQ / 16)) * 8,
+                                    dq + (uint64_t)(((ks >> 2) * kMtSlab + (ks & 3) * 32) >> 4), idesc, i ? 1u : 0u);
+                    }
                 }
+                __syncwarp();
             }
             constexpr uint32_t idesc = kIdesc | kAmn | kBmn | ((uint32_t)(KD >> 3) << 17);
             const uint64_t da = make_sw128_desc(smem_base + L::kVw, kMtSlab, 1024), db = make_sw128_desc(smem_base + L::kK + off_k, kMtSlab, 1024);
+            if (elect_one()) {
 #pragma unroll
-            for (int i = 0; i < 2 * (kChunk / 16); i++) {
-                const int hp = i / (kChunk / 16), ks = i % (kChunk / 16);
-                umma_f16(tm, da + (uint64_t)((hp * 2 * kMtSlab + ks * 2048) >> 4), db + (uint64_t)((ks * 2048) >> 4), idesc, i ? 1u : 0u);
+                for (int i = 0; i < 2 * (kChunk / 16); i++) {
+                    const int hp = i / (kChunk / 16), ks = i % (kChunk / 16);
+                    umma_f16(tm, da + (uint64_t)((hp * 2 * kMtSlab + ks * 2048) >> 4), db + (uint64_t)((ks * 2048) >> 4), idesc, i ? 1u : 0u);
+                }
+                umma_commit(&bar_s);
             }
-            umma_commit(&bar_s);
+            __syncwarp();
         } else if (!OUT && threadIdx.x == 32 && c > c_beg && c + 2 < c_end) {
             fetch(c + 2);  // over chunk c - 1
         }

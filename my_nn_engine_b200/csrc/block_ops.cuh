@@ -193,7 +193,7 @@ struct MoeRoute {
     int32_t *count;     // [E] scratch, zero between calls
     int32_t *tile_e, *tile_row, *n_tiles;  // tiles of kMoeTileRows places that do not cross experts (tensor-core kernel)
 };
-constexpr int kMoeTileRows = 128;
+constexpr int kMoeTileRows = 256;
 size_t moe_route_bytes(int M, int experts, int top);
 MoeRoute moe_route_bind(void *base, int M, int experts, int top);
 int launch_moe_route(cudaStream_t st, const MoeRoute &r, const float *logits, int M, int experts, int top, int groups, int keep);

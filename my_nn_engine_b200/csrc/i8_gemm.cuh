@@ -40,7 +40,12 @@ int launch_swiglu_limbs(cudaStream_t st, int dtype, void *workspace, size_t work
 int make_map(CUtensorMap *map, const void *base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows);
 bool tensor_map_api_available();
 
-// Large-M (prefill) variant: activations as two int8 limbs per element, 128 x 128-token tiles, persistent CTAs.
+int sm_count();  // of the current device
+// Products of many rows on pairs of CTAs (i8_gemm_prefill.cu, dense_gemm_tc.cu): how many accumulator columns a tile of 256 weight rows gets, `limbs` per
+// activation row, for `groups` groups of M rows.
+int pair_tile_columns(int limbs, int M, int groups, int w_tiles, int pairs);
+
+// Large-M (prefill) variant: activations as two int8 limbs per element, persistent pairs of CTAs.
 // Scratch layout: [0,256) status word, then M row scales (rounded up to 256 bytes), then the [2M][K] limb matrix.
 size_t i8_prefill_workspace_bytes(int M, int K);
 bool i8_prefill_supported(int M, int N, int K, const void *wq, int act_dtype, int out_dtype);

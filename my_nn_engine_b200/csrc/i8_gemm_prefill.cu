@@ -507,22 +507,22 @@ bool i8_prefill_supported(int M, int N, int K, const void *wq, int act_dtype, in
            tensor_map_api_available();
 }
 
-static int pf_sms() {
+int sm_count() {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     return sms;
 }
 
-// How many columns a tile gets: the width whose slowest pair has the least to do.  A stage brings 128 weight rows and half of the columns into
-// each SM at about 64 bytes per clock, so a tile costs its columns plus 256 (the tensor core, at two clocks per column, is not slower up to 256
-// columns); full tiles are dealt out first, ragged ones behind them.
-static int pf_columns(int limbs, int M, int w_tiles, int pairs) {
+// The width whose slowest pair has the least to do.  A stage brings 128 weight rows and half of the columns into each SM at about 64 bytes per
+// clock, so a tile costs its columns plus 256 (the tensor core, at two clocks per column, is not slower up to 256 columns); full tiles are
+// dealt out first, ragged ones behind them.
+int pair_tile_columns(int limbs, int M, int groups, int w_tiles, int pairs) {
     int best = kPfCols;
     long long best_cost = -1;
     for (int cols = kPfCols; cols >= 96; cols -= 32) {
         const int tok = cols / limbs, full_t = M / tok, rest = M - full_t * tok;
-        const long long full = (long long)w_tiles * full_t, all = full + (rest ? w_tiles : 0), r = full % pairs;
+        const long long full = (long long)w_tiles * groups * full_t, all = full + (rest ? (long long)w_tiles * groups : 0), r = full % pairs;
         const int unit = cols + 256, rest_unit = (rest * limbs + 31) / 32 * 32 + 256;
         const long long f0 = (full + pairs - 1) / pairs, c0 = f0 * unit + ((all + pairs - 1) / pairs - f0) * rest_unit;  // the first pair
         const long long f1 = full / pairs, c1 = f1 * unit + (all > r ? (all - r + pairs - 1) / pairs - f1 : 0) * rest_unit;  // the first with one full tile less
@@ -533,7 +533,7 @@ static int pf_columns(int limbs, int M, int w_tiles, int pairs) {
 }
 static void pf_tiles(PfParams &p, int limbs) {
     p.w_tiles = (p.N + 2 * kPfRows - 1) / (2 * kPfRows);
-    p.cols = pf_columns(limbs, p.M, p.w_tiles, pf_sms() / 2);
+    p.cols = pair_tile_columns(limbs, p.M, 1, p.w_tiles, sm_count() / 2);
     const int tok = p.cols / limbs;
     p.stages = std::min<int>(kPfMaxStages, kPfRingBytes / (kPfWBytes + p.cols * (kPfBlockK / 2)));
     p.t_full = p.M / tok;
@@ -546,7 +546,7 @@ static int launch_pf(cudaStream_t st, const CUtensorMap &mw, const CUtensorMap &
     auto kern = i8_prefill_gemm_kernel<OutT, LIMBS>;
     static SmemLimit limit;
     MYNN_CUDA_OK(limit.raise((const void *)kern, smem));
-    const int tiles = p.w_tiles * p.t_tiles, pairs = pf_sms() / 2;
+    const int tiles = p.w_tiles * p.t_tiles, pairs = sm_count() / 2;
     MYNN_CUDA_OK(launch_dependent_cluster(2, kern, dim3(2 * (tiles < pairs ? tiles : pairs)), dim3(kPfThreads), smem, st, mw, ma, p));
     MYNN_LAUNCH_OK("i8_prefill_gemm_kernel");
     return MYNN_OK;

@@ -6,7 +6,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-from my_nn_engine_b200 import ops  # noqa: E402
+from my_nn_engine_b200 import ffi, ops  # noqa: E402
 from oracle import ref_ops as R  # noqa: E402
 from oracle import ref_vebisun as V  # noqa: E402
 
@@ -104,6 +104,30 @@ def test_prompt_product_rounds_like_float64(dt, m, n, k):
     assert torch.isnan(got[m - 1]).all()
     ulp = 2.0 ** (-7 if dt == "bf16" else -10)
     assert (got[:-1].double() - want[:-1]).abs().max() <= ulp * want[:-1].abs().max()
+
+
+# ---- products of many rows over unquantised weights: pairs of CTAs own 256 weight rows (gating: 128 outputs) and up to 256 activation rows ----
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("m,n,k", [(33, 1, 8), (97, 64, 72), (128, 65, 448), (257, 129, 392), (300, 257, 64), (513, 200, 1032), (2500, 640, 136)])
+def test_dense_products_of_cta_pairs(dt, m, n, k):
+    g, word = gen(m + n), torch.zeros(1, dtype=torch.int32, device="cuda")
+    act, w = randn(g, m, k).to(DT[dt]), (randn(g, 2 * n, k) * k ** -0.5).to(DT[dt])
+    act[m - 1] = float("nan")  # stays in its own row
+    full = act.double() @ w.double().t()
+    # sums of size one: f32 accumulation (k 2^-24) is nothing beside the rounding of the result
+    eps = 2.0 ** (-8 if dt == "bf16" else -11)
+
+    def close(got, want, nan=True):
+        assert word.item() == 0 and (not nan or torch.isnan(got[m - 1]).all())
+        assert (got[:-1].double() - want[:-1]).abs().max() <= (eps + 1e-5) * want[:-1].abs().max()
+
+    close(ops.dense_matmul(act, w, status=word), full)
+    close(ops.dense_matmul(act, w, out_dtype=torch.float32, status=word), full)
+    gate, up = full[:, :n], full[:, n:]
+    close(ops.dense_matmul(act, w, glu=True, status=word), torch.nn.functional.silu(gate) * up)
+    got, extra = ops.dense_matmul_ex(act, w, act_fn=ffi.ACT_SQUARE_RELU, f32_columns=n, status=word)
+    close(got, torch.relu(gate).square(), nan=False)  # the larger of NaN and 0 is 0 here
+    assert torch.isnan(extra[m - 1]).all() and (extra[:-1].double() - up[:-1]).abs().max() <= 1e-5 * up[:-1].abs().max()
 
 
 @pytest.mark.parametrize("dt", ["bf16", "f16"])

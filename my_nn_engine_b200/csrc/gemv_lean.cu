@@ -24,6 +24,7 @@
 // two per SM (4.7 us).
 #include "common.cuh"
 #include "i8_gemm.cuh"
+#include "limbs.cuh"
 
 namespace mynn {
 
@@ -64,111 +65,82 @@ __device__ __forceinline__ void lean_unpack(const uint4 &raw, float (&v)[8]) {
 // The activation rows as limbs in shared memory (and from CTA 0 in the workspace), with the arithmetic of the limb pre-pass of
 // the tensor-core kernel: |a| * 2^(22-e) rounded to an integer below 2^22, split into three signed bytes.  Every CTA does this for
 // itself: all rows at once, eight elements per thread and round, two barriers and no launch in between.  (The norm or the SiLU product in
-// front taken inside as well cost as much as the launch it saved at one row and more at three: 10.2 us for norm and gate/up against 3.0 + 6.0.)
+// front taken inside as well cost as much as the launch it saved at one row and more at three: 10.2 us for norm and gate/up against 3.0 + 6.0.
+// The SiLU product belongs behind the product that makes its operands: see GATED below.)
 template <typename ActT, int M, int NB>
-__device__ __forceinline__ void lean_rows_to_limbs(const LeanParams &p, int pitch, int8_t *sm_limbs, float *sm_ascale, unsigned *sm_max) {
+__device__ __forceinline__ void lean_rows_to_limbs(const LeanParams &p, int pitch, int8_t *sm_limbs, float *sm_ascale, unsigned (*sm_max)[kLeanWarps]) {
+    static_assert(M <= 2, "rows of a warp's chunks");
     constexpr int ROUNDS = (M * NB * 128 + kLeanThreads - 1) / kLeanThreads;
     constexpr bool HALF = sizeof(ActT) == 2;  // 16-bit rows stay in registers between the passes
-    const int per = p.K >> 3, total = M * per, lane = threadIdx.x & 31;
-    const bool even = per % 32 == 0;  // a warp's chunks belong to one row
+    const int per = p.K >> 3, total = M * per, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const ActT *act = reinterpret_cast<const ActT *>(p.act);
     const bool vec = (uintptr_t)act % 16 == 0;
-    uint4 keep[HALF ? ROUNDS : 1];
-    auto fetch = [&](const ActT *src, float (&v)[8], uint4 &raw) {
-        if constexpr (HALF) {
-            if (vec) {
-                raw = __ldcg(reinterpret_cast<const uint4 *>(src));
-            } else {
-                __align__(16) ActT e[8];
+    auto fetch = [&](int i, uint4 &raw) {  // eight 16-bit elements
+        const ActT *src = act + 8 * (size_t)i;
+        if (vec) {
+            raw = __ldcg(reinterpret_cast<const uint4 *>(src));
+        } else {
+            __align__(16) ActT e[8];
 #pragma unroll
-                for (int j = 0; j < 8; j++) e[j] = src[j];
-                raw = *reinterpret_cast<const uint4 *>(e);
-            }
+            for (int j = 0; j < 8; j++) e[j] = src[j];
+            raw = *reinterpret_cast<const uint4 *>(e);
+        }
+    };
+    auto values = [&](int i, const uint4 &raw, float (&v)[8]) {
+        if constexpr (HALF) {
             lean_unpack<ActT>(raw, v);
         } else {
 #pragma unroll
-            for (int j = 0; j < 8; j++) v[j] = to_f32<ActT>(src[j]);
+            for (int j = 0; j < 8; j++) v[j] = to_f32<ActT>(act[8 * (size_t)i + j]);
         }
     };
-    auto chunk = [&](int k, int &m, int &c) {
-        const int i = threadIdx.x + k * kLeanThreads;
-        m = min(i / per, M - 1);
-        c = i - m * per;
-        return i < total;
-    };
+    uint4 keep[ROUNDS];
 #pragma unroll
     for (int k = 0; k < ROUNDS; k++) {  // all loads first
-        int m, c;
-        const bool in = chunk(k, m, c);
-        if constexpr (HALF) {
-            keep[k] = make_uint4(0u, 0u, 0u, 0u);
-            float v[8];
-            if (in) fetch(act + (size_t)m * p.K + 8 * c, v, keep[k]);
-        }
+        const int i = threadIdx.x + k * kLeanThreads;
+        keep[k] = make_uint4(0u, 0u, 0u, 0u);
+        if (HALF && i < total) fetch(i, keep[k]);
     }
+    unsigned mx[M] = {};
 #pragma unroll
     for (int k = 0; k < ROUNDS; k++) {
-        int m, c;
-        const bool in = chunk(k, m, c);
+        const int i = threadIdx.x + k * kLeanThreads;
+        if (i >= total) continue;
         float v[8];
-        if constexpr (HALF) {
-            lean_unpack<ActT>(keep[k], v);
-        } else {
-            uint4 none;
+        values(i, keep[k], v);
+        const unsigned top = max_bits8(v);
+        if (M == 1 || i < per) mx[0] = max(mx[0], top);
+        else mx[M - 1] = max(mx[M - 1], top);
+    }
 #pragma unroll
-            for (int j = 0; j < 8; j++) v[j] = 0.f;
-            if (in) fetch(act + (size_t)m * p.K + 8 * c, v, none);
-        }
-        unsigned mx = 0u;  // magnitudes as integers: infinities and NaN above every number
-#pragma unroll
-        for (int j = 0; j < 8; j++) mx = max(mx, __float_as_uint(v[j]) & 0x7fffffffu);
-        if (!in) mx = 0u;
-        if (even) {
-            mx = __reduce_max_sync(0xffffffffu, mx);
-            if (lane == 0 && mx) atomicMax(&sm_max[m], mx);
-        } else if (mx) {
-            atomicMax(&sm_max[m], mx);
-        }
+    for (int m = 0; m < M; m++) {
+        mx[m] = __reduce_max_sync(0xffffffffu, mx[m]);
+        if (lane == 0) sm_max[m][warp] = mx[m];
     }
     __syncthreads();
-    const bool publish = blockIdx.x == 0;
+    float sc[M];
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+        sc[m] = limb_scale(__reduce_max_sync(0xffffffffu, sm_max[m][lane & (kLeanWarps - 1)]));
+        if (threadIdx.x == m) {
+            const float as = limb_unscale(sc[m]);
+            sm_ascale[m] = as;
+            if (blockIdx.x == 0) p.ascale_g[m] = as;
+        }
+    }
 #pragma unroll
     for (int k = 0; k < ROUNDS; k++) {
-        int m, c;
-        if (!chunk(k, m, c)) break;
-        const float t = __uint_as_float(sm_max[m]);
-        const bool bad = !(t <= 3.0e38f);
-        int e = 0;
-        if (t > 0.f && !bad) frexpf(t, &e);
-        const float sc = bad ? 0.f : t > 0.f ? ldexpf(1.0f, 22 - e) : 1.0f;
-        if (c == 0) {
-            const float as = bad ? __int_as_float(0x7fc00000) : 1.0f / sc;  // a non-finite input row gives NaN outputs
-            sm_ascale[m] = as;
-            if (publish) p.ascale_g[m] = as;
-        }
+        const int i = threadIdx.x + k * kLeanThreads, m = M > 1 && i >= per ? 1 : 0, c = i - m * per;
+        if (i >= total) break;
         float v[8];
-        if constexpr (HALF) {
-            lean_unpack<ActT>(keep[k], v);
-        } else {
-            uint4 none;
-            fetch(act + (size_t)m * p.K + 8 * c, v, none);
-        }
-        uint32_t l[3][2] = {};
+        values(i, keep[k], v);
+        uint32_t l[3][2];
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            int A = bad ? 0 : __float2int_rn(v[j] * sc);
-            const int d0 = (int)(int8_t)(A & 0xFF);
-            A = (A - d0) >> 8;
-            const int d1 = (int)(int8_t)(A & 0xFF);
-            A = (A - d1) >> 8;
-            l[0][j >> 2] |= (uint32_t)(d0 & 0xFF) << (8 * (j & 3));
-            l[1][j >> 2] |= (uint32_t)(d1 & 0xFF) << (8 * (j & 3));
-            l[2][j >> 2] |= (uint32_t)(A & 0xFF) << (8 * (j & 3));
-        }
+        for (int h = 0; h < 2; h++) limbs_of_4(v + 4 * h, M > 1 && m ? sc[M - 1] : sc[0], l[0][h], l[1][h], l[2][h]);
 #pragma unroll
         for (int x = 0; x < 3; x++) {
             *reinterpret_cast<uint2 *>(sm_limbs + (size_t)(3 * m + x) * pitch + 8 * c) = make_uint2(l[x][0], l[x][1]);
-            if (publish) *reinterpret_cast<uint2 *>(p.limbs_g + (size_t)(3 * m + x) * p.K + 8 * c) = make_uint2(l[x][0], l[x][1]);
+            if (blockIdx.x == 0) *reinterpret_cast<uint2 *>(p.limbs_g + (size_t)(3 * m + x) * p.K + 8 * c) = make_uint2(l[x][0], l[x][1]);
         }
     }
 }
@@ -182,15 +154,20 @@ __device__ __forceinline__ void mma_i8(int (&c)[4], uint32_t a0, uint32_t a1, ui
 // One CTA per SM owns a contiguous range of weight rows, so that the whole grid is one balanced wave.  A warp owns NB blocks of 64 along K
 // (K <= 1024 NB) of all of them; TG tiles of 16 rows are in flight (2 NB TG <= 20 loads per lane, issued before anything else happens).
 // K % 16 == 0; wq and limbs 16-byte aligned.  Dynamic shared memory: limbs [3 M][pitch] (ACT), partial sums [warp][3 M][kLeanPitch].
-template <typename OutT, int M, int NB, int TG, bool ACT>
+// GATED: wq holds 2 N rows, N gate rows and behind them the N up rows of the same outputs, and out[m,n] = round(swish(gate) * up) of the two sums,
+// each rounded first.  A tile is eight gate rows and their eight up rows, so both sums of an output lie in one column of the partial sums.
+// TinyLlama shapes, us per layer at 1 / 3 rows: gate/up, SiLU product to limbs, down 3.1 + 3.1 + 2.0 / 4.8 + 3.6 + 2.8; gated, row to limbs, down
+// 2.9 + 1.6 + 2.4 / 4.8 + 1.7 + 2.8.
+template <typename OutT, int M, int NB, int TG, bool ACT, bool GATED>
 __global__ void __launch_bounds__(kLeanThreads, 1) gemv_lean_kernel(const LeanParams p) {
     extern __shared__ __align__(16) int8_t sm_dyn[];
     __shared__ float sm_ascale[8];
-    __shared__ unsigned sm_max[8];
+    __shared__ unsigned sm_max[2][kLeanWarps];
     constexpr int C = 3 * M, NT = (C + 7) / 8;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, t = lane & 3;
     const int K = p.K, chunks = K >> 4, pitch = lean_limb_pitch(K);
-    const int row0 = blockIdx.x * p.rows_per_cta, rows = min(p.rows_per_cta, p.N - row0), tiles = (rows + 15) >> 4;
+    constexpr int kTileOut = GATED ? 8 : 16;  // outputs per tile of 16 rows
+    const int row0 = blockIdx.x * p.rows_per_cta, rows = min(p.rows_per_cta, p.N - row0), tiles = (rows + kTileOut - 1) / kTileOut;  // in outputs
     int8_t *sm_limbs = sm_dyn;
     int *sm_sum = reinterpret_cast<int *>(sm_dyn + (ACT ? (size_t)C * pitch : 0));
     const OutT *scale_p = reinterpret_cast<const OutT *>(p.scale);
@@ -202,8 +179,8 @@ __global__ void __launch_bounds__(kLeanThreads, 1) gemv_lean_kernel(const LeanPa
     auto load_tile = [&](uint4 (&x)[NB][2], int tile) {
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-            const int row = 16 * tile + gq + 8 * h;
-            const int8_t *wr = p.wq + (size_t)(row0 + (row < rows ? row : 0)) * K;
+            const int row = kTileOut * tile + gq + (GATED ? 0 : 8 * h);
+            const int8_t *wr = p.wq + (size_t)(row0 + (row < rows ? row : 0) + (GATED && h ? p.N : 0)) * K;
 #pragma unroll
             for (int j = 0; j < NB; j++) {
                 const int c = c0 + 4 * j;
@@ -213,7 +190,7 @@ __global__ void __launch_bounds__(kLeanThreads, 1) gemv_lean_kernel(const LeanPa
     };
     // settled: the first tiles of weights and the row scale of this thread's output depend on nothing an earlier kernel writes; else the
     // weights only travel to L2 ahead of the wait
-    if (!p.settled) {
+    if (!GATED && !p.settled) {
         const int8_t *w0 = p.wq + (size_t)row0 * K;
 #pragma unroll 1
         for (int i = 128 * threadIdx.x; i < min(rows, 16 * TG) * K; i += 128 * kLeanThreads) prefetch_l2(w0 + i);
@@ -223,16 +200,13 @@ __global__ void __launch_bounds__(kLeanThreads, 1) gemv_lean_kernel(const LeanPa
     for (int i = 0; i < TG; i++)
         if (i < tiles) load_tile(w[i], i);
     // outputs of the first pass: thread -> (row, activation row)
-    const int pass_rows = min(rows, 16 * kLeanTiles), my_m = threadIdx.x / pass_rows, my_r = threadIdx.x - my_m * pass_rows;
-    float wscale_first = 0.f, resv_first = 0.f;
+    const int pass_rows = min(rows, kTileOut * kLeanTiles), my_m = threadIdx.x / pass_rows, my_r = threadIdx.x - my_m * pass_rows;
+    float wscale_first = 0.f, resv_first = 0.f;  // GATED: the gate's and the up row's scale
     if (my_m < M) wscale_first = to_f32<OutT>(scale_p[row0 + my_r]);
-    if constexpr (ACT) {
-        if (threadIdx.x < 8) sm_max[threadIdx.x] = 0u;
-        __syncthreads();
-    }
+    if (GATED && my_m < M) resv_first = to_f32<OutT>(scale_p[p.N + row0 + my_r]);
     pdl_trigger();
     pdl_wait();
-    if (my_m < M && resid_p) resv_first = to_f32<OutT>(resid_p[(size_t)my_m * p.N + row0 + my_r]);
+    if (!GATED && my_m < M && resid_p) resv_first = to_f32<OutT>(resid_p[(size_t)my_m * p.N + row0 + my_r]);
     // limbs of this warp's piece of K: column gq (and gq + 8) of the MMAs is limb row gq (gq + 8) = 3 m + l
     uint4 b[NT][NB];
     if constexpr (ACT) {
@@ -293,20 +267,32 @@ __global__ void __launch_bounds__(kLeanThreads, 1) gemv_lean_kernel(const LeanPa
             }
         }
         __syncthreads();
-        const int beg = 16 * first, n_rows = min(rows, 16 * last) - beg;
+        const int beg = kTileOut * first, n_rows = min(rows, kTileOut * last) - beg;
         for (int i = threadIdx.x; i < n_rows * M; i += kLeanThreads) {
             const int m = i / n_rows, r = i - m * n_rows, row = row0 + beg + r;
             const bool known = first == 0 && i == (int)threadIdx.x;  // requested at the top of the kernel
             const float wscale = known ? wscale_first : to_f32<OutT>(scale_p[row]);
-            const float resv = known ? resv_first : resid_p ? to_f32<OutT>(resid_p[(size_t)m * p.N + row]) : 0.f;
-            int v[3] = {0, 0, 0};
+            // the sum of one row of the tiles, times both scales
+            auto row_value = [&](int at, float ws) {
+                int v[3] = {0, 0, 0};
 #pragma unroll
-            for (int x = 0; x < kLeanWarps; x++)
+                for (int x = 0; x < kLeanWarps; x++)
 #pragma unroll
-                for (int l = 0; l < 3; l++) v[l] += sm_sum[(x * C + 3 * m + l) * kLeanPitch + r];
-            const long long sum = (long long)v[2] * 65536 + (long long)v[1] * 256 + (long long)v[0];
-            float y = __fmul_rn(__fmul_rn((float)sum, sm_ascale[m]), wscale);
-            if (resid_p) y = __fadd_rn(round_store<OutT>(y), resv);
+                    for (int l = 0; l < 3; l++) v[l] += sm_sum[(x * C + 3 * m + l) * kLeanPitch + at];
+                const long long sum = (long long)v[2] * 65536 + (long long)v[1] * 256 + (long long)v[0];
+                return __fmul_rn(__fmul_rn((float)sum, sm_ascale[m]), ws);
+            };
+            float y;
+            if constexpr (GATED) {
+                const float uscale = known ? resv_first : to_f32<OutT>(scale_p[p.N + row]);
+                const int at = 16 * (r >> 3) + (r & 7);
+                const float g = round_store<OutT>(row_value(at, wscale)), u = round_store<OutT>(row_value(at + 8, uscale));
+                y = (g / (1.0f + expf(-g))) * u;
+            } else {
+                const float resv = known ? resv_first : resid_p ? to_f32<OutT>(resid_p[(size_t)m * p.N + row]) : 0.f;
+                y = row_value(r, wscale);
+                if (resid_p) y = __fadd_rn(round_store<OutT>(y), resv);
+            }
             out_p[(size_t)m * p.N + row] = from_f32<OutT>(y);
         }
         if (last < tiles) __syncthreads();  // the sums are read before the next tiles' replace them
@@ -326,10 +312,10 @@ bool gemv_lean_supported(int M, int N, int K, const void *wq) {
     return M >= 1 && M <= kLeanMaxRows && K >= 16 && K % 16 == 0 && K <= 6144 && (size_t)N * K <= ((size_t)(M <= 2 ? 160 : 32) << 20) && ((uintptr_t)wq % 16) == 0;
 }
 
-template <typename OutT, int M, int NB, int TG, bool ACT>
+template <typename OutT, int M, int NB, int TG, bool ACT, bool GATED>
 static int launch_lean(cudaStream_t st, LeanParams p) {
     const size_t smem = lean_smem(ACT, M, p.K);
-    auto kern = gemv_lean_kernel<OutT, M, NB, TG, ACT>;
+    auto kern = gemv_lean_kernel<OutT, M, NB, TG, ACT, GATED>;
     static SmemLimit limit;
     MYNN_CUDA_OK(limit.raise((const void *)kern, kLeanMaxSmem));
     static int sms = 0;
@@ -340,7 +326,12 @@ static int launch_lean(cudaStream_t st, LeanParams p) {
     }
     // One CTA per SM, each with an equal share of the rows; a few SMs stay free, where the CTAs of the row kernel behind this one (launched
     // as its dependent) are resident by the time it ends.
-    const int ctas = sms > 4 * kLeanFreeSms ? sms - kLeanFreeSms : sms, rpc = (p.N + ctas - 1) / ctas;
+    const int ctas = sms > 4 * kLeanFreeSms ? sms - kLeanFreeSms : sms;
+    int rpc = (p.N + ctas - 1) / ctas;
+    // Whole tiles where half of the free SMs pay for them: 11264 rows are 139 x 81, the last row of each share a tile of its own that is
+    // loaded behind the others, or 141 x 80.
+    const int tile = GATED ? 8 : 16, whole = rpc / tile * tile;
+    if (whole > 0 && (p.N + whole - 1) / whole <= ctas + kLeanFreeSms / 2) rpc = whole;
     p.rows_per_cta = rpc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((p.N + rpc - 1) / rpc);
@@ -358,12 +349,12 @@ static int launch_lean(cudaStream_t st, LeanParams p) {
 }
 
 // blocks of 64 per warp (K <= 1024 / 2048 / 4096 / 6144) and row tiles in flight
-template <typename OutT, int M, bool ACT>
+template <typename OutT, int M, bool ACT, bool GATED = false>
 static int launch_by_k(cudaStream_t st, const LeanParams &p) {
-    if (p.K <= 1024) return launch_lean<OutT, M, 1, 8, ACT>(st, p);
-    if (p.K <= 2048) return launch_lean<OutT, M, 2, 5, ACT>(st, p);
-    if (p.K <= 4096) return launch_lean<OutT, M, 4, 2, ACT>(st, p);
-    return launch_lean<OutT, M, 6, 1, ACT>(st, p);
+    if (p.K <= 1024) return launch_lean<OutT, M, 1, 8, ACT, GATED>(st, p);
+    if (p.K <= 2048) return launch_lean<OutT, M, 2, 5, ACT, GATED>(st, p);
+    if (p.K <= 4096) return launch_lean<OutT, M, 4, 2, ACT, GATED>(st, p);
+    return launch_lean<OutT, M, 6, 1, ACT, GATED>(st, p);
 }
 template <typename OutT>
 static int launch_by_rows(cudaStream_t st, const LeanParams &p, int M) {
@@ -375,6 +366,34 @@ static int launch_by_rows(cudaStream_t st, const LeanParams &p, int M) {
         default: return launch_by_k<OutT, 5, false>(st, p);
     }
 }
+template <typename OutT>
+static int launch_gated_by_rows(cudaStream_t st, const LeanParams &p, int M) {
+    switch (M) {
+        case 1: return launch_by_k<OutT, 1, false, true>(st, p);
+        case 2: return launch_by_k<OutT, 2, false, true>(st, p);
+        case 3: return launch_by_k<OutT, 3, false, true>(st, p);
+        case 4: return launch_by_k<OutT, 4, false, true>(st, p);
+        default: return launch_by_k<OutT, 5, false, true>(st, p);
+    }
+}
+
+int gemv_lean_gated_launch(cudaStream_t st, void *out, const int8_t *wq, const void *scale, int M, int F, int K, int dtype, void *workspace, size_t workspace_bytes) {
+    const size_t need = i8_gemm_workspace_bytes(M, K);
+    if (!workspace || workspace_bytes < need || (uintptr_t)workspace % 256)
+        return fail(MYNN_E_ARG, "gated product: workspace of %zu bytes (256-byte aligned) needed", need);
+    LeanParams p = {};
+    p.out = out;
+    p.wq = wq;
+    p.scale = scale;
+    p.ascale_g = (float *)((char *)workspace + 256);
+    p.limbs_g = (int8_t *)workspace + 512;
+    p.N = F;
+    p.K = K;
+    p.act_dtype = dtype;
+    p.settled = 1;
+    MYNN_DISPATCH_DTYPE(dtype, T, return launch_gated_by_rows<T>(st, p, M));
+    return MYNN_OK;
+}
 
 // Same contract as i8_gemm_launch: `workspace` holds status word, row scales and the limb matrix; act == nullptr means a fused
 // producer (or the previous call) left the limbs there.
@@ -383,8 +402,10 @@ int gemv_lean_launch(cudaStream_t st, void *out, const void *act, const int8_t *
     const size_t need = i8_gemm_workspace_bytes(M, K);
     if (!workspace || workspace_bytes < need || (uintptr_t)workspace % 256)
         return fail(MYNN_E_ARG, "dequant_matmul: workspace of %zu bytes (256-byte aligned) needed", need);
-    // Every CTA makes the limbs of one or two rows itself; of more, a kernel in front does (three rows of 2048: 5.0 us inside, 2.2 + 2.3 so).
-    if (act && M > 2) {
+    // In a step the limbs are made by a row kernel in front, which is resident when the kernel before it ends (1.6 us; inside, a row of 2048 takes 0.5 to
+    // 0.9 us more than without and a row of 5632 2.7).  Operators come one by one and make those of one or two rows inside (5632 x 2048, one row: 4.4 us
+    // against 4.9; 4096 x 4096 5.4 against 5.9), of more in front (three rows of 2048: 5.0 us inside, 2.2 + 2.3 so).
+    if (act && (M > 2 || settled)) {
         if (int rc = launch_act_limbs(st, act, M, K, act_dtype, (int8_t *)workspace + 512, (float *)((char *)workspace + 256))) return rc;
         act = nullptr;
     }

@@ -31,6 +31,7 @@
 
 #include "common.cuh"
 #include "i8_gemm.cuh"
+#include "limbs.cuh"
 #include "tcgen05.cuh"
 #include "tp_fused.cuh"
 
@@ -463,18 +464,8 @@ __global__ void __launch_bounds__(256) act_to_limbs_kernel(int8_t *limbs, float 
     if (threadIdx.x == 0) ascale[m] = anybad ? __int_as_float(0x7fc00000) : 1.0f / sc;  // non-finite input -> NaN outputs
     int8_t *l0 = limbs + (size_t)(3 * m) * K, *l1 = l0 + K, *l2 = l1 + K;
     auto split4 = [&](const float (&x)[4], int gi) {
-        uint32_t w0 = 0, w1 = 0, w2 = 0;
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            int A = anybad ? 0 : __float2int_rn(x[i] * sc);
-            const int d0 = (int)(int8_t)(A & 0xFF);
-            A = (A - d0) >> 8;
-            const int d1 = (int)(int8_t)(A & 0xFF);
-            A = (A - d1) >> 8;
-            w0 |= (uint32_t)(d0 & 0xFF) << (8 * i);
-            w1 |= (uint32_t)(d1 & 0xFF) << (8 * i);
-            w2 |= (uint32_t)(A & 0xFF) << (8 * i);
-        }
+        uint32_t w0, w1, w2;
+        limbs_of_4(x, anybad ? 0.f : sc, w0, w1, w2);
         reinterpret_cast<uint32_t *>(l0)[gi] = w0;
         reinterpret_cast<uint32_t *>(l1)[gi] = w1;
         reinterpret_cast<uint32_t *>(l2)[gi] = w2;
@@ -550,18 +541,8 @@ __device__ __forceinline__ void smem_row_to_limbs(const float *row_s, int K, int
     for (int gi = threadIdx.x; gi < (K >> 2); gi += blockDim.x) {
         const float4 x4 = reinterpret_cast<const float4 *>(row_s)[gi];
         const float x[4] = {x4.x, x4.y, x4.z, x4.w};
-        uint32_t w0 = 0, w1 = 0, w2 = 0;
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            int A = sc == 0.f ? 0 : __float2int_rn(x[i] * sc);
-            const int d0 = (int)(int8_t)(A & 0xFF);
-            A = (A - d0) >> 8;
-            const int d1 = (int)(int8_t)(A & 0xFF);
-            A = (A - d1) >> 8;
-            w0 |= (uint32_t)(d0 & 0xFF) << (8 * i);
-            w1 |= (uint32_t)(d1 & 0xFF) << (8 * i);
-            w2 |= (uint32_t)(A & 0xFF) << (8 * i);
-        }
+        uint32_t w0, w1, w2;
+        limbs_of_4(x, sc, w0, w1, w2);
         l0[gi] = w0;
         l1[gi] = w1;
         l2[gi] = w2;
@@ -628,13 +609,31 @@ rms_norm_limbs_kernel(int8_t *limbs, float *ascale, T *norm_out, T *sum_out, con
     MYNN_GLUE_END();
 }
 
+// Eight elements per thread of a row in registers -> limbs (out: this thread's place in the first limb row).
+__device__ __forceinline__ void row_registers_to_limbs(const float (&v)[8], bool in, uint32_t *red /* 32 */, int warps, float *ascale_m, int8_t *out, int K) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t mine = __reduce_max_sync(0xffffffffu, in ? max_bits8(v) : 0u);
+    if (lane == 0) red[warp] = mine;
+    __syncthreads();
+    const float sc = limb_scale(__reduce_max_sync(0xffffffffu, lane < warps ? red[lane] : 0u));
+    if (threadIdx.x == 0) *ascale_m = limb_unscale(sc);
+    if (in) {
+        uint32_t l[3][2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) limbs_of_4(v + 4 * h, sc, l[0][h], l[1][h], l[2][h]);
+#pragma unroll
+        for (int k = 0; k < 3; k++) *reinterpret_cast<uint2 *>(out + (size_t)k * K) = make_uint2(l[k][0], l[k][1]);
+    }
+}
+
 // The same for rows of at most 8 elements per thread, which stay in registers (blockDim.x = D / 8 rounded up to whole warps).  A row or a
 // few is a chain of dependent steps, so they are kept short: the norm's weights, which belong to the model, are requested in front of the
 // wait for the preceding kernel, and both block reductions are finished by every thread for itself.
 template <typename T>
 __global__ void __launch_bounds__(kRowThreads)
 rms_norm_limbs_row_kernel(int8_t *limbs, float *ascale, T *norm_out, T *sum_out, const T *x, const float *part, const T *w, float eps, int D) {
-    __shared__ float red_s[32], red_m[32];
+    __shared__ float red_s[32];
+    __shared__ uint32_t red_m[32];
     MYNN_GLUE_BEGIN(1);
     pdl_trigger();
     const int m = blockIdx.x, i0 = 8 * threadIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
@@ -664,41 +663,10 @@ rms_norm_limbs_row_kernel(int8_t *limbs, float *ascale, T *norm_out, T *sum_out,
     float tot = 0.f;
     for (int i = 0; i < warps; i++) tot += red_s[i];
     const float inv = 1.0f / sqrtf(tot / (float)D + eps);
-    float mx = 0.f;
-    bool bad = false;
 #pragma unroll
-    for (int j = 0; j < 8; j++) {
-        v[j] = round_store<T>(v[j] * inv * wv[j]);
-        bad |= !(fabsf(v[j]) <= 3.0e38f);
-        mx = fmaxf(mx, fabsf(v[j]));
-    }
+    for (int j = 0; j < 8; j++) v[j] = round_store<T>(v[j] * inv * wv[j]);
     if (in && norm_out != nullptr) store8<T>(norm_out + base + i0, v);
-    mx = warp_max(mx);
-    if (lane == 0) red_m[warp] = mx;
-    const unsigned anybad = __syncthreads_or(in && bad);
-    float top = red_m[0];
-    for (int i = 1; i < warps; i++) top = fmaxf(top, red_m[i]);
-    int e = 0;
-    if (top > 0.f) frexpf(top, &e);
-    const float sc1 = top > 0.f ? ldexpf(1.0f, 22 - e) : 1.0f, sc = anybad ? 0.f : sc1;
-    if (threadIdx.x == 0) ascale[m] = anybad ? __int_as_float(0x7fc00000) : 1.0f / sc1;  // non-finite input -> NaN outputs
-    if (in) {
-        uint32_t l[3][2] = {};
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            int A = sc == 0.f ? 0 : __float2int_rn(v[j] * sc);
-            const int d0 = (int)(int8_t)(A & 0xFF);
-            A = (A - d0) >> 8;
-            const int d1 = (int)(int8_t)(A & 0xFF);
-            A = (A - d1) >> 8;
-            l[0][j >> 2] |= (uint32_t)(d0 & 0xFF) << (8 * (j & 3));
-            l[1][j >> 2] |= (uint32_t)(d1 & 0xFF) << (8 * (j & 3));
-            l[2][j >> 2] |= (uint32_t)(A & 0xFF) << (8 * (j & 3));
-        }
-        int8_t *out = limbs + (size_t)(3 * m) * D + i0;
-#pragma unroll
-        for (int k = 0; k < 3; k++) *reinterpret_cast<uint2 *>(out + (size_t)k * D) = make_uint2(l[k][0], l[k][1]);
-    }
+    row_registers_to_limbs(v, in, red_m, warps, ascale + m, limbs + (size_t)(3 * m) * D + i0, D);
     MYNN_GLUE_END();
 }
 
@@ -788,9 +756,22 @@ swiglu_limbs_cluster_kernel(int8_t *limbs, float *ascale, const T *gate, const T
     MYNN_GLUE_END_C();
 }
 
-// Plain pre-pass in the same style (one 1024-thread CTA per row, 16-byte loads): act -> limbs.  K % 8 == 0.
+// Plain pre-pass: act -> limbs.  K % 8 == 0, rows 16-byte aligned.  Rows of at most 8 elements per thread stay in registers.
 template <typename T>
 __global__ void __launch_bounds__(kRowThreads) act_limbs_row_kernel(int8_t *limbs, float *ascale, const T *act, int K) {
+    __shared__ uint32_t red[32];
+    pdl_trigger();
+    pdl_wait();
+    const int m = blockIdx.x, i0 = 8 * threadIdx.x;
+    const bool in = i0 < K;
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) v[j] = 0.f;
+    if (in) load8<T>(act + (size_t)m * K + i0, v);
+    row_registers_to_limbs(v, in, red, blockDim.x >> 5, ascale + m, limbs + (size_t)(3 * m) * K + i0, K);
+}
+template <typename T>
+__global__ void __launch_bounds__(kRowThreads) act_limbs_long_row_kernel(int8_t *limbs, float *ascale, const T *act, int K) {
     extern __shared__ __align__(16) float row_s[];
     __shared__ float red[40];
     pdl_trigger();
@@ -918,8 +899,10 @@ int launch_act_limbs(cudaStream_t st, const void *act, int M, int K, int act_dty
     const bool row_kernel = K % 8 == 0 && (size_t)K * 4 <= 200 * 1024 && ((uintptr_t)act % 16) == 0;
     const size_t smem = (size_t)K * 4;
 #define PREP(T)                                                                                                          \
-    if (row_kernel) {                                                                                                    \
-        auto kern = act_limbs_row_kernel<T>;                                                                             \
+    if (row_kernel && K <= 8 * kRowThreads) {                                                                            \
+        MYNN_CUDA_OK(launch_dependent(act_limbs_row_kernel<T>, dim3(M), dim3((K / 8 + 31) / 32 * 32), 0, st, limbs, ascale, (const T *)act, K)); \
+    } else if (row_kernel) {                                                                                             \
+        auto kern = act_limbs_long_row_kernel<T>;                                                                        \
         if (smem > 48 * 1024) MYNN_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
         MYNN_CUDA_OK(launch_dependent(kern, dim3(M), dim3(kRowThreads), smem, st, limbs, ascale, (const T *)act, K));    \
     } else {                                                                                                             \

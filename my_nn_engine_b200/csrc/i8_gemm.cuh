@@ -21,6 +21,10 @@ int i8_gemm_launch(cudaStream_t st, void *out, const void *act, const int8_t *wq
 bool gemv_lean_supported(int M, int N, int K, const void *wq);
 int gemv_lean_launch(cudaStream_t st, void *out, const void *act, const int8_t *wq, const void *scale, const void *resid, int M, int N,
                      int K, int act_dtype, int out_dtype, void *workspace, size_t workspace_bytes, bool settled);
+// Gate and up products of a model's step with the SiLU product in the finish: wq [2 F, K], F gate rows and behind them the up rows, scale [2 F];
+// out[m,f] = round(swish(round(gate)) * round(up)), M rows of F.  Limbs and row scales are in the workspace, weights and scales settled; sizes as for
+// gemv_lean_supported(M, 2 F, K, wq).
+int gemv_lean_gated_launch(cudaStream_t st, void *out, const int8_t *wq, const void *scale, int M, int F, int K, int dtype, void *workspace, size_t workspace_bytes);
 int launch_act_limbs(cudaStream_t st, const void *act, int M, int K, int act_dtype, int8_t *limbs, float *ascale);
 struct I8Tp;  // tp_fused.cuh
 int i8_gemm_launch_tp(cudaStream_t st, void *out, const void *act, const int8_t *wq, const void *scale, const void *resid,

@@ -242,9 +242,14 @@ static int enqueue_forward(Model &m, cudaStream_t st, int S, int head_rows = 0) 
             RC(norm(L.ln2, m.part, M, m.x));  // x = round(x + round(sum of partials)), then the norm
         }
         // --- MLP block ---
-        const bool fuse_mlp = fused && L.gu_fused;
+        // A few rows: the lean gate/up product finishes the SiLU product as well, and the limbs of its rows are made inside the down product, or by the
+        // row kernel in front of it.
+        const bool gated = fused && L.gu_fused && tp == 1 && !reduced_limbs && gemv_lean_supported(M, 2 * m.ffn, H, L.wg);
+        const bool fuse_mlp = fused && L.gu_fused && !gated;
         bool h_limbs2 = false;  // Swish*Mul left two-limb rows in the workspace instead of m.h
-        if (L.gu_fused) {
+        if (gated) {
+            RC(gemv_lean_gated_launch(st, m.h, L.wg, L.sg, M, m.ffn, H, dt, m.gemm_ws, m.gemm_ws_bytes));
+        } else if (L.gu_fused) {
             RC(gemm_n(m.gu, L.wg, L.sg, M, 2 * m.ffn, dt));
             const char *up_ = (char *)m.gu + (size_t)m.ffn * esz;
             if (fuse_mlp) {

@@ -68,6 +68,23 @@ def test_small_batches_step_like_a_large_one(dt, hidden, ffn):
         assert torch.equal(rows[batch], rows[8][:batch])
 
 
+# gate/up products with the SiLU product in their finish: more than one pass over the partial sums, last shares of a few outputs, each number of blocks along K
+@pytest.mark.parametrize("dt", ["bf16", "f16", "f32"])
+@pytest.mark.parametrize("hidden,ffn", [(128, 9104), (1152, 1136), (2112, 304), (4160, 80)])
+def test_gated_products_step_like_a_large_batch(dt, hidden, ffn):
+    from my_nn_engine_b200.decoder import DecoderModel
+    from my_nn_engine_b200.quantize import random_llama_state
+    cfg = dict(hidden_size=hidden, num_hidden_layers=1, num_attention_heads=2, num_key_value_heads=1, head_dim=64, intermediate_size=ffn, vocab_size=300,
+               rms_norm_eps=1e-5, rope_theta=1e4)
+    state, tokens, rows = random_llama_state(cfg, seed=5), np.arange(8) * 37 % 300, {}
+    for batch in (1, 2, 3, 4, 5, 8):
+        model = DecoderModel(cfg, state, dtype=dt, max_seq_len=32, batch=batch)
+        rows[batch] = model.step(tokens[:batch], 0).clone()
+        model.close()
+    for batch in (1, 2, 3, 4, 5):
+        assert torch.equal(rows[batch], rows[8][:batch])
+
+
 # ---- products of many int8 rows: tile widths, ragged last tiles ----
 @pytest.mark.parametrize("m,n,k", [(257, 3001, 1040), (520, 128, 2064), (777, 14336, 256), (2047, 640, 512), (1500, 5632, 128), (40, 130, 16)])
 def test_w8a8_product_is_exact(m, n, k):

@@ -48,7 +48,9 @@ MYNN_DEFINE_WAIT_BUDGET_SETTER(attention_decode)
 
 // WIN: a sliding window over a ring cache and a score soft cap (DecodeParams::window, ring_cache, softcap).
 // W: warps per CTA.
-template <typename T, int D, bool RING, bool WIN, int W>
+// STREAM: the fused form over a streaming cache (DecodeParams::kvpos).  The tables of a tile are fetched while the tile before it is computed.  (In
+// front of it stood a kernel that wrote rotated copies of all live keys, and one for the append: 3.6 + 1.8 us of a layer's step at two sequences of 1024 rows.)
+template <typename T, int D, bool RING, bool WIN, int W, bool STREAM = false>
 __global__ void __launch_bounds__(W * 32, W > kAttnWarps ? 1 : RING ? 2 : 4)
 attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const DecodeParams p) {
     constexpr int KS = D / 16;   // k16 steps of QK^T
@@ -65,7 +67,11 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     // rows [lo, active) are seen; the walk starts at the 16-row tile that holds lo (0 without a window)
     const int lo = WIN ? max(active > 0 ? first_visible(active - 1, p.window, p.chunk) : 0, p.ring_cache ? active - p.cache_seq : 0) : 0, walk0 = lo & ~15;
     // whole rounds of the CTA's warps (64 rows of four): a split that ends inside a round leaves some warps a tile short
-    const int rows_per_split = (((active - walk0 + p.splits - 1) / p.splits) + 16 * W - 1) / (16 * W) * (16 * W);
+    // A cluster whose rows are two rounds or less leaves them to its first CTA: the merge takes about as long as a round.
+    const bool solo = p.cluster && active - walk0 <= 2 * 16 * W;
+    if (solo && split > 0) return;
+    const int splits = solo ? 1 : p.splits;
+    const int rows_per_split = (((active - walk0 + splits - 1) / splits) + 16 * W - 1) / (16 * W) * (16 * W);
     const int row_beg = walk0 + split * rows_per_split;
     const int row_end = min(row_beg + rows_per_split, active);
 
@@ -77,7 +83,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     const size_t tab = fused ? (size_t)(*p.fused_pos) * D : 0;
     const T *cos_t = reinterpret_cast<const T *>(p.cos_t), *sin_t = reinterpret_cast<const T *>(p.sin_t);
     // the rows this CTA reads from the cache: with the fused append the new row is not there yet
-    const int cache_end = fused ? min(row_end, new_row) : row_end;
+    const int cache_end = fused && !STREAM ? min(row_end, new_row) : row_end;
 
     // Ring set-up and the copies of the first tiles come first: they travel while the query fragments are built.
     extern __shared__ __align__(1024) uint8_t ring_raw[];
@@ -104,6 +110,37 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
             }
         }
     };
+    // STREAM: table rows of the two keys of this lane in the next tile, and the position of those in the tile after it
+    uint4 key_cos[STREAM ? 2 : 1][KCH], key_sin[STREAM ? 2 : 1][KCH];
+    int key_pos[2] = {};
+    auto fetch_positions = [&](int j) {
+#pragma unroll
+        for (int nt = 0; nt < 2; nt++) key_pos[nt] = (int)p.kvpos[min(first + 16 * W * j + 8 * nt + g, p.cache_seq - 1)];
+    };
+    auto fetch_tables = [&]() {
+        if constexpr (STREAM) {
+#pragma unroll
+            for (int nt = 0; nt < 2; nt++)
+#pragma unroll
+                for (int i = 0; i < KCH; i++) {
+                    const size_t at = (size_t)key_pos[nt] * D + 8 * t + 32 * i;
+                    key_cos[nt][i] = *reinterpret_cast<const uint4 *>(cos_t + at);
+                    key_sin[nt][i] = *reinterpret_cast<const uint4 *>(sin_t + at);
+                }
+        }
+    };
+    // eight elements x of a key against their partners half a head away
+    auto rotate_key = [](const uint4 &x, const uint4 &xp, const uint4 &c, const uint4 &sn, bool low) {
+        const T *xe = reinterpret_cast<const T *>(&x), *pe = reinterpret_cast<const T *>(&xp), *ce = reinterpret_cast<const T *>(&c), *se = reinterpret_cast<const T *>(&sn);
+        uint4 r;
+        T *re = reinterpret_cast<T *>(&r);
+#pragma unroll
+        for (int e = 0; e < 8; e++) {
+            const float a = to_f32<T>(xe[e]), b_ = to_f32<T>(pe[e]), ce_ = to_f32<T>(ce[e]), se_ = to_f32<T>(se[e]);
+            re[e] = from_f32<T>(low ? a * ce_ - b_ * se_ : a * ce_ + b_ * se_);
+        }
+        return r;
+    };
     if constexpr (RING) {
         if (threadIdx.x == 0) abort_flag = 0;
         if (lane == 0) {
@@ -118,6 +155,11 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         if (lane == 0 && settled) {
             const int written = fused ? 0 : slot(*p.appended);
             for (; j < min(ntile, kRingDepth) && (fused || (unsigned)(written - slot(first + 16 * W * j)) >= 16u); j++) issue(j);
+        }
+        if constexpr (STREAM) {  // positions and tables were there before the step
+            fetch_positions(0);
+            fetch_tables();
+            fetch_positions(1);
         }
         pdl_wait();
         if (lane == 0)
@@ -188,8 +230,8 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         for (int i = 0; i < 4; i++) o[j][i] = 0.f;
     float m_run = -INFINITY, l_run = 0.f;
 
-    // One 16-row tile whose K / V fragments are in registers: rows base .. base+15, of which those below `end` count.
-    auto tile = [&](const uint4 (&kr)[2][KCH], const uint4 (&vr)[4][VH], int base, int end) {
+    // One 16-row tile whose K / V fragments are in registers: rows base .. base+15, of which those below `end` count (STREAM: but row `skip`).
+    auto tile = [&](const uint4 (&kr)[2][KCH], const uint4 (&vr)[4][VH], int base, int end, int skip = -1) {
         // ---- S = Q K^T: s[nt][e] = S[head g][kv row base + 8nt + 2t + e] ----
         float s[2][4];
 #pragma unroll
@@ -211,19 +253,19 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                 const int row = base + 8 * nt + 2 * t + e;
                 const float x = s[nt][e] * p.scale;
                 if constexpr (WIN) pv[nt][e] = row < end && row >= lo ? (p.softcap > 0.f ? fast_soft_cap(x, p.softcap) : x) : -INFINITY;
-                else pv[nt][e] = row < end ? x : -INFINITY;
+                else pv[nt][e] = row < end && (!STREAM || row != skip) ? x : -INFINITY;
                 tmax = fmaxf(tmax, pv[nt][e]);
             }
         tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 1));
         tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 2));
-        const float m_new = fmaxf(m_run, tmax);  // finite: the tile has at least one valid row
-        const float alpha = __expf(m_run - m_new);
+        const float m_new = fmaxf(m_run, tmax);  // finite: the tile has at least one valid row (STREAM: unless that is the skipped one)
+        const float m_ref = STREAM && m_new == -INFINITY ? 0.f : m_new, alpha = __expf(m_run - m_ref);
         float psum = 0.f;
 #pragma unroll
         for (int nt = 0; nt < 2; nt++)
 #pragma unroll
             for (int e = 0; e < 2; e++) {
-                pv[nt][e] = __expf(pv[nt][e] - m_new);
+                pv[nt][e] = __expf(pv[nt][e] - m_ref);
                 psum += pv[nt][e];
             }
         l_run = l_run * alpha + psum;  // per-lane partial; lanes of a group are summed at the end
@@ -287,7 +329,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
 #pragma unroll
             for (int r = 0; r < 4; r++) {
                 const int row = 2 * t + (r & 1) + 8 * (r >> 1);
-                const bool live = base + row < cache_end;  // rows past the end may hold anything: keep them out of P V
+                const bool live = base + row < cache_end && (!STREAM || base + row != new_row);  // rows past the end may hold anything: keep them out of P V
 #pragma unroll
                 for (int h = 0; h < VH; h++) {
                     const uint4 w = *reinterpret_cast<const uint4 *>(st + (NB + h) * kBox + row * 128 + ((g ^ (row & 7)) << 4));
@@ -299,7 +341,18 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 issue(j + kRingDepth);
             }
-            tile(kr, vr, base, cache_end);
+            if constexpr (STREAM) {
+                uint4 rot[2][KCH];
+#pragma unroll
+                for (int nt = 0; nt < 2; nt++)
+#pragma unroll
+                    for (int i = 0; i < KCH; i++) rot[nt][i] = rotate_key(kr[nt][i], kr[nt][i ^ (KCH / 2)], key_cos[nt][i], key_sin[nt][i], i < KCH / 2);
+                fetch_tables();
+                fetch_positions(j + 2);
+                tile(rot, vr, base, cache_end, new_row);
+            } else {
+                tile(kr, vr, base, cache_end);
+            }
         }
     } else {
     for (int base = row_beg + 16 * warp; base < cache_end; base += 16 * W) {
@@ -336,7 +389,15 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
 #pragma unroll
             for (int h = 0; h < VH; h++) vr[r][h] = make_uint4(0u, 0u, 0u, 0u);
         T *kcache = const_cast<T *>(kbase) + (size_t)new_row * D, *vcache = const_cast<T *>(vbase) + (size_t)new_row * D;
-        if (g == 0) {
+        if (STREAM && g == 0) {  // cached as it is, rotated for its score
+            const size_t at = (size_t)p.kvpos[new_row] * D;
+#pragma unroll
+            for (int i = 0; i < KCH; i++) {
+                const int d0 = 8 * t + 32 * i;
+                kr[0][i] = rotate_key(new_k[i], new_k[i ^ (KCH / 2)], *reinterpret_cast<const uint4 *>(cos_t + at + d0), *reinterpret_cast<const uint4 *>(sin_t + at + d0), i < KCH / 2);
+                *reinterpret_cast<uint4 *>(kcache + d0) = new_k[i];
+            }
+        } else if (g == 0) {
             const uint4(&raw)[KCH] = new_k;
 #pragma unroll
             for (int i = 0; i < KCH; i++) {
@@ -361,9 +422,9 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     if constexpr (RING) {
         // the warps' staging rows for the merge reuse each warp's own ring (all of its copies have landed and been read)
         __syncwarp();
-        decode_tail<T, D, VH * 4, Map16, true, W>(p, o, m_run, l_run, reinterpret_cast<float *>(ring_raw), (int)(kRingDepth * kTile / 4));
+        decode_tail<T, D, VH * 4, Map16, true, W>(p, o, m_run, l_run, splits, reinterpret_cast<float *>(ring_raw), (int)(kRingDepth * kTile / 4));
     } else {
-        decode_tail<T, D, VH * 4, Map16, false, W>(p, o, m_run, l_run);
+        decode_tail<T, D, VH * 4, Map16, false, W>(p, o, m_run, l_run, splits);
     }
 }
 
@@ -494,23 +555,32 @@ static bool decode_ring_possible(int B, int Hkv, int cache_seq) {
 static int decode_ctas_per_sm(bool ring, int D) { return ring && D == 128 ? 2 : kAttnCtasPerSm; }
 
 // Few (batch, kv head) pairs leave SMs without a CTA, and then the time is the number of rounds its warps take one after the other (0.85 us
-// each) plus, with splits, the merge through L2 (2.5 us).  Up to half as many pairs as SMs take CTAs of twice (head_dim 128; registers) or
-// four times the warps (head_dim 64), whose round is as many times longer, so that fewer than 1024 / 2048 rows (decode_splits: four rounds a split)
-// need no split; rows are those of the cache or window, since the live ones are known on the device only.  A model's steps
-// do; the operator by itself keeps four warps, with which its ring and its direct form give the same bits.
+// each) plus the merge of splits.  Up to half as many pairs as SMs take CTAs of twice (head_dim 128; registers) or
+// four times the warps (head_dim 64), whose round is as many times longer, and from four rounds on the CTAs of a cluster share a pair: they merge
+// through distributed shared memory (1.0 us; through L2 2.5 us), as many as SMs are there, up to eight, the largest portable cluster.  510 rows, 8 pairs,
+// head_dim 128: 1 / 2 / 4 / 8 CTAs 8.3 / 7.3 / 6.4 / 5.7 us; streaming, 1024 rows, 8 pairs, head_dim 64: 11.4 / 9.8 / 8.2 / 8.2 us; 337 rows, 12 pairs, head_dim 64
+// (two rounds): 4.9 / 5.8 us, so two rounds stay with one CTA.  Rows are those of the cache or window here, since the live ones are known on
+// the device only, where the kernel leaves clusters of few live rows to their first CTA.  More splits than a cluster has go through L2.  A model's steps
+// do all this; the operator by itself keeps four warps, with which its ring and its direct form give the same bits.
 constexpr int decode_wide_warps(int D) { return D == 64 ? 16 : 8; }
 static void decode_plan(DecodeParams &p, bool ring, bool step, int B, int D, int rows_bound) {
     p.wide = step && ring && 2 * B * p.Hkv <= 148;
     p.splits = p.wide ? decode_splits(B, p.Hkv, rows_bound, 16, 1, decode_wide_warps(D)) : decode_splits(B, p.Hkv, rows_bound, 16, decode_ctas_per_sm(ring, D));
+    p.cluster = 0;
+    if (!p.wide) return;
+    const int round = 16 * decode_wide_warps(D), rounds = (rows_bound + round - 1) / round;
+    if (rounds < 4) return;
+    const int room = 148 / (B * p.Hkv), s = room >= 8 ? 8 : room >= 4 ? 4 : 2;
+    if (s >= p.splits) p.splits = s, p.cluster = 1;
 }
 
-template <typename T, int D, bool WIN, int W>
+template <typename T, int D, bool WIN, int W, bool STREAM>
 static int launch_decode_ring(cudaStream_t st, const DecodeParams &p, int B, const CUtensorMap &mk, const CUtensorMap &mv) {
     constexpr size_t smem = (size_t)W * kRingDepth * 2 * (D / 64) * 16 * 128;
-    auto kern = attention_decode_kernel<T, D, true, WIN, W>;
+    auto kern = attention_decode_kernel<T, D, true, WIN, W, STREAM>;
     static SmemLimit limit;  // with the kernel's static shared memory every head_dim is past the 48 KB that need no opt-in
     MYNN_CUDA_OK(limit.raise((const void *)kern, smem));
-    MYNN_CUDA_OK(launch_dependent(kern, dim3(p.splits, p.Hkv, B), dim3(W * 32), smem, st, mk, mv, p));
+    MYNN_CUDA_OK(launch_dependent_cluster(p.cluster ? p.splits : 1, kern, dim3(p.splits, p.Hkv, B), dim3(W * 32), smem, st, mk, mv, p));
     MYNN_LAUNCH_OK("attention_decode_kernel");
     return MYNN_OK;
 }
@@ -525,9 +595,14 @@ static int launch_decode(cudaStream_t st, const DecodeParams &p, int B, bool rin
         const uint64_t rows = (uint64_t)B * p.Hkv * p.cache_seq, row_bytes = (uint64_t)D * sizeof(T);
         if (int rc = make_map(&mk, p.k, rows, row_bytes, row_bytes, 16)) return rc;
         if (int rc = make_map(&mv, p.v, rows, row_bytes, row_bytes, 16)) return rc;
-        return p.wide ? launch_decode_ring<T, D, WIN, decode_wide_warps(D)>(st, p, B, mk, mv)
-                      : launch_decode_ring<T, D, WIN, kAttnWarps>(st, p, B, mk, mv);
+        if constexpr (!WIN) {
+            if (p.kvpos)
+                return p.wide ? launch_decode_ring<T, D, false, decode_wide_warps(D), true>(st, p, B, mk, mv) : launch_decode_ring<T, D, false, kAttnWarps, true>(st, p, B, mk, mv);
+        }
+        return p.wide ? launch_decode_ring<T, D, WIN, decode_wide_warps(D), false>(st, p, B, mk, mv)
+                      : launch_decode_ring<T, D, WIN, kAttnWarps, false>(st, p, B, mk, mv);
     }
+    if (p.kvpos) return fail(MYNN_E_UNSUPPORTED, "attention: the streaming form with the append needs the ring kernel");
     MYNN_CUDA_OK(launch_plain(attention_decode_kernel<T, D, false, WIN, kAttnWarps>, dim3(p.splits, p.Hkv, B), dim3(kAttnWarps * 32), 0, st, mk, mv, p));
     MYNN_LAUNCH_OK("attention_decode_kernel");
     return MYNN_OK;
@@ -608,6 +683,8 @@ extern "C" int mynn_b200_attention_ring(void *stream, void *out, const void *q, 
     return launch_generic<__half>(st, out, q, k, v, scale, B, Hq, Hkv, Sq, cache_seq_len, D, active_seq_kv, nullptr, is_causal, 0, rs, rw, r0);
 }
 
+bool mynn::attention_decode_stream_supported(int B, int Hkv, int cache_seq) { return decode_ring_possible(B, Hkv, cache_seq); }
+
 bool mynn::attention_decode_fast_path(int Sq, int D, int Hq, int Hkv, int dtype, const void *q, const void *k, const void *v) {
     const bool aligned = (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v) % 16) == 0;
     return Sq == 1 && (D == 64 || D == 128) && Hkv > 0 && Hq % Hkv == 0 && Hq / Hkv <= 8 && dtype != MYNN_F32 && aligned;
@@ -672,6 +749,7 @@ int mynn::launch_attention(cudaStream_t st, void *out, const void *q, const void
         p.fused_pos = fuse->pos;
         p.fused_row = fuse->row;
         p.appended = fuse->row;
+        p.kvpos = fuse->kvpos;
     }
     if (int rc = decode_bind_workspace(p, B, D, workspace, workspace_bytes)) return rc;
     if (dtype == MYNN_BF16) return D == 64 ? launch_decode<__nv_bfloat16, 64>(st, p, B, ring) : launch_decode<__nv_bfloat16, 128>(st, p, B, ring);

@@ -4,6 +4,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace mynn {
 
@@ -112,6 +113,9 @@ struct DecodeParams {
     const void *cos_t = nullptr, *sin_t = nullptr;
     const int64_t *fused_pos = nullptr;
     const int32_t *fused_row = nullptr;
+    // With kvpos, the fused form of a streaming cache: keys are cached unrotated, and the key of row r is rotated at table row kvpos[r] on its
+    // way into the product; *fused_row may be any row below `active`, whatever it held before is left out.
+    const int64_t *kvpos = nullptr;
     // Optional (16-bit decode kernel): only the last `window` positions are seen; position p lives in cache row p % cache_seq
     // (ring_cache: `active` may then exceed cache_seq, which is a multiple of 16); scores pass through a soft cap.
     int window = 0, ring_cache = 0;
@@ -122,6 +126,7 @@ struct DecodeParams {
     // read while they still run.  Null: nothing may.  (With the fused append the kernel writes that row itself.)
     const int32_t *appended = nullptr;
     int wide = 0;           // host side: CTAs of more than four warps
+    int cluster = 0;        // the splits of a pair are the CTAs of one cluster and merge through distributed shared memory
     int *status = nullptr;  // ring kernel: where a timed-out wait is recorded (null: the library's own word, see attention_check)
 };
 
@@ -209,10 +214,12 @@ __device__ __forceinline__ void decode_row_limbs(const DecodeParams &p, int b, u
 // (head 2t, d), (head 2t+1, d), (head 2t, d+1), (head 2t+1, d+1) with d = DMap::d(i, g).  The warps are merged through
 // shared memory; with more than one split the partial result goes to the workspace and the last CTA of the
 // (batch, kv head) pair to arrive (atomic ticket, no spinning) combines the splits and writes the output.
+// splits: of this pair (p.splits, or 1 where one CTA has all rows).
+// The splits of a cluster keep their partial results in shared memory instead, and behind a cluster barrier each merges its share of the outputs.
 // ext != nullptr: the per-warp output staging rows live in caller-provided shared memory, warp w's [8][D] floats at
 // ext + w * ext_stride (the ring kernel hands every warp a piece of its own, by then idle, ring).
 template <typename T, int D, int NACC, typename DMap, bool EXT = false, int W = kAttnWarps>
-__device__ __forceinline__ void decode_tail(const DecodeParams &p, const float (&o)[NACC][4], float m_run, float l_run,
+__device__ __forceinline__ void decode_tail(const DecodeParams &p, const float (&o)[NACC][4], float m_run, float l_run, int splits,
                                             float *ext = nullptr, int ext_stride = 0) {
     float *so_base;
     int so_stride;
@@ -226,7 +233,7 @@ __device__ __forceinline__ void decode_tail(const DecodeParams &p, const float (
     }
     __shared__ float sm_m[W][8], sm_l[W][8];
     __shared__ unsigned sm_last, sm_row_last;
-    __shared__ float sm_red[W];
+    __shared__ float sm_red[W], sm_cm[8], sm_cl[8];
     const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int G = p.G;
@@ -264,10 +271,13 @@ __device__ __forceinline__ void decode_tail(const DecodeParams &p, const float (
                 O += so_base[(size_t)w * so_stride + hd * D + d] * f;
             }
         }
-        if (p.splits == 1) {
+        if (splits == 1) {
             outp[(size_t)hd * D + d] = from_f32<T>(O / L);
+        } else if (p.cluster) {
+            so_base[hd * D + d] = O;  // over warp 0's part of this element, which no other thread reads
+            if (d == 0) sm_cm[hd] = mx, sm_cl[hd] = L;
         } else {
-            const size_t slot = (pair * p.splits + split) * 8 + hd;
+            const size_t slot = (pair * splits + split) * 8 + hd;
             p.ws_o[slot * D + d] = O;
             if (d == 0) {
                 p.ws_ml[slot * 2] = mx;
@@ -275,14 +285,43 @@ __device__ __forceinline__ void decode_tail(const DecodeParams &p, const float (
             }
         }
     }
-    if (p.splits == 1) {
+    if (splits == 1) {
         decode_row_limbs<T, D, W>(p, b, &sm_row_last, sm_red);
         return;
     }
 
+    if (p.cluster) {
+        cluster_sync_all();  // the partial results of all splits are in place
+        const int share = (G * D + splits - 1) / splits, end = min(G * D, (split + 1) * share);
+        for (int idx = split * share + threadIdx.x; idx < end; idx += blockDim.x) {
+            const int hd = idx / D;
+            float ms[8], ls[8], os[8], mx = -INFINITY, L = 0.f, O = 0.f;
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const uint32_t r = j < splits ? j : 0;
+                ms[j] = ld_cluster_f32(map_rank(smem_u32(&sm_cm[hd]), r));
+                ls[j] = ld_cluster_f32(map_rank(smem_u32(&sm_cl[hd]), r));
+                os[j] = ld_cluster_f32(map_rank(smem_u32(&so_base[idx]), r));
+                if (j >= splits) ms[j] = -INFINITY;
+            }
+#pragma unroll
+            for (int j = 0; j < 8; j++) mx = fmaxf(mx, ms[j]);
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                if (ms[j] == -INFINITY) continue;
+                const float f = __expf(ms[j] - mx);
+                L += ls[j] * f;
+                O += os[j] * f;
+            }
+            outp[idx] = from_f32<T>(O / L);
+        }
+        cluster_sync_all();  // nobody leaves while its partial results may still be read; the outputs of all are ordered before what follows
+        if (split == 0) decode_row_limbs<T, D, W>(p, b, &sm_row_last, sm_red);
+        return;
+    }
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) sm_last = (atomicAdd(&p.ws_ticket[pair], 1u) == (unsigned)(p.splits - 1)) ? 1u : 0u;
+    if (threadIdx.x == 0) sm_last = (atomicAdd(&p.ws_ticket[pair], 1u) == (unsigned)(splits - 1)) ? 1u : 0u;
     __syncthreads();
     if (!sm_last) return;
     __threadfence();
@@ -291,12 +330,12 @@ __device__ __forceinline__ void decode_tail(const DecodeParams &p, const float (
         // eight splits at a time, all of their loads issued before any is used: the combine costs one L2 round trip per
         // eight splits instead of four dependent ones per split
         float mx = -INFINITY, L = 0.f, O = 0.f;
-        for (int s0 = 0; s0 < p.splits; s0 += 8) {
+        for (int s0 = 0; s0 < splits; s0 += 8) {
             float ms[8], ls[8], os[8];
 #pragma unroll
             for (int j = 0; j < 8; j++) {
-                const bool in = s0 + j < p.splits;
-                const size_t slot = (pair * p.splits + (in ? s0 + j : s0)) * 8 + hd;
+                const bool in = s0 + j < splits;
+                const size_t slot = (pair * splits + (in ? s0 + j : s0)) * 8 + hd;
                 ms[j] = in ? __ldcg(&p.ws_ml[slot * 2]) : -INFINITY;
                 ls[j] = in ? __ldcg(&p.ws_ml[slot * 2 + 1]) : 0.f;
                 os[j] = in ? __ldcg(&p.ws_o[slot * D + d]) : 0.f;

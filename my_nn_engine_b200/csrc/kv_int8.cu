@@ -478,9 +478,9 @@ attention_decode_q8_kernel(const __grid_constant__ CUtensorMap map_k, const __gr
     }
     if constexpr (RING) {
         __syncwarp();
-        decode_tail<T, D, NACC, MapQ8<VB>, true>(p, o, m_run, l_run, reinterpret_cast<float *>(ring_raw), (int)(kQ8RingDepth * kTile / 4));
+        decode_tail<T, D, NACC, MapQ8<VB>, true>(p, o, m_run, l_run, p.splits, reinterpret_cast<float *>(ring_raw), (int)(kQ8RingDepth * kTile / 4));
     } else {
-        decode_tail<T, D, NACC, MapQ8<VB>>(p, o, m_run, l_run);
+        decode_tail<T, D, NACC, MapQ8<VB>>(p, o, m_run, l_run, p.splits);
     }
 }
 

@@ -174,6 +174,13 @@ static int enqueue_forward(Model &m, cudaStream_t st, int S, int head_rows = 0) 
                 RC(launch_attention_q8(st, m.attn, m.q_rot, L.kc, L.vc, L.ksc, L.vsc, attn_scale, B, m.Hq, m.Hkv, S, D,
                                        c.max_seq_len, c.max_seq_len, m.active_dev, S > 1, dt, m.attn_ws, m.attn_ws_bytes, 1, S == 1 ? m.past_dev : nullptr));
             }
+        } else if (c.stream_window > 0 && S == 1 && g_fuse_rope && L.qkv_fused && qs % 8 == 0 && D % 32 == 0 && (((uintptr_t)kb | (uintptr_t)vb) % 16) == 0 &&
+                   attention_decode_fast_path(S, D, m.Hq, m.Hkv, dt, qb, L.kc, L.vc) && attention_decode_stream_supported(B, m.Hkv, c.max_seq_len)) {
+            // streaming cache, one token: the attention kernel appends the row (unrotated, at the slot in past_dev), and rotates q, the new key and
+            // every live key at its recency rank.  The live rows are the slots [0, active).
+            const AttentionFuse fz = {kb, vb, qs, m.cos_t, m.sin_t, m.pos0_dev, m.past_dev, m.kvpos_dev};
+            RC(launch_attention(st, m.attn, qb, L.kc, L.vc, attn_scale, B, m.Hq, m.Hkv, S, D, c.max_seq_len, c.max_seq_len, m.active_dev, 0, dt, m.attn_ws,
+                                m.attn_ws_bytes, 1, nullptr, nullptr, &fz, (int *)m.gemm_ws));
         } else if (c.stream_window > 0) {
             // streaming cache: K is appended unrotated at the slot in past_dev; the live rows are rotated at their
             // recency rank into the scratch copy that attention reads.  The live rows are the slots [0, active).

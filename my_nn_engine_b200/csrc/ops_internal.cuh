@@ -60,6 +60,7 @@ struct AttentionFuse {
     const void *cos_t, *sin_t;
     const int64_t *pos;
     const int32_t *row;
+    const int64_t *kvpos = nullptr;  // a streaming cache (DecodeParams::kvpos); needs attention_decode_stream_supported
 };
 int launch_attention(cudaStream_t st, void *out, const void *q, const void *k, const void *v, float scale, int B,
                      int Hq, int Hkv, int Sq, int D, int cache_seq_len, int active_seq_kv,
@@ -71,6 +72,7 @@ int launch_attention(cudaStream_t st, void *out, const void *q, const void *k, c
 int attention_decode_take_status(int *status);
 int attention_decode_q8_take_status(int *status);
 bool attention_decode_fast_path(int Sq, int D, int Hq, int Hkv, int dtype, const void *q, const void *k, const void *v);
+bool attention_decode_stream_supported(int B, int Hkv, int cache_seq);
 
 // Tiled tensor-core attention for several query rows (prefill chunks); see attention_prefill.cu.
 bool attention_prefill_supported(int Sq, int D, int dtype, const void *q, const void *k, const void *v, const void *out);

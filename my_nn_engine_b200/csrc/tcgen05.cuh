@@ -158,6 +158,17 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
+// A shared-memory address of this CTA, as the same place in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+    return v;
+}
 __device__ __forceinline__ int ld_dsmem_s32(uint32_t local_addr, uint32_t rank) {
     uint32_t remote;
     int v;
@@ -237,12 +248,6 @@ __device__ __forceinline__ uint64_t make_sw128_desc(uint32_t smem_addr, uint32_t
 // ---- CTA pairs (cta_group::2): a cluster of two CTAs works on one tile.  The CTA of rank 0 issues the MMAs and holds the barriers that they wait
 // for; each CTA brings its half of A's rows and of B's rows into its own shared memory, at the same offsets, and each has its half of the
 // accumulator's rows in its own tensor memory.
-// A shared-memory address of this CTA, as the same place in CTA `rank` of the cluster.
-__device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
 // A tile into this CTA's shared memory, counted on a barrier of either CTA of the pair (bar: a shared::cluster address).
 __device__ __forceinline__ void tma_load_2d_pair(void *smem_dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(

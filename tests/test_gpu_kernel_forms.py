@@ -250,3 +250,36 @@ def test_fused_append_over_a_long_cache(head_dim, kv_heads, batch):
         assert torch.equal(ca[0], cb[0]) and torch.equal(ca[1], cb[1]), past
         assert not torch.equal(ca[0][:, :, past], k[:, :, past]) and torch.equal(ca[0][:, :, past + 1:], k[:, :, past + 1:])
         assert (a - b).abs().max() <= 8 * 2.0 ** -7 * a.abs().max(), past
+
+
+# ---- streaming steps: rotation and append inside the attention kernel, one CTA or a cluster per kv head, against the kernels of their own ----
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("d,batch,window", [(64, 1, 15), (64, 3, 509), (64, 2, 1100), (128, 1, 300), (128, 2, 1300), (64, 30, 90)])
+def test_streaming_step_with_the_append_inside(dt, d, batch, window):
+    from my_nn_engine_b200.decoder import DecoderModel
+    from my_nn_engine_b200.quantize import random_llama_state
+    cfg = dict(hidden_size=256, num_hidden_layers=1, num_attention_heads=6, num_key_value_heads=2 if batch < 30 else 3, head_dim=d, intermediate_size=512, vocab_size=300,
+               rms_norm_eps=1e-5, rope_theta=1e4)
+    sink, tokens = 4, np.arange(batch) * 37 % 300
+    model = {}
+    try:
+        for fused in (1, 0):
+            ffi.set_option(ffi.OPT_FUSE_ROPE, fused)  # read when a step is captured
+            model[fused] = DecoderModel(cfg, random_llama_state(cfg, seed=7), dtype=dt, max_seq_len=-(-(sink + window) // 8) * 8, batch=batch, streaming=(sink, window))
+            model[fused].stream(tokens, 0)
+    finally:
+        ffi.set_option(ffi.OPT_FUSE_ROPE, 1)
+    g = gen(window)
+    for pos in (0, 1, 3, 17, sink + window - 1, sink + window, 3 * window + 5):
+        past = randn(g, *model[1].k_cache[0].shape).to(DT[dt]), randn(g, *model[1].k_cache[0].shape).to(DT[dt])
+        for m in model.values():
+            m.k_cache[0].copy_(past[0])
+            m.v_cache[0].copy_(past[1])
+        torch.cuda.synchronize()
+        got, want = (model[f].stream(tokens, pos).clone().double() for f in (1, 0))
+        torch.cuda.synchronize()
+        assert torch.equal(model[1].k_cache[0], model[0].k_cache[0]) and torch.equal(model[1].v_cache[0], model[0].v_cache[0])
+        # the sums of the attention in another order: a rounding of its output here and there, carried through the rest of the layer
+        assert (got - want).abs().max() <= 2.0 ** (-6 if dt == "bf16" else -9) * want.abs().max(), pos
+    for m in model.values():
+        m.close()

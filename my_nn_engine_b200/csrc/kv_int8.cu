@@ -14,6 +14,8 @@
 //     (row 2t, row 2t+1) pairs of two head-dim values, i.e. two A-fragment registers;
 //   * k_scale multiplies S per kv row after the MMA, v_scale multiplies P per kv row before it, so the tensor cores
 //     only ever see exact small integers on the cache side.
+#include <algorithm>
+
 #include "attention_internal.cuh"
 #include "i8_cvt.cuh"
 #include "i8_gemm.cuh"
@@ -188,6 +190,9 @@ __device__ __forceinline__ uint32_t load_scale_pair(const T *sc, int row, int la
 // engine fills: one 32-row x 128-byte box of K and one of V per tile (2-D maps of the caches, 128-byte swizzle) plus the 32
 // row scales of each by an untiled bulk copy; the fragments and scales are then taken from shared memory.  Lane 0 of the
 // consuming warp issues the copies of tile j + depth once the warp has tile j in registers.
+// Fused (DecodeParams::fused_k, RING only): q comes unrotated from the projection and is rotated on its way into limbs; the CTA whose split holds the
+// new row rotates and quantizes it, stores it, and puts it over its place in the tile that the copies brought.  (A kernel of its own for that took
+// 5.4 us per layer at five sequences.)
 constexpr int kQ8RingDepth = 3;
 __device__ int g_q8_ring_status;  // 32: a wait for a tile ran out of time
 MYNN_DEFINE_WAIT_BUDGET_SETTER(kv_int8)
@@ -212,8 +217,12 @@ attention_decode_q8_kernel(const __grid_constant__ CUtensorMap map_k, const __gr
     const int G = p.G;
     int active = p.active_dev ? *p.active_dev : p.active_host;
     active = max(0, min(active, p.cache_seq));
+    // A cluster with one round of rows leaves them to its first CTA.
+    const bool solo = p.cluster && active <= 32 * kAttnWarps;
+    if (solo && split > 0) return;
+    const int splits = solo ? 1 : p.splits;
     // whole rounds of the CTA's four warps (128 rows): a split that ends inside a round leaves some warps a tile short
-    const int rows_per_split = (((active + p.splits - 1) / p.splits) + 32 * kAttnWarps - 1) / (32 * kAttnWarps) * (32 * kAttnWarps);
+    const int rows_per_split = (((active + splits - 1) / splits) + 32 * kAttnWarps - 1) / (32 * kAttnWarps) * (32 * kAttnWarps);
     const int row_beg = split * rows_per_split;
     const int row_end = min(row_beg + rows_per_split, active);
 
@@ -230,6 +239,12 @@ attention_decode_q8_kernel(const __grid_constant__ CUtensorMap map_k, const __gr
     __shared__ uint64_t full[RING ? kAttnWarps : 1][kQ8RingDepth];
     __shared__ __align__(16) T sm_sc[RING ? kAttnWarps : 1][kQ8RingDepth][2][32];
     __shared__ int abort_flag;
+    __shared__ uint32_t sm_new[RING ? 2 : 1][32];  // fused: the new key and value as stored
+    __shared__ T sm_new_sc[2];
+    const bool fused = RING && p.fused_k != nullptr;
+    const int new_row = fused ? *p.fused_row : -1;
+    const size_t tab = fused ? (size_t)(*p.fused_pos) * D : 0;
+    const T *cos_t = reinterpret_cast<const T *>(p.cos_t), *sin_t = reinterpret_cast<const T *>(p.sin_t);
     uint8_t *ring = ring_raw + (size_t)warp * kQ8RingDepth * kTile;
     const int first = row_beg + 32 * warp;
     const int ntile = first < row_end ? (row_end - first + 32 * kAttnWarps - 1) / (32 * kAttnWarps) : 0;
@@ -258,7 +273,7 @@ attention_decode_q8_kernel(const __grid_constant__ CUtensorMap map_k, const __gr
         int j = 0;
         if (lane == 0 && settled) {
             const int written = *p.appended;
-            for (; j < min(ntile, kQ8RingDepth) && (unsigned)(written - first - 32 * kAttnWarps * j) >= 32u; j++) issue(j);
+            for (; j < min(ntile, kQ8RingDepth) && (fused || (unsigned)(written - first - 32 * kAttnWarps * j) >= 32u); j++) issue(j);
         }
         pdl_wait();
         if (lane == 0)
@@ -272,12 +287,28 @@ attention_decode_q8_kernel(const __grid_constant__ CUtensorMap map_k, const __gr
         constexpr int E = D / 16;
         const int h = threadIdx.x >> 4, part = threadIdx.x & 15;
         float qv[E];
-        const T *qrow = reinterpret_cast<const T *>(p.q) + (size_t)(b * p.Hq + kvh * G + min(h, G - 1)) * D + part * E;
+        const T *qhead = fused ? reinterpret_cast<const T *>(p.q) + (size_t)b * p.qkv_stride + (size_t)(kvh * G + min(h, G - 1)) * D
+                               : reinterpret_cast<const T *>(p.q) + (size_t)(b * p.Hq + kvh * G + min(h, G - 1)) * D;
+        const T *qrow = qhead + part * E;
         float mx = 0.f;
         bool bad = false;
+        if (RING && fused && h < G) {
+            T x[E], xp[E], c[E], sn[E];  // E = 8
+            *reinterpret_cast<uint4 *>(x) = *reinterpret_cast<const uint4 *>(qrow);
+            *reinterpret_cast<uint4 *>(xp) = *reinterpret_cast<const uint4 *>(qhead + (part ^ 8) * E);
+            *reinterpret_cast<uint4 *>(c) = *reinterpret_cast<const uint4 *>(cos_t + tab + part * E);
+            *reinterpret_cast<uint4 *>(sn) = *reinterpret_cast<const uint4 *>(sin_t + tab + part * E);
+#pragma unroll
+            for (int i = 0; i < E; i++) {
+                const float a = to_f32<T>(x[i]), o_ = to_f32<T>(xp[i]), cc = to_f32<T>(c[i]), ss = to_f32<T>(sn[i]);
+                qv[i] = round_store<T>(part < 8 ? rope_low(a, o_, cc, ss) : rope_high(o_, a, cc, ss));
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < E; i++) qv[i] = h < G ? to_f32<T>(qrow[i]) : 0.f;
+        }
 #pragma unroll
         for (int i = 0; i < E; i++) {
-            qv[i] = h < G ? to_f32<T>(qrow[i]) : 0.f;
             bad |= !(fabsf(qv[i]) <= 3.0e38f);
             mx = fmaxf(mx, fabsf(qv[i]));
         }
@@ -308,6 +339,41 @@ attention_decode_q8_kernel(const __grid_constant__ CUtensorMap map_k, const __gr
         // a query row with a NaN or an infinity gives NaN scores, hence a NaN output row, as plain arithmetic would
         if (part == 0) sm_qinv[h] = bad ? __int_as_float(0x7fc00000) : (sc > 0.f ? 1.0f / sc : 0.f);
     }
+    // The new row: warp 0 takes the key, warp 1 the value, four elements per lane.  A row that no split holds (not seen by this step) is stored by the first.
+    if constexpr (RING) {
+        const bool mine = fused && ((new_row >= row_beg && new_row < row_end) || (split == 0 && new_row >= active)) && new_row >= 0 && new_row < p.cache_seq;
+        if (mine && warp < 2) {
+            const T *src = (warp == 0 ? reinterpret_cast<const T *>(p.fused_k) : reinterpret_cast<const T *>(p.fused_v)) + (size_t)b * p.qkv_stride + (size_t)kvh * D + 4 * lane;
+            T x[4], c[4], sn[4];
+            *reinterpret_cast<uint2 *>(x) = *reinterpret_cast<const uint2 *>(src);
+            float v[4], mx = 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; i++) v[i] = to_f32<T>(x[i]);
+            if (warp == 0) {
+                *reinterpret_cast<uint2 *>(c) = *reinterpret_cast<const uint2 *>(cos_t + tab + 4 * lane);
+                *reinterpret_cast<uint2 *>(sn) = *reinterpret_cast<const uint2 *>(sin_t + tab + 4 * lane);
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const float other = __shfl_xor_sync(0xffffffffu, v[i], 16);
+                    v[i] = round_store<T>(lane < 16 ? rope_low(v[i], other, to_f32<T>(c[i]), to_f32<T>(sn[i])) : rope_high(other, v[i], to_f32<T>(c[i]), to_f32<T>(sn[i])));
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) mx = fmaxf(mx, fabsf(v[i]));
+            mx = warp_max(mx);
+            const float inv = mx == 0.f ? 0.f : __fdiv_rn(127.0f, mx);
+            uint32_t word = 0u;
+#pragma unroll
+            for (int i = 0; i < 4; i++) word |= (uint32_t)(uint8_t)quantize_kv_value(v[i], inv) << (8 * i);
+            const T sc = from_f32<T>(__fmul_rn(mx, 1.0f / 127.0f));
+            *reinterpret_cast<uint32_t *>(const_cast<int8_t *>(warp == 0 ? kbase : vbase) + (size_t)new_row * D + 4 * lane) = word;
+            sm_new[warp][lane] = word;
+            if (lane == 0) {
+                const_cast<T *>(warp == 0 ? ksc : vsc)[new_row] = sc;
+                sm_new_sc[warp] = sc;
+            }
+        }
+    }
     __syncthreads();
     const float qinv = sm_qinv[g] * p.scale;
 
@@ -334,7 +400,14 @@ attention_decode_q8_kernel(const __grid_constant__ CUtensorMap map_k, const __gr
                 }
                 break;
             }
-            const uint8_t *st = ring + (size_t)s * kTile;
+            uint8_t *st = ring + (size_t)s * kTile;
+            if (fused && (unsigned)(new_row - base) < 32u) {
+                const int r = new_row - base, at = r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + 4 * (lane & 3);
+                *reinterpret_cast<uint32_t *>(st + at) = sm_new[0][lane];
+                *reinterpret_cast<uint32_t *>(st + kBox + at) = sm_new[RING ? 1 : 0][lane];
+                if (lane < 2) sm_sc[warp][s][lane][r] = sm_new_sc[lane];
+                __syncwarp();
+            }
 #pragma unroll
             for (int u = 0; u < 2; u++)
 #pragma unroll
@@ -478,9 +551,9 @@ attention_decode_q8_kernel(const __grid_constant__ CUtensorMap map_k, const __gr
     }
     if constexpr (RING) {
         __syncwarp();
-        decode_tail<T, D, NACC, MapQ8<VB>, true>(p, o, m_run, l_run, p.splits, reinterpret_cast<float *>(ring_raw), (int)(kQ8RingDepth * kTile / 4));
+        decode_tail<T, D, NACC, MapQ8<VB>, true>(p, o, m_run, l_run, splits, reinterpret_cast<float *>(ring_raw), (int)(kQ8RingDepth * kTile / 4));
     } else {
-        decode_tail<T, D, NACC, MapQ8<VB>>(p, o, m_run, l_run, p.splits);
+        decode_tail<T, D, NACC, MapQ8<VB>>(p, o, m_run, l_run, splits);
     }
 }
 
@@ -591,7 +664,7 @@ static int launch_decode_q8(cudaStream_t st, const DecodeParams &p, int B, bool 
             auto kern = attention_decode_q8_kernel<T, D, true>;
             static SmemLimit limit;
             MYNN_CUDA_OK(limit.raise((const void *)kern, smem));
-            MYNN_CUDA_OK(launch_dependent(kern, dim3(p.splits, p.Hkv, B), dim3(kAttnWarps * 32), smem, st, mk, mv, p));
+            MYNN_CUDA_OK(launch_dependent_cluster(p.cluster ? p.splits : 1, kern, dim3(p.splits, p.Hkv, B), dim3(kAttnWarps * 32), smem, st, mk, mv, p));
             MYNN_LAUNCH_OK("attention_decode_q8_kernel");
             return MYNN_OK;
         }
@@ -640,10 +713,16 @@ int launch_dequant_kv_rows(cudaStream_t st, int dtype, void *out, const void *ca
     return MYNN_OK;
 }
 
+bool attention_q8_fused_supported(int B, int Hkv, int D, int cache_seq, const void *k_scale, const void *v_scale) {
+    DecodeParams p;
+    p.Hkv = Hkv, p.cache_seq = cache_seq, p.k_scale = k_scale, p.v_scale = v_scale;
+    return q8_ring_possible(p, B, D);
+}
+
 int launch_attention_q8(cudaStream_t st, void *out, const void *q, const void *k, const void *v, const void *k_scale,
                         const void *v_scale, float scale, int B, int Hq, int Hkv, int Sq, int D, int cache_seq_len,
                         int active_seq_kv, const int32_t *active_seq_kv_dev, int is_causal, int dtype, void *workspace,
-                        size_t workspace_bytes, int out_bshd, const int32_t *appended) {
+                        size_t workspace_bytes, int out_bshd, const int32_t *appended, const AttentionFuse *fuse) {
     if (B < 0 || Hq <= 0 || Hkv <= 0 || Sq < 0 || D <= 0 || cache_seq_len < 0 || active_seq_kv < 0)
         return fail(MYNN_E_ARG, "attention_q8: bad shape");
     if (Hq % Hkv != 0) return fail(MYNN_E_ARG, "attention_q8: %d query heads are not a multiple of %d kv heads", Hq, Hkv);
@@ -653,6 +732,7 @@ int launch_attention_q8(cudaStream_t st, void *out, const void *q, const void *k
     const int G = Hq / Hkv;
     const bool aligned = (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v) % 16) == 0;
     const bool fast = Sq == 1 && (D == 64 || D == 128) && G <= 8 && dtype != MYNN_F32 && aligned;
+    if (!fast && fuse) return fail(MYNN_E_UNSUPPORTED, "attention_q8: the fused RoPE + append exists only on the decode fast path");
     if (!fast) {
         if (dtype == MYNN_F32) return launch_q8_generic<float>(st, out, q, k, v, k_scale, v_scale, scale, B, Hq, Hkv, Sq, cache_seq_len, D, active_seq_kv, active_seq_kv_dev, is_causal, out_bshd);
         if (dtype == MYNN_BF16) return launch_q8_generic<__nv_bfloat16>(st, out, q, k, v, k_scale, v_scale, scale, B, Hq, Hkv, Sq, cache_seq_len, D, active_seq_kv, active_seq_kv_dev, is_causal, out_bshd);
@@ -678,6 +758,29 @@ int launch_attention_q8(cudaStream_t st, void *out, const void *q, const void *k
     const bool ring = q8_ring_possible(p, B, D);
     p.splits = decode_splits(B, Hkv, rows_bound, 32, ring ? 2 : kAttnCtasPerSm);
     p.appended = appended;
+    if (appended && ring) {
+        // A step of a model, few pairs: the splits of a pair are a cluster, as many as are resident at once, up to eight, each with a whole number of rounds.
+        const int rounds = (rows_bound + 32 * kAttnWarps - 1) / (32 * kAttnWarps), most = std::min(std::min(8, 2 * 148 / (B * Hkv)), rounds);
+        if (most > 1) {
+            const int per = (rounds + most - 1) / most, s = (rounds + per - 1) / per;
+            if (s >= p.splits) p.splits = s, p.cluster = 1;
+        }
+    }
+    if (fuse) {
+        if (!ring || !attention_q8_fused_supported(B, Hkv, D, cache_seq_len, k_scale, v_scale))
+            return fail(MYNN_E_UNSUPPORTED, "attention_q8: the fused RoPE + append needs the ring form");
+        if (!fuse->k_new || !fuse->v_new || !fuse->cos_t || !fuse->sin_t || !fuse->pos || !fuse->row || fuse->qkv_stride % 8 ||
+            (((uintptr_t)fuse->k_new | (uintptr_t)fuse->v_new | (uintptr_t)fuse->cos_t | (uintptr_t)fuse->sin_t) % 16))
+            return fail(MYNN_E_ARG, "attention_q8: fused RoPE + append needs 16-byte aligned rows, tables and device scalars");
+        p.fused_k = fuse->k_new;
+        p.fused_v = fuse->v_new;
+        p.qkv_stride = fuse->qkv_stride;
+        p.cos_t = fuse->cos_t;
+        p.sin_t = fuse->sin_t;
+        p.fused_pos = fuse->pos;
+        p.fused_row = fuse->row;
+        p.appended = fuse->row;
+    }
     if (int rc = decode_bind_workspace(p, B, D, workspace, workspace_bytes)) return rc;
     if (dtype == MYNN_BF16) return D == 64 ? launch_decode_q8<__nv_bfloat16, 64>(st, p, B, ring) : launch_decode_q8<__nv_bfloat16, 128>(st, p, B, ring);
     return D == 64 ? launch_decode_q8<__half, 64>(st, p, B, ring) : launch_decode_q8<__half, 128>(st, p, B, ring);

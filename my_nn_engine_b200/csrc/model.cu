@@ -159,6 +159,11 @@ static int enqueue_forward(Model &m, cudaStream_t st, int S, int head_rows = 0) 
                                         S == 1 ? m.pos0_dev : m.pos_dev, B, S, m.Hq, m.Hkv, D, c.max_seq_len, m.past_dev, 0));
             RC(launch_attention_streaming(st, m.attn, m.q_rot, L.kc, L.vc, L.ksc, L.vsc, attn_scale, B, m.Hq, m.Hkv, S, D, c.max_seq_len,
                                           c.max_seq_len, m.active_dev, S > 1, 0, 0, 0, m.cos_t, m.sin_t, m.kvpos_dev, dt, 1, 1));
+        } else if (c.kv_int8 && S == 1 && g_fuse_rope && L.qkv_fused && qs % 8 == 0 && (((uintptr_t)kb | (uintptr_t)vb) % 16) == 0 &&
+                   attention_decode_fast_path(S, D, m.Hq, m.Hkv, dt, qb, L.kc, L.vc) && attention_q8_fused_supported(B, m.Hkv, D, c.max_seq_len, L.ksc, L.vsc)) {
+            const AttentionFuse fz = {kb, vb, qs, m.cos_t, m.sin_t, m.pos0_dev, m.past_dev};
+            RC(launch_attention_q8(st, m.attn, qb, L.kc, L.vc, L.ksc, L.vsc, attn_scale, B, m.Hq, m.Hkv, S, D, c.max_seq_len, c.max_seq_len, m.active_dev, 0, dt,
+                                   m.attn_ws, m.attn_ws_bytes, 1, m.past_dev, &fz));
         } else if (c.kv_int8) {
             RC(launch_rope_kv_append_q8(st, dt, m.q_rot, L.kc, L.vc, L.ksc, L.vsc, qb, kb, vb, qs, ks, vs, m.cos_t, m.sin_t,
                                         S == 1 ? m.pos0_dev : m.pos_dev, B, S, m.Hq, m.Hkv, D, c.max_seq_len, m.past_dev));

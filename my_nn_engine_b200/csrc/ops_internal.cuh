@@ -35,10 +35,12 @@ int launch_rope_kv_append_q8(cudaStream_t st, int dtype, void *q_out, void *k_ca
                              const int32_t *past_len_dev, int rotate_k = 1);
 
 // Attention over an int8 KV cache (per-token scales), with the output-layout choice of launch_attention.  appended: see DecodeParams.
+struct AttentionFuse;
+bool attention_q8_fused_supported(int B, int Hkv, int D, int cache_seq, const void *k_scale, const void *v_scale);
 int launch_attention_q8(cudaStream_t st, void *out, const void *q, const void *k, const void *v, const void *k_scale,
                         const void *v_scale, float scale, int B, int Hq, int Hkv, int Sq, int D, int cache_seq_len,
                         int active_seq_kv, const int32_t *active_seq_kv_dev, int is_causal, int dtype, void *workspace,
-                        size_t workspace_bytes, int out_bshd, const int32_t *appended = nullptr);
+                        size_t workspace_bytes, int out_bshd, const int32_t *appended = nullptr, const AttentionFuse *fuse = nullptr);
 
 // out[m, f] = swish(gate[m, f]) * up[m, f] with gate/up rows `in_stride` elements apart.
 int launch_swiglu_strided(cudaStream_t st, int dtype, void *out, const void *gate, const void *up, int M, int F,

@@ -283,3 +283,35 @@ def test_streaming_step_with_the_append_inside(dt, d, batch, window):
         assert (got - want).abs().max() <= 2.0 ** (-6 if dt == "bf16" else -9) * want.abs().max(), pos
     for m in model.values():
         m.close()
+
+
+# ---- int8 cache, the same: rounds of 128 rows, one CTA, clusters of whole rounds, more pairs than SMs; the new row anywhere in its tile ----
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("batch,hkv,rows", [(1, 1, 128), (1, 2, 2048), (5, 8, 768), (32, 5, 256)])
+def test_int8_step_with_the_append_inside(dt, batch, hkv, rows):
+    from my_nn_engine_b200.decoder import DecoderModel
+    from my_nn_engine_b200.quantize import random_llama_state
+    cfg = dict(hidden_size=256, num_hidden_layers=1, num_attention_heads=2 * hkv, num_key_value_heads=hkv, head_dim=128, intermediate_size=512, vocab_size=300,
+               rms_norm_eps=1e-5, rope_theta=1e4)
+    tokens, model, g = np.arange(batch) * 37 % 300, {}, gen(rows + batch)
+    try:
+        for fused in (1, 0):
+            ffi.set_option(ffi.OPT_FUSE_ROPE, fused)  # read when a step is captured
+            model[fused] = DecoderModel(cfg, random_llama_state(cfg, seed=9), dtype=dt, max_seq_len=rows, batch=batch, kv_int8=True)
+            model[fused].step(tokens, 0)
+    finally:
+        ffi.set_option(ffi.OPT_FUSE_ROPE, 1)
+    for pos in (0, 1, 31, 32, 100, 127, rows // 2 + 3, rows - 1):
+        past = [int8(g, *model[1].k_cache[0].shape) for _ in range(2)] + [scales(g, model[1].k_scale[0].numel(), DT[dt]).view_as(model[1].k_scale[0]) for _ in range(2)]
+        for m in model.values():
+            for to, t in zip((m.k_cache, m.v_cache, m.k_scale, m.v_scale), past):
+                to[0].copy_(t)
+        torch.cuda.synchronize()
+        got, want = (model[f].step(tokens, pos).clone().double() for f in (1, 0))
+        torch.cuda.synchronize()
+        for a, b in zip(*((m.k_cache[0], m.v_cache[0], m.k_scale[0], m.v_scale[0]) for m in model.values())):
+            assert torch.equal(a, b)
+        # the sums of the attention in another order: a rounding of its output here and there, carried through the rest of the layer
+        assert (got - want).abs().max() <= 2.0 ** (-6 if dt == "bf16" else -9) * want.abs().max(), pos
+    for m in model.values():
+        m.close()

@@ -556,22 +556,46 @@ static int decode_ctas_per_sm(bool ring, int D) { return ring && D == 128 ? 2 : 
 
 // Few (batch, kv head) pairs leave SMs without a CTA, and then the time is the number of rounds its warps take one after the other (0.85 us
 // each) plus the merge of splits.  Up to half as many pairs as SMs take CTAs of twice (head_dim 128; registers) or
-// four times the warps (head_dim 64), whose round is as many times longer, and from four rounds on the CTAs of a cluster share a pair: they merge
-// through distributed shared memory (1.0 us; through L2 2.5 us), as many as SMs are there, up to eight, the largest portable cluster.  510 rows, 8 pairs,
+// four times the warps (head_dim 64), whose round is as many times longer, and the CTAs of a cluster share a pair (decode_step_splits).  510 rows, 8 pairs,
 // head_dim 128: 1 / 2 / 4 / 8 CTAs 8.3 / 7.3 / 6.4 / 5.7 us; streaming, 1024 rows, 8 pairs, head_dim 64: 11.4 / 9.8 / 8.2 / 8.2 us; 337 rows, 12 pairs, head_dim 64
 // (two rounds): 4.9 / 5.8 us, so two rounds stay with one CTA.  Rows are those of the cache or window here, since the live ones are known on
-// the device only, where the kernel leaves clusters of few live rows to their first CTA.  More splits than a cluster has go through L2.  A model's steps
+// the device only, where the kernel leaves clusters of few live rows to their first CTA.  A model's steps
 // do all this; the operator by itself keeps four warps, with which its ring and its direct form give the same bits.
 constexpr int decode_wide_warps(int D) { return D == 64 ? 16 : 8; }
 static void decode_plan(DecodeParams &p, bool ring, bool step, int B, int D, int rows_bound) {
     p.wide = step && ring && 2 * B * p.Hkv <= 148;
-    p.splits = p.wide ? decode_splits(B, p.Hkv, rows_bound, 16, 1, decode_wide_warps(D)) : decode_splits(B, p.Hkv, rows_bound, 16, decode_ctas_per_sm(ring, D));
-    p.cluster = 0;
-    if (!p.wide) return;
-    const int round = 16 * decode_wide_warps(D), rounds = (rows_bound + round - 1) / round;
-    if (rounds < 4) return;
-    const int room = 148 / (B * p.Hkv), s = room >= 8 ? 8 : room >= 4 ? 4 : 2;
-    if (s >= p.splits) p.splits = s, p.cluster = 1;
+    const int warps = p.wide ? decode_wide_warps(D) : kAttnWarps, per_sm = p.wide ? 1 : decode_ctas_per_sm(ring, D);
+    p.splits = decode_splits(B, p.Hkv, rows_bound, 16, per_sm, warps);
+    if (step && ring) p.splits = decode_step_splits(B * p.Hkv, rows_bound, 16 * warps, per_sm, p.splits);
+    p.cluster = decode_cluster(B * p.Hkv, p.splits, per_sm);
+}
+
+int mynn::decode_resident_clusters(int size, int ctas_per_sm) {
+    static std::atomic<int> known[64][kMaxClusterSplits + 1];  // per device, one more than the number; of kernels that fill an SM
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return 0;
+    int n = known[dev][size].load(std::memory_order_relaxed);
+    if (n == 0) {
+        auto kern = attention_decode_kernel<__nv_bfloat16, 128, true, false, decode_wide_warps(128)>;
+        constexpr size_t smem = (size_t)decode_wide_warps(128) * kRingDepth * 2 * 2 * 16 * 128;
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = size;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(size);
+        cfg.blockDim = dim3(32 * decode_wide_warps(128));
+        cfg.dynamicSmemBytes = smem;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            n = 0;
+        }
+        known[dev][size].store(++n, std::memory_order_relaxed);
+    }
+    return (n - 1) * ctas_per_sm;
 }
 
 template <typename T, int D, bool WIN, int W, bool STREAM>
@@ -580,7 +604,7 @@ static int launch_decode_ring(cudaStream_t st, const DecodeParams &p, int B, con
     auto kern = attention_decode_kernel<T, D, true, WIN, W, STREAM>;
     static SmemLimit limit;  // with the kernel's static shared memory every head_dim is past the 48 KB that need no opt-in
     MYNN_CUDA_OK(limit.raise((const void *)kern, smem));
-    MYNN_CUDA_OK(launch_dependent_cluster(p.cluster ? p.splits : 1, kern, dim3(p.splits, p.Hkv, B), dim3(W * 32), smem, st, mk, mv, p));
+    MYNN_CUDA_OK(launch_ex(true, p.cluster ? p.splits : 1, kern, dim3(p.splits, p.Hkv, B), dim3(W * 32), smem, st, mk, mv, p));
     MYNN_LAUNCH_OK("attention_decode_kernel");
     return MYNN_OK;
 }
@@ -603,7 +627,7 @@ static int launch_decode(cudaStream_t st, const DecodeParams &p, int B, bool rin
                       : launch_decode_ring<T, D, WIN, kAttnWarps, false>(st, p, B, mk, mv);
     }
     if (p.kvpos) return fail(MYNN_E_UNSUPPORTED, "attention: the streaming form with the append needs the ring kernel");
-    MYNN_CUDA_OK(launch_plain(attention_decode_kernel<T, D, false, WIN, kAttnWarps>, dim3(p.splits, p.Hkv, B), dim3(kAttnWarps * 32), 0, st, mk, mv, p));
+    MYNN_CUDA_OK(launch_ex(false, p.cluster ? p.splits : 1, attention_decode_kernel<T, D, false, WIN, kAttnWarps>, dim3(p.splits, p.Hkv, B), dim3(kAttnWarps * 32), 0, st, mk, mv, p));
     MYNN_LAUNCH_OK("attention_decode_kernel");
     return MYNN_OK;
 }

@@ -364,10 +364,9 @@ __device__ __forceinline__ void decode_tail(const DecodeParams &p, const float (
 
 // How many CTAs share the rows of one (batch, kv head) pair.  All CTAs of a launch last equally long, so the grid should fit
 // in ONE wave of resident CTAs (148 SMs): a partly filled second wave would cost as much time as a full one.  A split is not
-// free either: its partial result goes through the merge (a round trip through L2 per eight splits, plus the tail of one
-// more CTA), so a split gets at least four tiles per warp, and more than eight splits are only used when a split would
-// otherwise be longer than 32 tiles per warp.  (Measured, 2048 rows, 32 pairs: 1 / 2 / 4 / 8 / 16 / 32 splits = 30 / 21 / 15 /
-// 16 / 22 / 33 us; 256 rows, 4 pairs: 1 / 2 / 4 splits = 4.8 / 7.4 / 7.2 us.)
+// free either: its partial result goes through the merge, so a split gets at least four tiles per warp, and more than eight splits are only used
+// when a split would otherwise be longer than 32 tiles per warp.  This is the rule of the operators; steps of a model have one of their own behind it
+// (decode_step_splits).
 inline int decode_splits(int B, int Hkv, int rows_bound, int tile_rows = 16, int ctas_per_sm = kAttnCtasPerSm, int warps = kAttnWarps) {
     const int pairs = B * Hkv;
     const int round = tile_rows * warps;  // rows the warps of a CTA take at a time
@@ -384,6 +383,27 @@ inline int decode_splits(int B, int Hkv, int rows_bound, int tile_rows = 16, int
     }
     if (s > kMaxSplits) s = kMaxSplits;
     return s;
+}
+// Up to eight splits (the largest portable cluster) are the CTAs of one cluster and merge through distributed shared memory, 1.0 us, where all
+// clusters are resident at once; through L2 and a ticket the merge takes 4 to 6 us (five sequences over an int8 cache, 8 kv heads: 512 rows in one split
+// 8.8 us, 1024 in two 15.4 and in a cluster 12.8; 40 clusters of eight do not fit, 4096 rows 20.4 and 27.6).
+constexpr int kMaxClusterSplits = 8;
+// How many clusters of so many CTAs are resident on the current device at once: a cluster lies in one of the parts that the SMs come in, which the
+// driver knows (attention.cu).
+int decode_resident_clusters(int size, int ctas_per_sm);
+inline bool decode_cluster(int pairs, int splits, int ctas_per_sm) {
+    return splits > 1 && splits <= kMaxClusterSplits && decode_resident_clusters(splits, ctas_per_sm) >= pairs;
+}
+// In a step of a model: as many CTAs per pair as fit so, each with the same whole number of rounds (1.3 us each over the int8 cache, 0.85 us over the
+// 16-bit one), where that saves two rounds; `operators`: what decode_splits gives, which very long rows keep.
+inline int decode_step_splits(int pairs, int rows_bound, int round, int ctas_per_sm, int operators) {
+    const int rounds = (rows_bound + round - 1) / round;
+    for (int s = rounds < kMaxClusterSplits ? rounds : kMaxClusterSplits; s > 1; s--) {
+        const int per = (rounds + s - 1) / s, n = (rounds + per - 1) / per;
+        if (!decode_cluster(pairs, n, ctas_per_sm)) continue;
+        return rounds - per < 2 || per > 16 ? operators : n;
+    }
+    return operators;
 }
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }

@@ -114,42 +114,38 @@ extern int g_fuse_rope;                  // see MYNN_OPT_FUSE_ROPE
 extern int g_decode_ring;                // see MYNN_OPT_DECODE_RING
 extern std::atomic<int> g_inject_stall;  // see MYNN_OPT_INJECT_STALL; consumed by the next launch it applies to
 
-// A plain launch through cudaLaunchKernelEx (no attributes): everything in front has completed when it starts.
+// A launch in clusters of `cluster` CTAs along x (1: none).  dependent: it may begin while the kernel in front of it drains; what the kernel may
+// do before its pdl_wait stands above.  Else everything in front has completed when it starts.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_plain(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cfg.attrs = nullptr;
-    cfg.numAttrs = 0;
-    return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
-}
-
-// A launch that may begin while the kernel in front of it drains; what the kernel may do before its pdl_wait stands above.  Clusters of
-// `cluster` CTAs along x.
-template <typename... KArgs, typename... Args>
-inline cudaError_t launch_dependent_cluster(unsigned cluster, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+inline cudaError_t launch_ex(bool dependent, unsigned cluster, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
     cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = cluster;
-    attr[1].val.clusterDim.y = 1;
-    attr[1].val.clusterDim.z = 1;
+    unsigned n = 0;
+    if (dependent) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = cluster;
+        attr[n].val.clusterDim.y = 1;
+        attr[n++].val.clusterDim.z = 1;
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cfg.attrs = attr;
-    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    cfg.numAttrs = n;
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 template <typename... KArgs, typename... Args>
+inline cudaError_t launch_plain(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+    return launch_ex(false, 1, kern, grid, block, smem, st, args...);
+}
+template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
-    return launch_dependent_cluster(1, kern, grid, block, smem, st, args...);
+    return launch_ex(true, 1, kern, grid, block, smem, st, args...);
 }
 
 // Dispatch a launcher template over the three storage dtypes.

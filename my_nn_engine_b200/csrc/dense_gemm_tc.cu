@@ -308,7 +308,7 @@ static int launch_dg(cudaStream_t st, const CUtensorMap &ma, const CUtensorMap &
     static SmemLimit limit;
     MYNN_CUDA_OK(limit.raise((const void *)kern, smem));
     const int pairs = sm_count() / 2;
-    MYNN_CUDA_OK(launch_dependent_cluster(2, kern, dim3((unsigned)(2 * (tiles_bound < pairs ? tiles_bound : pairs))), dim3(kDgThreads), smem, st, ma, mw, p));
+    MYNN_CUDA_OK(launch_ex(true, 2, kern, dim3((unsigned)(2 * (tiles_bound < pairs ? tiles_bound : pairs))), dim3(kDgThreads), smem, st, ma, mw, p));
     MYNN_LAUNCH_OK("dense_gemm_tc_kernel");
     return MYNN_OK;
 }

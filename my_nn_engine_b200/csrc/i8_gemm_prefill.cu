@@ -547,7 +547,7 @@ static int launch_pf(cudaStream_t st, const CUtensorMap &mw, const CUtensorMap &
     static SmemLimit limit;
     MYNN_CUDA_OK(limit.raise((const void *)kern, smem));
     const int tiles = p.w_tiles * p.t_tiles, pairs = sm_count() / 2;
-    MYNN_CUDA_OK(launch_dependent_cluster(2, kern, dim3(2 * (tiles < pairs ? tiles : pairs)), dim3(kPfThreads), smem, st, mw, ma, p));
+    MYNN_CUDA_OK(launch_ex(true, 2, kern, dim3(2 * (tiles < pairs ? tiles : pairs)), dim3(kPfThreads), smem, st, mw, ma, p));
     MYNN_LAUNCH_OK("i8_prefill_gemm_kernel");
     return MYNN_OK;
 }

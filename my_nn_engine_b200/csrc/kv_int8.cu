@@ -14,8 +14,6 @@
 //     (row 2t, row 2t+1) pairs of two head-dim values, i.e. two A-fragment registers;
 //   * k_scale multiplies S per kv row after the MMA, v_scale multiplies P per kv row before it, so the tensor cores
 //     only ever see exact small integers on the cache side.
-#include <algorithm>
-
 #include "attention_internal.cuh"
 #include "i8_cvt.cuh"
 #include "i8_gemm.cuh"
@@ -217,7 +215,7 @@ attention_decode_q8_kernel(const __grid_constant__ CUtensorMap map_k, const __gr
     const int G = p.G;
     int active = p.active_dev ? *p.active_dev : p.active_host;
     active = max(0, min(active, p.cache_seq));
-    // A cluster with one round of rows leaves them to its first CTA.
+    // A cluster whose rows are a round or less leaves them to its first CTA.
     const bool solo = p.cluster && active <= 32 * kAttnWarps;
     if (solo && split > 0) return;
     const int splits = solo ? 1 : p.splits;
@@ -664,12 +662,12 @@ static int launch_decode_q8(cudaStream_t st, const DecodeParams &p, int B, bool 
             auto kern = attention_decode_q8_kernel<T, D, true>;
             static SmemLimit limit;
             MYNN_CUDA_OK(limit.raise((const void *)kern, smem));
-            MYNN_CUDA_OK(launch_dependent_cluster(p.cluster ? p.splits : 1, kern, dim3(p.splits, p.Hkv, B), dim3(kAttnWarps * 32), smem, st, mk, mv, p));
+            MYNN_CUDA_OK(launch_ex(true, p.cluster ? p.splits : 1, kern, dim3(p.splits, p.Hkv, B), dim3(kAttnWarps * 32), smem, st, mk, mv, p));
             MYNN_LAUNCH_OK("attention_decode_q8_kernel");
             return MYNN_OK;
         }
     }
-    MYNN_CUDA_OK(launch_plain(attention_decode_q8_kernel<T, D, false>, dim3(p.splits, p.Hkv, B), dim3(kAttnWarps * 32), 0, st, mk, mv, p));
+    MYNN_CUDA_OK(launch_ex(false, p.cluster ? p.splits : 1, attention_decode_q8_kernel<T, D, false>, dim3(p.splits, p.Hkv, B), dim3(kAttnWarps * 32), 0, st, mk, mv, p));
     MYNN_LAUNCH_OK("attention_decode_q8_kernel");
     return MYNN_OK;
 }
@@ -758,14 +756,8 @@ int launch_attention_q8(cudaStream_t st, void *out, const void *q, const void *k
     const bool ring = q8_ring_possible(p, B, D);
     p.splits = decode_splits(B, Hkv, rows_bound, 32, ring ? 2 : kAttnCtasPerSm);
     p.appended = appended;
-    if (appended && ring) {
-        // A step of a model, few pairs: the splits of a pair are a cluster, as many as are resident at once, up to eight, each with a whole number of rounds.
-        const int rounds = (rows_bound + 32 * kAttnWarps - 1) / (32 * kAttnWarps), most = std::min(std::min(8, 2 * 148 / (B * Hkv)), rounds);
-        if (most > 1) {
-            const int per = (rounds + most - 1) / most, s = (rounds + per - 1) / per;
-            if (s >= p.splits) p.splits = s, p.cluster = 1;
-        }
-    }
+    if (appended && ring) p.splits = decode_step_splits(B * Hkv, rows_bound, 32 * kAttnWarps, 2, p.splits);
+    p.cluster = decode_cluster(B * Hkv, p.splits, ring ? 2 : kAttnCtasPerSm);
     if (fuse) {
         if (!ring || !attention_q8_fused_supported(B, Hkv, D, cache_seq_len, k_scale, v_scale))
             return fail(MYNN_E_UNSUPPORTED, "attention_q8: the fused RoPE + append needs the ring form");

@@ -7,13 +7,13 @@
 // This kernel has none of it (the engine's counterpart is dequant_gemv, src/codegen/cuda/cpp/dequant_gemv.cuh:11-59: one
 // warp per row, one 16-byte load in flight per lane):
 //   * one CTA per SM with an equal share of the rows, so the grid is a single balanced wave.  Its rows are tiles of 16; the sixteen warps
-//     deal out the contraction, so that every warp has the same piece of every row, and each lane issues all its 128-bit loads (up to 20)
+//     deal out the contraction, so that every warp has the same piece of every row, and each lane issues all its loads (up to 320 bytes)
 //     before it touches anything else and, where the weights are settled (i8_gemm.cuh), before the programmatic-dependent-launch wait: they
 //     are in flight while the preceding kernel drains;
 //   * the activation row(s) are the same three signed 8-bit limbs of a 23-bit fixed-point value the tensor-core kernel uses, either read
 //     from the workspace, where a fused producer left them, or computed here in shared memory (no extra launch).  Three limbs of up to
-//     five rows are the columns of mma.m16n8k32 (int8, exact int32 sums).  The contraction index is permuted so that the 16 bytes a lane
-//     loads are its fragments of two MMAs, for weights and limbs alike; a warp needs its own piece of the limbs only;
+//     five rows are the columns of mma.m16n8k32 (int8, exact int32 sums).  The contraction index is permuted so that each 16 bytes of a
+//     lane are its fragments of two MMAs, for weights and limbs alike; a warp needs its own piece of the limbs only;
 //   * the warps' int32 sums meet in shared memory once, limbs recombined in int64, the same two roundings as the tensor-core kernel:
 //     the outputs are bit-identical to that kernel's, whichever of the two a shape is dispatched to.
 // The legacy tensor path is enough here: 156 KB of weights per SM (gate/up of a 1B model) are 312 MMAs per eight columns, 0.3 us.  With
@@ -34,8 +34,8 @@ constexpr int kLeanWarps = kLeanThreads / 32;
 constexpr int kLeanTiles = 8;                       // row tiles whose partial sums are kept at a time
 constexpr int kLeanFreeSms = 8;
 constexpr int kLeanPitch = 16 * kLeanTiles + 4;     // int32 per (warp, column): no two lanes of a store in one bank
-// limb rows in shared memory are this far apart: eight rows of a fragment load fall into different banks
-__host__ __device__ __forceinline__ int lean_limb_pitch(int K) { return (K + 127) / 128 * 128 + 64; }
+// limb rows in shared memory are this far apart: a phase of a fragment load covers four 16-byte chunks of two rows, 32 bytes apart in pairs, and the two rows interleave
+__host__ __device__ __forceinline__ int lean_limb_pitch(int K) { return (K + 127) / 128 * 128 + (K > 1024 ? 16 : 64); }
 
 struct LeanParams {
     void *out;
@@ -53,6 +53,12 @@ __device__ __forceinline__ uint4 ldg_stream_16(const void *p) {
     uint4 v;
     asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
+}
+
+__device__ __forceinline__ void ldg_stream_32(uint4 &a, uint4 &b, const void *p) {
+    asm volatile("ld.global.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+                 : "l"(p));
 }
 
 template <typename T>
@@ -154,11 +160,15 @@ __device__ __forceinline__ void mma_i8(int (&c)[4], uint32_t a0, uint32_t a1, ui
 // One CTA per SM owns a contiguous range of weight rows, so that the whole grid is one balanced wave.  A warp owns NB blocks of 64 along K
 // (K <= 1024 NB) of all of them; TG tiles of 16 rows are in flight (2 NB TG <= 20 loads per lane, issued before anything else happens).
 // K % 16 == 0; wq and limbs 16-byte aligned.  Dynamic shared memory: limbs [3 M][pitch] (ACT), partial sums [warp][3 M][kLeanPitch].
+// PAIRS (rows of weights that begin on 32 bytes): a lane's chunks come in pairs, so that the four lanes of a row read a whole line of 128 bytes with one
+// load; with loads of 16 bytes the two halves of a line are two requests.  Steps over 700 rows, 1 / 2 / 3 / 4 sequences: Llama-3-8B shapes 1997 -> 1861,
+// 2004 -> 1875, 1916 -> 1914, 1929 -> 1922 us, TinyLlama shapes 563 -> 558, 575 -> 553, 598 -> 587, 609 -> 597.  (A choice at every load instead of a form of the
+// kernel lost it at one row of TinyLlama, 573 us: code that runs once per launch; loads of 32 bytes for the limbs, too.)
 // GATED: wq holds 2 N rows, N gate rows and behind them the N up rows of the same outputs, and out[m,n] = round(swish(gate) * up) of the two sums,
 // each rounded first.  A tile is eight gate rows and their eight up rows, so both sums of an output lie in one column of the partial sums.
 // TinyLlama shapes, us per layer at 1 / 3 rows: gate/up, SiLU product to limbs, down 3.1 + 3.1 + 2.0 / 4.8 + 3.6 + 2.8; gated, row to limbs, down
 // 2.9 + 1.6 + 2.4 / 4.8 + 1.7 + 2.8.
-template <typename OutT, int M, int NB, int TG, bool ACT, bool GATED>
+template <typename OutT, int M, int NB, int TG, bool ACT, bool GATED, bool PAIRS>
 __global__ void __launch_bounds__(kLeanThreads, 1) gemv_lean_kernel(const LeanParams p) {
     extern __shared__ __align__(16) int8_t sm_dyn[];
     __shared__ float sm_ascale[8];
@@ -174,7 +184,8 @@ __global__ void __launch_bounds__(kLeanThreads, 1) gemv_lean_kernel(const LeanPa
     const OutT *resid_p = reinterpret_cast<const OutT *>(p.resid);
     OutT *out_p = reinterpret_cast<OutT *>(p.out);
 
-    const int c0 = warp * 4 * NB + t;  // this lane's 16-byte chunks of a row: c0 + 4 j
+    // this lane's 16-byte chunks of a row
+    auto chunk = [&](int j) { return warp * 4 * NB + (PAIRS ? 8 * (j / 2) + 2 * t + j % 2 : 4 * j + t); };
     uint4 w[TG][NB][2];
     auto load_tile = [&](uint4 (&x)[NB][2], int tile) {
 #pragma unroll
@@ -182,9 +193,14 @@ __global__ void __launch_bounds__(kLeanThreads, 1) gemv_lean_kernel(const LeanPa
             const int row = kTileOut * tile + gq + (GATED ? 0 : 8 * h);
             const int8_t *wr = p.wq + (size_t)(row0 + (row < rows ? row : 0) + (GATED && h ? p.N : 0)) * K;
 #pragma unroll
-            for (int j = 0; j < NB; j++) {
-                const int c = c0 + 4 * j;
-                x[j][h] = row < rows && c < chunks ? ldg_stream_16(wr + 16 * (size_t)c) : make_uint4(0u, 0u, 0u, 0u);
+            for (int j = 0; j < NB; j += PAIRS ? 2 : 1) {
+                const int c = chunk(j);
+                if constexpr (PAIRS) {
+                    x[j][h] = x[j + 1][h] = make_uint4(0u, 0u, 0u, 0u);
+                    if (row < rows && c < chunks) ldg_stream_32(x[j][h], x[j + 1][h], wr + 16 * (size_t)c);
+                } else {
+                    x[j][h] = row < rows && c < chunks ? ldg_stream_16(wr + 16 * (size_t)c) : make_uint4(0u, 0u, 0u, 0u);
+                }
             }
         }
     };
@@ -218,7 +234,7 @@ __global__ void __launch_bounds__(kLeanThreads, 1) gemv_lean_kernel(const LeanPa
         for (int n = 0; n < NT; n++)
 #pragma unroll
             for (int j = 0; j < NB; j++) {
-                const int c = c0 + 4 * j, col = 8 * n + gq;
+                const int c = chunk(j), col = 8 * n + gq;
                 b[n][j] = col < C && c < chunks ? *reinterpret_cast<const uint4 *>(sm_limbs + (size_t)col * pitch + 16 * c) : make_uint4(0u, 0u, 0u, 0u);
             }
     } else {
@@ -226,7 +242,7 @@ __global__ void __launch_bounds__(kLeanThreads, 1) gemv_lean_kernel(const LeanPa
         for (int n = 0; n < NT; n++)
 #pragma unroll
             for (int j = 0; j < NB; j++) {
-                const int c = c0 + 4 * j, col = 8 * n + gq;
+                const int c = chunk(j), col = 8 * n + gq;
                 b[n][j] = col < C && c < chunks ? __ldcg(reinterpret_cast<const uint4 *>(p.limbs_g + (size_t)col * K + 16 * (size_t)c)) : make_uint4(0u, 0u, 0u, 0u);
             }
         if (threadIdx.x < M) sm_ascale[threadIdx.x] = __ldcg(p.ascale_g + threadIdx.x);
@@ -312,10 +328,10 @@ bool gemv_lean_supported(int M, int N, int K, const void *wq) {
     return M >= 1 && M <= kLeanMaxRows && K >= 16 && K % 16 == 0 && K <= 6144 && (size_t)N * K <= ((size_t)(M <= 2 ? 160 : 32) << 20) && ((uintptr_t)wq % 16) == 0;
 }
 
-template <typename OutT, int M, int NB, int TG, bool ACT, bool GATED>
+template <typename OutT, int M, int NB, int TG, bool ACT, bool GATED, bool PAIRS>
 static int launch_lean(cudaStream_t st, LeanParams p) {
     const size_t smem = lean_smem(ACT, M, p.K);
-    auto kern = gemv_lean_kernel<OutT, M, NB, TG, ACT, GATED>;
+    auto kern = gemv_lean_kernel<OutT, M, NB, TG, ACT, GATED, PAIRS>;
     static SmemLimit limit;
     MYNN_CUDA_OK(limit.raise((const void *)kern, kLeanMaxSmem));
     static int sms = 0;
@@ -351,10 +367,11 @@ static int launch_lean(cudaStream_t st, LeanParams p) {
 // blocks of 64 per warp (K <= 1024 / 2048 / 4096 / 6144) and row tiles in flight
 template <typename OutT, int M, bool ACT, bool GATED = false>
 static int launch_by_k(cudaStream_t st, const LeanParams &p) {
-    if (p.K <= 1024) return launch_lean<OutT, M, 1, 8, ACT, GATED>(st, p);
-    if (p.K <= 2048) return launch_lean<OutT, M, 2, 5, ACT, GATED>(st, p);
-    if (p.K <= 4096) return launch_lean<OutT, M, 4, 2, ACT, GATED>(st, p);
-    return launch_lean<OutT, M, 6, 1, ACT, GATED>(st, p);
+    const bool pairs = p.K % 32 == 0 && (uintptr_t)p.wq % 32 == 0;
+    if (p.K <= 1024) return launch_lean<OutT, M, 1, 8, ACT, GATED, false>(st, p);
+    if (p.K <= 2048) return pairs ? launch_lean<OutT, M, 2, 5, ACT, GATED, true>(st, p) : launch_lean<OutT, M, 2, 5, ACT, GATED, false>(st, p);
+    if (p.K <= 4096) return pairs ? launch_lean<OutT, M, 4, 2, ACT, GATED, true>(st, p) : launch_lean<OutT, M, 4, 2, ACT, GATED, false>(st, p);
+    return pairs ? launch_lean<OutT, M, 6, 1, ACT, GATED, true>(st, p) : launch_lean<OutT, M, 6, 1, ACT, GATED, false>(st, p);
 }
 template <typename OutT>
 static int launch_by_rows(cudaStream_t st, const LeanParams &p, int M) {

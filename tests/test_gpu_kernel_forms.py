@@ -123,6 +123,20 @@ def test_prompt_product_rounds_like_float64(dt, m, n, k):
     assert (got[:-1].double() - want[:-1]).abs().max() <= ulp * want[:-1].abs().max()
 
 
+# ---- lean products: rows of weights that begin on 32 bytes are read in pieces of 32, others in pieces of 16; the same sums, so the same bits ----
+@pytest.mark.parametrize("m", [1, 2, 5])
+@pytest.mark.parametrize("n,k", [(300, 1024), (300, 1056), (1121, 2048), (37, 2080), (700, 4096), (145, 4128), (260, 5632)])
+def test_lean_products_of_aligned_and_unaligned_rows(m, n, k):
+    g = gen(n + k)
+    w, s, act = int8(g, n, k), scales(g, n, torch.bfloat16), randn(g, m, k).bfloat16()
+    moved = torch.empty(n * k + 16, dtype=torch.int8, device="cuda")[16:].view(n, k)
+    moved.copy_(w)
+    assert w.data_ptr() % 32 == 0 and moved.data_ptr() % 32 == 16
+    got, want = ops.dequant_matmul(act, w, s), act.double() @ w.double().t() * s.double()
+    assert torch.equal(got, ops.dequant_matmul(act, moved, s))
+    assert (got.double() - want).abs().max() <= 2.0 ** -7 * want.abs().max()
+
+
 # ---- products of many rows over unquantised weights: pairs of CTAs own 256 weight rows (gating: 128 outputs) and up to 256 activation rows ----
 @pytest.mark.parametrize("dt", ["bf16", "f16"])
 @pytest.mark.parametrize("m,n,k", [(33, 1, 8), (97, 64, 72), (128, 65, 448), (257, 129, 392), (300, 257, 64), (513, 200, 1032), (2500, 640, 136)])

@@ -139,7 +139,9 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t *v) {
                  : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// The aligned forms are defined for whole warps only, and callers come here out of loops and branches in which lanes went different ways.
 __device__ __forceinline__ void cluster_sync_all() {
+    __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // True in one lane of the (converged) warp.  A role's loop is walked by its whole warp and only what one thread has to issue stands behind this: the

@@ -22,7 +22,7 @@ rms_norm_kernel(T *sum_out, T *norm_out, const T *a, const T *b, const T *w, flo
     float ss = 0.f;
     if constexpr (VEC) {
         for (int i = 8 * threadIdx.x; i < D; i += 8 * blockDim.x) {
-            T av[8], bv[8], sv[8];
+            __align__(16) T av[8], bv[8], sv[8];
             *reinterpret_cast<uint4 *>(av) = *reinterpret_cast<const uint4 *>(a + base + i);
             if constexpr (ADD) *reinterpret_cast<uint4 *>(bv) = *reinterpret_cast<const uint4 *>(b + base + i);
 #pragma unroll
@@ -60,7 +60,7 @@ rms_norm_kernel(T *sum_out, T *norm_out, const T *a, const T *b, const T *w, flo
     const float inv = inv_s;
     if constexpr (VEC) {
         for (int i = 8 * threadIdx.x; i < D; i += 8 * blockDim.x) {
-            T wv[8], ov[8];
+            __align__(16) T wv[8], ov[8];
             *reinterpret_cast<uint4 *>(wv) = *reinterpret_cast<const uint4 *>(w + i);
 #pragma unroll
             for (int j = 0; j < 8; j++) ov[j] = from_f32<T>(row[i + j] * inv * to_f32<T>(wv[j]));
@@ -112,7 +112,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) add_vec_kernel(T *out, const T *a, const T *b, long long n8) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n8) return;
-    T av[8], bv[8], ov[8];
+    __align__(16) T av[8], bv[8], ov[8];
     *reinterpret_cast<uint4 *>(av) = reinterpret_cast<const uint4 *>(a)[i];
     *reinterpret_cast<uint4 *>(bv) = reinterpret_cast<const uint4 *>(b)[i];
 #pragma unroll
@@ -277,7 +277,7 @@ rope_kv_append_vec_kernel(T *q_out, T *k_cache, T *v_cache, const T *q, const T 
         return;
     }
     const size_t to = (size_t)positions[s] * D;
-    T xl[8], xh[8], cl[8], ch[8], sl[8], sh[8], ol[8], oh[8];
+    __align__(16) T xl[8], xh[8], cl[8], ch[8], sl[8], sh[8], ol[8], oh[8];
     *reinterpret_cast<uint4 *>(xl) = lo;
     *reinterpret_cast<uint4 *>(xh) = hi;
     *reinterpret_cast<uint4 *>(cl) = *reinterpret_cast<const uint4 *>(cos_t + to + j0);
@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(256) swiglu_strided_vec_kernel(T *out, const T
     const int m = blockIdx.y;
     const int f = 8 * (blockIdx.x * blockDim.x + threadIdx.x);
     if (f >= F) return;
-    T g[8], u[8], o[8];
+    __align__(16) T g[8], u[8], o[8];
     *reinterpret_cast<uint4 *>(g) = *reinterpret_cast<const uint4 *>(gate + (size_t)m * in_stride + f);
     *reinterpret_cast<uint4 *>(u) = *reinterpret_cast<const uint4 *>(up + (size_t)m * in_stride + f);
 #pragma unroll

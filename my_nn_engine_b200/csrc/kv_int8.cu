@@ -290,18 +290,20 @@ attention_decode_q8_kernel(const __grid_constant__ CUtensorMap map_k, const __gr
         const T *qrow = qhead + part * E;
         float mx = 0.f;
         bool bad = false;
-        if (RING && fused && h < G) {
-            T x[E], xp[E], c[E], sn[E];  // E = 8
-            *reinterpret_cast<uint4 *>(x) = *reinterpret_cast<const uint4 *>(qrow);
-            *reinterpret_cast<uint4 *>(xp) = *reinterpret_cast<const uint4 *>(qhead + (part ^ 8) * E);
-            *reinterpret_cast<uint4 *>(c) = *reinterpret_cast<const uint4 *>(cos_t + tab + part * E);
-            *reinterpret_cast<uint4 *>(sn) = *reinterpret_cast<const uint4 *>(sin_t + tab + part * E);
+        if constexpr (RING) {
+            static_assert(E == 8, "a thread's elements are 16 bytes");
+            if (fused && h < G) {
+                const uint4 xr = *reinterpret_cast<const uint4 *>(qrow), xpr = *reinterpret_cast<const uint4 *>(qhead + (part ^ 8) * E);
+                const uint4 cr = *reinterpret_cast<const uint4 *>(cos_t + tab + part * E), snr = *reinterpret_cast<const uint4 *>(sin_t + tab + part * E);
+                const T *x = reinterpret_cast<const T *>(&xr), *xp = reinterpret_cast<const T *>(&xpr), *c = reinterpret_cast<const T *>(&cr), *sn = reinterpret_cast<const T *>(&snr);
 #pragma unroll
-            for (int i = 0; i < E; i++) {
-                const float a = to_f32<T>(x[i]), o_ = to_f32<T>(xp[i]), cc = to_f32<T>(c[i]), ss = to_f32<T>(sn[i]);
-                qv[i] = round_store<T>(part < 8 ? rope_low(a, o_, cc, ss) : rope_high(o_, a, cc, ss));
+                for (int i = 0; i < E; i++) {
+                    const float a = to_f32<T>(x[i]), o_ = to_f32<T>(xp[i]), cc = to_f32<T>(c[i]), ss = to_f32<T>(sn[i]);
+                    qv[i] = round_store<T>(part < 8 ? rope_low(a, o_, cc, ss) : rope_high(o_, a, cc, ss));
+                }
             }
-        } else {
+        }
+        if (!fused || h >= G) {
 #pragma unroll
             for (int i = 0; i < E; i++) qv[i] = h < G ? to_f32<T>(qrow[i]) : 0.f;
         }
@@ -342,14 +344,14 @@ attention_decode_q8_kernel(const __grid_constant__ CUtensorMap map_k, const __gr
         const bool mine = fused && ((new_row >= row_beg && new_row < row_end) || (split == 0 && new_row >= active)) && new_row >= 0 && new_row < p.cache_seq;
         if (mine && warp < 2) {
             const T *src = (warp == 0 ? reinterpret_cast<const T *>(p.fused_k) : reinterpret_cast<const T *>(p.fused_v)) + (size_t)b * p.qkv_stride + (size_t)kvh * D + 4 * lane;
-            T x[4], c[4], sn[4];
-            *reinterpret_cast<uint2 *>(x) = *reinterpret_cast<const uint2 *>(src);
+            const uint2 xr = *reinterpret_cast<const uint2 *>(src);
+            const T *x = reinterpret_cast<const T *>(&xr);
             float v[4], mx = 0.f;
 #pragma unroll
             for (int i = 0; i < 4; i++) v[i] = to_f32<T>(x[i]);
             if (warp == 0) {
-                *reinterpret_cast<uint2 *>(c) = *reinterpret_cast<const uint2 *>(cos_t + tab + 4 * lane);
-                *reinterpret_cast<uint2 *>(sn) = *reinterpret_cast<const uint2 *>(sin_t + tab + 4 * lane);
+                const uint2 cr = *reinterpret_cast<const uint2 *>(cos_t + tab + 4 * lane), snr = *reinterpret_cast<const uint2 *>(sin_t + tab + 4 * lane);
+                const T *c = reinterpret_cast<const T *>(&cr), *sn = reinterpret_cast<const T *>(&snr);
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
                     const float other = __shfl_xor_sync(0xffffffffu, v[i], 16);
@@ -684,9 +686,9 @@ dequant_kv_rows_kernel(T *out, const int8_t *cache, const T *scale, int cache_se
     const int s = (int)(idx / groups), g = (int)(idx - (long long)s * groups);
     const size_t row = (size_t)blockIdx.y * cache_seq + s;
     const float sc = to_f32<T>(scale[row]);
-    int8_t q[16];
+    __align__(16) int8_t q[16];
     *reinterpret_cast<uint4 *>(q) = *reinterpret_cast<const uint4 *>(cache + row * D + 16 * g);
-    T o[16];
+    __align__(16) T o[16];
 #pragma unroll
     for (int i = 0; i < 16; i++) o[i] = from_f32<T>((float)q[i] * sc);
     uint4 *dst = reinterpret_cast<uint4 *>(out + row * D + 16 * g);

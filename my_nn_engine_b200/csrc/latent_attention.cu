@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(lat_warps(R) * 32, R == 128 ? 2 : 1) latent_at
                 w0[i] = lat_exp2(w0[i] - m_new), w1[i] = lat_exp2(w1[i] - m_new), al[i] = lat_exp2(m_old - m_new);
                 top[i] = m_new;
                 sum[i] = w0[i] + w1[i];
-                T two[2] = {from_f32<T>(w0[i]), from_f32<T>(w1[i])};
+                __align__(4) T two[2] = {from_f32<T>(w0[i]), from_f32<T>(w1[i])};
                 *reinterpret_cast<uint32_t *>(&sm.p[r][k]) = *reinterpret_cast<const uint32_t *>(two);
             }
 #pragma unroll
@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(lat_warps(R) * 32, R == 128 ? 2 : 1) latent_at
                 T *out = reinterpret_cast<T *>(p.out) + (slot0 + r) * R + warp * (R / WARPS) + 2 * t4;
 #pragma unroll
                 for (int n = 0; n < NT; n++) {
-                    T two[2] = {from_f32<T>(o[i][n][2 * x] * inv), from_f32<T>(o[i][n][2 * x + 1] * inv)};
+                    __align__(4) T two[2] = {from_f32<T>(o[i][n][2 * x] * inv), from_f32<T>(o[i][n][2 * x + 1] * inv)};
                     *reinterpret_cast<uint32_t *>(out + 8 * n) = *reinterpret_cast<const uint32_t *>(two);
                 }
             } else if (tiles > 0) {
@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(256) latent_merge_kernel(const LatParams p, in
             if (s0 + j < p.splits && f[s0 + j] != 0.f) acc.x += f[s0 + j] * v[j].x, acc.y += f[s0 + j] * v[j].y;
     }
     const float inv = total > 0.f ? 1.0f / total : 0.f;
-    T two[2] = {from_f32<T>(acc.x * inv), from_f32<T>(acc.y * inv)};
+    __align__(4) T two[2] = {from_f32<T>(acc.x * inv), from_f32<T>(acc.y * inv)};
     *reinterpret_cast<uint32_t *>(reinterpret_cast<T *>(p.out) + slot * R + 2 * threadIdx.x) = *reinterpret_cast<const uint32_t *>(two);
 }
 

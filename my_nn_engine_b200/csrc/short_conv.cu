@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(128) conv_step_vec_kernel(const ConvStep p, in
                 y[2 * i + 1] = rope_high(u, v, cs, sn);
             }
         }
-        T o[8];
+        __align__(16) T o[8];
 #pragma unroll
         for (int i = 0; i < 8; i++) o[i] = from_f32<T>(y[i]);
         *reinterpret_cast<uint4 *>(dst + (size_t)(rows ? pos % rows : s) * width) = *reinterpret_cast<const uint4 *>(o);

@@ -45,7 +45,7 @@ __global__ void rope_cache_rows_kernel(T *out, const T *x, const T *cos_t, const
     if (idx >= (long long)active * groups) return;
     const int s = (int)(idx / groups), j0 = 8 * (int)(idx - (long long)s * groups);
     const size_t ro = ((size_t)blockIdx.y * cache_seq + s) * D, to = (size_t)kv_position[s] * D;
-    T xl[8], xh[8], cl[8], ch[8], sl[8], sh[8], ol[8], oh[8];
+    __align__(16) T xl[8], xh[8], cl[8], ch[8], sl[8], sh[8], ol[8], oh[8];
     *reinterpret_cast<uint4 *>(xl) = *reinterpret_cast<const uint4 *>(x + ro + j0);
     *reinterpret_cast<uint4 *>(xh) = *reinterpret_cast<const uint4 *>(x + ro + j0 + half);
     *reinterpret_cast<uint4 *>(cl) = *reinterpret_cast<const uint4 *>(cos_t + to + j0);

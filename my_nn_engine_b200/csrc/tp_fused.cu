@@ -113,7 +113,7 @@ tp_reduce_norm_limbs_kernel(int8_t *limbs, float *ascale, T *x, const T *w, floa
                 acc.w += v[r].w;
             }
         const float s4[4] = {acc.x, acc.y, acc.z, acc.w};
-        T xv[4];  // four residual elements with one access each way
+        __align__(16) T xv[4];  // four residual elements with one access each way
         if constexpr (sizeof(T) == 2) *reinterpret_cast<uint2 *>(xv) = *reinterpret_cast<const uint2 *>(xrow + i);
         else *reinterpret_cast<float4 *>(xv) = *reinterpret_cast<const float4 *>(xrow + i);
 #pragma unroll

@@ -20,3 +20,14 @@ def test_aligned_cluster_barriers_are_reached_by_whole_warps():
             found += 1
             assert text[:m.start()].rstrip().endswith("__syncwarp();"), name
     assert found
+
+
+def test_local_arrays_are_aligned_for_the_pieces_they_are_accessed_in():
+    """A local array of small elements that is read or written through a wider type says so by its alignment: in registers it makes no difference, in a
+    debug build or after a spill it is a misaligned access."""
+    element = r"(?:T|O|OutT|ActT|__half|__nv_bfloat16|u?int8_t)"
+    for name, text in sources():
+        for m in re.finditer(r"reinterpret_cast<(?:const )?(?:u?int[248]|float[24]|u?int(?:32|64)_t) \*>\((\w+)", text):
+            declared = list(re.finditer(r"^.*?\b%s(\[|\b)[^;\n]*" % m.group(1), text[:m.start()], re.M))
+            arrays = [d.group(0).strip() for d in declared if re.match(r"\s*(?:__align__\(\d+\) )?%s (?:\w+\[\w+\], )*%s\[" % (element, m.group(1)), d.group(0))]
+            assert not arrays or arrays[-1].startswith("__align__"), (name, arrays[-1])

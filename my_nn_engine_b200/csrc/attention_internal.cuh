@@ -210,12 +210,16 @@ __device__ __forceinline__ void decode_row_limbs(const DecodeParams &p, int b, u
     if (threadIdx.x == 0) p.row_ticket[b] = 0u;
 }
 
+__device__ __forceinline__ float merge_reference(float mx) { return mx == -INFINITY ? 0.f : mx; }
+
 // Tail of a decode CTA.  Every lane holds NACC accumulator tiles of O^T: tile i, registers {0,1,2,3} are
 // (head 2t, d), (head 2t+1, d), (head 2t, d+1), (head 2t+1, d+1) with d = DMap::d(i, g).  The warps are merged through
 // shared memory; with more than one split the partial result goes to the workspace and the last CTA of the
 // (batch, kv head) pair to arrive (atomic ticket, no spinning) combines the splits and writes the output.
 // splits: of this pair (p.splits, or 1 where one CTA has all rows).
 // The splits of a cluster keep their partial results in shared memory instead, and behind a cluster barrier each merges its share of the outputs.
+// A part whose maximum is -inf has no rows, and sums of 0, or scores that are all NaN, and sums of NaN.  It is not left out: its factor is 0, which
+// adds nothing in the one case and keeps the NaN in the other.
 // ext != nullptr: the per-warp output staging rows live in caller-provided shared memory, warp w's [8][D] floats at
 // ext + w * ext_stride (the ring kernel hands every warp a piece of its own, by then idle, ring).
 template <typename T, int D, int NACC, typename DMap, bool EXT = false, int W = kAttnWarps>
@@ -263,13 +267,12 @@ __device__ __forceinline__ void decode_tail(const DecodeParams &p, const float (
 #pragma unroll
         for (int w = 0; w < W; w++) mx = fmaxf(mx, sm_m[w][hd]);
         float L = 0.f, O = 0.f;
-        if (mx > -INFINITY) {
+        const float ref = merge_reference(mx);
 #pragma unroll
-            for (int w = 0; w < W; w++) {
-                const float f = __expf(sm_m[w][hd] - mx);
-                L += sm_l[w][hd] * f;
-                O += so_base[(size_t)w * so_stride + hd * D + d] * f;
-            }
+        for (int w = 0; w < W; w++) {
+            const float f = __expf(sm_m[w][hd] - ref);
+            L += sm_l[w][hd] * f;
+            O += so_base[(size_t)w * so_stride + hd * D + d] * f;
         }
         if (splits == 1) {
             outp[(size_t)hd * D + d] = from_f32<T>(O / L);
@@ -302,14 +305,14 @@ __device__ __forceinline__ void decode_tail(const DecodeParams &p, const float (
                 ms[j] = ld_cluster_f32(map_rank(smem_u32(&sm_cm[hd]), r));
                 ls[j] = ld_cluster_f32(map_rank(smem_u32(&sm_cl[hd]), r));
                 os[j] = ld_cluster_f32(map_rank(smem_u32(&so_base[idx]), r));
-                if (j >= splits) ms[j] = -INFINITY;
+                if (j >= splits) ms[j] = -INFINITY, ls[j] = os[j] = 0.f;
             }
 #pragma unroll
             for (int j = 0; j < 8; j++) mx = fmaxf(mx, ms[j]);
+            const float ref = merge_reference(mx);
 #pragma unroll
             for (int j = 0; j < 8; j++) {
-                if (ms[j] == -INFINITY) continue;
-                const float f = __expf(ms[j] - mx);
+                const float f = __expf(ms[j] - ref);
                 L += ls[j] * f;
                 O += os[j] * f;
             }
@@ -343,14 +346,12 @@ __device__ __forceinline__ void decode_tail(const DecodeParams &p, const float (
             float cm = mx;
 #pragma unroll
             for (int j = 0; j < 8; j++) cm = fmaxf(cm, ms[j]);
-            if (cm == -INFINITY) continue;  // nothing but empty splits so far
-            const float f0 = __expf(mx - cm);  // 0 while mx is still -inf
+            const float ref = merge_reference(cm), f0 = __expf(mx - ref);  // 0 while mx is still -inf
             L *= f0;
             O *= f0;
 #pragma unroll
             for (int j = 0; j < 8; j++) {
-                if (ms[j] == -INFINITY) continue;
-                const float f = __expf(ms[j] - cm);
+                const float f = __expf(ms[j] - ref);
                 L += ls[j] * f;
                 O += os[j] * f;
             }

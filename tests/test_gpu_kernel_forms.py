@@ -329,3 +329,30 @@ def test_int8_step_with_the_append_inside(dt, batch, hkv, rows):
         assert (got - want).abs().max() <= 2.0 ** (-6 if dt == "bf16" else -9) * want.abs().max(), pos
     for m in model.values():
         m.close()
+
+
+# ---- decode attention whose splits meet: scores that are NaN in all rows of a warp or of a split are not lost, and stay with their sequence ----
+@pytest.mark.parametrize("form", ["int8", "plain", "window"])
+@pytest.mark.parametrize("d,batch,rows", [(64, 2, 64), (128, 3, 512), (64, 2, 2048), (128, 2, 2048), (64, 2, 3072), (128, 20, 1024), (128, 2, 40960)])
+def test_nan_rows_reach_the_output_through_every_merge(form, d, batch, rows):
+    """One CTA; clusters of two to eight splits; through L2 (40960 rows, 16 splits).  Only a range of whole splits shows a loss."""
+    hq, g, scale, dt = 4, gen(rows + d), d ** -0.5, torch.bfloat16
+    q, k, v = randn(g, batch, hq, 1, d).to(dt), randn(g, batch, 2, rows, d).to(dt), randn(g, batch, 2, rows, d).to(dt)
+    if form == "int8":
+        k, v, ks, vs = int8(g, *k.shape), int8(g, *k.shape), *(scales(g, batch * 2 * rows, dt).view(batch, 2, rows) for _ in range(2))
+
+    def run(where):
+        if form == "int8":
+            bad = ks.clone()
+            bad[1, 0, where] = float("nan")
+            return ops.attention_q8(q, k, v, bad, vs, scale)
+        bad = k.clone()
+        bad[1, 0, where] = float("nan")
+        return ops.attention(q, bad, v, scale) if form == "plain" else ops.window_attention(q, bad, v, scale, rows).transpose(1, 2)
+
+    clean = run(slice(0, 0))
+    assert torch.isfinite(clean).all()
+    for where in (slice(0, 16), slice(0, rows // 8 * 3), slice(0, rows // 2), slice(rows // 4, rows // 2), slice(rows // 2, rows), slice(rows - 1, rows)):
+        got, want = run(where), clean.clone()
+        want[1, :hq // 2] = float("nan")
+        assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.nan_to_num(), want.nan_to_num()), where

@@ -34,8 +34,17 @@ constexpr int kLeanWarps = kLeanThreads / 32;
 constexpr int kLeanTiles = 8;                       // row tiles whose partial sums are kept at a time
 constexpr int kLeanFreeSms = 8;
 constexpr int kLeanPitch = 16 * kLeanTiles + 4;     // int32 per (warp, column): no two lanes of a store in one bank
-// limb rows in shared memory are this far apart: a phase of a fragment load covers four 16-byte chunks of two rows, 32 bytes apart in pairs, and the two rows interleave
-__host__ __device__ __forceinline__ int lean_limb_pitch(int K) { return (K + 127) / 128 * 128 + (K > 1024 ? 16 : 64); }
+// Limb rows in shared memory are this far apart.  A phase of a fragment load is eight lanes, four chunks of 16 bytes in each of two rows: 32 bytes apart
+// with pairs, where the second row fills the gaps, side by side without, where it takes the other half of the banks.
+__host__ __device__ constexpr int lean_limb_pitch(int K, bool pairs) { return (K + 127) / 128 * 128 + (pairs ? 16 : 64); }
+constexpr bool lean_phase_has_all_banks(int K, bool pairs) {
+    unsigned banks = 0;  // in groups of four: the 16 bytes of a lane
+    for (int row = 0; row < 2; row++)
+        for (int t = 0; t < 4; t++) banks |= 1u << (row * lean_limb_pitch(K, pairs) + (pairs ? 32 : 16) * t) / 16 % 8;
+    return banks == 0xffu;
+}
+static_assert(lean_phase_has_all_banks(1024, false) && lean_phase_has_all_banks(2064, false) && lean_phase_has_all_banks(2080, true) && lean_phase_has_all_banks(4096, true),
+              "two lanes of a phase in one bank");
 
 struct LeanParams {
     void *out;
@@ -175,7 +184,7 @@ __global__ void __launch_bounds__(kLeanThreads, 1) gemv_lean_kernel(const LeanPa
     __shared__ unsigned sm_max[2][kLeanWarps];
     constexpr int C = 3 * M, NT = (C + 7) / 8;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, t = lane & 3;
-    const int K = p.K, chunks = K >> 4, pitch = lean_limb_pitch(K);
+    const int K = p.K, chunks = K >> 4, pitch = lean_limb_pitch(K, PAIRS);
     constexpr int kTileOut = GATED ? 8 : 16;  // outputs per tile of 16 rows
     const int row0 = blockIdx.x * p.rows_per_cta, rows = min(p.rows_per_cta, p.N - row0), tiles = (rows + kTileOut - 1) / kTileOut;  // in outputs
     int8_t *sm_limbs = sm_dyn;
@@ -316,7 +325,7 @@ __global__ void __launch_bounds__(kLeanThreads, 1) gemv_lean_kernel(const LeanPa
 }
 
 constexpr int kLeanMaxSmem = 226 * 1024;
-static size_t lean_smem(bool act, int M, int K) { return (act ? (size_t)3 * M * lean_limb_pitch(K) : 0) + (size_t)kLeanWarps * 3 * M * kLeanPitch * sizeof(int); }
+static size_t lean_smem(bool act, bool pairs, int M, int K) { return (act ? (size_t)3 * M * lean_limb_pitch(K, pairs) : 0) + (size_t)kLeanWarps * 3 * M * kLeanPitch * sizeof(int); }
 
 // Up to two rows all matrices of a layer (28672 x 4096, 112 MB, as an operator at one row: 20.5 us against 23.5 us with the tcgen05 kernel and
 // its pre-pass; Llama-3-8B steps of one and two sequences over 1000 rows 2356 -> 2232 and 2342 -> 2265 us).  The line at 160 MB lies above the
@@ -330,7 +339,7 @@ bool gemv_lean_supported(int M, int N, int K, const void *wq) {
 
 template <typename OutT, int M, int NB, int TG, bool ACT, bool GATED, bool PAIRS>
 static int launch_lean(cudaStream_t st, LeanParams p) {
-    const size_t smem = lean_smem(ACT, M, p.K);
+    const size_t smem = lean_smem(ACT, PAIRS, M, p.K);
     auto kern = gemv_lean_kernel<OutT, M, NB, TG, ACT, GATED, PAIRS>;
     static SmemLimit limit;
     MYNN_CUDA_OK(limit.raise((const void *)kern, kLeanMaxSmem));

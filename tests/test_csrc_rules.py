@@ -12,14 +12,15 @@ def sources():
             yield os.path.basename(path), re.sub(r"//[^\n]*", "", f.read())
 
 
-def test_aligned_cluster_barriers_are_reached_by_whole_warps():
-    """barrier.cluster.*.aligned is undefined unless the whole warp executes it together: a warp barrier stands right in front."""
+def test_aligned_instructions_are_reached_by_whole_warps():
+    """barrier.cluster.*.aligned and the loads, stores and waits of tensor memory are undefined unless the whole warp executes them together: a warp barrier
+    stands right in front of each."""
     found = 0
     for name, text in sources():
-        for m in re.finditer(r'asm volatile\(\s*"barrier\.cluster\.[a-z.]*aligned', text):
+        for m in re.finditer(r'asm volatile\(\s*"(?:barrier\.cluster|tcgen05\.(?:ld|st|wait))[a-z.:]*aligned', text):
             found += 1
-            assert text[:m.start()].rstrip().endswith("__syncwarp();"), name
-    assert found
+            assert text[:m.start()].rstrip().endswith("__syncwarp();"), (name, m.group(0))
+    assert found >= 8
 
 
 def test_local_arrays_are_aligned_for_the_pieces_they_are_accessed_in():

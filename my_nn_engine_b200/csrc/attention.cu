@@ -136,8 +136,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         T *re = reinterpret_cast<T *>(&r);
 #pragma unroll
         for (int e = 0; e < 8; e++) {
-            const float a = to_f32<T>(xe[e]), b_ = to_f32<T>(pe[e]), ce_ = to_f32<T>(ce[e]), se_ = to_f32<T>(se[e]);
-            re[e] = from_f32<T>(low ? a * ce_ - b_ * se_ : a * ce_ + b_ * se_);
+            re[e] = from_f32<T>(rope_cached(to_f32<T>(xe[e]), to_f32<T>(pe[e]), to_f32<T>(ce[e]), to_f32<T>(se[e]), low));
         }
         return r;
     };

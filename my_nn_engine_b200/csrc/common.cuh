@@ -71,10 +71,13 @@ template <>
 __device__ __forceinline__ __half from_f32<__half>(float v) { return __float2half_rn(v); }
 
 // One RoPE pair (xl, xh = the elements half a head apart) with the roundings of the engine's CPU kernel: two products and
-// one sum, each rounded to f32, never contracted into a fused multiply-add.  Every kernel that rotates uses these, so the
+// one sum, each rounded to f32, never contracted into a fused multiply-add.  Every kernel that rotates what it stores uses these, so the
 // stand-alone RoPE kernel and the rotation inside the decode attention kernel give the same bits.
 __device__ __forceinline__ float rope_low(float xl, float xh, float c, float s) { return __fsub_rn(__fmul_rn(xl, c), __fmul_rn(xh, s)); }
 __device__ __forceinline__ float rope_high(float xl, float xh, float c, float s) { return __fadd_rn(__fmul_rn(xh, c), __fmul_rn(xl, s)); }
+// The exception: the 16-bit keys of a streaming cache, which are rotated anew at each step, by a kernel of their own or on their way into the product, with
+// the first product not rounded.  An element against its partner half a head away.
+__device__ __forceinline__ float rope_cached(float x, float partner, float c, float s, bool low) { return __fmaf_rn(x, c, low ? -__fmul_rn(partner, s) : __fmul_rn(partner, s)); }
 
 // One store point: round to storage dtype and come back to f32.
 template <typename T>

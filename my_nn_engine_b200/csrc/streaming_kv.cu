@@ -55,8 +55,8 @@ __global__ void rope_cache_rows_kernel(T *out, const T *x, const T *cos_t, const
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         const float a = to_f32<T>(xl[i]), b = to_f32<T>(xh[i]);
-        ol[i] = from_f32<T>(a * to_f32<T>(cl[i]) - b * to_f32<T>(sl[i]));
-        oh[i] = from_f32<T>(b * to_f32<T>(ch[i]) + a * to_f32<T>(sh[i]));
+        ol[i] = from_f32<T>(rope_cached(a, b, to_f32<T>(cl[i]), to_f32<T>(sl[i]), true));
+        oh[i] = from_f32<T>(rope_cached(b, a, to_f32<T>(ch[i]), to_f32<T>(sh[i]), false));
     }
     *reinterpret_cast<uint4 *>(out + ro + j0) = *reinterpret_cast<const uint4 *>(ol);
     *reinterpret_cast<uint4 *>(out + ro + j0 + half) = *reinterpret_cast<const uint4 *>(oh);

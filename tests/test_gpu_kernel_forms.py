@@ -29,6 +29,26 @@ def scales(g, n, dt):
     return (0.002 + 0.018 * torch.rand(n, generator=g, device="cuda")).to(dt)
 
 
+def oracle_steps(cfg, state, dt, batch, rows, **options):
+    """step(pos, tokens, caches) -> logits of the CPU oracle over given caches (torch tensors by attribute name, of the first layer), and the oracle."""
+    from oracle.ref_model import LlamaConfig, OracleLlama
+    weights = {n: t.cpu().numpy() if t.dtype == torch.int8 else R.store_round(t.float().cpu().numpy(), dt) for n, t in state.items()}
+    oracle = OracleLlama(LlamaConfig.from_hf(cfg), weights, dt, rows, batch, c_attention="streaming" not in options, **options)
+
+    def step(pos, tokens, caches):
+        for name, t in caches.items():
+            getattr(oracle, name)[0] = t.cpu().numpy() if t.dtype == torch.int8 else t.float().cpu().numpy()
+        oracle.past_len = pos
+        oracle.decode_step(tokens)
+        return torch.from_numpy(oracle.last_logits).double()
+
+    return step, oracle
+
+
+# a layer and the head store about a dozen roundings of half an ulp (2^-9, 2^-12) on the way from the attention to the logits, which add up like a random walk
+LAYER = {"bf16": 2.0 ** -6, "f16": 2.0 ** -9}
+
+
 # ---- DequantMatMul of a few rows: up to five go to the lean kernel, eight to the tcgen05 one ----
 @pytest.mark.parametrize("dt", ["bf16", "f16", "f32"])
 @pytest.mark.parametrize("n,k", [(1, 16), (130, 1040), (2561, 2048), (2100, 4096), (700, 4112), (5000, 6144), (40001, 512), (9000, 4096)])
@@ -266,69 +286,159 @@ def test_fused_append_over_a_long_cache(head_dim, kv_heads, batch):
         assert (a - b).abs().max() <= 8 * 2.0 ** -7 * a.abs().max(), past
 
 
-# ---- streaming steps: rotation and append inside the attention kernel, one CTA or a cluster per kv head, against the kernels of their own ----
+# ---- streaming steps: rotation and append inside the attention kernel, one CTA or a cluster per kv head, against the kernels of their own and the oracle ----
 @pytest.mark.parametrize("dt", ["bf16", "f16"])
 @pytest.mark.parametrize("d,batch,window", [(64, 1, 15), (64, 3, 509), (64, 2, 1100), (128, 1, 300), (128, 2, 1300), (64, 30, 90)])
 def test_streaming_step_with_the_append_inside(dt, d, batch, window):
+    """Rows that the step overwrites, and those that are not live yet, hold NaN and infinities."""
     from my_nn_engine_b200.decoder import DecoderModel
     from my_nn_engine_b200.quantize import random_llama_state
     cfg = dict(hidden_size=256, num_hidden_layers=1, num_attention_heads=6, num_key_value_heads=2 if batch < 30 else 3, head_dim=d, intermediate_size=512, vocab_size=300,
                rms_norm_eps=1e-5, rope_theta=1e4)
     sink, tokens = 4, np.arange(batch) * 37 % 300
-    model = {}
+    rows, state, model = -(-(sink + window) // 8) * 8, random_llama_state(cfg, seed=7), {}
     try:
         for fused in (1, 0):
             ffi.set_option(ffi.OPT_FUSE_ROPE, fused)  # read when a step is captured
-            model[fused] = DecoderModel(cfg, random_llama_state(cfg, seed=7), dtype=dt, max_seq_len=-(-(sink + window) // 8) * 8, batch=batch, streaming=(sink, window))
+            model[fused] = DecoderModel(cfg, state, dtype=dt, max_seq_len=rows, batch=batch, streaming=(sink, window))
             model[fused].stream(tokens, 0)
     finally:
         ffi.set_option(ffi.OPT_FUSE_ROPE, 1)
+    want_step, _ = oracle_steps(cfg, state, dt, batch, rows, streaming=(sink, window))
     g = gen(window)
     for pos in (0, 1, 3, 17, sink + window - 1, sink + window, 3 * window + 5):
-        past = randn(g, *model[1].k_cache[0].shape).to(DT[dt]), randn(g, *model[1].k_cache[0].shape).to(DT[dt])
+        past = [randn(g, *model[1].k_cache[0].shape).to(DT[dt]) for _ in range(2)]
+        slot = pos if pos < sink else sink + (pos - sink) % window
+        for t in past:
+            t[:, :, pos + 1:] = float("nan")
+            t[:, :, slot, ::2], t[:, :, slot, 1::2] = float("nan"), float("inf")
         for m in model.values():
             m.k_cache[0].copy_(past[0])
             m.v_cache[0].copy_(past[1])
         torch.cuda.synchronize()
-        got, want = (model[f].stream(tokens, pos).clone().double() for f in (1, 0))
+        got, apart = (model[f].stream(tokens, pos).clone().double() for f in (1, 0))
         torch.cuda.synchronize()
-        assert torch.equal(model[1].k_cache[0], model[0].k_cache[0]) and torch.equal(model[1].v_cache[0], model[0].v_cache[0])
+        for a, b in zip(*((m.k_cache[0], m.v_cache[0]) for m in model.values())):
+            assert torch.equal(a.view(torch.int16), b.view(torch.int16)) and torch.isfinite(a[:, :, slot]).all()
+        want = want_step(pos, tokens, dict(k_cache=past[0], v_cache=past[1]))
         # the sums of the attention in another order: a rounding of its output here and there, carried through the rest of the layer
-        assert (got - want).abs().max() <= 2.0 ** (-6 if dt == "bf16" else -9) * want.abs().max(), pos
+        assert (got - apart).abs().max() <= LAYER[dt] * apart.abs().max(), pos
+        assert (got - want).abs().max() <= LAYER[dt] * want.abs().max(), pos
     for m in model.values():
         m.close()
 
 
-# ---- int8 cache, the same: rounds of 128 rows, one CTA, clusters of whole rounds, more pairs than SMs; the new row anywhere in its tile ----
+# ---- int8 cache, the same: rounds of 128 rows, one CTA, clusters of whole rounds, more pairs than SMs; the new row anywhere in its tile, also a short one ----
 @pytest.mark.parametrize("dt", ["bf16", "f16"])
-@pytest.mark.parametrize("batch,hkv,rows", [(1, 1, 128), (1, 2, 2048), (5, 8, 768), (32, 5, 256)])
+@pytest.mark.parametrize("batch,hkv,rows", [(1, 1, 128), (2, 1, 40), (3, 2, 136), (1, 2, 2048), (5, 8, 768), (2, 3, 3008), (32, 5, 256)])
 def test_int8_step_with_the_append_inside(dt, batch, hkv, rows):
+    """The same splits, tiles and sums as with a kernel in front that rotates and quantizes, so the same bits."""
     from my_nn_engine_b200.decoder import DecoderModel
     from my_nn_engine_b200.quantize import random_llama_state
     cfg = dict(hidden_size=256, num_hidden_layers=1, num_attention_heads=2 * hkv, num_key_value_heads=hkv, head_dim=128, intermediate_size=512, vocab_size=300,
                rms_norm_eps=1e-5, rope_theta=1e4)
-    tokens, model, g = np.arange(batch) * 37 % 300, {}, gen(rows + batch)
+    tokens, model, g, state = np.arange(batch) * 37 % 300, {}, gen(rows + batch), random_llama_state(cfg, seed=9)
+    names = ("k_cache", "v_cache", "k_scale", "v_scale")
     try:
         for fused in (1, 0):
             ffi.set_option(ffi.OPT_FUSE_ROPE, fused)  # read when a step is captured
-            model[fused] = DecoderModel(cfg, random_llama_state(cfg, seed=9), dtype=dt, max_seq_len=rows, batch=batch, kv_int8=True)
+            model[fused] = DecoderModel(cfg, state, dtype=dt, max_seq_len=rows, batch=batch, kv_int8=True)
             model[fused].step(tokens, 0)
     finally:
         ffi.set_option(ffi.OPT_FUSE_ROPE, 1)
-    for pos in (0, 1, 31, 32, 100, 127, rows // 2 + 3, rows - 1):
+    want_step, _ = oracle_steps(cfg, state, dt, batch, rows, kv_int8=True)
+    for pos in sorted({0, 1, 31, 32, 100, 127, rows // 2 + 3, rows - 9, rows - 1}):
+        if pos >= rows:
+            continue
         past = [int8(g, *model[1].k_cache[0].shape) for _ in range(2)] + [scales(g, model[1].k_scale[0].numel(), DT[dt]).view_as(model[1].k_scale[0]) for _ in range(2)]
         for m in model.values():
-            for to, t in zip((m.k_cache, m.v_cache, m.k_scale, m.v_scale), past):
-                to[0].copy_(t)
+            for name, t in zip(names, past):
+                getattr(m, name)[0].copy_(t)
         torch.cuda.synchronize()
-        got, want = (model[f].step(tokens, pos).clone().double() for f in (1, 0))
+        got, apart = (model[f].step(tokens, pos).clone().double() for f in (1, 0))
         torch.cuda.synchronize()
-        for a, b in zip(*((m.k_cache[0], m.v_cache[0], m.k_scale[0], m.v_scale[0]) for m in model.values())):
-            assert torch.equal(a, b)
-        # the sums of the attention in another order: a rounding of its output here and there, carried through the rest of the layer
-        assert (got - want).abs().max() <= 2.0 ** (-6 if dt == "bf16" else -9) * want.abs().max(), pos
+        for name in names:
+            assert torch.equal(getattr(model[1], name)[0], getattr(model[0], name)[0])
+        assert torch.equal(got, apart), pos
+        want = want_step(pos, tokens, dict(zip(names, past)))
+        assert (got - want).abs().max() <= LAYER[dt] * want.abs().max(), pos
     for m in model.values():
         m.close()
+
+
+# ---- more sequences than the lean products take: the attention leaves its rows as limbs, behind the merge of a cluster too ----
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("d,batch,hkv,rows", [(128, 6, 1, 1024), (64, 6, 1, 2048), (128, 9, 2, 1536), (64, 20, 1, 1536)])
+def test_clusters_leave_limbs_like_the_oracle(dt, d, batch, hkv, rows):
+    """Both sides of the two rounds (256 rows of eight warps, 512 of sixteen) that a cluster leaves to its first CTA."""
+    from my_nn_engine_b200.decoder import DecoderModel
+    from my_nn_engine_b200.quantize import random_llama_state
+    cfg = dict(hidden_size=256, num_hidden_layers=1, num_attention_heads=4 * hkv, num_key_value_heads=hkv, head_dim=d, intermediate_size=512, vocab_size=300,
+               rms_norm_eps=1e-5, rope_theta=1e4)
+    state, g, tokens = random_llama_state(cfg, seed=3), gen(rows + d), np.arange(batch) * 37 % 300
+    model = DecoderModel(cfg, state, dtype=dt, max_seq_len=rows, batch=batch)
+    want_step, _ = oracle_steps(cfg, state, dt, batch, rows)
+    for pos in (0, 70, 254, 255, 256, 511, 512, 513, 900, rows - 1):
+        past = [randn(g, *model.k_cache[0].shape).to(DT[dt]) for _ in range(2)]
+        model.k_cache[0].copy_(past[0])
+        model.v_cache[0].copy_(past[1])
+        torch.cuda.synchronize()
+        got, want = model.step(tokens, pos).clone().double(), want_step(pos, tokens, dict(k_cache=past[0], v_cache=past[1]))
+        assert (got - want).abs().max() <= LAYER[dt] * want.abs().max(), pos
+    model.close()
+
+
+# ---- windows over a ring: clusters whose first visible row lies inside a tile, rows on both sides of the two rounds that one CTA takes ----
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("d,window", [(128, 241), (128, 255), (128, 256), (128, 257), (128, 700), (64, 497), (64, 511), (64, 512), (64, 513), (64, 1000)])
+def test_windows_that_clusters_share(dt, d, window):
+    g, rows, batch, hkv, hq = gen(window), 1024, 2, 2, 6
+    q, k, v = (randn(g, batch, h, n, d).to(DT[dt]) for h, n in ((hq, 1), (hkv, rows), (hkv, rows)))
+    for active in (window - 3, window + 5, 800, 1000, 1024, 1031, 5003):
+        at = torch.arange(max(0, active - window), active) % rows
+        kk, vv = (t[:, :, at].double().repeat_interleave(hq // hkv, 1) for t in (k, v))
+        for cap in (0.0, 6.0):
+            s = q.double() @ kk.transpose(2, 3) * d ** -0.5
+            want = ((cap * torch.tanh(s / cap) if cap else s).softmax(-1) @ vv).transpose(1, 2)
+            got = ops.window_attention(q, k, v, d ** -0.5, active, window, cap)
+            # weights carry 16 bits, the soft cap 2^-10 of itself; what counts is the rounding of the output
+            assert (got.double() - want).abs().max() <= {"bf16": 2.0 ** -7, "f16": 2.0 ** -9}[dt] * want.abs().max(), (active, cap)
+
+
+# ---- products of experts on pairs of CTAs: experts of one tile, of one and a row, and rows of another expert that a tile's copies bring along ----
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("sizes", [(256, 257, 31, 56), (0, 512, 1, 33), (225, 32, 513, 16)])
+def test_experts_of_whole_tiles_keep_to_their_rows(dt, sizes):
+    n, k, experts = 130, 72, len(sizes)
+    g, of = gen(sum(sizes)), torch.repeat_interleave(torch.arange(experts), torch.tensor(sizes))
+    of = of[torch.randperm(len(of), generator=torch.Generator().manual_seed(1))].cuda()
+    routing = ops.MoeRouting(torch.nn.functional.one_hot(of, experts).float() * 9, 1)
+    place = routing.rows().reshape(-1).long()
+    act, gu, dn = randn(g, len(of), k).to(DT[dt]), (randn(g, experts, 2 * n, k) * k ** -0.5).to(DT[dt]), (randn(g, experts, k, n) * n ** -0.5).to(DT[dt])
+    hidden = randn(g, len(of), n).to(DT[dt])
+
+    def run(a, h):
+        out = []
+        for args in (dict(act=a, w=gu, gather=True, glu=True), dict(act=h, w=dn, gather=False, out_dtype=torch.float32)):
+            out.append(routing.matmul(**args))
+            assert int(routing.status.item()) == 0
+        return out
+
+    clean = run(act, hidden)
+    by_place = torch.empty_like(of)
+    by_place[place] = of
+    for e in range(experts):
+        full = act[of == e].double() @ gu[e].double().t()
+        want = torch.nn.functional.silu(full[:, :n]) * full[:, n:]
+        eps = 2.0 ** (-8 if dt == "bf16" else -11)
+        if len(want):
+            assert (clean[0][place[of == e]].double() - want).abs().max() <= (eps + 1e-5) * want.abs().max()
+            want = hidden[by_place == e].double() @ dn[e].double().t()
+            assert (clean[1][by_place == e].double() - want).abs().max() <= 1e-5 * want.abs().max()
+        bad_act, bad_hidden = act.clone(), hidden.clone()
+        bad_act[of == e], bad_hidden[by_place == e] = float("nan"), float("nan")
+        for got, was in zip(run(bad_act, bad_hidden), clean):
+            assert torch.isnan(got[by_place == e]).all() and torch.equal(got[by_place != e], was[by_place != e])
 
 
 # ---- decode attention whose splits meet: scores that are NaN in all rows of a warp or of a split are not lost, and stay with their sequence ----

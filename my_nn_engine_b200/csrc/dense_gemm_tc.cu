@@ -130,7 +130,6 @@ dense_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             const uint32_t bytes = 2 * (kDgWBytes + (uint32_t)(boxes * p.box) * (kDgK * 2));  // what both CTAs bring into a stage
             for (int kb = 0; kb < kblocks; kb++) {
                 if (use > 0 && !__all_sync(0xffffffffu, mbar_wait_spin(&empty_bar[s], (use - 1) & 1, &abort_flag))) {
-                    if (lane == 0) give_up(41);
                     ok = false;
                     break;
                 }
@@ -146,6 +145,12 @@ dense_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 if (++s == kDgStages) s = 0, use++;
             }
         }
+        // The commits that give the last stages back arrive in both CTAs: neither is left before its own have.
+        for (int i = 0; i < kDgStages && ok; i++) {
+            if (use > 0) ok = __all_sync(0xffffffffu, mbar_wait_spin(&empty_bar[s], (use - 1) & 1, &abort_flag));
+            if (++s == kDgStages) s = 0, use++;
+        }
+        if (!ok && lane == 0) give_up(41);
         __syncwarp();
     } else if (warp == 1) {
         // ---------------- MMA issuer of the pair ----------------

@@ -318,10 +318,6 @@ i8_prefill_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             const int w_row = (2 * wt + (int)rank) * kPfRows, a_row = tt * p.cols + (int)rank * (tile_cols(tt) >> 1);
             for (int kb = 0; kb < kblocks; kb++) {
                 if (use > 0 && !__all_sync(0xffffffffu, mbar_wait_spin(&empty_bar[s], (use - 1) & 1, &abort_flag))) {
-                    if (lane == 0) {
-                        atomicExch(&abort_flag, 1);
-                        atomicExch(p.status, 11);
-                    }
                     ok = false;
                     break;
                 }
@@ -336,6 +332,16 @@ i8_prefill_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                 if (++s == p.stages) s = 0, use++;
             }
         }
+        // The commits that give the last stages back arrive in both CTAs: neither is left before its own have.
+        for (int i = 0; i < p.stages && ok; i++) {
+            if (use > 0) ok = __all_sync(0xffffffffu, mbar_wait_spin(&empty_bar[s], (use - 1) & 1, &abort_flag));
+            if (++s == p.stages) s = 0, use++;
+        }
+        if (!ok && lane == 0) {
+            atomicExch(&abort_flag, 1);
+            atomicExch(p.status, 11);
+        }
+        __syncwarp();
     } else if (warp == 1) {
         // ---------------- MMA issuer of the pair ----------------
         if (rank == 0) {

@@ -66,11 +66,11 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     active = max(0, WIN && p.ring_cache ? active : min(active, p.cache_seq));
     // rows [lo, active) are seen; the walk starts at the 16-row tile that holds lo (0 without a window)
     const int lo = WIN ? max(active > 0 ? first_visible(active - 1, p.window, p.chunk) : 0, p.ring_cache ? active - p.cache_seq : 0) : 0, walk0 = lo & ~15;
-    // whole rounds of the CTA's warps (64 rows of four): a split that ends inside a round leaves some warps a tile short
     // A cluster whose rows are two rounds or less leaves them to its first CTA: the merge takes about as long as a round.
     const bool solo = p.cluster && active - walk0 <= 2 * 16 * W;
     if (solo && split > 0) return;
     const int splits = solo ? 1 : p.splits;
+    // whole rounds of the CTA's warps (64 rows of four): a split that ends inside a round leaves some warps a tile short
     const int rows_per_split = (((active - walk0 + splits - 1) / splits) + 16 * W - 1) / (16 * W) * (16 * W);
     const int row_beg = walk0 + split * rows_per_split;
     const int row_end = min(row_beg + rows_per_split, active);

@@ -103,7 +103,7 @@ __device__ __forceinline__ float warp_max(float v) {
 // fixed_weights).  A prefetch into L2 is no read.  What the kernel in front triggers, and when, makes no difference to this.
 // pdl_wait() returns when the grid in front has completed and is visible; since the kernels of a chain wait, that covers all before it.  The
 // one that does not, tp_reduce_norm_limbs_kernel, polls for each word it takes from the grid in front.
-// pdl_trigger() says when the next kernel may become resident: at the start where this kernel leaves room beside it (lean products leave eight SMs to the row kernels), when the
+// pdl_trigger() says when the next kernel may become resident: at the start where this kernel leaves room beside it (lean products leave eight SMs, where whole tiles of rows ask for it four, to the row kernels), when the
 // accumulators are complete in the tcgen05 products (step of batch 32: 3.98 -> 3.85 ms; a trigger at their start made the kernels two and three
 // places ahead take registers and shared memory from the running one, 4.63 -> 5.31 ms), when its own loads are here in the norms of few rows.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

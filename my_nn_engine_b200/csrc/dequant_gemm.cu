@@ -482,7 +482,7 @@ int launch_dequant_matmul(cudaStream_t st, void *out, const void *act, const int
     // With scratch memory the tcgen05 int8 kernel takes every [N,K] problem of up to 32 rows.
     if (workspace && w_layout == MYNN_W_NK && i8_gemm_supported(M, N, K, wq, act_dtype, out_dtype))
         return i8_gemm_launch(st, out, act, wq, scale, resid, M, N, K, act_dtype, out_dtype, workspace, workspace_bytes, settled);
-    // More rows: the prefill kernel (two activation limbs, 128 x 128-token tiles) if the scratch is large enough.
+    // More rows: the prefill kernel (two activation limbs, tiles of 256 weight rows x up to 128 tokens) if the scratch is large enough.
     if (workspace && w_layout == MYNN_W_NK && i8_prefill_supported(M, N, K, wq, act_dtype, out_dtype) &&
         workspace_bytes >= i8_prefill_workspace_bytes(M, K))
         return i8_prefill_launch(st, out, act, wq, scale, resid, M, N, K, act_dtype, out_dtype, workspace, workspace_bytes);

@@ -10,9 +10,9 @@
 //
 // Kernel: persistent pairs of CTAs (clusters of two, one CTA per SM), tile = 256 weight rows x up to 128 tokens (256 limb columns), UMMA
 // cta_group::2 M=256 N<=256 K=32.  Each CTA of a pair owns 128 of the weight rows, and brings them and half of the limb rows to its
-// shared memory: 32 KB per 128 of K where a CTA on its own needs 48.  That is what bounds this kernel: an SM gets about 64 bytes per clock from
-// L2 (220 ns per stage of 128 columns, 24 KB, and of 332 ns, 32 KB, at the clock that full tiles leave), and at the int8 rate of 128 x 256 x 32
-// per 128 clocks a CTA alone would take in 96.  Full tiles run at the power cap.
+// shared memory: 32 KB per 128 of K, 64 bytes per clock at the int8 rate of 128 x 256 x 32 per 128 clocks, where a CTA on its own needs 48 KB and 96.
+// An SM gets about 60 from L2 (ncu): full tiles keep the tensor pipe 95 % busy and run at the power cap, narrower ones wait for their copies (160
+// columns ask for 83 bytes per clock: 57 arrive, the pipe is 69 % busy).
 // 2048 rows: 28672 x 4096 325 -> 272 us (3.54 POP/s), 4096 x 14336 198 -> 166, 6144 x 4096 76 -> 69, 4096 x 4096 52 -> 48; one limb,
 // 777 rows of 14336 x 4096, 48 -> 36.  About half of it came from walking the two issuing loops with whole warps (see elect_one).
 // Warp 0 of both CTAs streams by TMA through a ring of six to nine mbarrier stages, warp 1 of the first issues the MMAs of both into one

@@ -202,8 +202,8 @@ static int enqueue_forward(Model &m, cudaStream_t st, int S, int head_rows = 0) 
             // the projection output is one block whose rows and heads are 16-byte aligned
             const bool fuse_rope = g_fuse_rope && attn_limbs && L.qkv_fused && qs % 8 == 0 && D % 32 == 0 &&
                                    (((uintptr_t)kb | (uintptr_t)vb) % 16) == 0;
-            // A lean o_proj takes the rows as they are: limbs made there, or by a row kernel in front, cost less than a last CTA of the attention
-            // that collects the heads (TinyLlama shapes, one sequence: 3.8 us for product and limbs against 2.2 + 3.5).
+            // A lean o_proj takes the rows as they are: a row kernel in front of it costs less than a last CTA of the attention that collects the heads
+            // (TinyLlama shapes, one sequence: 3.8 us for product and limbs against 2.2 + 3.5).
             if (tp == 1 && fuse_rope && gemv_lean_supported(M, H, Nq, L.wo)) attn_limbs = false;
             if (fuse_rope) {
                 const AttentionFuse fz = {kb, vb, qs, m.cos_t, m.sin_t, m.pos0_dev, m.past_dev};
@@ -254,8 +254,7 @@ static int enqueue_forward(Model &m, cudaStream_t st, int S, int head_rows = 0) 
             RC(norm(L.ln2, m.part, M, m.x));  // x = round(x + round(sum of partials)), then the norm
         }
         // --- MLP block ---
-        // A few rows: the lean gate/up product finishes the SiLU product as well, and the limbs of its rows are made inside the down product, or by the
-        // row kernel in front of it.
+        // A few rows: the lean gate/up product finishes the SiLU product as well, and a row kernel in front of the down product makes the limbs of its rows.
         const bool gated = fused && L.gu_fused && tp == 1 && !reduced_limbs && gemv_lean_supported(M, 2 * m.ffn, H, L.wg);
         const bool fuse_mlp = fused && L.gu_fused && !gated;
         bool h_limbs2 = false;  // Swish*Mul left two-limb rows in the workspace instead of m.h

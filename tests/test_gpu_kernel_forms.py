@@ -252,7 +252,7 @@ def test_dense_products(M, N, K):
 @pytest.mark.parametrize("head_dim,kv_heads,batch", [(64, 1, 1), (64, 2, 3), (128, 1, 1), (128, 2, 2)])
 def test_fused_append_over_a_long_cache(head_dim, kv_heads, batch):
     """Against the rotation and append in front of the attention, over caches whose rows are given.  Few pairs and 4096 rows: eight warps (head_dim
-    128) and sixteen (64), eight and four splits of 4096 rows, rounds of 128 and 256; the contexts put the new row on both sides of warp, round and split borders."""
+    128) and sixteen (64), clusters of eight splits, rounds of 128 and 256 rows; the contexts put the new row on both sides of warp, round and split borders."""
     from my_nn_engine_b200 import ffi
     from my_nn_engine_b200.decoder import DecoderModel
     from my_nn_engine_b200.quantize import random_llama_state
